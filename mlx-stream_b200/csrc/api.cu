@@ -193,6 +193,7 @@ extern "C" int mlxs_moe_create(const mlxs_moe_config* c, mlxs_moe** out) {
             if ((rc = h->alloc(&h->pf_tiles, prefill_tile_words(h->pf_max_tiles) * 4)) || (rc = h->alloc(&h->pf_xa, xa_bytes)) ||
                 (rc = h->alloc(&h->pf_xd, xd_bytes)))
                 return bail(rc);
+            if (exl3 && (rc = h->alloc(&h->pf_act, exl3_prefill_act_bytes(h->sm_count)))) return bail(rc);
         }
     }
     if (c->shared_expert) {
@@ -658,8 +659,7 @@ int mlxs_run_routed(mlxs_moe* h, uint32_t layer, const void* x_dev, const int32_
             pa.x = static_cast<const __nv_bfloat16*>(x_dev); pa.top_k = top_k; pa.tiles = h->pf_tiles; pa.max_tiles = h->pf_max_tiles;
             pa.xa = h->pf_xa; pa.xd = h->pf_xd; pa.rows_cap = h->rows_cap; pa.ro = static_cast<float*>(ro);
             pa.limit = limit; pa.status = h->status; pa.sm_count = h->sm_count;
-            // side by side with the streaming lane: the large-tile kernels also beside the small-tile ones
-            if (lane_aside) { pa.side = h->lane2_stream; pa.side_fork = h->lane2_fork; pa.side_join = h->lane2_join; }
+            pa.act = h->pf_act;
             StageTimer tm(h, MLXS_STAGE_TENSOR_LANE, tl);
             CU(launch_exl3_prefill(pa, tl));
         }
@@ -916,8 +916,8 @@ extern "C" int mlxs_moe_exl3_gemv(mlxs_moe* h, uint32_t layer, uint32_t expert, 
     const uint32_t in_dim = proj == 2 ? c.inter : c.hidden, out_dim = proj == 2 ? c.hidden : c.inter;
     CU(launch_exl3_prep_raw(xh_dev, in_dim, h->tabs, h->xa_gu, st));
     const uint32_t* code = proj == 2 ? L.d_code + (size_t)le * exl3_code_words(d) : L.gu_code + (size_t)le * 2 * exl3_code_words(d);
-    const uint32_t tw8 = 8u * exl3_tile_words(d);   // words of one projection's eight tiles of a k-tile
-    CU(launch_exl3_raw(code, in_dim, out_dim, proj == 2 ? tw8 : 2u * tw8, proj == 1 ? tw8 : 0u, (int)d.K, h->tabs, h->xa_gu, z_dev,
+    const uint32_t block = (in_dim / 16) * 8u * exl3_tile_words(d);   // words of one projection's k-tiles of an output block
+    CU(launch_exl3_raw(code + (proj == 1 ? block : 0u), in_dim, out_dim, proj == 2 ? block : 2u * block, (int)d.K, h->tabs, h->xa_gu, z_dev,
                        h->status, h->sm_count, st));
     return MLXS_OK;
 }

@@ -32,32 +32,38 @@ __device__ __forceinline__ void mbar_fence_init() { asm volatile("fence.mbarrier
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+__device__ __forceinline__ void mbar_arrive_at(uint32_t bar) {   // by shared-memory address
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) { mbar_arrive_at(smem_u32(bar)); }
+__device__ __forceinline__ bool mbar_try_wait_at(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
+        : "r"(bar), "r"(parity)
         : "memory");
     return ok != 0;
 }
+__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) { return mbar_try_wait_at(smem_u32(bar), parity); }
 // Bounded wait: gives up after `limit` polls (each poll itself blocks for a hardware-defined slice) or as soon as
 // *abort_flag is set by another thread of the CTA.  Returns false when it gave up.
 // sleep_ns > 0: back off between polls (the single-lane producer / MMA-issuer roles wait most of the time; polling
 // flat out would take issue slots from the warps that do the arithmetic).
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
-                                                  uint32_t sleep_ns = 0, uint32_t limit = (1u << 20)) {
+__device__ __forceinline__ bool mbar_wait_bounded_at(uint32_t bar, uint32_t parity, volatile int* abort_flag,
+                                                     uint32_t sleep_ns = 0, uint32_t limit = (1u << 20)) {
     for (uint32_t i = 0; i < limit; ++i) {
-        if (mbar_try_wait(bar, parity)) return true;
+        if (mbar_try_wait_at(bar, parity)) return true;
         if (sleep_ns) __nanosleep(sleep_ns);
         if ((i & 63u) == 63u && *abort_flag) return false;
     }
     return false;
+}
+__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
+                                                  uint32_t sleep_ns = 0, uint32_t limit = (1u << 20)) {
+    return mbar_wait_bounded_at(smem_u32(bar), parity, abort_flag, sleep_ns, limit);
 }
 // global -> this CTA's shared memory, completion counted in bytes on `bar`; 16-byte aligned addresses and size
 __device__ __forceinline__ void bulk_g2s(void* dst_smem, const void* src_gmem, uint32_t bytes, uint64_t* bar) {

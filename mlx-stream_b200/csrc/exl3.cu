@@ -23,6 +23,8 @@ constexpr int ZS_STRIDE = 132;    // padded row stride of the epilogue's f32 sta
 // ------------------------------------------------------------------------------------------------------------
 // load-time repack: reference record -> kernel layout (bit-preserving: words move, no bit changes)
 // ------------------------------------------------------------------------------------------------------------
+// V = uint4 (the record is 16-byte aligned: eight tiles of a k-tile are 48 or 32 vectors, contiguous on both sides) or uint32_t
+template <class V>
 __global__ void exl3_repack_kernel(const uint8_t* __restrict__ rec, uint32_t H, uint32_t I, uint32_t TW,
                                    uint32_t* __restrict__ gu, uint32_t* __restrict__ dn, __half* __restrict__ sc) {
     const size_t code_bytes = (size_t)(H / 16) * (I / 16) * TW * 4;   // TW words per 16x16 tile (24 at K = 3, 16 at K = 2)
@@ -30,28 +32,23 @@ __global__ void exl3_repack_kernel(const uint8_t* __restrict__ rec, uint32_t H, 
     const size_t off_g = 0, off_g_rout = code_bytes, off_g_rin = off_g_rout + 2 * (size_t)I;
     const size_t off_u = off_g_rin + 2 * (size_t)H, off_u_rout = off_u + code_bytes, off_u_rin = off_u_rout + 2 * (size_t)I;
     const size_t off_d = off_u_rin + 2 * (size_t)H, off_d_rout = off_d + code_bytes, off_d_rin = off_d_rout + 2 * (size_t)H;
-    const size_t words = code_bytes / 4;
-    const size_t n_gu = 2 * words, n_all = 3 * words, n_sc = (size_t)3 * H + 3 * I;
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_all + n_sc; i += stride) {
-        if (i < n_gu) {
-            // destination index -> (nb, kt, p, j, w)
-            size_t r = i;
-            const uint32_t w = r % TW; r /= TW;
-            const uint32_t j = r % 8; r /= 8;
-            const uint32_t p = r % 2; r /= 2;
-            const uint32_t kt = r % (H / 16); r /= (H / 16);
-            const uint32_t nb = (uint32_t)r;
-            const uint32_t* src = reinterpret_cast<const uint32_t*>(rec + (p ? off_u : off_g));
-            gu[i] = src[((size_t)kt * (I / 16) + nb * 8 + j) * TW + w];
-        } else if (i < n_all) {
-            size_t r = i - n_gu;
-            const uint32_t w = r % TW; r /= TW;
-            const uint32_t j = r % 8; r /= 8;
-            const uint32_t kt = r % (I / 16); r /= (I / 16);
-            const uint32_t nb = (uint32_t)r;
-            const uint32_t* src = reinterpret_cast<const uint32_t*>(rec + off_d);
-            dn[i - n_gu] = src[((size_t)kt * (H / 16) + nb * 8 + j) * TW + w];
+    const uint32_t per = 8u * TW * 4u / (uint32_t)sizeof(V);          // vectors of one k-tile of one 128-wide output block
+    const uint32_t n_code = (uint32_t)(code_bytes / sizeof(V)), n_all = 3 * n_code, n_sc = 3 * H + 3 * I;
+    const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_all + n_sc; i += stride) {
+        if (i < n_all) {
+            // destination: gate / up [block][projection][k-tile][vector], down [block][k-tile][vector]
+            const bool down = i >= 2 * n_code;
+            uint32_t r = down ? i - 2 * n_code : i;
+            const uint32_t v = r % per; r /= per;
+            const uint32_t nkt = (down ? I : H) / 16, n_out = (down ? H : I) / 16;
+            const uint32_t kt = r % nkt; r /= nkt;
+            uint32_t p = 2;
+            if (!down) { p = r % 2; r /= 2; }
+            const V* src = reinterpret_cast<const V*>(rec + (p == 0 ? off_g : p == 1 ? off_u : off_d));
+            const V w = src[((size_t)kt * n_out + r * 8) * TW * 4 / sizeof(V) + v];
+            if (down) reinterpret_cast<V*>(dn)[i - 2 * n_code] = w;
+            else reinterpret_cast<V*>(gu)[i] = w;
         } else {
             const size_t s = i - n_all;
             const __half* h;
@@ -70,7 +67,10 @@ __global__ void exl3_repack_kernel(const uint8_t* __restrict__ rec, uint32_t H, 
 
 cudaError_t launch_exl3_repack(const uint8_t* record_dev, Exl3Dims d, uint32_t* gu_code_e, uint32_t* d_code_e,
                                __half* scales_e, cudaStream_t st) {
-    exl3_repack_kernel<<<592, 256, 0, st>>>(record_dev, d.H, d.I, exl3_tile_words(d), gu_code_e, d_code_e, scales_e);
+    if (reinterpret_cast<uintptr_t>(record_dev) % 16 == 0)
+        exl3_repack_kernel<uint4><<<592, 256, 0, st>>>(record_dev, d.H, d.I, exl3_tile_words(d), gu_code_e, d_code_e, scales_e);
+    else
+        exl3_repack_kernel<uint32_t><<<592, 256, 0, st>>>(record_dev, d.H, d.I, exl3_tile_words(d), gu_code_e, d_code_e, scales_e);
     return cudaGetLastError();
 }
 
@@ -112,8 +112,7 @@ struct GemvParams {
     size_t expert_stride_words;
     uint32_t n_blocks;           // out / 128
     uint32_t nkt;                // in / 16
-    uint32_t kt_stride_words;    // words per k-tile in the block stream (192 per projection present)
-    uint32_t proj_off_words;     // where this kernel's (first) projection sits inside a k-tile
+    uint32_t block_stride_words; // words per 128-wide output block: a projection's k-tiles follow each other (8 tiles each)
     const uint32_t* xa;          // [chunk][NPROJ][nkt][128]
     DispatchTables t;
     uint32_t counter_idx;
@@ -145,9 +144,10 @@ struct GemvParams {
 struct StageMeta { int32_t item; uint32_t flags, mc, kt0, chunk0, expert, nb, part; };
 
 // one pipeline stage (KT k-tiles) of one warp's 16-column tile, MC chunks of activations
-template <int NPROJ, int KSTRIDE, int KB, int MC>
+template <int NPROJ, int KB, int MC>
 __device__ __forceinline__ void gemv_stage(const uint32_t* __restrict__ wt, const uint2* __restrict__ at, uint32_t mt_stride,
                                            uint32_t wi, uint32_t wj, uint32_t lp, float (&acc)[GROUP_CHUNKS][4]) {
+    constexpr int KSTRIDE = 64 * KB;   // words per k-tile: 8 tiles of 8 KB words
     // at: this projection's KT activation tiles of the first chunk (B-fragment order), the next chunk's mt_stride uint2 on
 #pragma unroll
     for (int kt = 0; kt < KT; ++kt) {
@@ -165,18 +165,19 @@ __device__ __forceinline__ void gemv_stage(const uint32_t* __restrict__ wt, cons
 }
 
 // SUB sub-stages of one ring slot, unrolled
-template <int NPROJ, int KSTRIDE, int KB, int MC, int SUB>
+template <int NPROJ, int KB, int MC, int SUB>
 __device__ __forceinline__ void gemv_slot(const uint32_t* __restrict__ wt, const uint2* __restrict__ at, uint32_t mt_stride,
                                           uint32_t wi, uint32_t wj, uint32_t lp, float (&acc)[GROUP_CHUNKS][4]) {
 #pragma unroll
     for (int u = 0; u < SUB; ++u)
-        gemv_stage<NPROJ, KSTRIDE, KB, MC>(wt + u * KT * KSTRIDE, at + u * KT * 32, mt_stride, wi, wj, lp, acc);
+        gemv_stage<NPROJ, KB, MC>(wt + u * KT * (64 * KB), at + u * KT * 32, mt_stride, wi, wj, lp, acc);
 }
 
-// KSTRIDE = words per k-tile of the block stream (8 tiles x 8 KB words per projection present), KB = bits per weight
-template <int NPROJ, int EPI, int KSTRIDE, int KB>
+// KB = bits per weight
+template <int NPROJ, int EPI, int KB>
 __global__ void __launch_bounds__(NPROJ * 256 + 32, NPROJ == 1 ? 3 : 2) exl3_gemv_kernel(const GemvParams P) {
     constexpr uint32_t TW = 8 * KB;        // words per 16x16 tile
+    constexpr uint32_t KT_WORDS = 8 * TW;  // words per k-tile of one projection's block stream
     extern __shared__ __align__(128) uint8_t smem_raw[];
     constexpr int NCW = NPROJ * 8;         // consumer warps: projection x 16-column tile of the 128 block
     constexpr int MAXS = 8;
@@ -222,7 +223,7 @@ __global__ void __launch_bounds__(NPROJ * 256 + 32, NPROJ == 1 ? 3 : 2) exl3_gem
                     chunk0 = P.t.group_chunk0[g]; mc = P.t.group_mc[g]; expert = P.t.chunk_expert[chunk0];
                 }
                 const uint32_t* wsrc = P.code + (size_t)expert * P.expert_stride_words +
-                                       (size_t)nb * P.nkt * P.kt_stride_words;
+                                       (size_t)nb * P.block_stride_words;
                 const uint32_t k_begin = share * share_kt, k_end = last ? k_begin + 1 : k_begin + share_kt;
                 // One barrier round trip serves `sub` sub-stages of KT k-tiles: the most (up to 3; 1 for rows in 3 or 4 chunks) that divide a part of
                 // the sum and fit the ring slot with this item's chunks of rows.
@@ -249,7 +250,9 @@ __global__ void __launch_bounds__(NPROJ * 256 + 32, NPROJ == 1 ? 3 : 2) exl3_gem
                     if (P.withhold && ++n_stage == P.withhold) continue;   // self-test: this stage never arrives
                     uint8_t* dst = ring + (size_t)s * P.stage_bytes;
                     mbar_expect_tx(&full_bar[s], sub * P.w_bytes + mc * NPROJ * xa_bytes);
-                    bulk_g2s(dst, wsrc + (size_t)kt0 * P.kt_stride_words, sub * P.w_bytes, &full_bar[s]);
+                    for (int p = 0; p < NPROJ; ++p)
+                        bulk_g2s(dst + p * (sub * KT * KT_WORDS * 4), wsrc + ((size_t)p * P.nkt + kt0) * KT_WORDS, sub * KT * KT_WORDS * 4,
+                                 &full_bar[s]);
                     for (uint32_t m = 0; m < mc; ++m)
                         for (int p = 0; p < NPROJ; ++p)
                             bulk_g2s(dst + sub * P.w_bytes + (m * NPROJ + p) * xa_bytes,
@@ -295,27 +298,27 @@ __global__ void __launch_bounds__(NPROJ * 256 + 32, NPROJ == 1 ? 3 : 2) exl3_gem
 #pragma unroll
                 for (int c = 0; c < 4; ++c) acc[a][c] = 0.f;
         }
-        // slot: [sub x KT k-tiles of codes][chunk][projection][sub x KT activation tiles]
+        // slot: [projection][sub x KT k-tiles of codes][chunk][projection][sub x KT activation tiles]
         const uint32_t sub = flags >> 16;
         const uint8_t* st = ring + (size_t)s * P.stage_bytes;
-        const uint32_t* wt = reinterpret_cast<const uint32_t*>(st) + P.proj_off_words + p * (8u * TW) + j * TW;
+        const uint32_t* wt = reinterpret_cast<const uint32_t*>(st) + p * (sub * KT * KT_WORDS) + j * TW;
         const uint2* at = reinterpret_cast<const uint2*>(st + sub * P.w_bytes) + p * (sub * KT * 32) + lane;
         const uint32_t mt_stride = NPROJ * sub * KT * 32;
         static_assert(GROUP_CHUNKS * CHUNK_ROWS == 16, "the K-split workspace is sized for 16 rows per item");
         static_assert(GROUP_CHUNKS == 4, "the stage dispatch below enumerates the chunk counts");
         // straight-line code per (chunks, sub-stages): rows in 3 or 4 chunks always come one sub-stage per slot
         if (stage_mc == 1) {
-            if (sub == 2) gemv_slot<NPROJ, KSTRIDE, KB, 1, 2>(wt, at, mt_stride, wi, wj, lp, acc);
-            else if (sub == 3) gemv_slot<NPROJ, KSTRIDE, KB, 1, 3>(wt, at, mt_stride, wi, wj, lp, acc);
-            else gemv_slot<NPROJ, KSTRIDE, KB, 1, 1>(wt, at, mt_stride, wi, wj, lp, acc);
+            if (sub == 2) gemv_slot<NPROJ, KB, 1, 2>(wt, at, mt_stride, wi, wj, lp, acc);
+            else if (sub == 3) gemv_slot<NPROJ, KB, 1, 3>(wt, at, mt_stride, wi, wj, lp, acc);
+            else gemv_slot<NPROJ, KB, 1, 1>(wt, at, mt_stride, wi, wj, lp, acc);
         } else if (stage_mc == 2) {
-            if (sub == 2) gemv_slot<NPROJ, KSTRIDE, KB, 2, 2>(wt, at, mt_stride, wi, wj, lp, acc);
-            else if (sub == 3) gemv_slot<NPROJ, KSTRIDE, KB, 2, 3>(wt, at, mt_stride, wi, wj, lp, acc);
-            else gemv_slot<NPROJ, KSTRIDE, KB, 2, 1>(wt, at, mt_stride, wi, wj, lp, acc);
+            if (sub == 2) gemv_slot<NPROJ, KB, 2, 2>(wt, at, mt_stride, wi, wj, lp, acc);
+            else if (sub == 3) gemv_slot<NPROJ, KB, 2, 3>(wt, at, mt_stride, wi, wj, lp, acc);
+            else gemv_slot<NPROJ, KB, 2, 1>(wt, at, mt_stride, wi, wj, lp, acc);
         } else if (stage_mc == 3) {
-            gemv_slot<NPROJ, KSTRIDE, KB, 3, 1>(wt, at, mt_stride, wi, wj, lp, acc);
+            gemv_slot<NPROJ, KB, 3, 1>(wt, at, mt_stride, wi, wj, lp, acc);
         } else {
-            gemv_slot<NPROJ, KSTRIDE, KB, 4, 1>(wt, at, mt_stride, wi, wj, lp, acc);
+            gemv_slot<NPROJ, KB, 4, 1>(wt, at, mt_stride, wi, wj, lp, acc);
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty_bar[s]);
@@ -446,7 +449,7 @@ static int tune_env(const char* name, int dflt, int lo, int hi) {
 
 static cudaError_t launch_gemv(int nproj, int epi, int kbits, GemvParams& P, int sm_count, cudaStream_t st) {
     const uint32_t zs_bytes = (uint32_t)(nproj * GROUP_CHUNKS * CHUNK_ROWS * ZS_STRIDE * sizeof(float));
-    P.w_bytes = KT * P.kt_stride_words * 4;
+    P.w_bytes = (uint32_t)(KT * nproj * 64 * kbits * 4);
     const uint32_t stage_one = P.w_bytes + GROUP_CHUNKS * nproj * KT * A_TILE_WORDS * 4;   // one sub-stage, 4 chunks of rows
     // resident CTAs per SM (tunable for experiments: MLXS_GU_CTAS 1..2, MLXS_DN_CTAS 1..3); the shared-memory ring
     // takes what the SM's 227 KB leave per CTA
@@ -468,22 +471,20 @@ static cudaError_t launch_gemv(int nproj, int epi, int kbits, GemvParams& P, int
     const int ctas = per_sm * sm_count;
     static const int k_parts = tune_env("MLXS_K_PARTS", 4, 1, 4);
     P.max_parts = (uint32_t)k_parts;
-#define MLXS_LAUNCH(NP, EP, KS, KBITS)                                                                            \
+#define MLXS_LAUNCH(NP, EP, KBITS)                                                                                \
     do {                                                                                                         \
-        e = cudaFuncSetAttribute(exl3_gemv_kernel<NP, EP, KS, KBITS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+        e = cudaFuncSetAttribute(exl3_gemv_kernel<NP, EP, KBITS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
         if (e != cudaSuccess) return e;                                                                          \
-        exl3_gemv_kernel<NP, EP, KS, KBITS><<<ctas, NP * 256 + 32, smem, st>>>(P);                               \
+        exl3_gemv_kernel<NP, EP, KBITS><<<ctas, NP * 256 + 32, smem, st>>>(P);                               \
     } while (0)
     if (kbits == 3) {
-        if (nproj == 2) MLXS_LAUNCH(2, EPI_GATE_UP, 384, 3);
-        else if (epi == EPI_DOWN) MLXS_LAUNCH(1, EPI_DOWN, 192, 3);
-        else if (P.kt_stride_words == 192) MLXS_LAUNCH(1, EPI_RAW, 192, 3);
-        else MLXS_LAUNCH(1, EPI_RAW, 384, 3);
+        if (nproj == 2) MLXS_LAUNCH(2, EPI_GATE_UP, 3);
+        else if (epi == EPI_DOWN) MLXS_LAUNCH(1, EPI_DOWN, 3);
+        else MLXS_LAUNCH(1, EPI_RAW, 3);
     } else if (kbits == 2) {
-        if (nproj == 2) MLXS_LAUNCH(2, EPI_GATE_UP, 256, 2);
-        else if (epi == EPI_DOWN) MLXS_LAUNCH(1, EPI_DOWN, 128, 2);
-        else if (P.kt_stride_words == 128) MLXS_LAUNCH(1, EPI_RAW, 128, 2);
-        else MLXS_LAUNCH(1, EPI_RAW, 256, 2);
+        if (nproj == 2) MLXS_LAUNCH(2, EPI_GATE_UP, 2);
+        else if (epi == EPI_DOWN) MLXS_LAUNCH(1, EPI_DOWN, 2);
+        else MLXS_LAUNCH(1, EPI_RAW, 2);
     } else {
         return cudaErrorInvalidValue;
     }
@@ -495,7 +496,7 @@ cudaError_t launch_exl3_gate_up(const Exl3GemvArgs& a, cudaStream_t st) {
     GemvParams P{};
     P.code = a.L.gu_code;
     P.expert_stride_words = 2 * exl3_code_words(a.d);
-    P.n_blocks = a.d.I / 128; P.nkt = a.d.H / 16; P.kt_stride_words = 16 * exl3_tile_words(a.d); P.proj_off_words = 0;
+    P.n_blocks = a.d.I / 128; P.nkt = a.d.H / 16; P.block_stride_words = 2 * P.nkt * 8 * exl3_tile_words(a.d);
     P.xa = a.xa_gu; P.t = a.t; P.counter_idx = HDR_CTR_GU;
     P.scales = a.L.scales; P.scales_stride = exl3_scales_per_expert(a.d);
     P.H = a.d.H; P.I = a.d.I; P.xa_d = a.xa_d; P.out = nullptr; P.out_dim = a.d.I; P.limit = a.limit; P.status = a.status;
@@ -508,7 +509,7 @@ cudaError_t launch_exl3_down(const Exl3GemvArgs& a, cudaStream_t st) {
     GemvParams P{};
     P.code = a.L.d_code;
     P.expert_stride_words = exl3_code_words(a.d);
-    P.n_blocks = a.d.H / 128; P.nkt = a.d.I / 16; P.kt_stride_words = 8 * exl3_tile_words(a.d); P.proj_off_words = 0;
+    P.n_blocks = a.d.H / 128; P.nkt = a.d.I / 16; P.block_stride_words = P.nkt * 8 * exl3_tile_words(a.d);
     P.xa = a.xa_d; P.t = a.t; P.counter_idx = HDR_CTR_DOWN;
     P.scales = a.L.scales; P.scales_stride = exl3_scales_per_expert(a.d);
     P.H = a.d.H; P.I = a.d.I; P.xa_d = nullptr; P.out = a.ro; P.out_dim = a.d.H; P.limit = a.limit; P.status = a.status;
@@ -517,12 +518,11 @@ cudaError_t launch_exl3_down(const Exl3GemvArgs& a, cudaStream_t st) {
     P.poll_limit = a.poll_limit ? a.poll_limit : (1u << 20); P.withhold = 0;
     return launch_gemv(1, EPI_DOWN, (int)a.d.K, P, a.sm_count, st);
 }
-cudaError_t launch_exl3_raw(const uint32_t* code_e, uint32_t in_dim, uint32_t out_dim, uint32_t ktile_stride_words,
-                            uint32_t proj_off_words, int kbits, DispatchTables t, const uint32_t* xa, float* z,
+cudaError_t launch_exl3_raw(const uint32_t* code_e, uint32_t in_dim, uint32_t out_dim, uint32_t block_stride_words, int kbits, DispatchTables t, const uint32_t* xa, float* z,
                             uint32_t* status, int sm_count, cudaStream_t st) {
     GemvParams P{};
     P.code = code_e; P.expert_stride_words = 0;
-    P.n_blocks = out_dim / 128; P.nkt = in_dim / 16; P.kt_stride_words = ktile_stride_words; P.proj_off_words = proj_off_words;
+    P.n_blocks = out_dim / 128; P.nkt = in_dim / 16; P.block_stride_words = block_stride_words;
     P.xa = xa; P.t = t; P.counter_idx = HDR_CTR_AUX;
     P.scales = nullptr; P.scales_stride = 0; P.H = 0; P.I = 0; P.xa_d = nullptr; P.out = z; P.out_dim = out_dim;
     P.limit = 0.f; P.status = status; P.poll_limit = 1u << 20; P.withhold = 0;

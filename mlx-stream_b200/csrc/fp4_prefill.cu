@@ -246,25 +246,24 @@ __global__ void __launch_bounds__(512 + 64, PER_SM) fp4_prefill_kernel(const QPa
             if (s_abort) for (int i = 0; i < 2000; ++i) __nanosleep(1000);
         }
     } else if (warp == NCW + 1) {
-        // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            // The issue loop is the pipeline's critical path: the tensor pipe queues only about two MMAs behind the one
-            // that runs, so every cycle this thread spends between two stages shows.  Per stage: one barrier wait (a
-            // ready mbarrier costs about 130 cycles to test), the MMAs, two commits.  The rows' barrier is waited on by
-            // decode warp 0 before it arrives.
-            uint32_t as = 0, aph = 0, bs = 0, nitem = 0;
-            const uint32_t b_ring_s = smem_u32(b_ring);
-            for (uint32_t item = blockIdx.x; item < n_items && !s_abort; item += gridDim.x, ++nitem) {
-                const uint32_t rows16 = (prefill_tile(P.tiles, LIST, P.max_tiles, item / nbg)[2] + 15) / 16 * 16;
-                const uint32_t idesc = umma_idesc(NV ? UMMA_F16 : UMMA_BF16, rows16), lbo_b = rows16 * 16;
-                const uint64_t bdesc0 = umma_smem_desc(b_ring_s, lbo_b, Q_SBO);   // + byte offset >> 4 in the low word
-                if (!mbar_wait_bounded(&acc_empty, (nitem & 1u) ^ 1u, &s_abort, 64)) { give_up(ST_WAIT_EMPTY); break; }
+        // ---------------- MMA issuer: the whole warp walks the loop, one elected lane issues ----------------
+        // The issue loop is the pipeline's critical path: the tensor pipe queues only about two MMAs behind the one
+        // that runs, so every cycle this warp spends between two stages shows.  Per stage: one barrier wait, the MMAs,
+        // one commit.  The rows' barrier is waited on by decode warp 0 before it arrives.
+        uint32_t as = 0, aph = 0, bs = 0, nitem = 0;
+        const uint32_t b_ring_s = smem_u32(b_ring);
+        for (uint32_t item = blockIdx.x; item < n_items && !s_abort; item += gridDim.x, ++nitem) {
+            const uint32_t rows16 = (prefill_tile(P.tiles, LIST, P.max_tiles, item / nbg)[2] + 15) / 16 * 16;
+            const uint32_t idesc = umma_idesc(NV ? UMMA_F16 : UMMA_BF16, rows16), lbo_b = rows16 * 16;
+            const uint64_t bdesc0 = umma_smem_desc(b_ring_s, lbo_b, Q_SBO);   // + byte offset >> 4 in the low word
+            if (!mbar_wait_warp(&acc_empty, (nitem & 1u) ^ 1u, &s_abort, 64)) { give_up(ST_WAIT_EMPTY); break; }
+            tc_fence_after();
+            bool ok = true;
+            const uint32_t nk = nstage * (Q_KS / KST);
+            for (uint32_t kk = 0; kk < nk; ++kk) {
+                if (!mbar_wait_warp(&a_full[as], aph, &s_abort)) { give_up(ST_WAIT_FULL); ok = false; break; }
                 tc_fence_after();
-                bool ok = true;
-                const uint32_t nk = nstage * (Q_KS / KST);
-                for (uint32_t kk = 0; kk < nk; ++kk) {
-                    if (!mbar_wait_bounded(&a_full[as], aph, &s_abort)) { give_up(ST_WAIT_FULL); ok = false; break; }
-                    tc_fence_after();
+                if (elect_one()) {
                     const uint64_t bd = bdesc0 + ((bs * B_SLOT) >> 4);
                     const uint32_t ta = tmem_a + as * (NG * A_COLS);
 #pragma unroll
@@ -277,12 +276,13 @@ __global__ void __launch_bounds__(512 + 64, PER_SM) fp4_prefill_kernel(const QPa
                     // one commit per stage (a commit costs the issuing thread about as much as an MMA): it frees the
                     // operand slot, and decode warp 0, when it sees that, frees the rows' slot of the same stage
                     umma_commit(&a_empty[as]);
-                    if (++as == A_STAGES) { as = 0; aph ^= 1u; }
-                    if (++bs == B_STAGES) bs = 0;
+                    if (kk + 1 == nk) umma_commit(&acc_full);
                 }
-                if (!ok) break;
-                umma_commit(&acc_full);
+                __syncwarp();
+                if (++as == A_STAGES) { as = 0; aph ^= 1u; }
+                if (++bs == B_STAGES) bs = 0;
             }
+            if (!ok) break;
         }
     } else {
         // ---------------- decode warps + epilogue ----------------

@@ -60,6 +60,7 @@ struct mlxs_moe {
     // prefill lane (EXL3): row-tile table and operand staging, allocated when the handle can see prefill-sized calls
     uint32_t* pf_tiles = nullptr;
     __half *pf_xa = nullptr, *pf_xd = nullptr;
+    float* pf_act = nullptr;    // EXL3: act(gate) between a CTA's two passes
     uint32_t pf_max_tiles = 0;
     uint32_t pf_min_rows = 0;   // experts with at least this many rows of a call take the tensor-core lane (0: lane off)
     uint32_t chunk_rows = CHUNK_ROWS, group_chunks = GROUP_CHUNKS;

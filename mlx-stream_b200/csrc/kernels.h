@@ -83,7 +83,7 @@ cudaError_t launch_usage_count(const int32_t* ids, uint64_t n, uint32_t E, unsig
 
 // ---- EXL3 ----
 struct Exl3Layer {            // one layer's resident bank, in the kernels' layout
-    const uint32_t* gu_code;  // [E][I/128][H/16][2][192] u32: per 128-wide output block, per k-tile, gate | up tiles
+    const uint32_t* gu_code;  // [E][I/128][2][H/16][192] u32: per 128-wide output block, gate's k-tiles, then up's
     const uint32_t* d_code;   // [E][H/128][I/16][192] u32
     const __half* scales;     // [E][2H + 2I + I + H]: suh_g, suh_u [H] | svh_g, svh_u [I] | suh_d [I] | svh_d [H]
 };
@@ -129,11 +129,9 @@ static inline uint32_t ksplit_cap_items(int sm_count, size_t zs_bytes) {
 }
 cudaError_t launch_exl3_gate_up(const Exl3GemvArgs& a, cudaStream_t st);
 cudaError_t launch_exl3_down(const Exl3GemvArgs& a, cudaStream_t st);
-// raw projection: z [rows, out] = xa . W_hat(code); `code` in the single-projection block layout with a k-tile
-// stride of `ktile_stride_words` and the projection at `proj_off_words` (at K = 3: 192/0 for down, 384/{0,192} for
-// gate/up; at K = 2: 128/0 and 256/{0,128}); kbits = bits per weight
-cudaError_t launch_exl3_raw(const uint32_t* code_e, uint32_t in_dim, uint32_t out_dim, uint32_t ktile_stride_words,
-                            uint32_t proj_off_words, int kbits, DispatchTables t, const uint32_t* xa, float* z,
+// raw projection: z [rows, out] = xa . W_hat(code); `code` = the projection's first k-tile of output block 0, the next
+// block block_stride_words further (one projection's block for down, two for gate and up); kbits = bits per weight
+cudaError_t launch_exl3_raw(const uint32_t* code_e, uint32_t in_dim, uint32_t out_dim, uint32_t block_stride_words, int kbits, DispatchTables t, const uint32_t* xa, float* z,
                             uint32_t* status, int sm_count, cudaStream_t st);
 
 // prefill-sized batches: tcgen05 MMA over trellis tiles decoded to f16 in tensor memory (exl3_prefill.cu)
@@ -174,17 +172,15 @@ struct Exl3PrefillArgs {
     float limit;
     uint32_t* status;
     int sm_count;
-    // optional: a stream for the kernels of the large tiles (they touch other experts than the small-tile kernels), with
-    // the two events that fork it from and join it into the call's stream; null: one stream
-    cudaStream_t side = nullptr;
-    cudaEvent_t side_fork = nullptr, side_join = nullptr;
+    float* act;              // exl3_prefill_act_bytes(sm_count): act(gate) between a CTA's gate and up passes
 };
+size_t exl3_prefill_act_bytes(int sm_count);
 // staging rows: every tile's rows padded to 16, tiles in sorted order
 static inline size_t exl3_prefill_staging_rows(size_t rows_cap, uint32_t max_tiles) { return rows_cap + 16 * (size_t)(2 * max_tiles + 1); }
 static inline size_t exl3_prefill_xa_bytes(Exl3Dims d, size_t rows_cap, uint32_t max_tiles) { return 2 * exl3_prefill_staging_rows(rows_cap, max_tiles) * d.H * 2; }
 static inline size_t exl3_prefill_xd_bytes(Exl3Dims d, size_t rows_cap, uint32_t max_tiles) { return exl3_prefill_staging_rows(rows_cap, max_tiles) * d.I * 2; }
 cudaError_t launch_exl3_prefill(const Exl3PrefillArgs& a, cudaStream_t st);
-bool exl3_prefill_supported(Exl3Dims d);  // the lane groups 2 (gate/up) and 4 (down) column blocks per CTA
+bool exl3_prefill_supported(Exl3Dims d);  // whole stages of 128 inputs
 
 // ---- MXFP4 / NVFP4 ----
 constexpr int FP4_CHUNK_ROWS = 8;
@@ -242,8 +238,8 @@ struct Fp4PrefillArgs {
     float limit;
     uint32_t* status;
     int sm_count;
-    // optional: a stream for the kernels of the large tiles, with the events that fork it from and join it into the
-    // call's stream (as in Exl3PrefillArgs); null: one stream
+    // optional: a stream for the kernels of the large tiles (they touch other experts than the small-tile kernels), with
+    // the events that fork it from and join it into the call's stream; null: one stream
     cudaStream_t side = nullptr;
     cudaEvent_t side_fork = nullptr, side_join = nullptr;
 };
