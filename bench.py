@@ -189,7 +189,7 @@ def own_launches_per_layer(wl, T, world):
     # the tensor-core lane's kernels launch when the local call has enough "tokens" for an expert to reach the threshold
     # (with expert parallelism every received assignment is a token of the local call)
     if (T if world == 1 else A) >= lane_min_rows(wl):
-        n += 6                              # tile plan, row prep, gate/up and down in two tile shapes each
+        n += 4                              # tile plan, row prep, gate/up and down
     if wl["shared"]:
         n += 2 if T <= 64 else 3            # skinny gate/up + down, or row staging + the two tcgen05 products
     if world > 1:
@@ -634,8 +634,8 @@ def measure(rig, args, sampler, want_e2e=True):
         # prefill-sized call: the tcgen05 lane (gate/up and down launches are timed together); tensor roofline
         flops = 6.0 * H * I * rows_heavy / NL
         tf = flops / (tl_ms / max(tl_n, 1) * 1e-3) / 1e12
-        native = wl["bank"] == "mxfp4" and os.environ.get("MLXS_MXFP4_NATIVE", "1") != "0"
-        kname = "exl3_prefill_kernel" if wl["bank"] == "exl3" else ("mxfp4_native_kernel" if native else "fp4_prefill_kernel")
+        native = wl["bank"] == "mxfp4" and os.environ.get("MLXS_MXFP4_NATIVE", "0") != "0"
+        kname = "mxfp4_native_kernel" if native else "lane_kernel<Exl3LaneBank>" if wl["bank"] == "exl3" else "lane_kernel<Fp4LaneBank>"
         out["roofline"] = {"kernel": kname + "<gate/up> + <down> (tcgen05" + (", kind::mxf8f6f4.block_scale" if native else ", kind::f16") + ")",
                            "bound": "tensor", "achieved": tf, "peak": tpeak,
                            "peak_source": "measured sustained bf16" if which == "measured" else "fallback", "unit": "TFLOP/s",

@@ -81,24 +81,27 @@ template <bool RAW>
 __global__ void __launch_bounds__(CHUNK_ROWS * 32) exl3_prep_kernel(const void* __restrict__ xin, uint32_t top_k, uint32_t in_dim,
                                                         const __half* __restrict__ scales, size_t scales_stride,
                                                         DispatchTables t, uint32_t* __restrict__ xa) {
-    const uint32_t chunk = blockIdx.x;
-    if (chunk >= t.header[HDR_NCHUNKS]) return;
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;  // warp = row of the chunk
-    const uint32_t e = t.chunk_expert[chunk], rows = t.chunk_rows[chunk];
-    const bool valid = warp < rows;
-    const uint32_t assign = valid ? t.order[t.chunk_row0[chunk] + warp] : 0u;
-    const uint32_t tok = x_row_of(t, assign, top_k);
-    for (uint32_t b = blockIdx.y; b < in_dim / 128; b += gridDim.y)
-        exl3_prep_row_block<RAW>(xin, tok, valid, e, in_dim, scales, scales_stride, chunk, warp, b, lane, xa);
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, n = t.header[HDR_NCHUNKS];  // warp = row of the chunk
+    for (uint32_t chunk = blockIdx.x; chunk < n; chunk += gridDim.x) {
+        const uint32_t e = t.chunk_expert[chunk], rows = t.chunk_rows[chunk];
+        const bool valid = warp < rows;
+        const uint32_t assign = valid ? t.order[t.chunk_row0[chunk] + warp] : 0u;
+        const uint32_t tok = x_row_of(t, assign, top_k);
+        for (uint32_t b = blockIdx.y; b < in_dim / 128; b += gridDim.y)
+            exl3_prep_row_block<RAW>(xin, tok, valid, e, in_dim, scales, scales_stride, chunk, warp, b, lane, xa);
+    }
 }
+// Chunks in flight: the tables' bound counts every row of a prefill call, of which the streaming lane gets few (one CTA per
+// possible chunk took 80 us at 8192 tokens to find that out)
+static inline uint32_t prep_grid(uint32_t max_chunks) { return max_chunks < 592u ? max_chunks : 592u; }
 
 cudaError_t launch_exl3_prep_in(const __nv_bfloat16* x, uint32_t top_k, Exl3Layer L, Exl3Dims d, DispatchTables t,
                                 uint32_t* xa_gu, cudaStream_t st) {
-    exl3_prep_kernel<false><<<dim3(t.max_chunks, 8), CHUNK_ROWS * 32, 0, st>>>(x, top_k, d.H, L.scales, exl3_scales_per_expert(d), t, xa_gu);
+    exl3_prep_kernel<false><<<dim3(prep_grid(t.max_chunks), 8), CHUNK_ROWS * 32, 0, st>>>(x, top_k, d.H, L.scales, exl3_scales_per_expert(d), t, xa_gu);
     return cudaGetLastError();
 }
 cudaError_t launch_exl3_prep_raw(const float* xh, uint32_t in_dim, DispatchTables t, uint32_t* xa, cudaStream_t st) {
-    exl3_prep_kernel<true><<<dim3(t.max_chunks, 8), CHUNK_ROWS * 32, 0, st>>>(xh, 1, in_dim, nullptr, 0, t, xa);
+    exl3_prep_kernel<true><<<dim3(prep_grid(t.max_chunks), 8), CHUNK_ROWS * 32, 0, st>>>(xh, 1, in_dim, nullptr, 0, t, xa);
     return cudaGetLastError();
 }
 

@@ -89,17 +89,18 @@ cudaError_t launch_fp4_repack(const uint8_t* record_dev, uint32_t H, uint32_t I,
 // which the conversion instruction hands out a word's eight codes
 __global__ void __launch_bounds__(256) fp4_prep_kernel(const __nv_bfloat16* __restrict__ x, uint32_t top_k, uint32_t H,
                                                        DispatchTables t, uint32_t* __restrict__ xa) {
-    const uint32_t chunk = blockIdx.x;
-    if (chunk >= t.header[HDR_NCHUNKS]) return;
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;  // warp = row slot
-    const bool valid = warp < t.chunk_rows[chunk];
-    const uint32_t tok = valid ? x_row_of(t, t.order[t.chunk_row0[chunk] + warp], top_k) : 0u;
-    fp4_prep_row(x, tok, valid, H, chunk, warp, blockIdx.y * 32 + lane, gridDim.y * 32, xa);
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, n = t.header[HDR_NCHUNKS];  // warp = row slot
+    for (uint32_t chunk = blockIdx.x; chunk < n; chunk += gridDim.x) {
+        const bool valid = warp < t.chunk_rows[chunk];
+        const uint32_t tok = valid ? x_row_of(t, t.order[t.chunk_row0[chunk] + warp], top_k) : 0u;
+        fp4_prep_row(x, tok, valid, H, chunk, warp, blockIdx.y * 32 + lane, gridDim.y * 32, xa);
+    }
 }
 
 cudaError_t launch_fp4_prep(const __nv_bfloat16* x, uint32_t top_k, uint32_t H, DispatchTables t, uint32_t* xa,
                             cudaStream_t st) {
-    fp4_prep_kernel<<<dim3(t.max_chunks, 4), 256, 0, st>>>(x, top_k, H, t, xa);
+    // not one CTA per possible chunk: a prefill call's bound is thousands, nearly all of them empty
+    fp4_prep_kernel<<<dim3(t.max_chunks < 592u ? t.max_chunks : 592u, 4), 256, 0, st>>>(x, top_k, H, t, xa);
     return cudaGetLastError();
 }
 

@@ -60,7 +60,7 @@ struct mlxs_moe {
     // prefill lane (EXL3): row-tile table and operand staging, allocated when the handle can see prefill-sized calls
     uint32_t* pf_tiles = nullptr;
     __half *pf_xa = nullptr, *pf_xd = nullptr;
-    float* pf_act = nullptr;    // EXL3: act(gate) between a CTA's two passes
+    void* pf_act = nullptr;     // act(gate) between a CTA's two passes
     uint32_t pf_max_tiles = 0;
     uint32_t pf_min_rows = 0;   // experts with at least this many rows of a call take the tensor-core lane (0: lane off)
     uint32_t chunk_rows = CHUNK_ROWS, group_chunks = GROUP_CHUNKS;
@@ -90,7 +90,7 @@ struct mlxs_moe {
     EpState* ep = nullptr;
     uint32_t* front_bar = nullptr;    // grid barrier of the fused front kernel (two words)
     bool front_done = false;          // the fused front kernel of this call has built the tables and staged the rows
-    bool mxfp4_native = true;         // MXFP4 tensor-core lane on the block-scaled kind (MLXS_MXFP4_NATIVE=0 at create: the decoded-operand lane)
+    bool mxfp4_native = false;        // MXFP4 tensor-core lane on the block-scaled kind (MLXS_MXFP4_NATIVE=1 at create) instead of the decoded-operand lane
     bool front_off = false;           // a cooperative launch was refused once: separate kernels from then on
     uint32_t dbg_poll_limit = 0, dbg_withhold = 0;  // mlxs_moe_debug_wait (self-test of the bounded waits)
     uint32_t rows_cap = 0;  // rows the expert kernels' workspaces hold (assignments of one call, or received rows)

@@ -141,16 +141,17 @@ constexpr int PREFILL_TILE_ROWS = 128;
 __host__ __device__ inline bool takes_tensor_lane(uint32_t rows, uint32_t min_rows, const uint8_t* flags, uint32_t e) {
     return min_rows && rows >= min_rows && !(flags && (flags[e] & 2u));
 }
-// Row tiles of the experts that take the tensor-core lane.  tiles[0], tiles[1] = tiles of list 0 (experts with up to
+// Row tiles of the experts that take the tensor-core lane.  tiles[2] = most rows of a tile of list 0, rounded up to 16;
+// tiles[0], tiles[1] = tiles of list 0 (experts with up to
 // cap0 rows; with cap1 = 0 all experts, in tiles of up to cap0 rows) and list 1 (the others, tiles of up to cap1 rows);
 // entries {expert, first sorted row, rows, first staging row}, list 1 from entry max_tiles.  The table holds
 // prefill_tile_words(max_tiles) words.
-__host__ __device__ inline size_t prefill_tile_words(uint32_t max_tiles) { return 2 + 8 * (size_t)max_tiles; }
+__host__ __device__ inline size_t prefill_tile_words(uint32_t max_tiles) { return 4 + 8 * (size_t)max_tiles; }
 __host__ __device__ inline uint32_t* prefill_tile(uint32_t* tiles, int list, uint32_t max_tiles, uint32_t i) {
-    return tiles + 2 + 4 * ((size_t)(list ? max_tiles : 0) + i);
+    return tiles + 4 + 4 * ((size_t)(list ? max_tiles : 0) + i);
 }
 __host__ __device__ inline const uint32_t* prefill_tile(const uint32_t* tiles, int list, uint32_t max_tiles, uint32_t i) {
-    return tiles + 2 + 4 * ((size_t)(list ? max_tiles : 0) + i);
+    return tiles + 4 + 4 * ((size_t)(list ? max_tiles : 0) + i);
 }
 cudaError_t launch_prefill_plan(DispatchTables t, uint32_t n_experts, const uint8_t* lane_flags, uint32_t min_rows,
                                 uint32_t cap0, uint32_t cap1, uint32_t max_tiles, uint32_t* tiles, uint32_t* status,
@@ -172,9 +173,9 @@ struct Exl3PrefillArgs {
     float limit;
     uint32_t* status;
     int sm_count;
-    float* act;              // exl3_prefill_act_bytes(sm_count): act(gate) between a CTA's gate and up passes
+    void* act;               // lane_act_bytes(sm_count): act(gate) between a CTA's gate and up passes
 };
-size_t exl3_prefill_act_bytes(int sm_count);
+size_t lane_act_bytes(int sm_count);
 // staging rows: every tile's rows padded to 16, tiles in sorted order
 static inline size_t exl3_prefill_staging_rows(size_t rows_cap, uint32_t max_tiles) { return rows_cap + 16 * (size_t)(2 * max_tiles + 1); }
 static inline size_t exl3_prefill_xa_bytes(Exl3Dims d, size_t rows_cap, uint32_t max_tiles) { return 2 * exl3_prefill_staging_rows(rows_cap, max_tiles) * d.H * 2; }
@@ -238,7 +239,8 @@ struct Fp4PrefillArgs {
     float limit;
     uint32_t* status;
     int sm_count;
-    // optional: a stream for the kernels of the large tiles (they touch other experts than the small-tile kernels), with
+    void* act;               // lane_act_bytes(sm_count): act(gate) between a CTA's gate and up passes (not used by launch_mxfp4_native)
+    // launch_mxfp4_native, optional: a stream for the kernels of the large tiles (they touch other experts than the small-tile kernels), with
     // the events that fork it from and join it into the call's stream; null: one stream
     cudaStream_t side = nullptr;
     cudaEvent_t side_fork = nullptr, side_join = nullptr;

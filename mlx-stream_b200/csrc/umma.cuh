@@ -40,6 +40,10 @@ __device__ __forceinline__ bool elect_one() {
     return p != 0;
 }
 // a bounded wait by all lanes of a warp: one answer for the warp
+__device__ __forceinline__ bool mbar_wait_warp_at(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+    if (__all_sync(0xFFFFFFFFu, mbar_try_wait_at(bar, parity))) return true;
+    return __all_sync(0xFFFFFFFFu, mbar_wait_bounded_at(bar, parity, abort_flag));
+}
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, uint32_t sleep_ns = 0,
                                                uint32_t limit = (1u << 20)) {
     return __all_sync(0xFFFFFFFFu, mbar_wait_bounded(bar, parity, abort_flag, sleep_ns, limit));
@@ -68,9 +72,10 @@ __device__ __forceinline__ void umma_f16_ts_lohi(uint32_t tmem_d, uint32_t tmem_
         ::"r"(tmem_d), "r"(tmem_a), "r"(db_lo), "r"(db_hi), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+__device__ __forceinline__ void umma_commit_at(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
+__device__ __forceinline__ void umma_commit(uint64_t* bar) { umma_commit_at(smem_u32(bar)); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
