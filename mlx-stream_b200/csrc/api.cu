@@ -671,7 +671,7 @@ int mlxs_run_routed(mlxs_moe* h, uint32_t layer, const void* x_dev, const int32_
         a.L = EL; a.d = d; a.t = h->tabs; a.xa_gu = h->xa_gu; a.xa_d = h->xa_d; a.ro = static_cast<float*>(ro); a.ro_bf16 = 0;
         a.limit = limit;
         a.status = h->status; a.sm_count = h->sm_count; a.ks_scratch = h->ks_scratch; a.ks_count = h->ks_count;
-        a.poll_limit = h->dbg_poll_limit; a.withhold = h->dbg_withhold;
+        a.poll_limit = h->dbg_poll_limit; a.withhold = h->dbg_withhold; a.dependent = !two_lanes;
         {
             StageTimer tm(h, MLXS_STAGE_GATE_UP, st);
             CU(launch_exl3_gate_up(a, st));
@@ -704,7 +704,7 @@ int mlxs_run_routed(mlxs_moe* h, uint32_t layer, const void* x_dev, const int32_
         Fp4GemvArgs a{};
         a.gu = L.f4_gu; a.dn = L.f4_dn; a.nv = c.bank_kind == MLXS_BANK_NVFP4; a.gscale = a.nv ? L.f4_gscale : nullptr;
         a.H = c.hidden; a.I = c.inter; a.t = h->tabs; a.xa = h->xa_gu; a.xa_d = h->xa_d; a.ro = ro;
-        a.ro_bf16 = ro_bf16; a.limit = limit;
+        a.ro_bf16 = ro_bf16; a.limit = limit; a.dependent = !two_lanes;
         a.status = h->status; a.sm_count = h->sm_count; a.ks_scratch = h->ks_scratch; a.ks_count = h->ks_count;
         {
             StageTimer tm(h, MLXS_STAGE_GATE_UP, st);
@@ -788,20 +788,10 @@ static int experts_impl(mlxs_moe* h, uint32_t layer, const void* x_dev, const in
         return MLXS_OK;
     };
     ForkGuard aux_guard(st);
-    if (shared_aside) {
-        CU(cudaEventRecord(h->aux_fork, st));
-        CU(cudaStreamWaitEvent(h->aux_stream, h->aux_fork, 0));
-        aux_guard.arm(h->aux_stream, h->aux_join);
-        {
-            StageTimer tm(h, MLXS_STAGE_SHARED, h->aux_stream);
-            if ((rc = run_shared(h->aux_stream))) return rc;
-        }
-        CU(aux_guard.record());
-        shared = h->sh_out;
-    }
+    // the fork is recorded before the front kernel and used after its launch: the front's few CTAs find their SMs first
+    if (shared_aside) CU(cudaEventRecord(h->aux_fork, st));
     if (front) {
-        // route (from the logits, or from x through the layer's router weight), sort and stage in one launch; the
-        // shared expert is already running beside it
+        // route (from the logits, or from x through the layer's router weight), sort and stage in one launch
         FrontArgs fa{};
         fa.w_router = front->logits ? nullptr : L.router_w; fa.logits_out = h->logits_ws; fa.logits = front->logits; fa.bias = L.bias;
         fa.E = (int)c.n_experts; fa.K = (int)c.top_k; fa.scoring = (int)c.scoring; fa.norm = (int)c.norm_topk; fa.scale = c.routed_scale;
@@ -829,6 +819,16 @@ static int experts_impl(mlxs_moe* h, uint32_t layer, const void* x_dev, const in
             CU(launch_router(lg, L.bias, (int)T, (int)c.n_experts, (int)c.top_k, (int)c.scoring, (int)c.norm_topk, c.routed_scale,
                              h->ids_ws, h->w_ws, st));
         }
+    }
+    if (shared_aside) {
+        CU(cudaStreamWaitEvent(h->aux_stream, h->aux_fork, 0));
+        aux_guard.arm(h->aux_stream, h->aux_join);
+        {
+            StageTimer tm(h, MLXS_STAGE_SHARED, h->aux_stream);
+            if ((rc = run_shared(h->aux_stream))) { h->front_done = false; return rc; }
+        }
+        CU(aux_guard.record());
+        shared = h->sh_out;
     }
     if (!ep_fused && (rc = run_routed(h, layer, x_dev, ids_dev, T, h->ro, ro_bf16, st))) { h->front_done = false; return rc; }
     if (c.shared_expert && !shared_aside) {

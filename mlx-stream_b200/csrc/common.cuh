@@ -72,6 +72,21 @@ __device__ __forceinline__ void bulk_g2s(void* dst_smem, const void* src_gmem, u
                  "l"(src_gmem), "r"(bytes), "r"(smem_u32(bar))
                  : "memory");
 }
+// Programmatic dependent launch (the chain router -> dispatch -> staging -> gate/up -> down -> combine): a kernel lets the
+// next one of the stream start while it still runs; the next one does what needs nothing of it (its prologue, the down
+// kernel its first weight copies) and then waits for the whole grid before it and for its memory.  A kernel allows its
+// successor only after its own wait, so whatever a successor reads before waiting comes from grids that are complete.
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <class... Params, class... Args>
+static inline cudaError_t launch_dependent(bool dependent, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st; cfg.attrs = &attr; cfg.numAttrs = dependent ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
@@ -93,11 +108,15 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
 // ---- EXL3 mul1: two 16-bit trellis states -> half2 (lo = a, hi = b) ----
 // value = f16( (1024 + bytesum(state * 0x83DCD12D)) * h(0x1EEE) + h(0xC931) ), one rounding
 // (src/exl3/kernels.zig:963-971; src/kernels/exl3/dsv41_exl3_mul1h_k3_2304.metal:27-31)
+// PRMT: the two halves are put together by a byte permute (logic pipe) instead of a multiply-add: with 16 of a tile's
+// instructions on the half-rate multiply pipe the streaming kernels are 1 % (K = 3) to 4 % (K = 2) faster that way, the
+// tensor-core lane, whose epilogue warps use the logic pipe, is not.
+template <bool PRMT>
 __device__ __forceinline__ uint32_t mul1_pair(uint32_t sa, uint32_t sb) {
     uint32_t xa = sa * MUL1, xb = sb * MUL1;
     uint32_t ha = __dp4a(xa, 0x01010101u, 0x6400u);  // 0x6400 + byte sum = the half bits of 1024 + s
     uint32_t hb = __dp4a(xb, 0x01010101u, 0x6400u);
-    uint32_t pk = hb * 65536u + ha;
+    uint32_t pk = PRMT ? __byte_perm(ha, hb, 0x5410) : hb * 65536u + ha;
     const uint32_t kinv = 0x1EEE1EEEu, kbias = 0xC931C931u;
     __half2 r = __hfma2(*reinterpret_cast<__half2*>(&pk), *reinterpret_cast<const __half2*>(&kinv),
                         *reinterpret_cast<const __half2*>(&kbias));
@@ -109,6 +128,7 @@ __device__ __forceinline__ uint32_t mul1_pair(uint32_t sa, uint32_t sb) {
 // distance of the last bit from the word's bit 0.  Returns the two B fragments (k16 x n8) of the tile's column
 // halves for mma m16n8k16: b[0], b[1] = columns 0..7, b[2], b[3] = columns 8..15 (the exllamav3 tensor-core order,
 // src/exl3/kernels.zig:978-986).
+template <bool PRMT = false>
 __device__ __forceinline__ void exl3_decode_lane(uint32_t lo, uint32_t hi, uint32_t lp, uint32_t (&b)[4]) {
     uint32_t v0 = __funnelshift_r(lo, hi, lp);  // stream bits, window m at bits [3m, 3m+16)
     uint32_t vh = hi >> lp;
@@ -122,10 +142,10 @@ __device__ __forceinline__ void exl3_decode_lane(uint32_t lo, uint32_t hi, uint3
     uint32_t w6 = v1 & 0xFFFFu;
     uint32_t w7 = (v1 >> 3) & 0xFFFFu;
     // code position j = 7 - m; positions (0,1),(2,3) -> columns 0..7 rows (r0,r0+1),(r0+8,r0+9); (4,5),(6,7) -> 8..15
-    b[0] = mul1_pair(w7, w6);
-    b[1] = mul1_pair(w5, w4);
-    b[2] = mul1_pair(w3, w2);
-    b[3] = mul1_pair(w1, w0);
+    b[0] = mul1_pair<PRMT>(w7, w6);
+    b[1] = mul1_pair<PRMT>(w5, w4);
+    b[2] = mul1_pair<PRMT>(w3, w2);
+    b[3] = mul1_pair<PRMT>(w1, w0);
 }
 __device__ __forceinline__ void exl3_lane_plan(uint32_t lane, uint32_t& wi, uint32_t& wj, uint32_t& lp) {
     wi = (3u * lane + 2u) >> 2;        // word of the lane's last stream bit
@@ -137,14 +157,15 @@ __device__ __forceinline__ void exl3_lane_plan(uint32_t lane, uint32_t& wi, uint
 // lp = 0 when halfword L is the word's low half, 16 when it is the high half; window m at bits [2m, 2m + 16).
 // Bit-level definition: src/exl3/kernels.zig:988-1020 (tileStates at K = 2), generic window formulas
 // scripts/dsv41_exl3_k2_gen.py:96-112.
+template <bool PRMT = false>
 __device__ __forceinline__ void exl3_decode_lane_k2(uint32_t lo, uint32_t hi, uint32_t lp, uint32_t (&b)[4]) {
     const uint32_t v0 = __funnelshift_r(lo, hi, lp);
     const uint32_t w0 = v0 & 0xFFFFu, w1 = (v0 >> 2) & 0xFFFFu, w2 = (v0 >> 4) & 0xFFFFu, w3 = (v0 >> 6) & 0xFFFFu;
     const uint32_t w4 = (v0 >> 8) & 0xFFFFu, w5 = (v0 >> 10) & 0xFFFFu, w6 = (v0 >> 12) & 0xFFFFu, w7 = (v0 >> 14) & 0xFFFFu;
-    b[0] = mul1_pair(w7, w6);
-    b[1] = mul1_pair(w5, w4);
-    b[2] = mul1_pair(w3, w2);
-    b[3] = mul1_pair(w1, w0);
+    b[0] = mul1_pair<PRMT>(w7, w6);
+    b[1] = mul1_pair<PRMT>(w5, w4);
+    b[2] = mul1_pair<PRMT>(w3, w2);
+    b[3] = mul1_pair<PRMT>(w1, w0);
 }
 __device__ __forceinline__ void exl3_lane_plan_k2(uint32_t lane, uint32_t& wi, uint32_t& wj, uint32_t& lp) {
     wi = lane >> 1;
@@ -152,10 +173,10 @@ __device__ __forceinline__ void exl3_lane_plan_k2(uint32_t lane, uint32_t& wi, u
     lp = (lane & 1u) ? 0u : 16u;
 }
 // by code width
-template <int KB>
+template <int KB, bool PRMT = false>
 __device__ __forceinline__ void exl3_decode_lane_kb(uint32_t lo, uint32_t hi, uint32_t lp, uint32_t (&b)[4]) {
-    if (KB == 3) exl3_decode_lane(lo, hi, lp, b);
-    else exl3_decode_lane_k2(lo, hi, lp, b);
+    if (KB == 3) exl3_decode_lane<PRMT>(lo, hi, lp, b);
+    else exl3_decode_lane_k2<PRMT>(lo, hi, lp, b);
 }
 template <int KB>
 __device__ __forceinline__ void exl3_lane_plan_kb(uint32_t lane, uint32_t& wi, uint32_t& wj, uint32_t& lp) {

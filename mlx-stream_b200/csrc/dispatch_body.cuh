@@ -82,7 +82,7 @@ __device__ __forceinline__ void build_tables(const uint32_t* cnt, uint32_t E, co
         }
         for (uint32_t i = 0; i < ng; ++i) {
             t.group_chunk0[ex[2] + i] = ex[1] + i * GROUP_CHUNKS;
-            t.group_mc[ex[2] + i] = min(GROUP_CHUNKS, nc - i * GROUP_CHUNKS);
+            t.group_mc[ex[2] + i] = min(GROUP_CHUNKS, nc - i * GROUP_CHUNKS) | e << 16;
         }
     }
 }

@@ -143,8 +143,10 @@ struct GemvParams {
 };
 
 // flags: 1 = first stage of a part of the sum, 2 = last stage of a part, 4 = last stage of this CTA's share of the item;
-// bits 16.. = sub-stages (of KT k-tiles each) this ring slot carries
-struct StageMeta { int32_t item; uint32_t flags, mc, kt0, chunk0, expert, nb, part; };
+// bits 3.. = the straight-line form that serves the slot (slot_form).  Only item and flags are read every stage.
+struct StageMeta { int32_t item; uint32_t flags, mc, chunk0, expert, nb, part, pad; };
+// (chunks of rows, sub-stages of KT k-tiles) -> 0 .. 7; rows in 3 or 4 chunks always come one sub-stage per slot
+__device__ __forceinline__ uint32_t slot_form(uint32_t mc, uint32_t sub) { return mc <= 2 ? (mc - 1) * 3 + sub - 1 : mc + 3; }
 
 // one pipeline stage (KT k-tiles) of one warp's 16-column tile, MC chunks of activations
 template <int NPROJ, int KB, int MC>
@@ -156,7 +158,7 @@ __device__ __forceinline__ void gemv_stage(const uint32_t* __restrict__ wt, cons
     for (int kt = 0; kt < KT; ++kt) {
         const uint32_t lo = wt[kt * KSTRIDE + wi], hi = wt[kt * KSTRIDE + wj];
         uint32_t b[4];
-        exl3_decode_lane_kb<KB>(lo, hi, lp, b);
+        exl3_decode_lane_kb<KB, true>(lo, hi, lp, b);
         // W^T as the A operand: rows = the tile's 16 output columns
         const uint32_t a[4] = {b[0], b[2], b[1], b[3]};
 #pragma unroll
@@ -167,13 +169,16 @@ __device__ __forceinline__ void gemv_stage(const uint32_t* __restrict__ wt, cons
     }
 }
 
-// SUB sub-stages of one ring slot, unrolled
+// SUB sub-stages of one ring slot, unrolled: [projection][SUB x KT k-tiles of codes][chunk][projection][SUB x KT row tiles]
 template <int NPROJ, int KB, int MC, int SUB>
-__device__ __forceinline__ void gemv_slot(const uint32_t* __restrict__ wt, const uint2* __restrict__ at, uint32_t mt_stride,
-                                          uint32_t wi, uint32_t wj, uint32_t lp, float (&acc)[GROUP_CHUNKS][4]) {
+__device__ __forceinline__ void gemv_slot(const uint8_t* __restrict__ st, uint32_t p, uint32_t lane, uint32_t wi, uint32_t wj,
+                                          uint32_t lp, float (&acc)[GROUP_CHUNKS][4]) {
+    constexpr uint32_t CODE = SUB * KT * (64 * KB) * 4, ROWS = SUB * KT * A_TILE_WORDS * 4;   // bytes of one projection
+    const uint32_t* wt = reinterpret_cast<const uint32_t*>(st + (NPROJ == 2 ? p * CODE : 0u));
+    const uint2* at = reinterpret_cast<const uint2*>(st + NPROJ * CODE + (NPROJ == 2 ? p * ROWS : 0u)) + lane;
 #pragma unroll
     for (int u = 0; u < SUB; ++u)
-        gemv_stage<NPROJ, KB, MC>(wt + u * KT * (64 * KB), at + u * KT * 32, mt_stride, wi, wj, lp, acc);
+        gemv_stage<NPROJ, KB, MC>(wt + u * KT * (64 * KB), at + u * KT * 32, NPROJ * SUB * KT * 32, wi, wj, lp, acc);
 }
 
 // KB = bits per weight
@@ -184,8 +189,9 @@ __global__ void __launch_bounds__(NPROJ * 256 + 32, NPROJ == 1 ? 3 : 2) exl3_gem
     extern __shared__ __align__(128) uint8_t smem_raw[];
     constexpr int NCW = NPROJ * 8;         // consumer warps: projection x 16-column tile of the 128 block
     constexpr int MAXS = 8;
-    __shared__ __align__(8) uint64_t full_bar[MAXS], empty_bar[MAXS], epi_bar;
-    __shared__ __align__(8) StageMeta meta[MAXS];
+    __shared__ __align__(8) uint64_t ring_bar[2 * MAXS], epi_bar;   // per slot: full, then (+ MAXS) empty
+    uint64_t *full_bar = ring_bar, *empty_bar = ring_bar + MAXS;
+    __shared__ __align__(16) StageMeta meta[MAXS];
     __shared__ volatile int s_abort;
     __shared__ volatile int s_last_part;
     // epilogue staging: [NPROJ][GROUP_CHUNKS][CHUNK_ROWS][ZS_STRIDE]
@@ -199,6 +205,12 @@ __global__ void __launch_bounds__(NPROJ * 256 + 32, NPROJ == 1 ? 3 : 2) exl3_gem
         mbar_init(&epi_bar, NCW);
         s_abort = 0;
         mbar_fence_init();
+    }
+    // The down kernel's prologue and first weight copies come before gate/up is complete (its producer waits, below);
+    // everything else after the grid before
+    if (EPI != EPI_DOWN) {
+        grid_dep_wait();
+        grid_dep_launch();
     }
     __syncthreads();
     const uint32_t n_items = P.t.header[HDR_NGROUPS] * P.n_blocks;
@@ -215,15 +227,19 @@ __global__ void __launch_bounds__(NPROJ * 256 + 32, NPROJ == 1 ? 3 : 2) exl3_gem
             uint32_t s = 0, ph = 0;     // ring slot and phase
             uint32_t n_stage = 0;       // stages this producer has filled (self-test: the withheld one)
             const uint32_t np_mask = NP - 1, np_shift = NP == 4 ? 2u : (NP == 2 ? 1u : 0u);
-            bool ok = true;
+            bool ok = true, first = true;
+            // down: the weights of the first ring slots go out before gate/up is complete, the slots' rows after the wait
+            bool dep_done = EPI != EPI_DOWN;
             while (ok) {
-                const uint32_t unit = atomicAdd(&P.t.header[P.counter_idx], 1u);
+                // the first unit is the CTA's own number (no round trip before the first copy), the others come from the counter
+                const uint32_t unit = first ? blockIdx.x : gridDim.x + atomicAdd(&P.t.header[P.counter_idx], 1u);
+                first = false;
                 const bool last = unit >= n_items * NP;
                 const uint32_t item = unit >> np_shift, share = unit & np_mask;
                 uint32_t g = 0, nb = 0, chunk0 = 0, mc = 0, expert = 0;
                 if (!last) {
                     g = item / P.n_blocks; nb = item % P.n_blocks;
-                    chunk0 = P.t.group_chunk0[g]; mc = P.t.group_mc[g]; expert = P.t.chunk_expert[chunk0];
+                    chunk0 = P.t.group_chunk0[g]; mc = P.t.group_mc[g]; expert = mc >> 16; mc &= 0xFFFFu;
                 }
                 const uint32_t* wsrc = P.code + (size_t)expert * P.expert_stride_words +
                                        (size_t)nb * P.block_stride_words;
@@ -243,10 +259,10 @@ __global__ void __launch_bounds__(NPROJ * 256 + 32, NPROJ == 1 ? 3 : 2) exl3_gem
                         s_abort = 1; ok = false; break;
                     }
                     meta[s].item = last ? -1 : (int32_t)item;
-                    meta[s].kt0 = kt0; meta[s].chunk0 = chunk0; meta[s].mc = mc; meta[s].expert = expert; meta[s].nb = nb;
+                    meta[s].chunk0 = chunk0; meta[s].mc = mc; meta[s].expert = expert; meta[s].nb = nb;
                     meta[s].part = part;
                     const bool part_ends = in_part + step == part_kt;
-                    meta[s].flags = (in_part == 0 ? 1u : 0u) | (part_ends ? 2u : 0u) | (kt0 + step >= k_end ? 4u : 0u) | (sub << 16);
+                    meta[s].flags = (in_part == 0 ? 1u : 0u) | (part_ends ? 2u : 0u) | (kt0 + step >= k_end ? 4u : 0u) | (slot_form(mc, sub) << 3);
                     in_part = part_ends ? 0u : in_part + step;
                     part += part_ends ? 1u : 0u;
                     if (last) { mbar_arrive(&full_bar[s]); ok = false; break; }
@@ -256,13 +272,24 @@ __global__ void __launch_bounds__(NPROJ * 256 + 32, NPROJ == 1 ? 3 : 2) exl3_gem
                     for (int p = 0; p < NPROJ; ++p)
                         bulk_g2s(dst + p * (sub * KT * KT_WORDS * 4), wsrc + ((size_t)p * P.nkt + kt0) * KT_WORDS, sub * KT * KT_WORDS * 4,
                                  &full_bar[s]);
-                    for (uint32_t m = 0; m < mc; ++m)
-                        for (int p = 0; p < NPROJ; ++p)
-                            bulk_g2s(dst + sub * P.w_bytes + (m * NPROJ + p) * xa_bytes,
-                                     P.xa + (((size_t)(chunk0 + m) * NPROJ + p) * P.nkt + kt0) * A_TILE_WORDS, xa_bytes,
-                                     &full_bar[s]);
+                    // the rows of this stage, or of the stages whose weights went ahead (slots 0, 1, ... of the first unit)
+                    uint32_t r_kt = kt0, r_s = s;
+                    if (!dep_done) {
+                        if (s + 1 < NS && kt0 + step < k_end) continue;
+                        grid_dep_wait();
+                        grid_dep_launch();
+                        dep_done = true; r_kt = k_begin; r_s = 0;
+                    }
+                    for (; r_kt <= kt0; r_kt += step, ++r_s) {
+                        uint8_t* rows = ring + (size_t)r_s * P.stage_bytes + sub * P.w_bytes;
+                        for (uint32_t m = 0; m < mc; ++m)
+                            for (int p = 0; p < NPROJ; ++p)
+                                bulk_g2s(rows + (m * NPROJ + p) * xa_bytes,
+                                         P.xa + (((size_t)(chunk0 + m) * NPROJ + p) * P.nkt + r_kt) * A_TILE_WORDS, xa_bytes, &full_bar[r_s]);
+                    }
                 }
             }
+            if (!dep_done) grid_dep_wait();   // no work: this grid is still not complete before the one before it
             // after a give-up: let copies already issued land before the CTA's shared memory is released
             if (s_abort) for (int i = 0; i < 2000; ++i) __nanosleep(1000);
         }
@@ -270,7 +297,7 @@ __global__ void __launch_bounds__(NPROJ * 256 + 32, NPROJ == 1 ? 3 : 2) exl3_gem
     }
 
     // ---------------- consumer warps ----------------
-    const uint32_t p = warp >> 3, j = warp & 7u;  // projection, 16-column tile
+    const uint32_t p = NPROJ == 2 ? warp >> 3 : 0u, j = warp & 7u;  // projection, 16-column tile
     uint32_t wi, wj, lp;
     exl3_lane_plan_kb<KB>(lane, wi, wj, lp);
     float acc[GROUP_CHUNKS][4];
@@ -285,46 +312,60 @@ __global__ void __launch_bounds__(NPROJ * 256 + 32, NPROJ == 1 ? 3 : 2) exl3_gem
         if (!ok) { if (!s_abort) atomicMax(P.status, (uint32_t)ST_WAIT_FULL); s_abort = 1; }
         return ok;
     };
-    // ring slot and its phase advance by increment-and-wrap (the ring depth is a run-time value: no division per stage)
-    for (uint32_t s = 0, ph = 0;; s = (s + 1 == NS) ? (ph ^= 1u, 0u) : s + 1) {
-        if (!mbar_wait_bounded(&full_bar[s], ph, &s_abort, 0, P.poll_limit)) {
+    // ring slot, its barriers, its meta and its phase advance by increment-and-wrap (the ring depth is a run-time value: no
+    // division per stage, and as little else as possible: the decode leaves no free issue slots)
+    const uint32_t full0 = smem_u32(&full_bar[0]), full_end = full0 + 8 * NS;
+    wi += j * TW; wj += j * TW;            // words of this warp's tile inside a k-tile
+    uint32_t bar = full0, ph = 0;
+    const uint8_t* st = ring;
+    const StageMeta* mp = &meta[0];
+    for (;;) {
+        if (!mbar_wait_bounded_at(bar, ph, &s_abort, 0, P.poll_limit)) {
             if (!s_abort) atomicMax(P.status, (uint32_t)ST_WAIT_FULL);
             s_abort = 1;
             break;
         }
-        const StageMeta m = meta[s];
-        if (m.item < 0) break;
-        const uint32_t flags = m.flags, stage_mc = m.mc;
+        const uint2 hot = *reinterpret_cast<const uint2*>(mp);   // item, flags
+        if ((int32_t)hot.x < 0) break;
+        const uint32_t flags = hot.y, form = hot.y >> 3;
         if (flags & 1u) {
 #pragma unroll
             for (int a = 0; a < GROUP_CHUNKS; ++a)
 #pragma unroll
                 for (int c = 0; c < 4; ++c) acc[a][c] = 0.f;
         }
-        // slot: [projection][sub x KT k-tiles of codes][chunk][projection][sub x KT activation tiles]
-        const uint32_t sub = flags >> 16;
-        const uint8_t* st = ring + (size_t)s * P.stage_bytes;
-        const uint32_t* wt = reinterpret_cast<const uint32_t*>(st) + p * (sub * KT * KT_WORDS) + j * TW;
-        const uint2* at = reinterpret_cast<const uint2*>(st + sub * P.w_bytes) + p * (sub * KT * 32) + lane;
-        const uint32_t mt_stride = NPROJ * sub * KT * 32;
         static_assert(GROUP_CHUNKS * CHUNK_ROWS == 16, "the K-split workspace is sized for 16 rows per item");
         static_assert(GROUP_CHUNKS == 4, "the stage dispatch below enumerates the chunk counts");
-        // straight-line code per (chunks, sub-stages): rows in 3 or 4 chunks always come one sub-stage per slot
-        if (stage_mc == 1) {
-            if (sub == 2) gemv_slot<NPROJ, KB, 1, 2>(wt, at, mt_stride, wi, wj, lp, acc);
-            else if (sub == 3) gemv_slot<NPROJ, KB, 1, 3>(wt, at, mt_stride, wi, wj, lp, acc);
-            else gemv_slot<NPROJ, KB, 1, 1>(wt, at, mt_stride, wi, wj, lp, acc);
-        } else if (stage_mc == 2) {
-            if (sub == 2) gemv_slot<NPROJ, KB, 2, 2>(wt, at, mt_stride, wi, wj, lp, acc);
-            else if (sub == 3) gemv_slot<NPROJ, KB, 2, 3>(wt, at, mt_stride, wi, wj, lp, acc);
-            else gemv_slot<NPROJ, KB, 2, 1>(wt, at, mt_stride, wi, wj, lp, acc);
-        } else if (stage_mc == 3) {
-            gemv_slot<NPROJ, KB, 3, 1>(wt, at, mt_stride, wi, wj, lp, acc);
+        // straight-line code per slot_form
+        if (form < 3) {
+            if (form == 1) gemv_slot<NPROJ, KB, 1, 2>(st, p, lane, wi, wj, lp, acc);
+            else if (form == 2) gemv_slot<NPROJ, KB, 1, 3>(st, p, lane, wi, wj, lp, acc);
+            else gemv_slot<NPROJ, KB, 1, 1>(st, p, lane, wi, wj, lp, acc);
+        } else if (form < 6) {
+            if (form == 4) gemv_slot<NPROJ, KB, 2, 2>(st, p, lane, wi, wj, lp, acc);
+            else if (form == 5) gemv_slot<NPROJ, KB, 2, 3>(st, p, lane, wi, wj, lp, acc);
+            else gemv_slot<NPROJ, KB, 2, 1>(st, p, lane, wi, wj, lp, acc);
+        } else if (form == 6) {
+            gemv_slot<NPROJ, KB, 3, 1>(st, p, lane, wi, wj, lp, acc);
         } else {
-            gemv_slot<NPROJ, KB, 4, 1>(wt, at, mt_stride, wi, wj, lp, acc);
+            gemv_slot<NPROJ, KB, 4, 1>(st, p, lane, wi, wj, lp, acc);
+        }
+        // the slot may be refilled once this warp has arrived below.  (Gate/up has 56 registers a thread: the copy of the
+        // whole struct spilled, 4 % at K = 2)
+        StageMeta m;
+        m.item = (int32_t)hot.x;
+        if (flags & 2u) {
+            if (NPROJ == 2) {
+                const uint4 q = reinterpret_cast<const uint4*>(mp)[1];
+                m.mc = mp->mc; m.chunk0 = mp->chunk0; m.expert = q.x; m.nb = q.y; m.part = q.z;
+            } else {
+                m = *mp;
+            }
         }
         __syncwarp();
-        if (lane == 0) mbar_arrive(&empty_bar[s]);
+        if (lane == 0) mbar_arrive_at(bar + 8 * MAXS);
+        bar += 8; st += P.stage_bytes; ++mp;
+        if (bar == full_end) { bar = full0; st = ring; mp = &meta[0]; ph ^= 1u; }
         if (!(flags & 2u)) continue;
 
         // ---------------- end of a part of the sum ----------------
@@ -450,7 +491,8 @@ static int tune_env(const char* name, int dflt, int lo, int hi) {
     return x < lo ? lo : (x > hi ? hi : x);
 }
 
-static cudaError_t launch_gemv(int nproj, int epi, int kbits, GemvParams& P, int sm_count, cudaStream_t st) {
+// dependent: the kernel may become resident while the one before it in the stream still runs (common.cuh)
+static cudaError_t launch_gemv(int nproj, int epi, int kbits, GemvParams& P, int sm_count, cudaStream_t st, bool dependent) {
     const uint32_t zs_bytes = (uint32_t)(nproj * GROUP_CHUNKS * CHUNK_ROWS * ZS_STRIDE * sizeof(float));
     P.w_bytes = (uint32_t)(KT * nproj * 64 * kbits * 4);
     const uint32_t stage_one = P.w_bytes + GROUP_CHUNKS * nproj * KT * A_TILE_WORDS * 4;   // one sub-stage, 4 chunks of rows
@@ -478,7 +520,8 @@ static cudaError_t launch_gemv(int nproj, int epi, int kbits, GemvParams& P, int
     do {                                                                                                         \
         e = cudaFuncSetAttribute(exl3_gemv_kernel<NP, EP, KBITS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
         if (e != cudaSuccess) return e;                                                                          \
-        exl3_gemv_kernel<NP, EP, KBITS><<<ctas, NP * 256 + 32, smem, st>>>(P);                               \
+        e = launch_dependent(dependent, exl3_gemv_kernel<NP, EP, KBITS>, ctas, NP * 256 + 32, smem, st, P);      \
+        if (e != cudaSuccess) return e;                                                                          \
     } while (0)
     if (kbits == 3) {
         if (nproj == 2) MLXS_LAUNCH(2, EPI_GATE_UP, 3);
@@ -506,7 +549,7 @@ cudaError_t launch_exl3_gate_up(const Exl3GemvArgs& a, cudaStream_t st) {
     P.ks_scratch = a.ks_scratch; P.ks_count = a.ks_count; P.n_sm = (uint32_t)a.sm_count;
     P.ks_cap_items = ksplit_cap_items(a.sm_count, (size_t)2 * GROUP_CHUNKS * CHUNK_ROWS * ZS_STRIDE * sizeof(float));
     P.poll_limit = a.poll_limit ? a.poll_limit : (1u << 20); P.withhold = a.withhold;
-    return launch_gemv(2, EPI_GATE_UP, (int)a.d.K, P, a.sm_count, st);
+    return launch_gemv(2, EPI_GATE_UP, (int)a.d.K, P, a.sm_count, st, true);
 }
 cudaError_t launch_exl3_down(const Exl3GemvArgs& a, cudaStream_t st) {
     GemvParams P{};
@@ -519,7 +562,7 @@ cudaError_t launch_exl3_down(const Exl3GemvArgs& a, cudaStream_t st) {
     P.ks_scratch = a.ks_scratch; P.ks_count = a.ks_count; P.n_sm = (uint32_t)a.sm_count;
     P.ks_cap_items = ksplit_cap_items(a.sm_count, (size_t)GROUP_CHUNKS * CHUNK_ROWS * ZS_STRIDE * sizeof(float));
     P.poll_limit = a.poll_limit ? a.poll_limit : (1u << 20); P.withhold = 0;
-    return launch_gemv(1, EPI_DOWN, (int)a.d.K, P, a.sm_count, st);
+    return launch_gemv(1, EPI_DOWN, (int)a.d.K, P, a.sm_count, st, a.dependent);
 }
 cudaError_t launch_exl3_raw(const uint32_t* code_e, uint32_t in_dim, uint32_t out_dim, uint32_t block_stride_words, int kbits, DispatchTables t, const uint32_t* xa, float* z,
                             uint32_t* status, int sm_count, cudaStream_t st) {
@@ -529,7 +572,7 @@ cudaError_t launch_exl3_raw(const uint32_t* code_e, uint32_t in_dim, uint32_t ou
     P.xa = xa; P.t = t; P.counter_idx = HDR_CTR_AUX;
     P.scales = nullptr; P.scales_stride = 0; P.H = 0; P.I = 0; P.xa_d = nullptr; P.out = z; P.out_dim = out_dim;
     P.limit = 0.f; P.status = status; P.poll_limit = 1u << 20; P.withhold = 0;
-    return launch_gemv(1, EPI_RAW, kbits, P, sm_count, st);
+    return launch_gemv(1, EPI_RAW, kbits, P, sm_count, st, false);
 }
 
 }  // namespace mlxs

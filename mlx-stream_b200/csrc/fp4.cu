@@ -249,6 +249,12 @@ __global__ void __launch_bounds__(NPROJ * 256 + 32, NPROJ == 1 ? 3 : 2) fp4_gemv
         const __half2 hv = e4m3_half2(threadIdx.x);
         s_lut[threadIdx.x] = *reinterpret_cast<const uint32_t*>(&hv);
     }
+    // The down kernel's prologue and first weight copies come before gate/up is complete (its producer waits, below);
+    // everything else after the grid before
+    if (NPROJ == 2) {
+        grid_dep_wait();
+        grid_dep_launch();
+    }
     __syncthreads();
     const uint32_t n_items = P.t.header[HDR_NGROUPS] * P.n_blocks;
     const uint32_t xa_chunk_words = (NPROJ == 2 ? P.H : P.I) / 32 * F4_XA_SB_WORDS;
@@ -263,15 +269,19 @@ __global__ void __launch_bounds__(NPROJ * 256 + 32, NPROJ == 1 ? 3 : 2) fp4_gemv
         if (lane == 0) {
             uint32_t s = 0, ph = 0;     // ring slot and phase
             const uint32_t np_mask = NP - 1, np_shift = NP == 4 ? 2u : (NP == 2 ? 1u : 0u);
-            bool ok = true;
+            bool ok = true, first = true;
+            // down: the weights of the first ring slots go out before gate/up is complete, the slots' rows after the wait
+            bool dep_done = NPROJ == 2;
             while (ok) {
-                const uint32_t unit = atomicAdd(&P.t.header[P.counter_idx], 1u);
+                // the first unit is the CTA's own number (no round trip before the first copy), the others come from the counter
+                const uint32_t unit = first ? blockIdx.x : gridDim.x + atomicAdd(&P.t.header[P.counter_idx], 1u);
+                first = false;
                 const bool last = unit >= n_items * NP;
                 const uint32_t item = unit >> np_shift, share = unit & np_mask;
                 uint32_t g = 0, nb = 0, chunk0 = 0, mc = 0, expert = 0;
                 if (!last) {
                     g = item / P.n_blocks; nb = item % P.n_blocks;
-                    chunk0 = P.t.group_chunk0[g]; mc = P.t.group_mc[g]; expert = P.t.chunk_expert[chunk0];
+                    chunk0 = P.t.group_chunk0[g]; mc = P.t.group_mc[g]; expert = mc >> 16; mc &= 0xFFFFu;
                 }
                 const uint8_t* wsrc = P.w + (size_t)expert * P.expert_stride + (size_t)nb * P.n_stages_k * P.w_bytes;
                 const uint32_t ks_begin = share * share_stages, ks_end = last ? ks_begin + 1 : ks_begin + share_stages;
@@ -293,12 +303,23 @@ __global__ void __launch_bounds__(NPROJ * 256 + 32, NPROJ == 1 ? 3 : 2) fp4_gemv
                     uint8_t* dst = ring + (size_t)s * P.stage_bytes;
                     mbar_expect_tx(&full_bar[s], sub * P.w_bytes + mc * xa_sub_bytes);
                     bulk_g2s(dst, wsrc + (size_t)ks * P.w_bytes, sub * P.w_bytes, &full_bar[s]);
-                    for (uint32_t m = 0; m < mc; ++m)
-                        bulk_g2s(dst + sub * P.w_bytes + m * xa_sub_bytes,
-                                 P.xa + (size_t)(chunk0 + m) * xa_chunk_words + (size_t)ks * 4 * F4_XA_SB_WORDS,
-                                 xa_sub_bytes, &full_bar[s]);
+                    // the rows of this stage, or of the stages whose weights went ahead (slots 0, 1, ... of the first unit)
+                    uint32_t r_ks = ks, r_s = s;
+                    if (!dep_done) {
+                        if (s + 1 < NS && ks + sub < ks_end) continue;
+                        grid_dep_wait();
+                        grid_dep_launch();
+                        dep_done = true; r_ks = ks_begin; r_s = 0;
+                    }
+                    for (; r_ks <= ks; r_ks += sub, ++r_s) {
+                        uint8_t* rows = ring + (size_t)r_s * P.stage_bytes + sub * P.w_bytes;
+                        for (uint32_t m = 0; m < mc; ++m)
+                            bulk_g2s(rows + m * xa_sub_bytes, P.xa + (size_t)(chunk0 + m) * xa_chunk_words + (size_t)r_ks * 4 * F4_XA_SB_WORDS,
+                                     xa_sub_bytes, &full_bar[r_s]);
+                    }
                 }
             }
+            if (!dep_done) grid_dep_wait();   // no work: this grid is still not complete before the one before it
             if (s_abort) for (int i = 0; i < 2000; ++i) __nanosleep(1000);
         }
         return;
@@ -499,7 +520,8 @@ cudaError_t launch_fp4_gemv(const Fp4GemvArgs& a, int down, cudaStream_t st) {
     do {                                                                                                      \
         e = cudaFuncSetAttribute(fp4_gemv_kernel<NP, NVV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
         if (e != cudaSuccess) return e;                                                                       \
-        fp4_gemv_kernel<NP, NVV><<<ctas, NP * 256 + 32, smem, st>>>(P);                                       \
+        e = launch_dependent(!down || a.dependent, fp4_gemv_kernel<NP, NVV>, ctas, NP * 256 + 32, smem, st, P); \
+        if (e != cudaSuccess) return e;                                                                       \
     } while (0)
     if (!down && a.nv) MLXS_F4_LAUNCH(2, true);
     else if (!down) MLXS_F4_LAUNCH(2, false);

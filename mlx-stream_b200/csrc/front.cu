@@ -1,15 +1,19 @@
 // The front of a decode-sized layer call in one launch: [router logits from x] -> router tail -> dispatch -> row
 // staging.  Four dependent kernels of a few microseconds each cost a decode step more in launch gaps than in work
-// (at one token: 37 us of a 175 us call); here they are phases of one cooperative kernel separated by grid barriers,
-// and the [T, E] logits, the ids and the tables never leave the L2 between them.
+// (at one token: 37 us of a 175 us call); here they are phases of one kernel.
 //   phase 0 (only when the layer starts from x): logits = f32(x) . f32(W_g)^T, four warps per expert row, 8 token rows
-//            staged in shared memory at a time (src/arch/deepseek_v41/graph.zig:2033; mimo_glue_router_rows.metal);
-//   phase 1: CTA t routes token t (the router kernel's code: scoring, bias, top-k, weights);
-//   phase 2: CTA 0 sorts the assignment rows by expert and builds the work tables (the dispatch kernel's code);
+//            staged in shared memory at a time (src/arch/deepseek_v41/graph.zig:2033; mimo_glue_router_rows.metal), then a
+//            grid barrier;
+//   phase 1: every CTA routes all tokens: scores by all threads, the selection by a warp per token (router_body.cuh);
+//   phase 2: every CTA sorts the assignment rows by expert and builds the work tables in its shared memory (the dispatch
+//            kernel's code); CTA 0 writes them out;
 //   phase 3: all warps stage the rows for the streaming lane (the prep kernels' code).
+// Phases 1 and 2 are a few microseconds whoever does them; done by every CTA for itself they cost no grid barrier (two of
+// them, with the round trips of ids and tables through L2, were half of the 17 us this kernel took at one token), and without
+// phase 0 the launch is an ordinary one.  More than 256 experts or top_k > 32: a CTA per token routes, then a barrier.
 // The grid barrier is a counter and a generation word in global memory: the last CTA to arrive resets the counter and
-// bumps the generation, the others poll the generation with a bound.  The launch is cooperative, so all CTAs are
-// resident together; a barrier that runs out still records the status word and lets the kernel finish.
+// bumps the generation, the others poll the generation with a bound.  A launch with a barrier is cooperative, so all CTAs
+// are resident together; a barrier that runs out still records the status word and lets the kernel finish.
 #include "common.cuh"
 #include "kernels.h"
 #include "dispatch_body.cuh"
@@ -48,6 +52,7 @@ struct FrontParams {
     uint32_t* bar;
     uint32_t poll_limit;
     int rthreads;
+    int by_warp;                     // phases 1 and 2 in every CTA
 };
 
 __device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p) {
@@ -86,6 +91,8 @@ __device__ __forceinline__ bool front_grid_sync(uint32_t* bar, uint32_t& gen, ui
 __global__ void __launch_bounds__(1024, 1) front_kernel(const FrontParams P) {
     extern __shared__ __align__(16) uint8_t fsm[];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, nwarp = blockDim.x >> 5;
+    grid_dep_wait();
+    grid_dep_launch();
     // the barrier's generation before this CTA's first arrival (it cannot advance until every CTA, this one too, arrives)
     __shared__ uint32_t s_gen;
     if (threadIdx.x == 0) s_gen = ld_acquire_gpu(&P.bar[1]);
@@ -99,36 +106,92 @@ __global__ void __launch_bounds__(1024, 1) front_kernel(const FrontParams P) {
         front_grid_sync(P.bar, gen, P.poll_limit, P.status);
     }
 
-    // ---- phase 1: the router's tail, a CTA per token ----
-    for (uint32_t t = blockIdx.x; t < T; t += gridDim.x)
-        route_row(P.logits, P.bias, P.E, P.K, P.scoring, P.norm, P.scale, P.ids, P.weights, (int)t, reinterpret_cast<float*>(fsm), P.rthreads);
-    front_grid_sync(P.bar, gen, P.poll_limit, P.status);
+    // ---- phase 1: the router's tail ----
+    // shared memory: ids and weights [A], the tables [E + 1 + 6 A + 16], the dispatch scratch [E + 99], the scores [T][E + 2]
+    const uint32_t A = T * (uint32_t)P.K, E = (uint32_t)P.E;
+    int32_t* s_ids = reinterpret_cast<int32_t*>(fsm);
+    float* s_w = reinterpret_cast<float*>(s_ids + A);
+    DispatchTables S = P.t;
+    S.header = reinterpret_cast<uint32_t*>(s_w + A);
+    S.offsets = S.header + 16;
+    S.order = S.offsets + E + 1;
+    S.chunk_expert = S.order + A; S.chunk_row0 = S.chunk_expert + A; S.chunk_rows = S.chunk_row0 + A;
+    S.group_chunk0 = S.chunk_rows + A; S.group_mc = S.group_chunk0 + A;
+    S.max_chunks = A < P.t.max_chunks ? A : P.t.max_chunks;
+    uint32_t* scratch = S.group_mc + A;
+    const int32_t* ids = s_ids;
+    if (P.by_warp) {
+        // one expert per thread: the scoring functions are long, and this kernel's code comes cold from memory
+        float* s_sc = reinterpret_cast<float*>(scratch + E + 99);     // [T][E], then per token {max, NaN flag}
+        float* s_max = s_sc + (size_t)T * E;
+        if (P.scoring == 2) {
+            for (uint32_t t = warp; t < T; t += nwarp) {
+                float xv[NE], m;
+                bool nan;
+#pragma unroll
+                for (int i = 0; i < NE; ++i) xv[i] = lane + 32 * i < E ? P.logits[(size_t)t * E + lane + 32 * i] : 0.0f;
+                route_max_warp(xv, P.E, m, nan);
+                if (lane == 0) { s_max[2 * t] = m; s_max[2 * t + 1] = nan ? 1.0f : 0.0f; }
+            }
+            __syncthreads();
+        }
+#pragma unroll 1
+        for (uint32_t i = threadIdx.x; i < T * E; i += blockDim.x) {
+            const float x = P.logits[i];
+            if (P.scoring == 2) {
+                const float* mx = s_max + 2 * (i / E);
+                s_sc[i] = mx[1] != 0.0f ? __int_as_float(0x7FC00000) : det_expf(__fsub_rn(x, mx[0]));
+            } else {
+                s_sc[i] = route_score(x, P.scoring);
+            }
+        }
+        __syncthreads();
+        for (uint32_t t = warp; t < T; t += nwarp)
+            route_row_warp<true>(s_sc + t * E, P.bias, P.E, P.K, P.scoring, P.norm, P.scale, s_ids + t * P.K, s_w + t * P.K);
+        __syncthreads();
+    } else {
+        for (uint32_t t = blockIdx.x; t < T; t += gridDim.x)
+            route_row(P.logits, P.bias, P.E, P.K, P.scoring, P.norm, P.scale, P.ids, P.weights, (int)t, reinterpret_cast<float*>(fsm), P.rthreads);
+        front_grid_sync(P.bar, gen, P.poll_limit, P.status);
+        ids = P.ids;
+    }
 
-    // ---- phase 2: dispatch by CTA 0 ----
-    if (blockIdx.x == 0)
-        dispatch_body(P.ids, T * (uint32_t)P.K, (uint32_t)P.E, P.loaded, P.t, P.chunk_rows, P.group_chunks, P.heavy, P.status,
-                      reinterpret_cast<uint32_t*>(fsm));
-    front_grid_sync(P.bar, gen, P.poll_limit, P.status);
+    // ---- phase 2: dispatch, by every CTA for itself ----
+    dispatch_body(ids, A, E, P.loaded, S, P.chunk_rows, P.group_chunks, P.heavy, P.status, scratch);
+    __syncthreads();
+    const uint32_t n_chunks = S.header[HDR_NCHUNKS];
+    if (blockIdx.x == 0) {
+        const uint32_t n_groups = S.header[HDR_NGROUPS];
+        if (threadIdx.x <= HDR_CTR_AUX) P.t.header[threadIdx.x] = S.header[threadIdx.x];
+        for (uint32_t i = threadIdx.x; i <= E; i += blockDim.x) P.t.offsets[i] = S.offsets[i];
+        for (uint32_t i = threadIdx.x; i < A; i += blockDim.x) {
+            P.t.order[i] = S.order[i];
+            if (P.by_warp) { P.ids[i] = s_ids[i]; P.weights[i] = s_w[i]; }
+        }
+        for (uint32_t i = threadIdx.x; i < n_chunks; i += blockDim.x) {
+            P.t.chunk_expert[i] = S.chunk_expert[i]; P.t.chunk_row0[i] = S.chunk_row0[i]; P.t.chunk_rows[i] = S.chunk_rows[i];
+        }
+        for (uint32_t i = threadIdx.x; i < n_groups; i += blockDim.x) { P.t.group_chunk0[i] = S.group_chunk0[i]; P.t.group_mc[i] = S.group_mc[i]; }
+    }
 
     // ---- phase 3: row staging, a warp per (chunk, row, 128-block) or per (chunk, row) ----
-    const uint32_t n_chunks = P.t.header[HDR_NCHUNKS];
     const uint32_t gw = blockIdx.x * nwarp + warp, gstride = gridDim.x * nwarp;
     if (P.bank_exl3) {
         const uint32_t nb = P.H / 128, per_chunk = P.chunk_rows * nb;
         for (uint32_t task = gw; task < n_chunks * per_chunk; task += gstride) {
             const uint32_t chunk = task / per_chunk, rem = task % per_chunk, row = rem / nb, b = rem % nb;
-            const uint32_t e = P.t.chunk_expert[chunk], rows = P.t.chunk_rows[chunk];
+            const uint32_t e = S.chunk_expert[chunk], rows = S.chunk_rows[chunk];
             const bool valid = row < rows;
-            const uint32_t assign = valid ? P.t.order[P.t.chunk_row0[chunk] + row] : 0u;
-            exl3_prep_row_block<false>(P.x, x_row_of(P.t, assign, (uint32_t)P.K), valid, e, P.H, P.scales, P.scales_stride, chunk, row, b,
+            const uint32_t assign = valid ? S.order[S.chunk_row0[chunk] + row] : 0u;
+            exl3_prep_row_block<false>(P.x, x_row_of(S, assign, (uint32_t)P.K), valid, e, P.H, P.scales, P.scales_stride, chunk, row, b,
                                        lane, P.xa);
         }
     } else {
         // a row's 8-input groups are split over 4 warps
         for (uint32_t task = gw; task < n_chunks * P.chunk_rows * 4u; task += gstride) {
             const uint32_t chunk = task / (P.chunk_rows * 4u), rem = task % (P.chunk_rows * 4u), row = rem / 4u, part = rem % 4u;
-            const bool valid = row < P.t.chunk_rows[chunk];
-            const uint32_t tok = valid ? x_row_of(P.t, P.t.order[P.t.chunk_row0[chunk] + row], (uint32_t)P.K) : 0u;
+            const bool valid = row < S.chunk_rows[chunk];
+            const uint32_t tok = valid ? x_row_of(S, S.order[S.chunk_row0[chunk] + row], (uint32_t)P.K) : 0u;
             fp4_prep_row(P.x, tok, valid, P.H, chunk, row, part * 32u + lane, 128u, P.xa);
         }
     }
@@ -137,7 +200,7 @@ __global__ void __launch_bounds__(1024, 1) front_kernel(const FrontParams P) {
 // smem: the larger of the phases' needs
 static size_t front_smem_bytes(const FrontArgs& a, int rthreads) {
     size_t s = router_smem_floats(a.E, a.K, rthreads) * sizeof(float);
-    const size_t d = ((size_t)a.E + 99) * sizeof(uint32_t);
+    const size_t d = ((size_t)8 * a.T * a.K + 2 * (size_t)a.E + 116 + (size_t)a.T * (a.E + 2)) * sizeof(uint32_t);
     if (d > s) s = d;
     if (a.w_router) { const size_t l = logits_smem_bytes(a.H, 32); if (l > s) s = l; }
     return s;
@@ -156,10 +219,18 @@ cudaError_t launch_front(const FrontArgs& a, cudaStream_t st) {
     const size_t smem = front_smem_bytes(a, rt);
     cudaError_t e = cudaFuncSetAttribute(front_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
+    P.by_warp = route_by_warp(a.E, a.K) ? 1 : 0;
+    const bool barrier = a.w_router || !P.by_warp;
+    // a warp per staging task (a row's 128-block, or a quarter of a row for the FP4 banks), at most a CTA per SM; with a
+    // barrier 32 to 64 CTAs: one round of expert rows, and room beside the shared expert's kernels
+    const unsigned sms = (unsigned)(a.sm_count > 0 ? a.sm_count : 32);
+    unsigned grid = ((unsigned)(a.T * a.K) * a.chunk_rows * (a.bank_exl3 ? a.H / 128 : 4u) + 31u) / 32u;
+    if (barrier) grid = grid < 32u ? 32u : grid > 64u ? 64u : grid;
+    if (grid > sms) grid = sms;
+    if (!barrier) {
+        return launch_dependent(true, front_kernel, grid, 1024, smem, st, P);
+    }
     void* args[] = {&P};
-    // enough CTAs for the staging of the call's rows (a CTA per SM above 16 tokens); every CTA of a cooperative launch
-    // is resident at once
-    const unsigned grid = a.T > 16 ? (unsigned)(a.sm_count > 0 ? a.sm_count : 32) : (a.T > 4 ? 32u : (a.T > 1 ? 16u : 8u));
     return cudaLaunchCooperativeKernel(reinterpret_cast<void*>(front_kernel), dim3(grid), dim3(1024), args, smem, st);
 }
 

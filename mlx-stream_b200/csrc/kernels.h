@@ -20,7 +20,7 @@ struct DispatchTables {
     uint32_t* chunk_row0;    // [max_chunks] first sorted row
     uint32_t* chunk_rows;    // [max_chunks] valid rows (1..8)
     uint32_t* group_chunk0;  // [max_chunks]
-    uint32_t* group_mc;      // [max_chunks]
+    uint32_t* group_mc;      // [max_chunks] chunks of the work item | its expert << 16
     uint32_t max_chunks;
     const uint32_t* xrow;    // optional [A]: row of x an assignment reads (null: assignment / top_k)
 };
@@ -118,6 +118,7 @@ struct Exl3GemvArgs {
     uint32_t* ks_count;     // [ksplit_count_words(sm_count)] zeroed once
     uint32_t poll_limit;    // polls after which a wait gives up (0: the default, 2^20)
     uint32_t withhold;      // self-test: the gate/up producers leave out their n-th ring stage (0: off)
+    bool dependent;         // down: may start under gate/up (not beside the tensor-core lane: its waiting CTAs would hold the lane's SMs)
 };
 // The fold's workspace: 12 slots per SM of the largest staging array (2 projections x 16 rows x 132 floats), and as many
 // arrival counters.  A kernel whose staging array is zs_bytes and whose sums have up to 4 parts can split this many items:
@@ -213,6 +214,7 @@ struct Fp4GemvArgs {
     int sm_count;
     float* ks_scratch;      // optional K-split workspace, exl3_ksplit_scratch_bytes(sm_count) bytes
     uint32_t* ks_count;     // [ksplit_count_words(sm_count)] zeroed once
+    bool dependent;         // as in Exl3GemvArgs
 };
 cudaError_t launch_fp4_gemv(const Fp4GemvArgs& a, int down, cudaStream_t st);
 // experts with many rows: tcgen05 MMA over codes decoded to 16-bit operands in tensor memory (fp4_prefill.cu)

@@ -1,5 +1,6 @@
 // Router tail: fp32 logits -> top-k expert ids (rank order) + normalised weights.
-// One CTA per token row, one thread per expert (n_experts <= 1024), top_k <= 64.
+// A warp per token row up to 256 experts and top_k 32; a CTA per token row, one thread per expert, above (n_experts <= 1024,
+// top_k <= 64).
 // Semantics: src/kernels/exl3/q3rc_router_tail.metal:12-40 (sqrt(softplus)), src/arch/mimo_v2/kernels/mimo_glue_top8.metal
 // and src/arch/glm5_next/kernels/glm5n_glue_top8.metal (sigmoid): key = score + bias, rank = number of experts that
 // precede (key descending, ties to the lower index, NaN last), ids[rank] = expert, weights from the unbiased score,
@@ -16,6 +17,14 @@ __global__ void router_kernel(const float* __restrict__ logits, const float* __r
                               float* __restrict__ weights) {
     extern __shared__ float sm[];
     route_row(logits, bias, E, K, scoring, norm, scale, ids, weights, (int)blockIdx.x, sm, (int)blockDim.x);
+}
+
+// a warp per token: 8 tokens per CTA and no barrier (16,384 tokens of 256 experts: 104 -> 37 us against a CTA per token)
+__global__ void __launch_bounds__(256) router_warp_kernel(const float* __restrict__ logits, const float* __restrict__ bias, int T,
+                                                          int E, int K, int scoring, int norm, float scale,
+                                                          int32_t* __restrict__ ids, float* __restrict__ weights) {
+    const int t = (int)(blockIdx.x * 8 + (threadIdx.x >> 5));
+    if (t < T) route_row_warp<false>(logits + (size_t)t * E, bias, E, K, scoring, norm, scale, ids + (size_t)t * K, weights + (size_t)t * K);
 }
 
 // Router logits for decode-sized batches: the shared device code of logits_body.cuh, two expert rows per CTA of 8 warps
@@ -42,9 +51,11 @@ cudaError_t launch_router_logits(const __nv_bfloat16* x, const __nv_bfloat16* w,
 cudaError_t launch_router(const float* logits, const float* bias, int T, int E, int K, int scoring, int norm,
                           float scale, int32_t* ids, float* weights, cudaStream_t st) {
     if (T == 0) return cudaSuccess;
+    if (route_by_warp(E, K)) {
+        router_warp_kernel<<<(T + 7) / 8, 256, 0, st>>>(logits, bias, T, E, K, scoring, norm, scale, ids, weights);
+        return cudaGetLastError();
+    }
     int threads = ((E > K ? E : K) + 31) / 32 * 32;
-    const int nwarps = threads / 32;
-    (void)nwarps;
     size_t smem = router_smem_floats(E, K, threads) * sizeof(float);
     router_kernel<<<T, threads, smem, st>>>(logits, bias, E, K, scoring, norm, scale, ids, weights);
     return cudaGetLastError();

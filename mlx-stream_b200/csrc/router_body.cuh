@@ -18,6 +18,99 @@ __device__ __forceinline__ float rt_softplus(float g) {
     return __fadd_rn(maxval, rt_log1p(det_expf(__fsub_rn(minval, maxval))));
 }
 
+// One token row by one warp, for up to 256 experts and top_k <= 32: lane l holds experts l, l + 32, ...  The same scores, the
+// same selection order (key descending, ties to the lower index, NaN last) and the same sums in the same order as
+// route_row, so the bits agree; no barrier, so a CTA routes as many tokens at once as it has warps.
+__host__ __device__ inline bool route_by_warp(int E, int K) { return E <= 256 && K <= 32; }
+constexpr int NE = 8;   // experts per lane
+__device__ __forceinline__ float route_score(float x, int scoring) {
+    if (scoring == 1) {
+        const float y = __fdiv_rn(1.0f, __fadd_rn(1.0f, det_expf(fabsf(x))));
+        return x < 0.0f ? y : __fsub_rn(1.0f, y);
+    }
+    return __fsqrt_rn(rt_softplus(x));
+}
+// softmax: the largest logit of a row and whether it holds a NaN
+__device__ __forceinline__ void route_max_warp(const float (&x)[NE], int E, float& m, bool& has_nan) {
+    const int lane = threadIdx.x & 31;
+    m = -__int_as_float(0x7F800000);
+    has_nan = false;
+#pragma unroll
+    for (int i = 0; i < NE; ++i)
+        if (lane + 32 * i < E) {
+            if (x[i] != x[i]) has_nan = true; else if (x[i] > m) m = x[i];
+        }
+    for (int o = 16; o >= 1; o >>= 1) {
+        const float om = __shfl_xor_sync(0xFFFFFFFFu, m, o);
+        m = om > m ? om : m;
+    }
+    has_nan = __any_sync(0xFFFFFFFFu, has_nan);
+}
+// SCORED: the row holds scores already (softmax: exp(x - max))
+template <bool SCORED>
+__device__ __forceinline__ void route_row_warp(const float* __restrict__ row, const float* __restrict__ bias, int E, int K,
+                                               int scoring, int norm, float scale, int32_t* ids, float* weights) {
+    const int lane = threadIdx.x & 31;
+    float score[NE];
+#pragma unroll
+    for (int i = 0; i < NE; ++i) score[i] = lane + 32 * i < E ? row[lane + 32 * i] : 0.0f;
+    if (scoring == 2) {
+        float m = 0.0f, p = 0.0f;
+        bool has_nan = false;
+        if (!SCORED) route_max_warp(score, E, m, has_nan);
+#pragma unroll
+        for (int i = 0; i < NE; ++i) {
+            if (32 * i >= E) break;
+            if (!SCORED) score[i] = has_nan ? __int_as_float(0x7FC00000) : det_expf(__fsub_rn(score[i], m));
+            if (lane + 32 * i < E) p = __fadd_rn(p, score[i]);
+        }
+        for (int o = 16; o >= 1; o >>= 1) p = __fadd_rn(p, __shfl_xor_sync(0xFFFFFFFFu, p, o));
+#pragma unroll
+        for (int i = 0; i < NE; ++i) {
+            if (32 * i >= E) break;
+            score[i] = __fdiv_rn(score[i], p);
+        }
+    } else if (!SCORED) {
+#pragma unroll
+        for (int i = 0; i < NE; ++i) {
+            if (32 * i >= E) break;
+            score[i] = route_score(score[i], scoring);
+        }
+    }
+    uint32_t key[NE], alive = 0;
+#pragma unroll
+    for (int i = 0; i < NE; ++i) {
+        key[i] = 0;
+        const int e = lane + 32 * i;
+        if (e >= E) continue;
+        alive |= 1u << i;
+        const float biased = bias ? __fadd_rn(score[i], bias[e]) : score[i];
+        if (biased == biased) {
+            const uint32_t b = __float_as_uint(__fadd_rn(biased, 0.0f));
+            key[i] = (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+        }
+    }
+    float total = 0.0f, mine = 0.0f;
+    for (int r = 0; r < K; ++r) {
+        // this lane's best live expert (a lower i is a lower index), then the warp's
+        uint32_t bk = 0, bi = 0xFFFFFFFFu;
+        float bs = 0.0f;
+#pragma unroll
+        for (int i = 0; i < NE; ++i)
+            if ((alive >> i & 1u) && (bi == 0xFFFFFFFFu || key[i] > bk)) { bk = key[i]; bi = (uint32_t)(lane + 32 * i); bs = score[i]; }
+        const uint32_t best = __reduce_max_sync(0xFFFFFFFFu, bk);
+        const uint32_t who = __reduce_min_sync(0xFFFFFFFFu, bk == best ? bi : 0xFFFFFFFFu);
+        const float sc = __shfl_sync(0xFFFFFFFFu, bs, (int)(who & 31u));
+        if (bi == who) alive &= ~(1u << (who >> 5));
+        total = __fadd_rn(sc, total);
+        if (lane == r) { mine = sc; ids[r] = (int32_t)who; }
+    }
+    if (lane < K) {
+        const float q = norm ? __fdiv_rn(mine, __fadd_rn(total, 1e-20f)) : mine;
+        weights[lane] = __fmul_rn(q, scale);
+    }
+}
+
 // One token row by the whole CTA: thread e < E scores expert e; `rthreads` = the E (and K) rounded up to whole warps,
 // the threads beyond it only keep the barriers company.  sm: router_smem_floats(E, K, rthreads) floats.
 __host__ __device__ inline size_t router_smem_floats(int E, int K, int rthreads) {

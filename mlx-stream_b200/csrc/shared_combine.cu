@@ -15,29 +15,31 @@ namespace mlxs {
 // warps of a CTA (they split the reduction dimension).  The down kernel has 320 row tiles for 148 SMs: with 4 warps
 // and about 100 registers every CTA is resident at once (2-3 per SM) instead of running in two waves.
 constexpr int sh_warps(int mode) { return mode == 0 ? 8 : 4; }
-constexpr int SH_TOK = 64;  // tokens per pass
 constexpr int SH_AHEAD = 2;  // weight chunks in flight per warp
 
-template <int MODE>  // 0: gate/up + activation -> h bf16 [T, N]; 1: down -> out f32 [T, N]
+// MODE 0: gate/up + activation -> h bf16 [T, N]; 1: down -> out f32 [T, N].  NT = token tiles of 8 per pass: a call of few
+// tokens takes the form that holds registers and reduction space for its own tiles only, so that its CTAs fit beside the
+// routed kernels' (gate/up at one token 35 -> 27 us).
+template <int MODE, int NT>
 __global__ void __launch_bounds__(sh_warps(MODE) * 32) shared_kernel(const __nv_bfloat16* __restrict__ x, uint32_t T,
                                                                uint32_t Kdim, uint32_t N,
                                                                const __nv_bfloat16* __restrict__ wa,
                                                                const __nv_bfloat16* __restrict__ wb, float limit,
                                                                __nv_bfloat16* __restrict__ h_out,
                                                                float* __restrict__ f_out) {
-    extern __shared__ float red[];  // [SH_WARPS][NW][8 tiles][32 lanes][4]
+    extern __shared__ float red[];  // [SH_WARPS][NW][NT tiles][32 lanes][4]
     constexpr int SH_WARPS = sh_warps(MODE);
     constexpr int NW = MODE == 0 ? 2 : 1;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, g = lane >> 2, c = lane & 3u;
     const uint32_t row0 = blockIdx.x * 16;
-    for (uint32_t t0 = 0; t0 < T; t0 += SH_TOK) {
-        const uint32_t nt_n = min((uint32_t)SH_TOK, T - t0);
+    for (uint32_t t0 = 0; t0 < T; t0 += NT * 8) {
+        const uint32_t nt_n = min((uint32_t)(NT * 8), T - t0);
         const uint32_t ntiles = (nt_n + 7) / 8;
-        float acc[NW][8][4];
+        float acc[NW][NT][4];
 #pragma unroll
         for (int w = 0; w < NW; ++w)
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
+            for (int i = 0; i < NT; ++i)
 #pragma unroll
                 for (int q = 0; q < 4; ++q) acc[w][i][q] = 0.f;
         // A warp walks its share of the reduction dimension 32 inputs at a time.  The weights come straight from HBM and
@@ -59,11 +61,11 @@ __global__ void __launch_bounds__(sh_warps(MODE) * 32) shared_kernel(const __nv_
         // the rows of a chunk's token tiles come from L2: they too are loaded one chunk ahead, all eight at once
         // (predicated, no branch between them)
         static_assert(SH_AHEAD == 2, "the row buffers alternate with the chunk's place in the weight ring");
-        uint4 xr[2][8];
-        auto load_rows = [&](uint4 (&dst)[8], uint32_t kc) {
+        uint4 xr[2][NT];
+        auto load_rows = [&](uint4 (&dst)[NT], uint32_t kc) {
             const size_t ko = (size_t)kc * 32 + c * 8;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
+            for (int i = 0; i < NT; ++i) {
                 const uint32_t tok = t0 + i * 8 + g;
                 dst[i] = make_uint4(0, 0, 0, 0);
                 if (kc < nchunk && i < (int)ntiles && tok < T) dst[i] = *reinterpret_cast<const uint4*>(x + (size_t)tok * Kdim + ko);
@@ -83,7 +85,7 @@ __global__ void __launch_bounds__(sh_warps(MODE) * 32) shared_kernel(const __nv_
                     load_chunk(ring[r], kc + SH_AHEAD * SH_WARPS);
                     load_rows(xr[r ^ 1], kc + SH_WARPS);
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
+                    for (int i = 0; i < NT; ++i) {
                         if (i < (int)ntiles) {
 #pragma unroll
                             for (int w = 0; w < NW; ++w) {
@@ -101,9 +103,9 @@ __global__ void __launch_bounds__(sh_warps(MODE) * 32) shared_kernel(const __nv_
 #pragma unroll
         for (int w = 0; w < NW; ++w)
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
+            for (int i = 0; i < NT; ++i)
                 if (i < (int)ntiles)
-                    *reinterpret_cast<float4*>(red + ((((size_t)warp * NW + w) * 8 + i) * 32 + lane) * 4) =
+                    *reinterpret_cast<float4*>(red + ((((size_t)warp * NW + w) * NT + i) * 32 + lane) * 4) =
                         make_float4(acc[w][i][0], acc[w][i][1], acc[w][i][2], acc[w][i][3]);
         __syncthreads();
         for (uint32_t idx = threadIdx.x; idx < ntiles * 128; idx += SH_WARPS * 32) {
@@ -112,7 +114,7 @@ __global__ void __launch_bounds__(sh_warps(MODE) * 32) shared_kernel(const __nv_
 #pragma unroll
             for (int w = 0; w < NW; ++w) {
                 float v = 0.f;
-                for (int ww = 0; ww < SH_WARPS; ++ww) v += red[((((size_t)ww * NW + w) * 8 + i) * 32 + ln) * 4 + q];
+                for (int ww = 0; ww < SH_WARPS; ++ww) v += red[((((size_t)ww * NW + w) * NT + i) * 32 + ln) * 4 + q];
                 s[w] = v;
             }
             const uint32_t row = row0 + (ln >> 2) + ((q & 2) ? 8 : 0);
@@ -136,18 +138,29 @@ __global__ void __launch_bounds__(sh_warps(MODE) * 32) shared_kernel(const __nv_
     }
 }
 
+template <int NT>
+static cudaError_t shared_launch(const __nv_bfloat16* x, const __nv_bfloat16* w1, const __nv_bfloat16* w3, const __nv_bfloat16* w2, uint32_t T,
+                                 uint32_t H, uint32_t I, float limit, __nv_bfloat16* h_ws, float* out, cudaStream_t st) {
+    const size_t smem0 = (size_t)sh_warps(0) * 2 * NT * 32 * 4 * sizeof(float), smem1 = (size_t)sh_warps(1) * NT * 32 * 4 * sizeof(float);
+    cudaError_t e = cudaFuncSetAttribute(shared_kernel<0, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem0);
+    if (e != cudaSuccess) return e;
+    // The routed kernels beside it take all of an SM's shared memory: an SM that had to change its split would drain first.
+    // (Not from 17 tokens on: the rows of eight token tiles then miss the L1, 27 -> 41 us at 64 tokens.)
+    if (NT < 8 && (e = cudaFuncSetAttribute(shared_kernel<0, NT>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared)) != cudaSuccess) return e;
+    if (NT < 8 && (e = cudaFuncSetAttribute(shared_kernel<1, NT>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared)) != cudaSuccess) return e;
+    shared_kernel<0, NT><<<I / 16, sh_warps(0) * 32, smem0, st>>>(x, T, H, I, w1, w3, limit, h_ws, nullptr);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    shared_kernel<1, NT><<<H / 16, sh_warps(1) * 32, smem1, st>>>(h_ws, T, I, H, w2, nullptr, 0.f, nullptr, out);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_shared_expert(const __nv_bfloat16* x, const __nv_bfloat16* w1, const __nv_bfloat16* w3,
                                  const __nv_bfloat16* w2, uint32_t T, uint32_t H, uint32_t I, float limit,
                                  __nv_bfloat16* h_ws, float* out, cudaStream_t st) {
     if (T == 0) return cudaSuccess;
-    const size_t smem0 = (size_t)sh_warps(0) * 2 * 8 * 32 * 4 * sizeof(float), smem1 = (size_t)sh_warps(1) * 8 * 32 * 4 * sizeof(float);
-    cudaError_t e = cudaFuncSetAttribute(shared_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem0);
-    if (e != cudaSuccess) return e;
-    shared_kernel<0><<<I / 16, sh_warps(0) * 32, smem0, st>>>(x, T, H, I, w1, w3, limit, h_ws, nullptr);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    shared_kernel<1><<<H / 16, sh_warps(1) * 32, smem1, st>>>(h_ws, T, I, H, w2, nullptr, 0.f, nullptr, out);
-    return cudaGetLastError();
+    if (T <= 8) return shared_launch<1>(x, w1, w3, w2, T, H, I, limit, h_ws, out, st);
+    if (T <= 16) return shared_launch<2>(x, w1, w3, w2, T, H, I, limit, h_ws, out, st);
+    return shared_launch<8>(x, w1, w3, w2, T, H, I, limit, h_ws, out, st);
 }
 
 // thread = 4 columns of one token
@@ -155,6 +168,7 @@ __global__ void combine_kernel(const void* __restrict__ ro, int ro_bf16, const f
                                const float* __restrict__ shared, uint32_t T, uint32_t K, uint32_t H, int chain,
                                __nv_bfloat16* __restrict__ y) {
     const uint32_t col = (blockIdx.x * blockDim.x + threadIdx.x) * 4, t = blockIdx.y;
+    grid_dep_wait();
     if (col >= H) return;
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
     for (uint32_t k = 0; k < K; ++k) {
@@ -196,8 +210,7 @@ cudaError_t launch_combine(const void* ro, int ro_bf16, const float* weights, co
                            uint32_t K, uint32_t H, int chain, __nv_bfloat16* y, cudaStream_t st) {
     if (T == 0) return cudaSuccess;
     dim3 grid((H / 4 + 255) / 256, T);
-    combine_kernel<<<grid, 256, 0, st>>>(ro, ro_bf16, weights, shared, T, K, H, chain, y);
-    return cudaGetLastError();
+    return launch_dependent(true, combine_kernel, grid, 256, 0, st, ro, ro_bf16, weights, shared, T, K, H, chain, y);
 }
 
 }  // namespace mlxs
