@@ -398,10 +398,6 @@ static int dense_workspace(mlxs_moe* h) {
     int rc;
     const size_t T16 = ((size_t)h->cfg.max_tokens + 15) / 16 * 16;
     if (!h->dg_xb && (rc = h->alloc(&h->dg_xb, T16 * h->cfg.hidden * 2))) return rc;
-    if (!h->dg_scratch) {
-        if ((rc = h->alloc(&h->dg_scratch, dense_gemm_scratch_bytes(h->sm_count))) || (rc = h->alloc(&h->dg_count, (size_t)h->sm_count * 4))) return rc;
-        CU(cudaMemset(h->dg_count, 0, (size_t)h->sm_count * 4));
-    }
     return 0;
 }
 
@@ -576,7 +572,9 @@ extern "C" int mlxs_moe_set_router_weight(mlxs_moe* h, uint32_t layer, const voi
     return MLXS_OK;
 }
 
-extern "C" int mlxs_moe_logits(mlxs_moe* h, uint32_t layer, const void* x_dev, uint32_t T, float* logits_dev, void* stream) {
+// staged_nt: rows per tile of the staged rows the dense product leaves behind (0: none)
+static int logits_impl(mlxs_moe* h, uint32_t layer, const void* x_dev, uint32_t T, float* logits_dev, void* stream, uint32_t* staged_nt) {
+    *staged_nt = 0;
     int rc = check_call(h, layer, T, "logits");
     if (rc) return rc;
     if (T == 0) return MLXS_OK;
@@ -587,12 +585,19 @@ extern "C" int mlxs_moe_logits(mlxs_moe* h, uint32_t layer, const void* x_dev, u
     cudaStream_t st = (cudaStream_t)stream;
     StageTimer tm(h, MLXS_STAGE_ROUTER, st);
     if (T > 64 && L.router_w_t) {
-        CU(launch_dense_logits(static_cast<const __nv_bfloat16*>(x_dev), L.router_w_t, T, c.n_experts, c.hidden, h->dg_xb, logits_dev,
-                               h->dg_scratch, h->dg_count, h->status, h->sm_count, st));
+        const uint32_t nt = dense_logits_rows(T, c.n_experts, c.hidden, h->sm_count);
+        *staged_nt = nt;
+        CU(launch_dense_logits(static_cast<const __nv_bfloat16*>(x_dev), L.router_w_t, T, c.n_experts, c.hidden, nt, h->dg_xb, logits_dev,
+                               h->status, h->sm_count, st));
     } else {
         CU(launch_router_logits(static_cast<const __nv_bfloat16*>(x_dev), L.router_w, T, c.n_experts, c.hidden, logits_dev, st));
     }
     return MLXS_OK;
+}
+
+extern "C" int mlxs_moe_logits(mlxs_moe* h, uint32_t layer, const void* x_dev, uint32_t T, float* logits_dev, void* stream) {
+    uint32_t staged = 0;
+    return logits_impl(h, layer, x_dev, T, logits_dev, stream, &staged);
 }
 
 extern "C" int mlxs_moe_forward_x(mlxs_moe* h, uint32_t layer, const void* x_dev, uint32_t T, void* y_dev, void* stream) {
@@ -604,9 +609,11 @@ extern "C" int mlxs_moe_forward_x(mlxs_moe* h, uint32_t layer, const void* x_dev
         const FrontCall fc{nullptr};
         return experts_impl(h, layer, x_dev, h->ids_ws, h->w_ws, T, y_dev, stream, &fc);
     }
-    int rc = mlxs_moe_logits(h, layer, x_dev, T, h->logits_ws, stream);
-    if (rc) return rc;
-    return mlxs_moe_forward(h, layer, x_dev, h->logits_ws, T, y_dev, stream);
+    // the logits product leaves the rows staged: the shared expert of this call reads them when its tiles are the same
+    int rc = logits_impl(h, layer, x_dev, T, h->logits_ws, stream, &h->dg_staged_nt);
+    if (!rc) rc = mlxs_moe_forward(h, layer, x_dev, h->logits_ws, T, y_dev, stream);
+    h->dg_staged_nt = 0;
+    return rc;
 }
 
 // dispatch + the bank's expert kernels -> ro (unweighted rows in assignment order)
@@ -764,13 +771,11 @@ static int experts_impl(mlxs_moe* h, uint32_t layer, const void* x_dev, const in
     // rows back (ep.cu); the chain combine needs every assignment's row in k order and keeps the per-assignment form
     static const bool per_assignment = getenv("MLXS_EP_PER_ASSIGNMENT") != nullptr;
     const bool ep_fused = c.ep_world > 1 && c.combine != MLXS_COMBINE_CHAIN && !per_assignment;
-    // The shared expert only reads x: it runs beside the routed kernels on the handle's second stream.  Decode-sized
-    // batches leave SMs idle in the routed kernels (T = 1: 144 work items for 296 CTA slots); larger ones still have
-    // the dispatch and the staging of the rows at their start, about as long as the shared expert itself.
-    // Prefill-sized calls keep it on the caller's stream after the routed kernels: its library GEMMs are full-GPU
-    // kernels, and running them among the tensor-core lane's persistent CTAs stretched that lane (C4 at 16384 tokens:
-    // 12.9 -> 14.6 ms).  MLXS_SHARED_ASIDE_MAX moves the limit (0: never aside).
-    static const uint32_t aside_max = getenv("MLXS_SHARED_ASIDE_MAX") ? (uint32_t)atoi(getenv("MLXS_SHARED_ASIDE_MAX")) : 64u;
+    // The shared expert only reads x: it runs on the handle's second stream beside the router's, dispatch's and staging's
+    // kernels, which leave the GPU nearly idle, and what is left of it beside the routed kernels.  Measured at every size up
+    // to 8192 tokens: 100 tokens 472 -> 447 us, 300 711 -> 677, 2048 2959 -> 2831, 4093 (NVFP4) 2968 -> 2840, 8192 1 %.
+    // MLXS_SHARED_ASIDE_MAX limits it (0: never aside).
+    static const uint32_t aside_max = getenv("MLXS_SHARED_ASIDE_MAX") ? (uint32_t)atoi(getenv("MLXS_SHARED_ASIDE_MAX")) : 65536u;
     const bool shared_aside = c.shared_expert && h->aux_stream && T <= aside_max;
     const float* shared = nullptr;
     auto run_shared = [&](cudaStream_t s) -> int {
@@ -779,7 +784,9 @@ static int experts_impl(mlxs_moe* h, uint32_t layer, const void* x_dev, const in
             DenseSharedArgs da{};
             da.x = static_cast<const __nv_bfloat16*>(x_dev); da.w_gu = L.sh_gu_t; da.w_d = L.sh_d_t;
             da.T = T; da.H = c.hidden; da.I = c.inter; da.limit = lim; da.xb = h->dg_xb; da.hb = h->dg_hb; da.out = h->sh_out;
-            da.part_scratch = h->dg_scratch; da.part_count = h->dg_count; da.status = h->status; da.sm_count = h->sm_count;
+            da.status = h->status; da.sm_count = h->sm_count;
+            da.nt = dense_shared_rows(T, c.hidden, c.inter, h->sm_count);
+            da.rows_staged = h->dg_staged_nt == da.nt;
             CU(launch_dense_shared_expert(da, s));
         } else {
             CU(launch_shared_expert(static_cast<const __nv_bfloat16*>(x_dev), L.sh_w1, L.sh_w3, L.sh_w2, T, c.hidden, c.inter,
@@ -931,7 +938,6 @@ extern "C" int mlxs_moe_status_clear(mlxs_moe* h) {
     CU(cudaMemset(h->status, 0, 16));
     // a call that gave up may have left arrivals of the K-split fold behind
     if (h->ks_count) CU(cudaMemset(h->ks_count, 0, ksplit_count_words(h->sm_count) * 4));
-    if (h->dg_count) CU(cudaMemset(h->dg_count, 0, (size_t)h->sm_count * 4));
     CU(cudaMemset(h->front_bar, 0, 16));
     h->stats.device_status = 0;
     return MLXS_OK;

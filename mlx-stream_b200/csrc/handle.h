@@ -68,8 +68,7 @@ struct mlxs_moe {
     // dense tensor-core products (shared expert, router logits): rows / h in the MMA's B-operand order, the scratch of
     // the split reduction
     uint16_t *dg_xb = nullptr, *dg_hb = nullptr;
-    float* dg_scratch = nullptr;
-    uint32_t* dg_count = nullptr;
+    uint32_t dg_staged_nt = 0;    // inside mlxs_moe_forward_x: dg_xb holds this call's rows in tiles of that many (0: it does not)
     // small batches: the shared expert runs beside the routed kernels on a second stream (they leave SMs free)
     float* logits_ws = nullptr;       // [max_tokens, E] logits of mlxs_moe_forward_x
     float* ks_scratch = nullptr;      // K-split workspace of the streaming kernels (exl3.cu)

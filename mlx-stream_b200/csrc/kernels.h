@@ -288,21 +288,22 @@ struct DenseSharedArgs {
     uint16_t* xb;            // [T rounded to 16, H] rows in the MMA's B-operand order (scratch)
     uint16_t* hb;            // [T rounded to 16, I] h in the same order (scratch)
     float* out;              // [T, H] f32
-    float* part_scratch;     // dense_gemm_scratch_bytes(sm_count), or null: never split the reduction
-    uint32_t* part_count;    // [sm_count] zeroed once
+    uint32_t nt;             // rows per token tile: dense_shared_rows(T, H, I, sm_count)
+    bool rows_staged;        // xb already holds x in tiles of nt rows
     uint32_t* status;
     int sm_count;
 };
-size_t dense_gemm_scratch_bytes(int sm_count);
+// rows per token tile of the shared expert's products, of the logits product alone
+uint32_t dense_shared_rows(uint32_t T, uint32_t H, uint32_t I, int sm_count);
+uint32_t dense_logits_rows(uint32_t T, uint32_t E, uint32_t H, int sm_count);
 bool dense_gemm_supported(uint32_t n_out, uint32_t K, int two_blocks);
 // W[n_out, K] row-major bf16 (w1 = a second matrix interleaved per 8-row group, or null) -> the tiled order
 cudaError_t launch_dense_retile(const __nv_bfloat16* w0, const __nv_bfloat16* w1, uint32_t n_out, uint32_t K, void* dst,
                                 cudaStream_t st);
 cudaError_t launch_dense_shared_expert(const DenseSharedArgs& a, cudaStream_t st);
 // logits[T, E] f32 = x . W_g^T with W_g re-tiled (single projection); E a multiple of 256
-cudaError_t launch_dense_logits(const __nv_bfloat16* x, const void* w_tiled, uint32_t T, uint32_t E, uint32_t H, uint16_t* xb,
-                                float* logits, float* part_scratch, uint32_t* part_count, uint32_t* status, int sm_count,
-                                cudaStream_t st);
+cudaError_t launch_dense_logits(const __nv_bfloat16* x, const void* w_tiled, uint32_t T, uint32_t E, uint32_t H, uint32_t nt, uint16_t* xb,
+                                float* logits, uint32_t* status, int sm_count, cudaStream_t st);
 // y[t] = sum_k ro[t,k] w[t,k] (+ shared[t]) -> bf16
 cudaError_t launch_combine(const void* ro, int ro_bf16, const float* weights, const float* shared, uint32_t T,
                            uint32_t K, uint32_t H, int chain, __nv_bfloat16* y, cudaStream_t st);
