@@ -132,9 +132,9 @@ struct Fp4Params {
     uint32_t n_sm, ks_cap_items; // SMs of the device; items the workspace and the counters hold
 };
 
-// flags: 1 = first stage of a part of the sum, 2 = last stage of a part, 4 = last stage of this CTA's share of the item
-// Only `item` and `flags` (with the chunk count in bits 8..) are read every stage, the rest at the end of a part.
-struct F4Meta { int32_t item; uint32_t flags, mc, ks, chunk0, expert, nb, part; };
+// flags: 1 = first stage of a part of the sum, 2 = last stage of a part, 4 = last stage of this CTA's share of the item;
+// bits 3.. = chunks of rows - 1.  Only `item` and `flags` are read every stage, the rest at the end of a part.
+struct F4Meta { int32_t item; uint32_t flags, mc, chunk0, expert, nb, part, pad; };
 
 // Eight e2m1 codes of a word -> four f16x2 through sm_100a's e2m1x2 conversion (one instruction per two codes, exact
 // values): h[i] = codes (2i, 2i + 1).  Measured against placing the code bits with shifts and masks (two logic ops per
@@ -149,75 +149,60 @@ __device__ __forceinline__ void fp4_decode8(uint32_t w, uint32_t (&h)[4]) {
         : "=r"(h[0]), "=r"(h[1]), "=r"(h[2]), "=r"(h[3])
         : "r"(w));
 }
-// E4M3 byte -> half2 (both halves) of its value (glm5n_e4m3: bits << 7 is the value x 2^-8 as f16; x 256 is exact)
-__device__ __forceinline__ __half2 e4m3_half2(uint32_t b) {
-    const uint32_t v = b & 127u;
-    const uint32_t u = (v << 7) | (((v + 1u) >> 7) << 14) | ((b & 128u) << 8);
-    const uint32_t uu = u * 0x00010001u;
-    const uint32_t k256 = 0x5C005C00u;
-    return __hmul2(*reinterpret_cast<const __half2*>(&uu), *reinterpret_cast<const __half2*>(&k256));
-}
 __device__ __forceinline__ uint32_t hmul2_u32(uint32_t a, __half2 s) {
     __half2 r = __hmul2(*reinterpret_cast<__half2*>(&a), s);
     return *reinterpret_cast<uint32_t*>(&r);
 }
 
-template <int NPROJ, bool NV, int MC>
-__device__ __forceinline__ void fp4_stage(const uint8_t* __restrict__ st, const uint8_t* __restrict__ xs, uint32_t x_mt_stride,
-                                          uint32_t p, uint32_t j, uint32_t lane, const uint32_t* __restrict__ lut,
-                                          float (&acc)[F4_GROUP][4]) {
-    // st: one 128-input sub-stage of codes and scales; xs: the same sub-stage of the first chunk's rows, the next
-    // chunk's x_mt_stride uint4 further
-    const uint32_t* wv = reinterpret_cast<const uint32_t*>(st + (size_t)p * F4_W_STAGE) + (j * 4) * 64 + lane;
-    const uint8_t* sc = st + (size_t)NPROJ * F4_W_STAGE + (size_t)p * f4_scale_stage_bytes(NV);
-    const uint4* xv = reinterpret_cast<const uint4*>(xs) + lane;
-    const uint32_t g = lane >> 2, c = lane & 3u;
+// One ring slot of SUB 128-input sub-stages: [sub-stage][projection codes, projection scales], then the rows [chunk][sub-stage].
+// w, sc: this lane's first code word and scale pair of the slot; xs: its first row word.  The block scales come through the
+// conversion instructions (two bytes at once: this lane's two output rows).
+template <int NPROJ, bool NV, int MC, int SUB>
+__device__ __forceinline__ void fp4_slot(const uint32_t* __restrict__ wv, const uint8_t* __restrict__ sc, const uint4* __restrict__ xv,
+                                         float (&acc)[F4_GROUP][4]) {
+    constexpr uint32_t W_BYTES = NPROJ * (F4_W_STAGE + (NV ? 1024u : 512u));
 #pragma unroll
-    for (int sb = 0; sb < 4; ++sb) {
-        const uint2 ww = make_uint2(wv[sb * 64], wv[sb * 64 + 32]);
-        uint32_t hx[4], hy[4];
-        fp4_decode8(ww.x, hx);
-        fp4_decode8(ww.y, hy);
-        float s_lo = 1.f, s_hi = 1.f;
-        if (NV) {
-            const uint32_t bb = *reinterpret_cast<const uint16_t*>(sc + (((j * 4 + sb) * 2 + (c >> 1)) * 8 + g) * 2);
-            const uint32_t u0 = lut[bb & 0xFFu], u1 = lut[bb >> 8];  // E4M3 byte -> f16x2 of its value
-            const __half2 sg = *reinterpret_cast<const __half2*>(&u0), sg8 = *reinterpret_cast<const __half2*>(&u1);
+    for (int u = 0; u < SUB; ++u) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) { hx[i] = hmul2_u32(hx[i], sg); hy[i] = hmul2_u32(hy[i], sg8); }
-        } else {
-            const uint32_t bb = *reinterpret_cast<const uint16_t*>(sc + ((j * 4 + sb) * 8 + g) * 2);
-            // 2^(b - 127); b = 0 is the subnormal 2^-127 (src/arch/mimo_v2/moe.zig:410-413)
-            const uint32_t b0 = bb & 0xFFu, b1 = bb >> 8;
-            s_lo = __uint_as_float(b0 ? b0 << 23 : 0x00400000u);
-            s_hi = __uint_as_float(b1 ? b1 << 23 : 0x00400000u);
-        }
-        const uint32_t a1[4] = {hx[0], hy[0], hx[1], hy[1]}, a2[4] = {hx[2], hy[2], hx[3], hy[3]};
-#pragma unroll
-        for (int mt = 0; mt < MC; ++mt) {
-            const uint4 xq = xv[mt * x_mt_stride + sb * 32];
+        for (int sb = 0; sb < 4; ++sb) {
+            const uint32_t wx = wv[u * (W_BYTES / 4) + sb * 64], wy = wv[u * (W_BYTES / 4) + sb * 64 + 32];
+            uint32_t hx[4], hy[4];
+            fp4_decode8(wx, hx);
+            fp4_decode8(wy, hy);
+            float s_lo = 1.f, s_hi = 1.f;
             if (NV) {
-                mma_f16(acc[mt], a1, xq.x, xq.y);
-                mma_f16(acc[mt], a2, xq.z, xq.w);
+                uint32_t s2;
+                const uint16_t bb = *reinterpret_cast<const uint16_t*>(sc + u * W_BYTES + sb * 32);
+                asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(s2) : "h"(bb));   // exact
+                const uint32_t u0 = __byte_perm(s2, s2, 0x1010), u1 = __byte_perm(s2, s2, 0x3232);
+                const __half2 sg = *reinterpret_cast<const __half2*>(&u0), sg8 = *reinterpret_cast<const __half2*>(&u1);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) { hx[i] = hmul2_u32(hx[i], sg); hy[i] = hmul2_u32(hy[i], sg8); }
             } else {
-                float tmp[4] = {0.f, 0.f, 0.f, 0.f};
-                mma_f16(tmp, a1, xq.x, xq.y);
-                mma_f16(tmp, a2, xq.z, xq.w);
-                acc[mt][0] = fmaf(tmp[0], s_lo, acc[mt][0]); acc[mt][1] = fmaf(tmp[1], s_lo, acc[mt][1]);
-                acc[mt][2] = fmaf(tmp[2], s_hi, acc[mt][2]); acc[mt][3] = fmaf(tmp[3], s_hi, acc[mt][3]);
+                // 2^(b - 127); b = 0 is the subnormal 2^-127 (src/arch/mimo_v2/moe.zig:410-413)
+                uint32_t s2;
+                const uint16_t bb = *reinterpret_cast<const uint16_t*>(sc + u * W_BYTES + sb * 16);
+                asm("cvt.rn.bf16x2.ue8m0x2 %0, %1;" : "=r"(s2) : "h"(bb));
+                s_lo = __uint_as_float(s2 << 16);
+                s_hi = __uint_as_float(s2 & 0xFFFF0000u);
+            }
+            const uint32_t a1[4] = {hx[0], hy[0], hx[1], hy[1]}, a2[4] = {hx[2], hy[2], hx[3], hy[3]};
+#pragma unroll
+            for (int mt = 0; mt < MC; ++mt) {
+                const uint4 xq = xv[(mt * SUB + u) * (4 * F4_XA_SB_WORDS / 4) + sb * 32];
+                if (NV) {
+                    mma_f16(acc[mt], a1, xq.x, xq.y);
+                    mma_f16(acc[mt], a2, xq.z, xq.w);
+                } else {
+                    float tmp[4] = {0.f, 0.f, 0.f, 0.f};
+                    mma_f16(tmp, a1, xq.x, xq.y);
+                    mma_f16(tmp, a2, xq.z, xq.w);
+                    acc[mt][0] = fmaf(tmp[0], s_lo, acc[mt][0]); acc[mt][1] = fmaf(tmp[1], s_lo, acc[mt][1]);
+                    acc[mt][2] = fmaf(tmp[2], s_hi, acc[mt][2]); acc[mt][3] = fmaf(tmp[3], s_hi, acc[mt][3]);
+                }
             }
         }
     }
-}
-
-// SUB sub-stages of one ring slot, unrolled
-template <int NPROJ, bool NV, int MC, int SUB>
-__device__ __forceinline__ void fp4_slot(const uint8_t* __restrict__ st, const uint8_t* __restrict__ xs, uint32_t w_bytes,
-                                         uint32_t x_mt_stride, uint32_t p, uint32_t j, uint32_t lane,
-                                         const uint32_t* __restrict__ lut, float (&acc)[F4_GROUP][4]) {
-#pragma unroll
-    for (int u = 0; u < SUB; ++u)
-        fp4_stage<NPROJ, NV, MC>(st + u * w_bytes, xs + u * (4 * F4_XA_SB_WORDS * 4), x_mt_stride, p, j, lane, lut, acc);
 }
 
 __device__ __forceinline__ float sigmoid_ref(float x) {  // src/arch/mimo_v2/moe.zig:341-344 (MLX's f32 sigmoid)
@@ -230,11 +215,11 @@ __global__ void __launch_bounds__(NPROJ * 256 + 32, NPROJ == 1 ? 3 : 2) fp4_gemv
     extern __shared__ __align__(128) uint8_t smem_raw[];
     constexpr int NCW = NPROJ * 8;
     constexpr int MAXS = 8;
-    __shared__ __align__(8) uint64_t full_bar[MAXS], empty_bar[MAXS], epi_bar;
-    __shared__ __align__(8) F4Meta meta[MAXS];
+    __shared__ __align__(8) uint64_t ring_bar[2 * MAXS], epi_bar;   // per slot: full, then (+ MAXS) empty
+    uint64_t *full_bar = ring_bar, *empty_bar = ring_bar + MAXS;
+    __shared__ __align__(16) F4Meta meta[MAXS];
     __shared__ volatile int s_abort;
     __shared__ volatile int s_last_part;
-    __shared__ uint32_t s_lut[NV ? 256 : 1];
     float* zs = reinterpret_cast<float*>(smem_raw);  // [NPROJ][F4_GROUP][8 rows][F4_ZS_STRIDE]
     uint8_t* ring = smem_raw + (size_t)NPROJ * F4_GROUP * F4_CHUNK * F4_ZS_STRIDE * sizeof(float);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
@@ -244,10 +229,6 @@ __global__ void __launch_bounds__(NPROJ * 256 + 32, NPROJ == 1 ? 3 : 2) fp4_gemv
         mbar_init(&epi_bar, NCW);
         s_abort = 0;
         mbar_fence_init();
-    }
-    if (NV && threadIdx.x < 256) {
-        const __half2 hv = e4m3_half2(threadIdx.x);
-        s_lut[threadIdx.x] = *reinterpret_cast<const uint32_t*>(&hv);
     }
     // The down kernel's prologue and first weight copies come before gate/up is complete (its producer waits, below);
     // everything else after the grid before
@@ -293,10 +274,10 @@ __global__ void __launch_bounds__(NPROJ * 256 + 32, NPROJ == 1 ? 3 : 2) fp4_gemv
                         s_abort = 1; ok = false; break;
                     }
                     meta[s].item = last ? -1 : (int32_t)item;
-                    meta[s].ks = ks; meta[s].chunk0 = chunk0; meta[s].mc = mc; meta[s].expert = expert; meta[s].nb = nb;
+                    meta[s].chunk0 = chunk0; meta[s].mc = mc; meta[s].expert = expert; meta[s].nb = nb;
                     meta[s].part = part;
                     const bool part_ends = in_part + sub == part_stages;
-                    meta[s].flags = (in_part == 0 ? 1u : 0u) | (part_ends ? 2u : 0u) | (ks + sub >= ks_end ? 4u : 0u) | (mc << 8);
+                    meta[s].flags = (in_part == 0 ? 1u : 0u) | (part_ends ? 2u : 0u) | (ks + sub >= ks_end ? 4u : 0u) | ((mc - 1u) << 3);
                     in_part = part_ends ? 0u : in_part + sub;
                     part += part_ends ? 1u : 0u;
                     if (last) { mbar_arrive(&full_bar[s]); ok = false; break; }
@@ -325,7 +306,7 @@ __global__ void __launch_bounds__(NPROJ * 256 + 32, NPROJ == 1 ? 3 : 2) fp4_gemv
         return;
     }
 
-    const uint32_t p = warp >> 3, j = warp & 7u;
+    const uint32_t p = NPROJ == 2 ? warp >> 3 : 0u, j = warp & 7u;
     float acc[F4_GROUP][4];
     uint32_t epi_ph = 0;
     auto epi_sync = [&]() -> bool {
@@ -336,38 +317,55 @@ __global__ void __launch_bounds__(NPROJ * 256 + 32, NPROJ == 1 ? 3 : 2) fp4_gemv
         if (!ok) { if (!s_abort) atomicMax(P.status, (uint32_t)ST_WAIT_FULL); s_abort = 1; }
         return ok;
     };
-    // ring slot and its phase advance by increment-and-wrap (the ring depth is a run-time value: no division per stage)
-    for (uint32_t s = 0, ph = 0;; s = (s + 1 == NS) ? (ph ^= 1u, 0u) : s + 1) {
-        if (!mbar_wait_bounded(&full_bar[s], ph, &s_abort)) {
+    // ring slot, its barriers, its meta and its phase advance by increment-and-wrap, and this lane's places inside a slot are
+    // worked out once: what a warp spends per slot beside the codes is what bounds the kernel (with one sub-stage per slot
+    // instead of two the MXFP4 gate/up of 61 tokens takes 512 us instead of 387)
+    const uint32_t full0 = smem_u32(&full_bar[0]), full_end = full0 + 8 * NS;
+    const uint32_t lg = lane >> 2, lc = lane & 3u;
+    const uint32_t w_off = p * F4_W_STAGE + (j * 4 * 64 + lane) * 4;
+    const uint32_t s_off = NPROJ * F4_W_STAGE + p * f4_scale_stage_bytes(NV) + (NV ? ((j * 8 + (lc >> 1)) * 8 + lg) * 2 : (j * 4 * 8 + lg) * 2);
+    const uint32_t x_off = P.sub * P.w_bytes + lane * 16;
+    uint32_t bar = full0, ph = 0;
+    const uint8_t* st = ring;
+    const F4Meta* mp = &meta[0];
+    for (;;) {
+        if (!mbar_wait_bounded_at(bar, ph, &s_abort)) {
             if (!s_abort) atomicMax(P.status, (uint32_t)ST_WAIT_FULL);
             s_abort = 1;
             break;
         }
-        const uint2 hot = *reinterpret_cast<const uint2*>(&meta[s]);   // item, flags | chunk count << 8
+        const uint2 hot = *reinterpret_cast<const uint2*>(mp);   // item, flags
         if ((int32_t)hot.x < 0) break;
-        const uint32_t flags = hot.y, stage_mc = hot.y >> 8;
+        const uint32_t flags = hot.y;
         if (flags & 1u) {
 #pragma unroll
             for (int a = 0; a < F4_GROUP; ++a)
 #pragma unroll
                 for (int q = 0; q < 4; ++q) acc[a][q] = 0.f;
         }
-        const uint8_t* st = ring + (size_t)s * P.stage_bytes;
-        const uint8_t* xs = st + P.sub * P.w_bytes;
-        const uint32_t x_mt_stride = P.sub * (4 * F4_XA_SB_WORDS / 4);
-        if (P.sub == 2) {
-            if (stage_mc == 1) fp4_slot<NPROJ, NV, 1, 2>(st, xs, P.w_bytes, x_mt_stride, p, j, lane, s_lut, acc);
-            else fp4_slot<NPROJ, NV, 2, 2>(st, xs, P.w_bytes, x_mt_stride, p, j, lane, s_lut, acc);
+        const uint32_t* wv = reinterpret_cast<const uint32_t*>(st + w_off);
+        const uint8_t* sc = st + s_off;
+        const uint4* xv = reinterpret_cast<const uint4*>(st + x_off);
+        if (flags & 8u) {
+            if (P.sub == 2) fp4_slot<NPROJ, NV, 2, 2>(wv, sc, xv, acc);
+            else if (P.sub == 4) fp4_slot<NPROJ, NV, 2, 4>(wv, sc, xv, acc);
+            else fp4_slot<NPROJ, NV, 2, 1>(wv, sc, xv, acc);
         } else {
-            for (uint32_t u = 0; u < P.sub; ++u, st += P.w_bytes, xs += 4 * F4_XA_SB_WORDS * 4) {
-                if (stage_mc == 1) fp4_stage<NPROJ, NV, 1>(st, xs, x_mt_stride, p, j, lane, s_lut, acc);
-                else fp4_stage<NPROJ, NV, 2>(st, xs, x_mt_stride, p, j, lane, s_lut, acc);
-            }
+            if (P.sub == 2) fp4_slot<NPROJ, NV, 1, 2>(wv, sc, xv, acc);
+            else if (P.sub == 4) fp4_slot<NPROJ, NV, 1, 4>(wv, sc, xv, acc);
+            else fp4_slot<NPROJ, NV, 1, 1>(wv, sc, xv, acc);
         }
+        // the slot may be refilled once this warp has arrived below
         F4Meta m;
-        if (flags & 2u) m = meta[s];       // the slot may be refilled once this warp has arrived below
+        m.item = (int32_t)hot.x;
+        if (flags & 2u) {
+            const uint4 q = reinterpret_cast<const uint4*>(mp)[1];
+            m.mc = mp->mc; m.chunk0 = mp->chunk0; m.expert = q.x; m.nb = q.y; m.part = q.z;
+        }
         __syncwarp();
-        if (lane == 0) mbar_arrive(&empty_bar[s]);
+        if (lane == 0) mbar_arrive_at(bar + 8 * MAXS);
+        bar += 8; st += P.stage_bytes; ++mp;
+        if (bar == full_end) { bar = full0; st = ring; mp = &meta[0]; ph ^= 1u; }
         if (!(flags & 2u)) continue;
 
         // ---- end of a part of the sum: D fragment = (output row g | g+8) x (token slots 2c, 2c+1) ----
