@@ -783,7 +783,7 @@ static int ep_combined_p2p(mlxs_moe* h, uint32_t layer, const void* x_dev, const
         StageTimer tm(h, MLXS_STAGE_EXCHANGE, st);
         if (A <= 2048) {
             // decode-sized calls: destination ranks, rank sort and dedup in one launch
-            mlxs::ep_plan_kernel<<<1, mlxs::DTHREADS, (W + 99) * sizeof(uint32_t), st>>>(ids_dev, A, c.n_experts, h->layers[layer].place_dev,
+            mlxs::ep_plan_kernel<<<1, mlxs::DTHREADS, mlxs::dispatch_words(A, W) * sizeof(uint32_t), st>>>(ids_dev, A, c.n_experts, h->layers[layer].place_dev,
                                                                                      ep->dest, ep->meta, ep->rtab, W, c.top_k, h->chunk_rows,
                                                                                      h->group_chunks, ep->urow, ep->ustart, ep->counts_dev,
                                                                                      h->status);

@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(1024, 1) front_kernel(const FrontParams P) {
     }
 
     // ---- phase 1: the router's tail ----
-    // shared memory: ids and weights [A], the tables [E + 1 + 6 A + 16], the dispatch scratch [E + 99], the scores [T][E + 2]
+    // shared memory: ids and weights [A], the tables [E + 1 + 6 A + 16], the dispatch scratch, the scores [T][E + 2]
     const uint32_t A = T * (uint32_t)P.K, E = (uint32_t)P.E;
     int32_t* s_ids = reinterpret_cast<int32_t*>(fsm);
     float* s_w = reinterpret_cast<float*>(s_ids + A);
@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(1024, 1) front_kernel(const FrontParams P) {
     const int32_t* ids = s_ids;
     if (P.by_warp) {
         // one expert per thread: the scoring functions are long, and this kernel's code comes cold from memory
-        float* s_sc = reinterpret_cast<float*>(scratch + E + 99);     // [T][E], then per token {max, NaN flag}
+        float* s_sc = reinterpret_cast<float*>(scratch + dispatch_words(A, E));     // [T][E], then per token {max, NaN flag}
         float* s_max = s_sc + (size_t)T * E;
         if (P.scoring == 2) {
             for (uint32_t t = warp; t < T; t += nwarp) {
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(1024, 1) front_kernel(const FrontParams P) {
 // smem: the larger of the phases' needs
 static size_t front_smem_bytes(const FrontArgs& a, int rthreads) {
     size_t s = router_smem_floats(a.E, a.K, rthreads) * sizeof(float);
-    const size_t d = ((size_t)8 * a.T * a.K + 2 * (size_t)a.E + 116 + (size_t)a.T * (a.E + 2)) * sizeof(uint32_t);
+    const size_t d = ((size_t)8 * a.T * a.K + (size_t)a.E + 17 + dispatch_words(a.T * (uint32_t)a.K, (uint32_t)a.E) + (size_t)a.T * (a.E + 2)) * sizeof(uint32_t);
     if (d > s) s = d;
     if (a.w_router) { const size_t l = logits_smem_bytes(a.H, 32); if (l > s) s = l; }
     return s;
