@@ -1,0 +1,141 @@
+"""Edges of the kernels' tiles and of the dispatch's ranges, against the CPU oracle or a plain product."""
+import numpy as np
+import pytest
+
+import oracle_lib as O
+from moe_cases import Exl3Case, Exl3K2Case, Mxfp4Case, Nvfp4Case, max_err_over_rms, rel_l2
+from test_parity_shapes_gpu import _shared_ref
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("rows", [(12, 13, 16, 17), (31, 32, 33, 1), (96, 97, 128, 129), (160, 161, 192, 193), (256, 257, 384, 385)])
+@pytest.mark.parametrize("cls,limit", [(Exl3Case, 10.0), (Exl3K2Case, 10.0), (Mxfp4Case, 0.0), (Nvfp4Case, 10.0)])
+def test_rows_of_an_expert_around_the_lanes_tiles(cls, limit, rows):
+    """Row counts on both sides of the lane choice and of the tensor-core lane's row tiles, three weight blocks of 128 wide
+    (an odd count: the last pass of the pair is short)."""
+    fp4 = cls in (Mxfp4Case, Nvfp4Case)
+    case = cls(768, 384, 4, 1, seed=21, shared=False, scoring=O.SCORE_SIGMOID, max_tokens=1300, routed_scale=1.0, limit=limit,
+               chain=fp4)
+    try:
+        ids = np.random.default_rng(rows[0]).permutation(np.repeat(np.arange(4), rows)).astype(np.int32)[:, None]
+        x, _ = case.inputs(ids.size, seed=40)
+        w = np.full(ids.shape, 0.75, np.float32)
+        y = case.gpu_experts(x, ids, w)
+        assert case.status() == 0
+        ref = case.cpu_layer(x, ids, w)
+        for e in range(4):   # every expert by itself: one wrong tile is not averaged away
+            m = ids[:, 0] == e
+            assert rel_l2(y[m], ref[m]) < 1e-2, (e, rows[e])
+    finally:
+        case.close()
+
+
+@pytest.mark.parametrize("E", [16, 64, 120, 256, 288])
+def test_router_logits_around_the_change_of_kernel(E):
+    """16 and 17 tokens (row kernel, tensor-core product) and the product's token tiles, the expert count padded to 256."""
+    import torch
+    case = Exl3Case(640, 256, E, 4, seed=2, shared=False, max_tokens=1030, experts_to_load=[])
+    try:
+        wg = O.f32_to_bf16_bits((np.random.default_rng(5).standard_normal((E, 640)) * 0.05).astype(np.float32))
+        case.moe.set_router_weight(0, wg.ctypes.data)
+        wf = O.bf16_bits_to_f32(wg).astype(np.float64)
+        for T in (1, 16, 17, 32, 33, 64, 65, 193, 1025):
+            x, _ = case.inputs(T, seed=70 + T)
+            lg = torch.full((T + 1, E), 7.0, dtype=torch.float32, device=case.dev)
+            case.moe.logits(0, case.to_dev_bf16(x).data_ptr(), T, lg.data_ptr(), None)
+            torch.cuda.synchronize()
+            got = lg.cpu().numpy()
+            assert np.allclose(got[:T], x.astype(np.float64) @ wf.T, rtol=2e-5, atol=1e-4), T
+            assert (got[T] == 7.0).all()        # the padding is not stored
+        assert case.status() == 0
+    finally:
+        case.close()
+
+
+@pytest.mark.parametrize("H,I", [(512, 256), (1280, 768)])
+def test_shared_expert_products_of_every_cluster_size(H, I):
+    case = Exl3Case(H, I, 2, 1, seed=11, shared=True, max_tokens=1030)
+    try:
+        for T in (65, 96, 97, 129, 192, 193, 257, 1025):
+            x, _ = case.inputs(T, seed=T)
+            y = case.gpu_experts(x, np.zeros((T, 1), np.int32), np.zeros((T, 1), np.float32))
+            assert case.status() == 0
+            assert rel_l2(y, _shared_ref(x, case.shared, case.limit)) < 4e-3, T
+    finally:
+        case.close()
+
+
+@pytest.mark.parametrize("cls,chain", [(Exl3Case, False), (Nvfp4Case, True)])
+@pytest.mark.parametrize("H,k", [(384, 1), (512, 3), (1152, 9), (2176, 8)])
+def test_combine_of_ragged_widths_and_counts(cls, chain, H, k):
+    """Columns that do not fill a block, and expert counts around the eight rows a thread holds in flight."""
+    case = cls(H, 256, 12, k, seed=5, shared=True, max_tokens=16, limit=10.0, chain=chain)
+    try:
+        x, logits = case.inputs(5, seed=3)
+        ids, w = case.cpu_route(logits)
+        y = case.gpu_forward(x, logits)
+        assert case.status() == 0
+        assert rel_l2(y, case.cpu_layer(x, ids, w)) < 1e-2
+    finally:
+        case.close()
+
+
+@pytest.mark.parametrize("E", [1, 33, 256, 1024])
+def test_dispatch_around_its_warps_and_blocks(E):
+    import torch
+    case = Exl3Case(128, 128, E, 1, seed=1, shared=False, max_tokens=17 * 1024 + 1, experts_to_load=[])
+    try:
+        rng = np.random.default_rng(E)
+        for n in (1, 31, 32, 33, 1023, 1024, 1025, 2047, 2048, 2049, 17 * 1024 + 1):
+            for slot in (rng.integers(0, E, n).astype(np.int32), np.full(n, E - 1, np.int32)):
+                d = torch.from_numpy(slot).cuda()
+                order = torch.full((n,), -1, dtype=torch.int32, device="cuda")
+                offs = torch.full((E + 1,), -1, dtype=torch.int32, device="cuda")
+                case.moe.sort_rows(d.data_ptr(), n, E, order.data_ptr(), offs.data_ptr(), None)
+                torch.cuda.synchronize()
+                assert (order.cpu().numpy() == np.argsort(slot, kind="stable")).all(), n
+                assert (offs.cpu().numpy()[1:] == np.cumsum(np.bincount(slot, minlength=E))).all(), n
+        assert case.status() == 0
+    finally:
+        case.close()
+
+
+@pytest.mark.parametrize("E,k", [(8, 8), (31, 4), (256, 8), (288, 8)])
+@pytest.mark.parametrize("scoring", [O.SCORE_SQRTSOFTPLUS, O.SCORE_SIGMOID, O.SCORE_SOFTMAX])
+def test_front_of_a_small_call_routes_as_the_router_alone(scoring, E, k):
+    """The fused front (one warp or one CTA per token) and the router kernel give the same layer, 1 to 17 tokens."""
+    case = Exl3Case(256, 128, E, k, seed=6, shared=False, scoring=scoring, max_tokens=32)
+    try:
+        for T in (1, 2, 16, 17):
+            x, logits = case.inputs(T, seed=T)
+            ids, w = case.gpu_route(logits)
+            assert (ids == case.cpu_route(logits)[0]).all()
+            assert (case.gpu_forward(x, logits) == case.gpu_experts(x, ids, w)).all(), T
+        assert case.status() == 0
+    finally:
+        case.close()
+
+
+@pytest.mark.parametrize("cls,scales", [(Mxfp4Case, [0, 1, 109, 126, 127, 128, 130]), (Nvfp4Case, [0, 1, 7, 8, 9, 119, 126])])
+def test_fp4_scale_bytes_at_the_ends_of_their_range(cls, scales):
+    """Zero, subnormal and the largest scales through the streaming kernels' conversions."""
+    nv = cls is Nvfp4Case
+    case = cls(512, 256, 2, 1, seed=4, shared=False, scoring=O.SCORE_SIGMOID, max_tokens=16, routed_scale=1.0,
+               limit=10.0 if nv else 0.0, chain=True)
+    try:
+        rec = case.records[0].copy()
+        off = (O.nvfp4_record_bytes if nv else O.mxfp4_record_bytes)(512, 256)[1]
+        n = 512 * 256 // (16 if nv else 32)
+        s = off[1]                                # the gate projection's scales
+        rec[s:s + n] = np.resize(np.array(scales, np.uint8), n)
+        case.records[0] = rec
+        case.moe.load_expert(0, 0, rec.ctypes.data, rec.size, on_device=False)
+        for T in (1, 7, 16):
+            x, _ = case.inputs(T, seed=T)
+            ids, w = np.zeros((T, 1), np.int32), np.ones((T, 1), np.float32)
+            y = case.gpu_experts(x, ids, w)
+            assert case.status() == 0 and np.isfinite(y).all()
+            assert rel_l2(y, case.cpu_layer(x, ids, w)) < 1e-2, T
+    finally:
+        case.close()
