@@ -331,7 +331,7 @@ static bool front_applies(const mlxs_moe* h, uint32_t T) {
 }
 
 static int experts_impl(mlxs_moe* h, uint32_t layer, const void* x_dev, const int32_t* ids_dev, const float* weights_dev,
-                        uint32_t T, void* y_dev, void* stream, const FrontCall* front);
+                        uint32_t T, void* y_dev, void* stream, const FrontCall* front, bool fork_recorded = false);
 
 int mlxs_bank_for_each_record(const char* dir, uint32_t bank_kind, uint64_t H, uint64_t I, uint64_t E, uint64_t n_layers,
                               uint32_t e_first, uint32_t e_count, int (*layer_begin)(void* ctx, uint32_t layer, uint32_t bits),
@@ -756,7 +756,7 @@ extern "C" int mlxs_moe_routed(mlxs_moe* h, uint32_t layer, const void* x_dev, c
 }
 
 static int experts_impl(mlxs_moe* h, uint32_t layer, const void* x_dev, const int32_t* ids_dev, const float* weights_dev,
-                        uint32_t T, void* y_dev, void* stream, const FrontCall* front) {
+                        uint32_t T, void* y_dev, void* stream, const FrontCall* front, bool fork_recorded) {
     int rc = check_call(h, layer, T, "experts");
     if (rc) return rc;
     if (T == 0 && h->cfg.ep_world == 1) return MLXS_OK;  // with expert parallelism an empty rank still serves its peers
@@ -799,7 +799,7 @@ static int experts_impl(mlxs_moe* h, uint32_t layer, const void* x_dev, const in
     };
     ForkGuard aux_guard(st);
     // the fork is recorded before the front kernel and used after its launch: the front's few CTAs find their SMs first
-    if (shared_aside) CU(cudaEventRecord(h->aux_fork, st));
+    if (shared_aside && !fork_recorded) CU(cudaEventRecord(h->aux_fork, st));
     if (front) {
         // route (from the logits, or from x through the layer's router weight), sort and stage in one launch
         FrontArgs fa{};
@@ -871,9 +871,14 @@ extern "C" int mlxs_moe_forward(mlxs_moe* h, uint32_t layer, const void* x_dev, 
         const FrontCall fc{logits_dev};
         return experts_impl(h, layer, x_dev, h->ids_ws, h->w_ws, T, y_dev, stream, &fc);
     }
-    int rc = mlxs_moe_route(h, layer, logits_dev, T, h ? h->ids_ws : nullptr, h ? h->w_ws : nullptr, stream);
+    int rc = check_call(h, layer, T, "route");
     if (rc) return rc;
-    return mlxs_moe_experts(h, layer, x_dev, h->ids_ws, h->w_ws, T, y_dev, stream);
+    // the shared expert needs nothing of the router: its stream forks off before it (its 128 or 144 large CTAs leave a few
+    // SMs, on which the router and the dispatch run; 64 tokens: the routed kernels start 10 us earlier)
+    const bool fork = h->cfg.shared_expert && h->aux_stream && T;
+    if (fork) CU(cudaEventRecord(h->aux_fork, (cudaStream_t)stream));
+    if ((rc = mlxs_moe_route(h, layer, logits_dev, T, h->ids_ws, h->w_ws, stream))) return rc;
+    return experts_impl(h, layer, x_dev, h->ids_ws, h->w_ws, T, y_dev, stream, nullptr, fork);
 }
 
 static int read_status(mlxs_moe* h, cudaStream_t st) {

@@ -24,7 +24,8 @@ namespace mlxs {
 // ------------------------------------------------------------------------------------------------------------
 // plan: row tiles per expert from the dispatch tables
 // ------------------------------------------------------------------------------------------------------------
-// Tile table: [2] = most rows of a tile of list 0 (a multiple of 16); [0] = tiles of list 0 (experts with up to cap0 rows: one tile each; with cap1 = 0 every expert, in tiles
+// Tile table: [2] = most rows of a tile of list 0 (a multiple of 16); [3], [4] = items that the gate/up, the down kernel has
+// given out; [0] = tiles of list 0 (experts with up to cap0 rows: one tile each; with cap1 = 0 every expert, in tiles
 // of up to cap0 rows), [1] = tiles of list 1 (the other experts, tiles of up to cap1 rows), then the entries {expert,
 // first sorted row, rows, first staging row}: list 0 from entry 0, list 1 from entry max_tiles.  An expert's rows are
 // split evenly over its tiles (a 16-row remainder tile would cost a full decode).
@@ -56,7 +57,7 @@ __global__ void pf_plan_kernel(DispatchTables t, uint32_t E, const uint8_t* __re
         base1[E] = n1;
         tiles[0] = n0;
         tiles[1] = n1;
-        tiles[2] = 0;
+        tiles[2] = tiles[3] = tiles[4] = 0;
     }
     __syncthreads();
     if (base0[E] + base1[E] == 0) return;
@@ -385,13 +386,14 @@ cudaError_t launch_prefill_plan(DispatchTables t, uint32_t n_experts, const uint
 template <int KB>
 static cudaError_t pf_launch_all(const Exl3PrefillArgs& a, cudaStream_t st) {
     LaneParams P{};
-    P.tiles = a.tiles; P.max_tiles = a.max_tiles; P.t = a.t; P.scales = a.L.scales; P.scales_stride = exl3_scales_per_expert(a.d);
+    P.tiles = a.tiles; P.next = a.tiles + 3; P.max_tiles = a.max_tiles; P.t = a.t; P.scales = a.L.scales; P.scales_stride = exl3_scales_per_expert(a.d);
     P.H = a.d.H; P.I = a.d.I; P.limit = a.limit; P.status = a.status; P.act = a.act;
     P.code = reinterpret_cast<const uint8_t*>(a.L.gu_code); P.expert_stride = 8 * exl3_code_words(a.d); P.n_blocks = a.d.I / 128; P.n_stages = a.d.H / LN_KST;
     P.xa = reinterpret_cast<const uint16_t*>(a.xa); P.xa_proj_stride = exl3_prefill_staging_rows(a.rows_cap, a.max_tiles) * a.d.H;
     P.xd = reinterpret_cast<uint16_t*>(a.xd);
     const cudaError_t e = lane_launch<Exl3LaneBank<KB>, 2>(P, a.sm_count, st);
     if (e != cudaSuccess) return e;
+    P.next = a.tiles + 4;
     P.code = reinterpret_cast<const uint8_t*>(a.L.d_code); P.expert_stride = 4 * exl3_code_words(a.d); P.n_blocks = a.d.H / 128; P.n_stages = a.d.I / LN_KST;
     P.xa = P.xd; P.xa_proj_stride = 0; P.xd = nullptr; P.out = a.ro;
     return lane_launch<Exl3LaneBank<KB>, 1>(P, a.sm_count, st);

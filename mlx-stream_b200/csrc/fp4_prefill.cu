@@ -241,12 +241,13 @@ static cudaError_t q_launch_all(const Fp4PrefillArgs& a, cudaStream_t st) {
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     LaneParams P{};
-    P.gscale = a.gscale; P.tiles = a.tiles; P.max_tiles = a.max_tiles; P.t = a.t; P.H = a.H; P.I = a.I; P.limit = a.limit;
+    P.gscale = a.gscale; P.tiles = a.tiles; P.next = a.tiles + 3; P.max_tiles = a.max_tiles; P.t = a.t; P.H = a.H; P.I = a.I; P.limit = a.limit;
     P.status = a.status; P.act = a.act;
     P.code = a.gu; P.n_blocks = a.I / 128; P.n_stages = a.H / LN_KST;
     P.expert_stride = (size_t)P.n_blocks * P.n_stages * 2 * Fp4LaneBank<NV>::RAW_BYTES;
     P.xa = a.xa; P.xa_proj_stride = 0; P.xd = a.xd;
     if ((e = lane_launch<Fp4LaneBank<NV>, 2>(P, a.sm_count, st)) != cudaSuccess) return e;
+    P.next = a.tiles + 4;
     P.code = a.dn; P.n_blocks = a.H / 128; P.n_stages = a.I / LN_KST;
     P.expert_stride = (size_t)P.n_blocks * P.n_stages * Fp4LaneBank<NV>::RAW_BYTES;
     P.xa = a.xd; P.xd = nullptr; P.out = a.ro; P.out_bf16 = a.ro_bf16;

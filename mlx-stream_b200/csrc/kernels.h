@@ -147,12 +147,12 @@ __host__ __device__ inline bool takes_tensor_lane(uint32_t rows, uint32_t min_ro
 // cap0 rows; with cap1 = 0 all experts, in tiles of up to cap0 rows) and list 1 (the others, tiles of up to cap1 rows);
 // entries {expert, first sorted row, rows, first staging row}, list 1 from entry max_tiles.  The table holds
 // prefill_tile_words(max_tiles) words.
-__host__ __device__ inline size_t prefill_tile_words(uint32_t max_tiles) { return 4 + 8 * (size_t)max_tiles; }
+__host__ __device__ inline size_t prefill_tile_words(uint32_t max_tiles) { return 8 + 8 * (size_t)max_tiles; }
 __host__ __device__ inline uint32_t* prefill_tile(uint32_t* tiles, int list, uint32_t max_tiles, uint32_t i) {
-    return tiles + 4 + 4 * ((size_t)(list ? max_tiles : 0) + i);
+    return tiles + 8 + 4 * ((size_t)(list ? max_tiles : 0) + i);
 }
 __host__ __device__ inline const uint32_t* prefill_tile(const uint32_t* tiles, int list, uint32_t max_tiles, uint32_t i) {
-    return tiles + 4 + 4 * ((size_t)(list ? max_tiles : 0) + i);
+    return tiles + 8 + 4 * ((size_t)(list ? max_tiles : 0) + i);
 }
 cudaError_t launch_prefill_plan(DispatchTables t, uint32_t n_experts, const uint8_t* lane_flags, uint32_t min_rows,
                                 uint32_t cap0, uint32_t cap1, uint32_t max_tiles, uint32_t* tiles, uint32_t* status,

@@ -17,6 +17,9 @@
 //   * The MMA warp runs its loop with all lanes and issues under elect.sync (see elect_one); one commit per stage frees the
 //     operand slot and the rows' slot.
 //   * One producer lane streams the code, another the rows: bulk copies into rings.
+//   * The code producer takes the CTA's items one by one from a counter and passes them on to the other roles.  Beside the
+//     streaming lane the CTAs start when SMs come free, up to a third of the kernel apart, and with items dealt out in
+//     advance the last CTA to start decided the time.
 // Every wait is bounded; on a give-up the CTA sets the status word, skips work and still frees its tensor memory.
 #pragma once
 #include "common.cuh"
@@ -39,6 +42,9 @@ constexpr int LN_A_COLS = LN_KST / 2;   // tensor-memory columns of a decoded st
 constexpr int LN_ROWS = 192;            // most rows of a tile
 constexpr int LN_RAW_STAGES = 4;        // stages of the code ring
 constexpr int LN_B_STAGES = 3;          // stages of the rows' ring
+// Items announced to the roles.  An entry is written again LN_ITEMS items later: the code ring, the operand slots and the two
+// accumulator buffers keep the slowest role (the epilogue) within 4 + 6 + 3 one-stage items of the code producer.
+constexpr uint32_t LN_ITEMS = 16, LN_NO_ITEM = 0xFFFFFFFFu;
 constexpr int LN_DONE = 4;              // barriers of the stages in flight: operands complete, MMAs complete
 constexpr int LN_DEC_WARPS = 16, LN_EPI_WARPS = 8;
 // warps 0 .. 3: MMA, code producer, rows' producer, none; then the decode warps, then the epilogue warps.  The scheduler
@@ -59,6 +65,7 @@ struct LaneParams {
     const uint16_t* xa;          // staged rows, pass p at p * xa_proj_stride elements
     size_t xa_proj_stride;
     const uint32_t* tiles;       // list 0 of the tile table
+    uint32_t* next;              // items given out so far
     uint32_t max_tiles;
     DispatchTables t;
     uint32_t H, I;
@@ -113,7 +120,9 @@ template <class BK, int NPASS>
 __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t raw_full[LN_RAW_STAGES], raw_empty[LN_RAW_STAGES];
-    __shared__ __align__(8) uint64_t bar_stage[2 * LN_DONE], acc_full[2], acc_empty[2], epi_bar;
+    __shared__ __align__(8) uint64_t bar_stage[2 * LN_DONE], acc_full[2], acc_empty[2], epi_bar, item_full[LN_ITEMS];
+    __shared__ uint4 s_tile[LN_ITEMS];       // the tile's entry
+    __shared__ uint32_t s_nb[LN_ITEMS];      // the column block, LN_NO_ITEM behind the last item
     uint64_t *full = bar_stage, *done = bar_stage + LN_DONE;             // of the stages in flight: operands complete, MMAs complete
     __shared__ uint32_t s_tmem;
     __shared__ volatile int s_abort;
@@ -121,7 +130,7 @@ __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P)
     uint8_t* raw_ring = b_ring + LN_B_STAGES * LN_B_SLOT;                // [stage][BK::RAW_BYTES]
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t n_items = P.tiles[0] * P.n_blocks;
-    // a CTA without work leaves before it takes tensor memory (the whole CTA reads the same count)
+    // a CTA that cannot get work leaves before it takes tensor memory (the whole CTA reads the same count)
     if (blockIdx.x >= n_items) return;
 
     if (threadIdx.x == 0) {
@@ -130,10 +139,12 @@ __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P)
         for (int s = 0; s < LN_DONE; ++s) { mbar_init(&full[s], LN_DEC_WARPS / 2 + 1); mbar_init(&done[s], 1); }
         for (int s = 0; s < 2; ++s) { mbar_init(&acc_full[s], 1); mbar_init(&acc_empty[s], LN_EPI_WARPS); }
         mbar_init(&epi_bar, LN_EPI_WARPS);
+        for (uint32_t s = 0; s < LN_ITEMS; ++s) mbar_init(&item_full[s], 1);
         s_abort = 0;
         mbar_fence_init();
     }
     if (warp == 0) tmem_alloc(&s_tmem, 512);
+    const uint32_t first = threadIdx.x == 32 ? atomicAdd(P.next, 1u) : 0u;   // the code producer's first item
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -141,14 +152,14 @@ __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P)
     const uint32_t acc_cols = P.tiles[2] <= 128u ? 128u : P.tiles[2] <= 160u ? 160u : 192u, slots = (512u - 2u * acc_cols) / LN_A_COLS;
     const uint32_t tmem = s_tmem, tmem_a = tmem + 2 * acc_cols;
     const uint32_t nstage = P.n_stages, width = nstage * LN_KST;
-    const uint32_t my_items = (n_items - blockIdx.x + gridDim.x - 1) / gridDim.x;
-    const uint32_t my_stages = my_items * NPASS * nstage;   // stages are numbered through over all passes of the CTA
     auto give_up = [&](uint32_t code) { if (!s_abort) atomicMax(P.status, code); s_abort = 1; };
-    // item number i of this CTA -> its tile entry {expert, first sorted row, rows, first staging row} and column block
-    auto item_tile = [&](uint32_t i, uint32_t& nb) {
-        const uint32_t item = blockIdx.x + i * gridDim.x;
-        nb = item % P.n_blocks;
-        return prefill_tile(P.tiles, 0, P.max_tiles, item / P.n_blocks);
+    // item number n of this CTA, once it is known; false: there is none (or the CTA has given up)
+    auto next_item = [&](uint32_t n, uint4& tile, uint32_t& nb, uint32_t sleep_ns) -> bool {
+        const uint32_t s = n % LN_ITEMS;
+        if (!mbar_wait_bounded(&item_full[s], (n / LN_ITEMS) & 1u, &s_abort, sleep_ns)) { give_up(ST_WAIT_FULL); return false; }
+        tile = s_tile[s];
+        nb = s_nb[s];
+        return nb != LN_NO_ITEM;
     };
 
     if (warp >= LN_SERVICE && warp < LN_SERVICE + LN_DEC_WARPS) {
@@ -161,13 +172,22 @@ __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P)
         // flip every second stage.  The instructions around the decode count (it is issue-bound), so those addresses advance
         // by an exclusive-or, and the tests of the two barriers that come next (the operand slot, the next stage's code) go
         // out together: a test of a barrier that is ready costs its latency.
-        const uint32_t n_i = (my_stages - team + 1) / 2, bar0 = smem_u32(&bar_stage[0]);
+        const uint32_t bar0 = smem_u32(&bar_stage[0]);
         uint32_t b_raw = smem_u32(&raw_full[team]), b_emp = smem_u32(&raw_empty[team]), b_full = bar0 + 8 * team;
         const uint32_t x_raw = b_raw ^ smem_u32(&raw_full[team + 2]), x_emp = b_emp ^ smem_u32(&raw_empty[team + 2]), x_full = b_full ^ (bar0 + 8 * (team + 2));
         bool code_ready = false;
         uint32_t woff = 0, slot = team;                    // slots >= 2
+        uint32_t items = 0, known = 0;                     // items so far and the stages they have
         LC(const long long c0 = clock64();)
-        for (uint32_t i = 0; i < n_i; ++i) {
+        for (uint32_t i = 0;; ++i) {
+            bool more = true;
+            while (more && team + 2 * i >= known) {
+                uint4 tile;
+                uint32_t nb;
+                more = next_item(items++, tile, nb, 0);
+                known += NPASS * nstage;
+            }
+            if (!more) break;
             if (!code_ready && !mbar_wait_bounded_at(b_raw, (i >> 1) & 1u, &s_abort)) { give_up(ST_WAIT_FULL); break; }
             uint32_t v[2][16];
             dec.decode(raw, woff, v);
@@ -188,7 +208,7 @@ __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P)
             b_emp ^= x_emp; b_full ^= x_full; woff ^= 2 * BK::RAW_BYTES;
             slot = slot + 2 >= slots ? slot + 2 - slots : slot + 2;
         }
-        LC(if (blockIdx.x == 3 && lane == 0 && warp == 13) printf("LANE<%d> decode warp: %u half stages of %u, cycles per stage: %lld\n", NPASS, n_i, 2 * my_stages, (clock64() - c0) / my_stages);)
+        LC(if (blockIdx.x == 3 && lane == 0 && warp == 13) printf("LANE<%d> decode warp: cycles per stage: %lld\n", NPASS, (clock64() - c0) / (known + 1));)
     } else if (warp >= LN_SERVICE + LN_DEC_WARPS) {
         // ---------------- epilogue warps ----------------
         LaneEpi E;
@@ -198,10 +218,11 @@ __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P)
         uint32_t pass_n = 0;
         LC(long long t_wait = 0, t_epi = 0;)
         bool ok = true;
-        for (uint32_t it = 0; it < my_items && ok; ++it) {
+        for (uint32_t it = 0; ok; ++it) {
             LanePass C;
-            const uint32_t* te = item_tile(it, C.nb);
-            C.expert = te[0]; C.row0 = te[1]; C.rows = te[2]; C.srow0 = te[3]; C.rows16 = (te[2] + 15) / 16 * 16;
+            uint4 te;
+            if (!next_item(it, te, C.nb, 200)) break;
+            C.expert = te.x; C.row0 = te.y; C.rows = te.z; C.srow0 = te.w; C.rows16 = (te.z + 15) / 16 * 16;
 #pragma unroll
             for (int p = 0; p < NPASS && ok; ++p, ++pass_n) {
                 const uint32_t buf = pass_n & 1u;
@@ -220,10 +241,16 @@ __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P)
         // ---------------- code producer ----------------
         if (lane == 0) {
             uint32_t g = 0;
-            for (uint32_t it = 0; it < my_items && !s_abort; ++it) {
-                uint32_t nb;
-                const uint32_t* te = item_tile(it, nb);
-                const uint8_t* src = P.code + (size_t)te[0] * P.expert_stride + (size_t)nb * NPASS * nstage * BK::RAW_BYTES;
+            for (uint32_t it = 0;; ++it) {
+                const uint32_t item = it ? atomicAdd(P.next, 1u) : first;
+                const bool more = item < n_items && !s_abort;
+                const uint32_t nb = more ? item % P.n_blocks : LN_NO_ITEM;
+                const uint4 te = *reinterpret_cast<const uint4*>(prefill_tile(P.tiles, 0, P.max_tiles, more ? item / P.n_blocks : 0u));
+                s_tile[it % LN_ITEMS] = te;
+                s_nb[it % LN_ITEMS] = nb;
+                mbar_arrive(&item_full[it % LN_ITEMS]);
+                if (!more) break;
+                const uint8_t* src = P.code + (size_t)te.x * P.expert_stride + (size_t)nb * NPASS * nstage * BK::RAW_BYTES;
                 for (uint32_t ks = 0; ks < NPASS * nstage; ++ks, ++g) {
                     const uint32_t rs = g % LN_RAW_STAGES;
                     if (!mbar_wait_bounded(&raw_empty[rs], ((g / LN_RAW_STAGES) & 1u) ^ 1u, &s_abort, 64)) { give_up(ST_WAIT_EMPTY); break; }
@@ -245,9 +272,11 @@ __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P)
         const uint32_t bars_end = bars + 8 * LN_DONE;
         bool ok = true;
         LC(long long m_a = 0, m_issue = 0; uint32_t g = 0;)
-        for (uint32_t it = 0; it < my_items && ok; ++it) {
+        for (uint32_t it = 0; ok; ++it) {
+            uint4 te;
             uint32_t nb;
-            const uint32_t idesc = umma_idesc(BK::FORMAT, (item_tile(it, nb)[2] + 15) / 16 * 16);
+            if (!__all_sync(0xFFFFFFFFu, next_item(it, te, nb, 0))) break;
+            const uint32_t idesc = umma_idesc(BK::FORMAT, (te.z + 15) / 16 * 16);
             for (int p = 0; p < NPASS && ok; ++p, ++pass_n) {
                 const uint32_t buf = pass_n & 1u, acc = tmem + buf * acc_cols;
                 if (!mbar_wait_warp(&acc_empty[buf], ((pass_n >> 1) & 1u) ^ 1u, &s_abort)) { give_up(ST_WAIT_EMPTY); ok = false; break; }
@@ -276,12 +305,13 @@ __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P)
         // ---------------- rows' producer ----------------
         if (lane == 0) {
             uint32_t g = 0, bs = 0;
-            for (uint32_t it = 0; it < my_items && !s_abort; ++it) {
+            for (uint32_t it = 0; !s_abort; ++it) {
+                uint4 te;
                 uint32_t nb;
-                const uint32_t* te = item_tile(it, nb);
-                const uint32_t rows16 = (te[2] + 15) / 16 * 16, b_bytes = rows16 * LN_KST * 2;
+                if (!next_item(it, te, nb, 64)) break;
+                const uint32_t rows16 = (te.z + 15) / 16 * 16, b_bytes = rows16 * LN_KST * 2;
                 for (int p = 0; p < NPASS; ++p) {
-                    const uint16_t* xsrc = P.xa + p * P.xa_proj_stride + (size_t)te[3] * width;
+                    const uint16_t* xsrc = P.xa + p * P.xa_proj_stride + (size_t)te.w * width;
                     for (uint32_t ks = 0; ks < nstage; ++ks, ++g) {
                         if (g >= LN_B_STAGES) {
                             const uint32_t d = g - LN_B_STAGES;
