@@ -241,8 +241,9 @@ struct Exl3LaneBank {
             exl3_lane_plan_kb<KB>(lane, wi, wj, lp);
             off = half * (LN_KST / 32) * KT_WORDS + 2 * q * TW;   // lanes 32 q .. hold the 16-column tiles 2 q, 2 q + 1
         }
-        __device__ __forceinline__ void decode(const uint8_t* raw, uint32_t slot_bytes, uint32_t (&v)[2][16]) const {
-            const uint32_t* w = reinterpret_cast<const uint32_t*>(raw + slot_bytes) + off;
+        // h: halves of a stage behind the constructor's
+        __device__ __forceinline__ void decode(const uint8_t* raw, uint32_t slot_bytes, uint32_t h, uint32_t (&v)[2][16]) const {
+            const uint32_t* w = reinterpret_cast<const uint32_t*>(raw + slot_bytes) + off + h * ((LN_KST / 32) * KT_WORDS);
             const uint32_t *tw_i = w + wi, *tw_j = w + wj;
 #pragma unroll
             for (int jj = 0; jj < 2; ++jj)

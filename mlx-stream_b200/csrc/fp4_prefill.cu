@@ -132,8 +132,9 @@ struct Fp4LaneBank {
             w_off = (((wr * 4 + sb) * 2 + r) * 32 + g * 4) * 4;                       // words [wr][block][r][g][4]
             s_off = Q_W_STAGE + (NV ? (wr * 4 + sb) * 32 + g * 2 + r : ((wr * 4 + sb) * 8 + g) * 2 + r);
         }
-        __device__ __forceinline__ void decode(const uint8_t* raw, uint32_t slot_bytes, uint32_t (&v)[2][16]) const {
-            const uint8_t *w = raw + slot_bytes + w_off, *s = raw + slot_bytes + s_off;
+        // h: halves of a stage behind the constructor's
+        __device__ __forceinline__ void decode(const uint8_t* raw, uint32_t slot_bytes, uint32_t h, uint32_t (&v)[2][16]) const {
+            const uint8_t *w = raw + slot_bytes + w_off + h * 512u, *s = raw + slot_bytes + s_off + h * (NV ? 64u : 32u);
 #pragma unroll
             for (int b = 0; b < 2; ++b) {
                 const uint4 ww = *reinterpret_cast<const uint4*>(w + b * 256);

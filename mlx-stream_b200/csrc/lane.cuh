@@ -11,9 +11,12 @@
 //     further ahead and a stage's round trip (decode, store, MMAs, slot free) no longer shows.
 //     With gate and up accumulated together (2 x 192, one buffer) the K loop stood still for the epilogue, a fifth of an
 //     item's time, and experts of 65 .. 96 rows paid for it most.
-//   * 16 decode warps in two teams take the stages alternately (team = stage parity).  A warp decodes its half
-//     stage into 32 registers and only then waits for its operand slot: the MMAs of the slot's last stage run under the
-//     decode.  (Decoding in halves of that, or with 5 or 6 warps per lane quarter, measured slower or equal.)
+//   * 16 decode warps in teams that take the stages in turn.  A warp decodes half a stage of its 32 columns into 32 registers
+//     and only then waits for its operand slot: the MMAs of the slot's last stage run under the decode.  With four operand
+//     slots there are four teams of four warps, a warp decoding both halves of a stage, else two of eight: the barriers
+//     around a stage are a quarter of the instructions of a warp that decodes one half (EXL3: 60 instructions per 16x16 tile,
+//     43 of them the decode), and the loop is bound by their issue; but a team of four keeps its slot for twice as long.
+//     (Decoding in smaller pieces, or with 5 or 6 warps per lane quarter, measured slower or equal.)
 //   * The MMA warp runs its loop with all lanes and issues under elect.sync (see elect_one); one commit per stage frees the
 //     operand slot and the rows' slot.
 //   * One producer lane streams the code, another the rows: bulk copies into rings.
@@ -22,6 +25,8 @@
 //     advance the last CTA to start decided the time.
 // Every wait is bounded; on a give-up the CTA sets the status word, skips work and still frees its tensor memory.
 #pragma once
+#include <type_traits>
+
 #include "common.cuh"
 #include "kernels.h"
 #include "umma.cuh"
@@ -40,11 +45,11 @@ namespace mlxs {
 constexpr int LN_KST = 128;             // inputs per stage
 constexpr int LN_A_COLS = LN_KST / 2;   // tensor-memory columns of a decoded stage
 constexpr int LN_ROWS = 192;            // most rows of a tile
-constexpr int LN_RAW_STAGES = 4;        // stages of the code ring
+constexpr int LN_RAW_STAGES = 8;        // most stages of the code ring: two per team
 constexpr int LN_B_STAGES = 3;          // stages of the rows' ring
 // Items announced to the roles.  An entry is written again LN_ITEMS items later: the code ring, the operand slots and the two
-// accumulator buffers keep the slowest role (the epilogue) within 4 + 6 + 3 one-stage items of the code producer.
-constexpr uint32_t LN_ITEMS = 16, LN_NO_ITEM = 0xFFFFFFFFu;
+// accumulator buffers keep the slowest role (the epilogue) within 8 + 4 + 3 one-stage items of the code producer.
+constexpr uint32_t LN_ITEMS = 32, LN_NO_ITEM = 0xFFFFFFFFu;
 constexpr int LN_DONE = 4;              // barriers of the stages in flight: operands complete, MMAs complete
 constexpr int LN_DEC_WARPS = 16, LN_EPI_WARPS = 8;
 // warps 0 .. 3: MMA, code producer, rows' producer, none; then the decode warps, then the epilogue warps.  The scheduler
@@ -126,17 +131,20 @@ __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P)
     uint64_t *full = bar_stage, *done = bar_stage + LN_DONE;             // of the stages in flight: operands complete, MMAs complete
     __shared__ uint32_t s_tmem;
     __shared__ volatile int s_abort;
-    uint8_t* b_ring = smem_raw;                                          // [stage][rows16 x 256 B]
-    uint8_t* raw_ring = b_ring + LN_B_STAGES * LN_B_SLOT;                // [stage][BK::RAW_BYTES]
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t n_items = P.tiles[0] * P.n_blocks;
     // a CTA that cannot get work leaves before it takes tensor memory (the whole CTA reads the same count)
     if (blockIdx.x >= n_items) return;
 
+    // columns of an accumulator buffer (the call's largest tile), operand slots in what is left
+    const uint32_t acc_cols = P.tiles[2] <= 128u ? 128u : P.tiles[2] <= 160u ? 160u : 192u, slots = (512u - 2u * acc_cols) / LN_A_COLS;
+    const uint32_t teams = slots == 4 ? 4u : 2u, raw_stages = 2u * teams, b_slot = acc_cols * (LN_KST * 2u);
+    uint8_t* b_ring = smem_raw;                                          // [stage][rows16 x 256 B]
+    uint8_t* raw_ring = b_ring + LN_B_STAGES * b_slot;                   // [stage][BK::RAW_BYTES]
     if (threadIdx.x == 0) {
-        for (int s = 0; s < LN_RAW_STAGES; ++s) { mbar_init(&raw_full[s], 1); mbar_init(&raw_empty[s], LN_DEC_WARPS / 2); }
+        for (int s = 0; s < LN_RAW_STAGES; ++s) { mbar_init(&raw_full[s], 1); mbar_init(&raw_empty[s], LN_DEC_WARPS / teams); }
         // a stage's operands: the team's warps have stored theirs, the rows have landed
-        for (int s = 0; s < LN_DONE; ++s) { mbar_init(&full[s], LN_DEC_WARPS / 2 + 1); mbar_init(&done[s], 1); }
+        for (int s = 0; s < LN_DONE; ++s) { mbar_init(&full[s], LN_DEC_WARPS / teams + 1); mbar_init(&done[s], 1); }
         for (int s = 0; s < 2; ++s) { mbar_init(&acc_full[s], 1); mbar_init(&acc_empty[s], LN_EPI_WARPS); }
         mbar_init(&epi_bar, LN_EPI_WARPS);
         for (uint32_t s = 0; s < LN_ITEMS; ++s) mbar_init(&item_full[s], 1);
@@ -148,8 +156,6 @@ __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P)
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    // columns of an accumulator buffer (the call's largest tile), operand slots in what is left
-    const uint32_t acc_cols = P.tiles[2] <= 128u ? 128u : P.tiles[2] <= 160u ? 160u : 192u, slots = (512u - 2u * acc_cols) / LN_A_COLS;
     const uint32_t tmem = s_tmem, tmem_a = tmem + 2 * acc_cols;
     const uint32_t nstage = P.n_stages, width = nstage * LN_KST;
     auto give_up = [&](uint32_t code) { if (!s_abort) atomicMax(P.status, code); s_abort = 1; };
@@ -162,26 +168,27 @@ __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P)
         return nb != LN_NO_ITEM;
     };
 
-    if (warp >= LN_SERVICE && warp < LN_SERVICE + LN_DEC_WARPS) {
-        // ---------------- decode warps: (lane quarter q, half of the stage's inputs, team) ----------------
-        const uint32_t q = warp & 3u, half = (warp >> 2) & 1u, team = (warp - LN_SERVICE) >> 3;
+    // a decode warp (lane quarter q, team; of two teams: half of the stage's inputs)
+    auto decode_stages = [&](auto teams_c) {
+        constexpr uint32_t TEAMS = decltype(teams_c)::value;
+        const uint32_t dw = warp - LN_SERVICE, q = warp & 3u, team = TEAMS == 4 ? dw >> 2 : dw >> 3, half = TEAMS == 4 ? 0u : (dw >> 2) & 1u;
         const typename BK::Decoder dec(q, half, lane);
         const uint8_t* raw = raw_ring + team * BK::RAW_BYTES;
         const uint32_t ta0 = tmem_a + ((q * 32u) << 16) + half * (LN_A_COLS / 2);
-        // The team's stages are g = team + 2 i: code slot and code barriers alternate between team and team + 2, their phases
-        // flip every second stage.  The instructions around the decode count (it is issue-bound), so those addresses advance
-        // by an exclusive-or, and the tests of the two barriers that come next (the operand slot, the next stage's code) go
-        // out together: a test of a barrier that is ready costs its latency.
+        // The team's stages are g = team + TEAMS i: code slot and code barriers alternate between team and team + TEAMS, their
+        // phases flip every second stage.  The instructions around the decode count (it is issue-bound), so those addresses
+        // advance by an exclusive-or, and the tests of the two barriers that come next (the operand slot, the next stage's
+        // code) go out together: a test of a barrier that is ready costs its latency.
         const uint32_t bar0 = smem_u32(&bar_stage[0]);
-        uint32_t b_raw = smem_u32(&raw_full[team]), b_emp = smem_u32(&raw_empty[team]), b_full = bar0 + 8 * team;
-        const uint32_t x_raw = b_raw ^ smem_u32(&raw_full[team + 2]), x_emp = b_emp ^ smem_u32(&raw_empty[team + 2]), x_full = b_full ^ (bar0 + 8 * (team + 2));
+        uint32_t b_raw = smem_u32(&raw_full[team]), b_emp = smem_u32(&raw_empty[team]);
+        const uint32_t x_raw = b_raw ^ smem_u32(&raw_full[team + TEAMS]), x_emp = b_emp ^ smem_u32(&raw_empty[team + TEAMS]);
         bool code_ready = false;
-        uint32_t woff = 0, slot = team;                    // slots >= 2
+        uint32_t woff = 0, slot = team;                    // slots >= 2; four with four teams
         uint32_t items = 0, known = 0;                     // items so far and the stages they have
-        LC(const long long c0 = clock64();)
         for (uint32_t i = 0;; ++i) {
+            const uint32_t g = team + TEAMS * i;
             bool more = true;
-            while (more && team + 2 * i >= known) {
+            while (more && g >= known) {
                 uint4 tile;
                 uint32_t nb;
                 more = next_item(items++, tile, nb, 0);
@@ -189,31 +196,47 @@ __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P)
             }
             if (!more) break;
             if (!code_ready && !mbar_wait_bounded_at(b_raw, (i >> 1) & 1u, &s_abort)) { give_up(ST_WAIT_FULL); break; }
-            uint32_t v[2][16];
-            dec.decode(raw, woff, v);
             // this slot's last MMAs are stage d = g - slots
-            const uint32_t d = team + 2 * i - slots, b_done = bar0 + 8 * LN_DONE + 8 * (d % LN_DONE), ph_done = (d / LN_DONE) & 1u;
-            const bool slot_ready = team + 2 * i < slots || mbar_try_wait_at(b_done, ph_done);
+            const uint32_t d = g - slots, b_done = bar0 + 8 * LN_DONE + 8 * (d % LN_DONE), ph_done = (d / LN_DONE) & 1u;
+            uint32_t v[2][16];
+            dec.decode(raw, woff, 0, v);
+            const bool slot_ready = g < slots || mbar_try_wait_at(b_done, ph_done);
             b_raw ^= x_raw;
-            code_ready = mbar_try_wait_at(b_raw, ((i + 1) >> 1) & 1u);
-            __syncwarp();
-            if (lane == 0) mbar_arrive_at(b_emp);
+            if (TEAMS == 2) {
+                code_ready = mbar_try_wait_at(b_raw, ((i + 1) >> 1) & 1u);
+                __syncwarp();
+                if (lane == 0) mbar_arrive_at(b_emp);
+            }
             if (!slot_ready && !mbar_wait_bounded_at(b_done, ph_done, &s_abort)) { give_up(ST_WAIT_EMPTY); break; }
             tc_fence_after();
             BK::Decoder::store(ta0 + slot * LN_A_COLS, v);
+            if (TEAMS == 4) {
+                dec.decode(raw, woff, 1, v);
+                code_ready = mbar_try_wait_at(b_raw, ((i + 1) >> 1) & 1u);
+                __syncwarp();
+                if (lane == 0) mbar_arrive_at(b_emp);
+                BK::Decoder::store(ta0 + slot * LN_A_COLS + LN_A_COLS / 2, v);
+            }
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive_at(b_full);
-            b_emp ^= x_emp; b_full ^= x_full; woff ^= 2 * BK::RAW_BYTES;
-            slot = slot + 2 >= slots ? slot + 2 - slots : slot + 2;
+            if (lane == 0) mbar_arrive_at(bar0 + 8 * (g % LN_DONE));
+            b_emp ^= x_emp; woff ^= TEAMS * BK::RAW_BYTES;
+            if (TEAMS == 2) slot = slot + 2 >= slots ? slot + 2 - slots : slot + 2;
         }
-        LC(if (blockIdx.x == 3 && lane == 0 && warp == 13) printf("LANE<%d> decode warp: cycles per stage: %lld\n", NPASS, (clock64() - c0) / (known + 1));)
+    };
+
+    if (warp >= LN_SERVICE && warp < LN_SERVICE + LN_DEC_WARPS) {
+        // ---------------- decode warps ----------------
+        LC(const long long c0 = clock64();)
+        if (teams == 4) decode_stages(std::integral_constant<uint32_t, 4>());
+        else decode_stages(std::integral_constant<uint32_t, 2>());
+        LC(if (blockIdx.x == 3 && lane == 0 && warp == 13) printf("LANE<%d> decode warp: %lld cycles\n", NPASS, clock64() - c0);)
     } else if (warp >= LN_SERVICE + LN_DEC_WARPS) {
         // ---------------- epilogue warps ----------------
         LaneEpi E;
         E.ew = warp - LN_SERVICE - LN_DEC_WARPS; E.q = warp & 3u; E.half = E.ew >> 2; E.lane = lane;
-        E.smem = raw_ring + LN_RAW_STAGES * BK::RAW_BYTES;
+        E.smem = smem_raw + LN_B_STAGES * LN_B_SLOT + 4 * BK::RAW_BYTES;
         E.sync_bar = &epi_bar; E.abort_flag = &s_abort; E.status = P.status; E.sync_ph = 0; E.batch = 0;
         uint32_t pass_n = 0;
         LC(long long t_wait = 0, t_epi = 0;)
@@ -252,8 +275,8 @@ __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P)
                 if (!more) break;
                 const uint8_t* src = P.code + (size_t)te.x * P.expert_stride + (size_t)nb * NPASS * nstage * BK::RAW_BYTES;
                 for (uint32_t ks = 0; ks < NPASS * nstage; ++ks, ++g) {
-                    const uint32_t rs = g % LN_RAW_STAGES;
-                    if (!mbar_wait_bounded(&raw_empty[rs], ((g / LN_RAW_STAGES) & 1u) ^ 1u, &s_abort, 64)) { give_up(ST_WAIT_EMPTY); break; }
+                    const uint32_t rs = g & (raw_stages - 1u);
+                    if (!mbar_wait_bounded(&raw_empty[rs], ((g >> (teams == 4 ? 3 : 2)) & 1u) ^ 1u, &s_abort, 64)) { give_up(ST_WAIT_EMPTY); break; }
                     mbar_expect_tx(&raw_full[rs], BK::RAW_BYTES);
                     BK::template copy_stage<NPASS>(raw_ring + rs * BK::RAW_BYTES, src, ks, nstage, &raw_full[rs]);
                 }
@@ -266,7 +289,7 @@ __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P)
         // everything a stage needs is worked out before the stage before it is issued.
         uint32_t pass_n = 0;
         const uint64_t bdesc = umma_smem_desc(smem_u32(b_ring), LN_LBO, LN_SBO);
-        const uint32_t bd_hi = (uint32_t)(bdesc >> 32), bd_lo0 = (uint32_t)bdesc, bd_end = bd_lo0 + LN_B_STAGES * (LN_B_SLOT >> 4);
+        const uint32_t bd_hi = (uint32_t)(bdesc >> 32), bd_lo0 = (uint32_t)bdesc, bd_step = b_slot >> 4, bd_end = bd_lo0 + LN_B_STAGES * bd_step;
         const uint32_t a_end = tmem_a + slots * LN_A_COLS;
         uint32_t bd_lo = bd_lo0, a0 = tmem_a, bars = smem_u32(&bar_stage[0]), par = 0;   // bars: full[g % 4] at + 0, done[g % 4] at + 32
         const uint32_t bars_end = bars + 8 * LN_DONE;
@@ -286,7 +309,7 @@ __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P)
                     tc_fence_after();
                     LC(const long long w2 = clock64();)
                     const uint32_t bars_n = bars + 8 == bars_end ? bars_end - 8 * LN_DONE : bars + 8, par_n = bars + 8 == bars_end ? par ^ 1u : par;
-                    const uint32_t bd_n = bd_lo + (LN_B_SLOT >> 4) == bd_end ? bd_lo0 : bd_lo + (LN_B_SLOT >> 4);
+                    const uint32_t bd_n = bd_lo + bd_step == bd_end ? bd_lo0 : bd_lo + bd_step;
                     if (elect_one()) {
                         umma_f16_ts_lohi(acc, a0, bd_lo, bd_hi, idesc, ks);
 #pragma unroll
@@ -318,7 +341,7 @@ __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P)
                             if (!mbar_wait_bounded(&done[d % LN_DONE], (d / LN_DONE) & 1u, &s_abort, 64)) { give_up(ST_WAIT_EMPTY); break; }
                         }
                         mbar_expect_tx(&full[g % LN_DONE], b_bytes);
-                        bulk_g2s(b_ring + bs * LN_B_SLOT, xsrc + (size_t)ks * (rows16 * LN_KST), b_bytes, &full[g % LN_DONE]);
+                        bulk_g2s(b_ring + bs * b_slot, xsrc + (size_t)ks * (rows16 * LN_KST), b_bytes, &full[g % LN_DONE]);
                         if (++bs == LN_B_STAGES) bs = 0;
                     }
                 }
@@ -335,7 +358,8 @@ __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P)
 
 template <class BK, int NPASS>
 static cudaError_t lane_launch(const LaneParams& P, int sm_count, cudaStream_t st) {
-    const size_t smem = (size_t)LN_B_STAGES * LN_B_SLOT + (size_t)LN_RAW_STAGES * BK::RAW_BYTES + BK::EPI_SMEM;
+    const size_t smem = (size_t)LN_B_STAGES * LN_B_SLOT + 4 * (size_t)BK::RAW_BYTES + BK::EPI_SMEM;   // four code stages beside the largest tiles, eight beside tiles of 128 rows
+    static_assert(LN_B_STAGES * (LN_B_SLOT - 128 * LN_KST * 2) >= 4 * BK::RAW_BYTES, "the eight code stages of four teams");
     cudaError_t e = cudaFuncSetAttribute(lane_kernel<BK, NPASS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     lane_kernel<BK, NPASS><<<sm_count, LN_THREADS, smem, st>>>(P);
