@@ -12,10 +12,11 @@
 //     With gate and up accumulated together (2 x 192, one buffer) the K loop stood still for the epilogue, a fifth of an
 //     item's time, and experts of 65 .. 96 rows paid for it most.
 //   * 16 decode warps in teams that take the stages in turn.  A warp decodes half a stage of its 32 columns into 32 registers
-//     and only then waits for its operand slot: the MMAs of the slot's last stage run under the decode.  With four operand
-//     slots there are four teams of four warps, a warp decoding both halves of a stage, else two of eight: the barriers
-//     around a stage are a quarter of the instructions of a warp that decodes one half (EXL3: 60 instructions per 16x16 tile,
-//     43 of them the decode), and the loop is bound by their issue; but a team of four keeps its slot for twice as long.
+//     and only then waits for its operand slot: the MMAs of the slot's last stage run under the decode.  With three or four
+//     operand slots there are four teams of four warps, a warp decoding both halves of a stage, with two slots two teams of
+//     eight (a team of four keeps its slot for twice as long).  The barriers around a stage were a quarter of the instructions
+//     of a warp that decoded one half (EXL3: 60 per 16x16 tile, 43 of them the decode), and their latencies showed where the
+//     decode is short: EXL3 at 2048 tokens 2927 -> 2690 us, at 8192 7660 -> 7355, MXFP4 at 2048 1649 -> 1315, at 3500 1840 -> 1625.
 //     (Decoding in smaller pieces, or with 5 or 6 warps per lane quarter, measured slower or equal.)
 //   * The MMA warp runs its loop with all lanes and issues under elect.sync (see elect_one); one commit per stage frees the
 //     operand slot and the rows' slot.
@@ -120,6 +121,14 @@ struct LanePass {
     }
 };
 
+// shared memory of the two rings: four code stages beside tiles of up to 192 rows, eight where four teams decode
+template <class BK>
+constexpr size_t ln_ring_bytes() {
+    constexpr size_t two = (size_t)LN_B_STAGES * LN_B_SLOT + 4 * BK::RAW_BYTES;
+    constexpr size_t four = (size_t)LN_B_STAGES * 160 * LN_KST * 2 + 8 * BK::RAW_BYTES;
+    return two > four ? two : four;
+}
+
 // NPASS = 2: gate then up of a column block; 1: down
 template <class BK, int NPASS>
 __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P) {
@@ -138,7 +147,7 @@ __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P)
 
     // columns of an accumulator buffer (the call's largest tile), operand slots in what is left
     const uint32_t acc_cols = P.tiles[2] <= 128u ? 128u : P.tiles[2] <= 160u ? 160u : 192u, slots = (512u - 2u * acc_cols) / LN_A_COLS;
-    const uint32_t teams = slots == 4 ? 4u : 2u, raw_stages = 2u * teams, b_slot = acc_cols * (LN_KST * 2u);
+    const uint32_t teams = slots >= 3 ? 4u : 2u, raw_stages = 2u * teams, b_slot = acc_cols * (LN_KST * 2u);
     uint8_t* b_ring = smem_raw;                                          // [stage][rows16 x 256 B]
     uint8_t* raw_ring = b_ring + LN_B_STAGES * b_slot;                   // [stage][BK::RAW_BYTES]
     if (threadIdx.x == 0) {
@@ -183,7 +192,7 @@ __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P)
         uint32_t b_raw = smem_u32(&raw_full[team]), b_emp = smem_u32(&raw_empty[team]);
         const uint32_t x_raw = b_raw ^ smem_u32(&raw_full[team + TEAMS]), x_emp = b_emp ^ smem_u32(&raw_empty[team + TEAMS]);
         bool code_ready = false;
-        uint32_t woff = 0, slot = team;                    // slots >= 2; four with four teams
+        uint32_t woff = 0, slot = team % slots;            // of stage g: g % slots
         uint32_t items = 0, known = 0;                     // items so far and the stages they have
         for (uint32_t i = 0;; ++i) {
             const uint32_t g = team + TEAMS * i;
@@ -222,7 +231,7 @@ __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P)
             __syncwarp();
             if (lane == 0) mbar_arrive_at(bar0 + 8 * (g % LN_DONE));
             b_emp ^= x_emp; woff ^= TEAMS * BK::RAW_BYTES;
-            if (TEAMS == 2) slot = slot + 2 >= slots ? slot + 2 - slots : slot + 2;
+            if (TEAMS == 4 && slots == 3) slot = slot == 2 ? 0u : slot + 1;   // else the slot stays the team's
         }
     };
 
@@ -236,7 +245,7 @@ __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P)
         // ---------------- epilogue warps ----------------
         LaneEpi E;
         E.ew = warp - LN_SERVICE - LN_DEC_WARPS; E.q = warp & 3u; E.half = E.ew >> 2; E.lane = lane;
-        E.smem = smem_raw + LN_B_STAGES * LN_B_SLOT + 4 * BK::RAW_BYTES;
+        E.smem = smem_raw + ln_ring_bytes<BK>();
         E.sync_bar = &epi_bar; E.abort_flag = &s_abort; E.status = P.status; E.sync_ph = 0; E.batch = 0;
         uint32_t pass_n = 0;
         LC(long long t_wait = 0, t_epi = 0;)
@@ -358,8 +367,7 @@ __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P)
 
 template <class BK, int NPASS>
 static cudaError_t lane_launch(const LaneParams& P, int sm_count, cudaStream_t st) {
-    const size_t smem = (size_t)LN_B_STAGES * LN_B_SLOT + 4 * (size_t)BK::RAW_BYTES + BK::EPI_SMEM;   // four code stages beside the largest tiles, eight beside tiles of 128 rows
-    static_assert(LN_B_STAGES * (LN_B_SLOT - 128 * LN_KST * 2) >= 4 * BK::RAW_BYTES, "the eight code stages of four teams");
+    const size_t smem = ln_ring_bytes<BK>() + BK::EPI_SMEM;
     cudaError_t e = cudaFuncSetAttribute(lane_kernel<BK, NPASS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     lane_kernel<BK, NPASS><<<sm_count, LN_THREADS, smem, st>>>(P);
