@@ -17,6 +17,7 @@
 // the lane that accumulated gate and up together.
 #include <cstdlib>
 
+#include "dispatch_body.cuh"
 #include "lane.cuh"
 
 namespace mlxs {
@@ -30,50 +31,39 @@ namespace mlxs {
 // first sorted row, rows, first staging row}: list 0 from entry 0, list 1 from entry max_tiles.  An expert's rows are
 // split evenly over its tiles (a 16-row remainder tile would cost a full decode).
 // Staging rows: a tile's rows padded to 16, tiles in sorted order, so tile number n starts at its first row + 16 n.
-__global__ void pf_plan_kernel(DispatchTables t, uint32_t E, const uint8_t* __restrict__ flags, uint32_t min_rows,
-                               uint32_t cap0, uint32_t cap1, uint32_t max_tiles, uint32_t* __restrict__ tiles,
-                               uint32_t* status) {
-    __shared__ uint32_t base0[1025], base1[1025];
-    const uint32_t tid = threadIdx.x;
-    // tiles per expert in parallel (base0 / base1 hold the counts first), then one thread turns them into offsets
-    for (uint32_t e = tid; e < E; e += blockDim.x) {
-        const uint32_t c = t.offsets[e + 1] - t.offsets[e];
-        const bool lane = takes_tensor_lane(c, min_rows, flags, e), list1 = cap1 && c > cap0;
-        base0[e] = lane && !list1 ? (c + cap0 - 1) / cap0 : 0u;
-        base1[e] = lane && list1 ? (c + cap1 - 1) / cap1 : 0u;
-    }
+// narrow: with tiles of up to that many rows the lane has another operand slot (lane.cuh), worth about as much as a
+// twentieth of the tiles: taken when the call gets at most one tile in sixteen more.  (300 Zipf-routed tokens, one expert
+// above 160 rows: 690 -> 665 us; 4500 tokens, one expert in 23 above: even; 6000 tokens, nearly all above: 5.5 -> 6.5 ms if
+// it were taken there.)
+// One thread per expert; with one thread adding up the tile counts the kernel took 8 us for 256 experts.
+__global__ void __launch_bounds__(DTHREADS) pf_plan_kernel(DispatchTables t, uint32_t E, const uint8_t* __restrict__ flags, uint32_t min_rows,
+                                                           uint32_t cap0, uint32_t cap1, uint32_t narrow, uint32_t max_tiles,
+                                                           uint32_t* __restrict__ tiles, uint32_t* status) {
+    __shared__ uint32_t ws[99], s_most;
+    const uint32_t e = threadIdx.x;
+    if (e == 0) s_most = 0;
+    const uint32_t r0 = e < E ? t.offsets[e] : 0u, c = e < E ? t.offsets[e + 1] - r0 : 0u;
+    const bool lane = e < E && takes_tensor_lane(c, min_rows, flags, e), list1 = cap1 && c > cap0;
+    const uint32_t v[3] = {lane && !list1 ? (c + cap0 - 1) / cap0 : 0u, lane && list1 ? (c + cap1 - 1) / cap1 : 0u,
+                           lane && narrow ? (c + narrow - 1) / narrow : 0u};
+    uint32_t base[3], tot[3];
+    block_scan3(v, base, tot, ws);
+    const int k = narrow && tot[2] * 16u <= tot[0] * 17u ? 2 : 0;   // the scan that list 0 goes by
+    const bool ok = tot[k] <= max_tiles && tot[1] <= max_tiles;
+    const uint32_t nt = list1 ? v[1] : v[k], first = list1 ? base[1] : base[k], ordinal = base[k] + base[1];
+    const uint32_t per = nt ? ((c + nt - 1) / nt + 15) / 16 * 16 : 0u;
+    if (!list1 && nt) atomicMax(&s_most, per);
+    if (ok)
+        for (uint32_t i = 0; i < nt; ++i)
+            *reinterpret_cast<uint4*>(prefill_tile(tiles, list1 ? 1 : 0, max_tiles, first + i)) =
+                make_uint4(e, r0 + i * per, min(per, c - i * per), r0 + i * per + 16 * (ordinal + i));
     __syncthreads();
-    if (tid == 0) {
-        uint32_t n0 = 0, n1 = 0;
-        for (uint32_t e = 0; e < E; ++e) {
-            const uint32_t c0 = base0[e], c1 = base1[e];
-            base0[e] = n0;
-            base1[e] = n1;
-            n0 += c0;
-            n1 += c1;
-        }
-        if (n0 > max_tiles || n1 > max_tiles) { atomicMax(status, (uint32_t)ST_WORKLIST_OVERFLOW); n0 = 0; n1 = 0; }
-        base0[E] = n0;
-        base1[E] = n1;
-        tiles[0] = n0;
-        tiles[1] = n1;
-        tiles[2] = tiles[3] = tiles[4] = 0;
-    }
-    __syncthreads();
-    if (base0[E] + base1[E] == 0) return;
-    for (uint32_t e = tid; e < E; e += blockDim.x) {
-        const uint32_t c = t.offsets[e + 1] - t.offsets[e], r0 = t.offsets[e];
-        if (!takes_tensor_lane(c, min_rows, flags, e)) continue;
-        const bool list1 = cap1 && c > cap0;
-        const uint32_t cap = list1 ? cap1 : cap0;
-        const uint32_t nt = (c + cap - 1) / cap;
-        const uint32_t per = ((c + nt - 1) / nt + 15) / 16 * 16;
-        if (!list1) atomicMax(&tiles[2], per);
-        const uint32_t first = list1 ? base1[e] : base0[e], ordinal = base0[e] + base1[e];
-        for (uint32_t i = 0; i < nt; ++i) {
-            uint32_t* d = prefill_tile(tiles, list1 ? 1 : 0, max_tiles, first + i);
-            d[0] = e; d[1] = r0 + i * per; d[2] = min(per, c - i * per); d[3] = r0 + i * per + 16 * (ordinal + i);
-        }
+    if (e == 0) {
+        if (!ok) atomicMax(status, (uint32_t)ST_WORKLIST_OVERFLOW);
+        tiles[0] = ok ? tot[k] : 0u;
+        tiles[1] = ok ? tot[1] : 0u;
+        tiles[2] = s_most;
+        tiles[3] = tiles[4] = 0;
     }
 }
 
@@ -378,9 +368,10 @@ bool exl3_prefill_supported(Exl3Dims d) { return d.I % LN_KST == 0 && d.H % LN_K
 size_t lane_act_bytes(int sm_count) { return (size_t)sm_count * LN_ACT_BYTES; }
 
 cudaError_t launch_prefill_plan(DispatchTables t, uint32_t n_experts, const uint8_t* lane_flags, uint32_t min_rows,
-                                uint32_t cap0, uint32_t cap1, uint32_t max_tiles, uint32_t* tiles, uint32_t* status,
-                                cudaStream_t st) {
-    pf_plan_kernel<<<1, 256, 0, st>>>(t, n_experts, lane_flags, min_rows, cap0, cap1, max_tiles, tiles, status);
+                                uint32_t cap0, uint32_t cap1, uint32_t narrow, uint32_t max_tiles, uint32_t* tiles,
+                                uint32_t* status, cudaStream_t st) {
+    if (n_experts > (uint32_t)DTHREADS) return cudaErrorInvalidValue;
+    pf_plan_kernel<<<1, DTHREADS, 0, st>>>(t, n_experts, lane_flags, min_rows, cap0, cap1, narrow, max_tiles, tiles, status);
     return cudaGetLastError();
 }
 
@@ -401,7 +392,7 @@ static cudaError_t pf_launch_all(const Exl3PrefillArgs& a, cudaStream_t st) {
 }
 
 cudaError_t launch_exl3_prefill(const Exl3PrefillArgs& a, cudaStream_t st) {
-    cudaError_t e = launch_prefill_plan(a.t, a.n_experts, nullptr, a.min_rows, LN_ROWS, 0, a.max_tiles, a.tiles, a.status, st);
+    cudaError_t e = launch_prefill_plan(a.t, a.n_experts, nullptr, a.min_rows, LN_ROWS, 0, LN_ROWS_NARROW, a.max_tiles, a.tiles, a.status, st);
     if (e != cudaSuccess) return e;
     pf_prep_kernel<<<dim3(a.max_tiles, 8), PREP_WARPS * 32, 0, st>>>(a.x, a.top_k, a.d.H, a.L.scales, exl3_scales_per_expert(a.d), a.t,
                                                                      a.tiles, a.max_tiles,

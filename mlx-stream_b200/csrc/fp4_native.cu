@@ -460,7 +460,7 @@ static cudaError_t nf_launch(NfParams P, int sm_count, cudaStream_t st) {
 }
 
 cudaError_t launch_mxfp4_native(const Fp4PrefillArgs& a, cudaStream_t st) {
-    cudaError_t e = launch_prefill_plan(a.t, a.n_experts, a.lane_flags, a.min_rows, NF_CAP0, NF_CAP1, a.max_tiles, a.tiles, a.status, st);
+    cudaError_t e = launch_prefill_plan(a.t, a.n_experts, a.lane_flags, a.min_rows, NF_CAP0, NF_CAP1, 0, a.max_tiles, a.tiles, a.status, st);
     if (e != cudaSuccess) return e;
     uint8_t* xa = reinterpret_cast<uint8_t*>(a.xa);
     uint8_t* xd = reinterpret_cast<uint8_t*>(a.xd);

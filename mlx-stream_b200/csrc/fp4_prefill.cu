@@ -256,7 +256,7 @@ static cudaError_t q_launch_all(const Fp4PrefillArgs& a, cudaStream_t st) {
 }
 
 cudaError_t launch_fp4_prefill(const Fp4PrefillArgs& a, cudaStream_t st) {
-    const cudaError_t e = launch_prefill_plan(a.t, a.n_experts, a.lane_flags, a.min_rows, LN_ROWS, 0, a.max_tiles, a.tiles, a.status, st);
+    const cudaError_t e = launch_prefill_plan(a.t, a.n_experts, a.lane_flags, a.min_rows, LN_ROWS, 0, LN_ROWS_NARROW, a.max_tiles, a.tiles, a.status, st);
     if (e != cudaSuccess) return e;
     return a.nv ? q_launch_all<true>(a, st) : q_launch_all<false>(a, st);
 }

@@ -155,8 +155,8 @@ __host__ __device__ inline const uint32_t* prefill_tile(const uint32_t* tiles, i
     return tiles + 8 + 4 * ((size_t)(list ? max_tiles : 0) + i);
 }
 cudaError_t launch_prefill_plan(DispatchTables t, uint32_t n_experts, const uint8_t* lane_flags, uint32_t min_rows,
-                                uint32_t cap0, uint32_t cap1, uint32_t max_tiles, uint32_t* tiles, uint32_t* status,
-                                cudaStream_t st);
+                                uint32_t cap0, uint32_t cap1, uint32_t narrow, uint32_t max_tiles, uint32_t* tiles,
+                                uint32_t* status, cudaStream_t st);
 struct Exl3PrefillArgs {
     Exl3Layer L;
     Exl3Dims d;

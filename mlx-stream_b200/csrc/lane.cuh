@@ -46,6 +46,7 @@ namespace mlxs {
 constexpr int LN_KST = 128;             // inputs per stage
 constexpr int LN_A_COLS = LN_KST / 2;   // tensor-memory columns of a decoded stage
 constexpr int LN_ROWS = 192;            // most rows of a tile
+constexpr int LN_ROWS_NARROW = 160;     // most rows that leave room for three operand slots
 constexpr int LN_RAW_STAGES = 8;        // most stages of the code ring: two per team
 constexpr int LN_B_STAGES = 3;          // stages of the rows' ring
 // Items announced to the roles.  An entry is written again LN_ITEMS items later: the code ring, the operand slots and the two
@@ -125,7 +126,7 @@ struct LanePass {
 template <class BK>
 constexpr size_t ln_ring_bytes() {
     constexpr size_t two = (size_t)LN_B_STAGES * LN_B_SLOT + 4 * BK::RAW_BYTES;
-    constexpr size_t four = (size_t)LN_B_STAGES * 160 * LN_KST * 2 + 8 * BK::RAW_BYTES;
+    constexpr size_t four = (size_t)LN_B_STAGES * LN_ROWS_NARROW * LN_KST * 2 + 8 * BK::RAW_BYTES;
     return two > four ? two : four;
 }
 
@@ -146,7 +147,7 @@ __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P)
     if (blockIdx.x >= n_items) return;
 
     // columns of an accumulator buffer (the call's largest tile), operand slots in what is left
-    const uint32_t acc_cols = P.tiles[2] <= 128u ? 128u : P.tiles[2] <= 160u ? 160u : 192u, slots = (512u - 2u * acc_cols) / LN_A_COLS;
+    const uint32_t acc_cols = P.tiles[2] <= 128u ? 128u : P.tiles[2] <= (uint32_t)LN_ROWS_NARROW ? (uint32_t)LN_ROWS_NARROW : (uint32_t)LN_ROWS, slots = (512u - 2u * acc_cols) / LN_A_COLS;
     const uint32_t teams = slots >= 3 ? 4u : 2u, raw_stages = 2u * teams, b_slot = acc_cols * (LN_KST * 2u);
     uint8_t* b_ring = smem_raw;                                          // [stage][rows16 x 256 B]
     uint8_t* raw_ring = b_ring + LN_B_STAGES * b_slot;                   // [stage][BK::RAW_BYTES]

@@ -9,22 +9,23 @@ from test_parity_shapes_gpu import _shared_ref
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("rows", [(12, 13, 16, 17), (31, 32, 33, 1), (96, 97, 128, 129), (160, 161, 192, 193), (256, 257, 384, 385)])
+@pytest.mark.parametrize("rows", [(12, 13, 16, 17), (31, 32, 33, 1), (96, 97, 128, 129), (160, 161, 192, 193), (256, 257, 384, 385),
+                                  (161,) + (17,) * 16])   # the last: one tile in sixteen more lets all tiles be narrow
 @pytest.mark.parametrize("cls,limit", [(Exl3Case, 10.0), (Exl3K2Case, 10.0), (Mxfp4Case, 0.0), (Nvfp4Case, 10.0)])
 def test_rows_of_an_expert_around_the_lanes_tiles(cls, limit, rows):
     """Row counts on both sides of the lane choice and of the tensor-core lane's row tiles, three weight blocks of 128 wide
     (an odd count: the last pass of the pair is short)."""
     fp4 = cls in (Mxfp4Case, Nvfp4Case)
-    case = cls(768, 384, 4, 1, seed=21, shared=False, scoring=O.SCORE_SIGMOID, max_tokens=1300, routed_scale=1.0, limit=limit,
+    case = cls(768, 384, len(rows), 1, seed=21, shared=False, scoring=O.SCORE_SIGMOID, max_tokens=1300, routed_scale=1.0, limit=limit,
                chain=fp4)
     try:
-        ids = np.random.default_rng(rows[0]).permutation(np.repeat(np.arange(4), rows)).astype(np.int32)[:, None]
+        ids = np.random.default_rng(rows[0]).permutation(np.repeat(np.arange(len(rows)), rows)).astype(np.int32)[:, None]
         x, _ = case.inputs(ids.size, seed=40)
         w = np.full(ids.shape, 0.75, np.float32)
         y = case.gpu_experts(x, ids, w)
         assert case.status() == 0
         ref = case.cpu_layer(x, ids, w)
-        for e in range(4):   # every expert by itself: one wrong tile is not averaged away
+        for e in range(len(rows)):   # every expert by itself: one wrong tile is not averaged away
             m = ids[:, 0] == e
             assert rel_l2(y[m], ref[m]) < 1e-2, (e, rows[e])
     finally:
