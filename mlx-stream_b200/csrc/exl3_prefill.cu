@@ -131,9 +131,12 @@ __device__ __forceinline__ void pf_load_scale4(const __half* p, uint32_t lane, f
 }
 
 // xa: [projection][staging rows][H] (a tile's rows start at its first staging row, padded to 16).  A warp stages eight
-// rows of one 128-block: lane = (row, s), with the 32 inputs 32 j + 8 s + i (j < 4, i < 8).  Five of the transform's seven
-// levels then stay in registers and two are shuffles (64 per eight rows; with four inputs per lane it was 160), four lanes
-// read 64 contiguous bytes of a row, and the 16-byte stores fill whole lines of core matrices.
+// rows of one 128-block: lane = (row, s), with the 32 inputs 32 j + 8 s + i (j < 4, i < 8).  The levels of i and j stay in
+// registers.  For a level of s the two lanes swap half their registers: each then has both sides of 16 butterflies, and the
+// lane bit has become a bit of i, whose level is done.  The kernel is bound by the L1's data path, which the shuffles share:
+// 32 of them per row group and projection (one per input and level, with a last exchange before the stores, was 72).
+// After both levels a lane holds exactly the four consecutive positions of pf_lane_off in every 16-block: with c = lane % 4,
+// {2 c', 2 c' + 1, 2 c' + 8, 2 c' + 9}, c' = c with its two bits swapped; the 8-byte stores of a warp fill whole lines.
 constexpr int PREP_WARPS = 8;
 __global__ void __launch_bounds__(PREP_WARPS * 32, 3) pf_prep_kernel(const __nv_bfloat16* __restrict__ x, uint32_t top_k, uint32_t H,
                                                                   const __half* __restrict__ scales, size_t scales_stride,
@@ -146,7 +149,9 @@ __global__ void __launch_bounds__(PREP_WARPS * 32, 3) pf_prep_kernel(const __nv_
     const uint32_t rows16 = (rows + 15) / 16 * 16, warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, nblk = H / 128;
     const uint32_t r8 = lane >> 2, seg = lane & 3u;
     const float S = __uint_as_float(SCALE_BITS);
-    const float sg0 = seg & 1u ? -1.0f : 1.0f, sg1 = seg & 2u ? -1.0f : 1.0f;
+    const bool odd = seg & 1u, high = seg & 2u;
+    // a difference comes out negated in the lane that kept the second halves: made good in the last scaling
+    const float S0 = odd ? -S : S, S1 = high ? -S : S, S01 = odd != high ? -S : S;
     const __half* sc_e = scales + (size_t)e * scales_stride + seg * 8;
     for (uint32_t task = blockIdx.y * PREP_WARPS + warp; task < nblk * (rows16 / 8); task += gridDim.y * PREP_WARPS) {
         const uint32_t b = task % nblk, r = task / nblk * 8 + r8;
@@ -184,23 +189,28 @@ __global__ void __launch_bounds__(PREP_WARPS * 32, 3) pf_prep_kernel(const __nv_
                     }
             };
             level_reg(1); level_reg(2); level_reg(4);
+            auto level_swap = [&](int m, bool second, int lane_mask) {
 #pragma unroll
-            for (int k = 0; k < 32; ++k) v[k] = __fmaf_rn(sg0, v[k], __shfl_xor_sync(0xFFFFFFFFu, v[k], 1));
-#pragma unroll
-            for (int k = 0; k < 32; ++k) v[k] = __fmaf_rn(sg1, v[k], __shfl_xor_sync(0xFFFFFFFFu, v[k], 2));
+                for (int k = 0; k < 32; ++k)
+                    if (!(k & m)) {
+                        const float keep = second ? v[k | m] : v[k], got = __shfl_xor_sync(0xFFFFFFFFu, second ? v[k] : v[k | m], lane_mask);
+                        v[k] = keep + got;
+                        v[k | m] = keep - got;
+                    }
+            };
+            level_swap(4, odd, 1);
+            level_swap(2, high, 2);
             level_reg(8); level_reg(16);
 #pragma unroll
-            for (int k = 0; k < 32; ++k) v[k] *= S;
+            for (int k = 0; k < 32; ++k) v[k] *= (k & 6) == 6 ? S01 : (k & 4) ? S0 : (k & 2) ? S1 : S;
             // src/kernels/exl3/dsv41_prefill_dig_take2v_5120.metal:57-58: the rotated input is rounded to f16
-            __half* dst = xa + p * proj_stride + (size_t)te[3] * H + (size_t)b * (rows16 * LN_KST) + (r >> 3) * 1024u + (r & 7u) * 8u;
-            // 16-block 2 j + s / 2: an even lane holds its inputs 0 .. 7, the odd one 8 .. 15; the block's first core matrix
-            // takes {0, 1, 8, 9, 2, 3, 10, 11}, its second the others, so the two lanes swap half of theirs
+            const uint32_t c = (seg & 1u) * 2u + (seg >> 1);
+            __half* dst = xa + p * proj_stride + (size_t)te[3] * H + (size_t)b * (rows16 * LN_KST) + ln_row_off(r, c >> 1) + (c & 1u) * 4u;
+            // registers 8 j + 4 (bit 3 of the input) + 2 (bit 4) + bit 0
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const uint2 a = pf_pack4(v[8 * j], v[8 * j + 1], v[8 * j + 2], v[8 * j + 3]), c = pf_pack4(v[8 * j + 4], v[8 * j + 5], v[8 * j + 6], v[8 * j + 7]);
-                const bool odd = seg & 1u;
-                const uint32_t g0 = __shfl_xor_sync(0xFFFFFFFFu, odd ? a.x : c.x, 1), g1 = __shfl_xor_sync(0xFFFFFFFFu, odd ? a.y : c.y, 1);
-                *reinterpret_cast<uint4*>(dst + (4 * j + seg) * 64) = odd ? make_uint4(g0, c.x, g1, c.y) : make_uint4(a.x, g0, a.y, g1);
+            for (int t16 = 0; t16 < 8; ++t16) {
+                const int k = (t16 >> 1) * 8 + (t16 & 1) * 2;
+                *reinterpret_cast<uint2*>(dst + t16 * 128) = pf_pack4(v[k], v[k + 1], v[k + 4], v[k + 5]);
             }
         }
     }
