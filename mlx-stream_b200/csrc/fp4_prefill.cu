@@ -45,19 +45,26 @@ __global__ void __launch_bounds__(256) q_prep_kernel(const __nv_bfloat16* __rest
         const uint32_t r = rg * 8 + r8;
         const bool valid = r < rows;
         const __nv_bfloat16* src = x + (valid ? (size_t)x_row_of(t, t.order[row0 + r], top_k) * H : 0);
-        for (uint32_t g = blockIdx.y * 4 + c; g < H / 8; g += gridDim.y * 4) {   // group of 8 inputs
-            uint4 raw = make_uint4(0, 0, 0, 0);
-            if (valid) raw = *reinterpret_cast<const uint4*>(src + (size_t)g * 8);
-            if (NV) {
-                uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+        const uint32_t step = gridDim.y * 4;
+        for (uint32_t g0 = blockIdx.y * 4 + c; g0 < H / 8; g0 += 4 * step) {   // groups of 8 inputs, four loads in flight
+            uint4 raw[4];
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const __half2 h = __floats2half2_rn(__uint_as_float(w[k] << 16), __uint_as_float(w[k] & 0xFFFF0000u));
-                    w[k] = *reinterpret_cast<const uint32_t*>(&h);
+            for (int i = 0; i < 4; ++i) raw[i] = valid && g0 + i * step < H / 8 ? *reinterpret_cast<const uint4*>(src + (size_t)(g0 + i * step) * 8) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint32_t g = g0 + i * step;
+                if (g >= H / 8) break;
+                if (NV) {
+                    uint32_t w[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const __half2 h = __floats2half2_rn(__uint_as_float(w[k] << 16), __uint_as_float(w[k] & 0xFFFF0000u));
+                        w[k] = *reinterpret_cast<const uint32_t*>(&h);
+                    }
+                    raw[i] = make_uint4(w[0], w[1], w[2], w[3]);
                 }
-                raw = make_uint4(w[0], w[1], w[2], w[3]);
+                *reinterpret_cast<uint4*>(dst + (size_t)(g / 16) * (rows16 * LN_KST) + ln_row_off(r, g % 16)) = q_order8<NV>(raw[i]);
             }
-            *reinterpret_cast<uint4*>(dst + (size_t)(g / 16) * (rows16 * LN_KST) + ln_row_off(r, g % 16)) = q_order8<NV>(raw);
         }
     }
 }
