@@ -11,9 +11,9 @@
 //   * the epilogue: transpose through shared memory, then row-wise Hadamard-128, svh, clamped SwiGLU, suh_d, Hadamard for
 //     gate / up (act(gate) waits in an L2-resident scratch between the two passes, read back by the threads that wrote it);
 //     Hadamard, svh_d for down.
-// What bounds it (61 -> 58 warp instructions per decoded tile, 43 of them the decode): up to about 128 rows per tile the
+// What bounds it (about 55 warp instructions per decoded tile, 43 of them the decode): up to about 128 rows per tile the
 // decode's instruction issue, above that the MMAs; calls of thousands of tokens run into the 1 kW power cap (1.55 GHz at
-// 8192 tokens).  Layer of H 5120, I 2304, 256 experts: 2048 tokens 4.05 -> 3.27 ms, 8192 tokens 10.64 -> 8.11 ms against
+// 8192 tokens).  Layer of H 5120, I 2304, 256 experts: 2048 tokens 4.06 -> 3.02 ms, 8192 tokens 10.6 -> 7.7 ms against
 // the lane that accumulated gate and up together.
 #include <cstdlib>
 
