@@ -19,7 +19,8 @@ constexpr int SH_AHEAD = 2;  // weight chunks in flight per warp
 
 // MODE 0: gate/up + activation -> h bf16 [T, N]; 1: down -> out f32 [T, N].  NT = token tiles of 8 per pass: a call of few
 // tokens takes the form that holds registers and reduction space for its own tiles only, so that its CTAs fit beside the
-// routed kernels' (gate/up at one token 35 -> 27 us).
+// routed kernels' (gate/up at one token 35 -> 27 us; four tiles for 17 .. 32 tokens: the layer of 20 NVFP4 tokens 528 -> 511,
+// four EXL3 layers of 32 tokens 1813 -> 1787).
 template <int MODE, int NT>
 __global__ void __launch_bounds__(sh_warps(MODE) * 32) shared_kernel(const __nv_bfloat16* __restrict__ x, uint32_t T,
                                                                uint32_t Kdim, uint32_t N,
@@ -145,9 +146,9 @@ static cudaError_t shared_launch(const __nv_bfloat16* x, const __nv_bfloat16* w1
     cudaError_t e = cudaFuncSetAttribute(shared_kernel<0, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem0);
     if (e != cudaSuccess) return e;
     // The routed kernels beside it take all of an SM's shared memory: an SM that had to change its split would drain first.
-    // (Not from 17 tokens on: the rows of eight token tiles then miss the L1, 27 -> 41 us at 64 tokens.)
-    if (NT < 8 && (e = cudaFuncSetAttribute(shared_kernel<0, NT>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared)) != cudaSuccess) return e;
-    if (NT < 8 && (e = cudaFuncSetAttribute(shared_kernel<1, NT>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared)) != cudaSuccess) return e;
+    // (Not from 17 tokens on: the rows then miss the L1, 27 -> 41 us at 64 tokens, four layers of 32 tokens 1787 -> 1804.)
+    if (NT < 4 && (e = cudaFuncSetAttribute(shared_kernel<0, NT>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared)) != cudaSuccess) return e;
+    if (NT < 4 && (e = cudaFuncSetAttribute(shared_kernel<1, NT>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared)) != cudaSuccess) return e;
     shared_kernel<0, NT><<<I / 16, sh_warps(0) * 32, smem0, st>>>(x, T, H, I, w1, w3, limit, h_ws, nullptr);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     shared_kernel<1, NT><<<H / 16, sh_warps(1) * 32, smem1, st>>>(h_ws, T, I, H, w2, nullptr, 0.f, nullptr, out);
@@ -160,6 +161,7 @@ cudaError_t launch_shared_expert(const __nv_bfloat16* x, const __nv_bfloat16* w1
     if (T == 0) return cudaSuccess;
     if (T <= 8) return shared_launch<1>(x, w1, w3, w2, T, H, I, limit, h_ws, out, st);
     if (T <= 16) return shared_launch<2>(x, w1, w3, w2, T, H, I, limit, h_ws, out, st);
+    if (T <= 32) return shared_launch<4>(x, w1, w3, w2, T, H, I, limit, h_ws, out, st);
     return shared_launch<8>(x, w1, w3, w2, T, H, I, limit, h_ws, out, st);
 }
 

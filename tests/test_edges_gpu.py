@@ -56,9 +56,10 @@ def test_router_logits_around_the_change_of_kernel(E):
 
 @pytest.mark.parametrize("H,I", [(512, 256), (1280, 768)])
 def test_shared_expert_products_of_every_cluster_size(H, I):
+    """The skinny kernel's token tiles, then the tensor-core products' tiles and clusters."""
     case = Exl3Case(H, I, 2, 1, seed=11, shared=True, max_tokens=1030)
     try:
-        for T in (65, 96, 97, 129, 192, 193, 257, 1025):
+        for T in (16, 17, 32, 33, 65, 96, 97, 129, 192, 193, 257, 1025):
             x, _ = case.inputs(T, seed=T)
             y = case.gpu_experts(x, np.zeros((T, 1), np.int32), np.zeros((T, 1), np.float32))
             assert case.status() == 0
