@@ -397,7 +397,9 @@ static uint32_t shared_dense_min() {
 static int dense_workspace(mlxs_moe* h) {
     int rc;
     const size_t T16 = ((size_t)h->cfg.max_tokens + 15) / 16 * 16;
-    if (!h->dg_xb && (rc = h->alloc(&h->dg_xb, T16 * h->cfg.hidden * 2))) return rc;
+    if (h->dg_xb) return 0;
+    CU(dense_caps(h->sm_count, &h->dg_caps));
+    if ((rc = h->alloc(&h->dg_xb, T16 * h->cfg.hidden * 2))) return rc;
     return 0;
 }
 
@@ -588,10 +590,10 @@ static int logits_impl(mlxs_moe* h, uint32_t layer, const void* x_dev, uint32_t 
     cudaStream_t st = (cudaStream_t)stream;
     StageTimer tm(h, MLXS_STAGE_ROUTER, st);
     if (T > LOGITS_DENSE_FROM && L.router_w_t) {
-        const uint32_t nt = dense_logits_rows(T, c.n_experts, c.hidden, h->sm_count);
+        const uint32_t nt = dense_logits_rows(T, c.n_experts, c.hidden, h->sm_count, h->dg_caps);
         *staged_nt = nt;
         CU(launch_dense_logits(static_cast<const __nv_bfloat16*>(x_dev), L.router_w_t, T, c.n_experts, c.hidden, nt, h->dg_xb, logits_dev,
-                               h->status, h->sm_count, st));
+                               h->status, h->sm_count, h->dg_caps, st));
     } else {
         CU(launch_router_logits(static_cast<const __nv_bfloat16*>(x_dev), L.router_w, T, c.n_experts, c.hidden, logits_dev, st));
     }
@@ -788,7 +790,8 @@ static int experts_impl(mlxs_moe* h, uint32_t layer, const void* x_dev, const in
             da.x = static_cast<const __nv_bfloat16*>(x_dev); da.w_gu = L.sh_gu_t; da.w_d = L.sh_d_t;
             da.T = T; da.H = c.hidden; da.I = c.inter; da.limit = lim; da.xb = h->dg_xb; da.hb = h->dg_hb; da.out = h->sh_out;
             da.status = h->status; da.sm_count = h->sm_count;
-            da.nt = dense_shared_rows(T, c.hidden, c.inter, h->sm_count);
+            da.nt = dense_shared_rows(T, c.hidden, c.inter, h->sm_count, h->dg_caps);
+            da.caps = &h->dg_caps;
             da.rows_staged = h->dg_staged_nt == da.nt;
             CU(launch_dense_shared_expert(da, s));
         } else {

@@ -14,10 +14,13 @@
 //     or two adjacent blocks of a single projection): 2 x 256 columns = all 512;
 //   * one producer thread (bulk copies into a ring, mbarriers), one MMA thread (tcgen05.mma.kind::f16 on bf16,
 //     K = 16 per instruction, commits free the stage), eight epilogue warps (tcgen05.ld, activation, stores);
-//   * calls with too few (token tile, feature block) items for the SMs take smaller token tiles and split the reduction
-//     dimension over the CTAs of a cluster (dg_plan): each leaves its f32 partial tile in its own shared memory, and every
-//     CTA folds a slice of the rows over the cluster in part order.  With one CTA folding all parts out of global scratch
-//     the fold was most of the time: gate/up at 300 tokens 90 us for 42 MB of weights.
+//   * calls with few tokens split the reduction into parts (dg_parts): every part is summed by itself and the parts are added
+//     in part order, so a sum's bits depend on the part count alone, which is the same for all calls of up to 256 tokens: a
+//     row's bits do not depend on the batch around it.  How the parts are spread is free (dg_cost): one CTA takes them in turn
+//     with tiles of up to 64 rows, the epilogue warps adding each to their registers under the next part's MMAs; or the CTAs of
+//     a cluster leave their parts' f32 tiles in their own shared memory and every CTA folds a slice of the rows over the
+//     cluster.  With one CTA folding all parts out of global scratch the fold was most of the time: gate/up at 300 tokens
+//     90 us for 42 MB of weights.
 // Every wait is bounded; on a give-up the CTA records the status word, skips its work and still frees tensor memory.
 #include <cstdlib>
 
@@ -29,7 +32,9 @@ namespace mlxs {
 
 constexpr int DG_KS = 64;                         // inputs per stage
 constexpr int DG_NT = 256;                        // most rows per token tile (MMA N)
-constexpr int DG_CL_NT = 192;                     // the same in a cluster: the partial tile has to fit the ring's shared memory
+constexpr int DG_CL_NT = 192;                     // most rows x parts of a CTA in a cluster: the partial tiles have to fit the ring's shared memory
+constexpr int DG_CL_MAX = 8;                      // most CTAs of a cluster
+constexpr int DG_FOLD_NT = 64;                    // most rows of a tile whose parts one CTA takes in turn: 64 sums per epilogue thread
 constexpr int DG_STAGES = 6;                      // most ring stages
 constexpr int DG_RING = 192 * 1024;               // ring bytes: 3 stages at 256 rows
 constexpr int DG_A_TILE = 128 * DG_KS * 2;        // one projection's (block, stage): 16 KB
@@ -100,7 +105,8 @@ struct DenseParams {
     uint32_t n_out;
     uint32_t nt;               // rows per token tile (a multiple of 16)
     uint32_t n_stages;         // ring stages
-    uint32_t k_parts;          // CTAs of a cluster that share one item's reduction dimension (1: no cluster)
+    uint32_t k_parts;          // parts of the reduction, each summed by itself
+    uint32_t n_cl;             // CTAs of a cluster that share an item's parts (1: no cluster)
     uint32_t* status;
     uint32_t poll_limit;
 };
@@ -130,11 +136,14 @@ __device__ __forceinline__ float4 ld_cluster4(uint32_t addr) {
 }
 
 // NPROJ = 2: gate and up of one feature block (activation epilogue -> hb); NPROJ = 1: two adjacent blocks -> out.
-// CL: a cluster of k_parts CTAs per item, one part of the reduction each; otherwise a CTA walks whole items.
-template <int NPROJ, bool CL>
+// MODE: how an item's parts are spread
+constexpr int DG_WHOLE = 0;     // one part; a CTA walks items
+constexpr int DG_FOLD = 1;      // a CTA walks items and takes their parts in turn
+constexpr int DG_CLUSTER = 2;   // a cluster of n_cl CTAs per item, an even share of its parts each
+template <int NPROJ, int MODE>
 __global__ void __launch_bounds__(64 + DG_EPI_WARPS * 32, 1) dense_gemm_kernel(const DenseParams P) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
-    __shared__ __align__(8) uint64_t full_bar[DG_STAGES], empty_bar[DG_STAGES], acc_full, acc_empty;
+    __shared__ __align__(8) uint64_t full_bar[DG_STAGES], empty_bar[DG_STAGES], acc_full[2], acc_empty[2];
     __shared__ uint32_t s_tmem;
     __shared__ volatile int s_abort;
     uint8_t* a_ring = smem_raw;                              // [stage][2 groups' tiles]
@@ -143,14 +152,14 @@ __global__ void __launch_bounds__(64 + DG_EPI_WARPS * 32, 1) dense_gemm_kernel(c
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t n_tt = (P.T + NT - 1) / NT;
     const uint32_t n_fb = NPROJ == 2 ? P.n_blocks : P.n_blocks / 2;     // feature-block groups
-    const uint32_t KP = CL ? P.k_parts : 1u;
-    const uint32_t n_units = n_tt * n_fb * KP;
+    constexpr bool CL = MODE == DG_CLUSTER;
+    const uint32_t KP = MODE == DG_WHOLE ? 1u : P.k_parts, NCL = CL ? P.n_cl : 1u;
+    const uint32_t n_units = n_tt * n_fb * NCL;
     if (blockIdx.x >= n_units) return;   // before any tensor memory is taken (the whole CTA reads the same count)
 
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < NS; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-        mbar_init(&acc_full, 1);
-        mbar_init(&acc_empty, DG_EPI_WARPS);
+        for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], DG_EPI_WARPS); }
         s_abort = 0;
         mbar_fence_init();
     }
@@ -162,11 +171,15 @@ __global__ void __launch_bounds__(64 + DG_EPI_WARPS * 32, 1) dense_gemm_kernel(c
     // part p of the reduction covers stages [p n_ks / KP, (p + 1) n_ks / KP): a function of the shape and the part count
     auto part_begin = [&](uint32_t part) { return (uint32_t)(((uint64_t)part * P.n_ks) / KP); };
     auto give_up = [&](uint32_t code) { if (!s_abort) atomicMax(P.status, code); s_abort = 1; };
-    // unit -> (token tile, feature-block group, part of the reduction); feature blocks vary fastest so that the CTAs
-    // running together share the rows of a few token tiles and the weights in L2
-    auto decode_unit = [&](uint32_t unit, uint32_t& tt, uint32_t& fb, uint32_t& part) {
-        part = unit % KP;
-        const uint32_t item = unit / KP;
+    // This CTA's parts: [part0, part1).  In a cluster all of them stay in tensor memory, number l in the columns from 2 l NT;
+    // otherwise they alternate between two buffers of 2 NT columns (one where only one fits)
+    const uint32_t n_buf = !CL && NT <= 128u ? 2u : 1u;
+    auto cl_part = [&](uint32_t rank) { return rank * KP / NCL; };
+    const uint32_t cl_rank = CL ? blockIdx.x % NCL : 0u, part0 = cl_part(cl_rank), part1 = cl_part(cl_rank + 1), n_parts = part1 - part0;
+    // unit -> (token tile, feature-block group); feature blocks vary fastest so that the CTAs running together share the
+    // rows of a few token tiles and the weights in L2
+    auto decode_unit = [&](uint32_t unit, uint32_t& tt, uint32_t& fb) {
+        const uint32_t item = unit / NCL;
         fb = item % n_fb;
         tt = item / n_fb;
     };
@@ -176,13 +189,13 @@ __global__ void __launch_bounds__(64 + DG_EPI_WARPS * 32, 1) dense_gemm_kernel(c
         if (lane == 0) {
             uint32_t s = 0, ph = 0;
             for (uint32_t unit = blockIdx.x; unit < n_units && !s_abort; unit += gridDim.x) {
-                uint32_t tt, fb, part;
-                decode_unit(unit, tt, fb, part);
+                uint32_t tt, fb;
+                decode_unit(unit, tt, fb);
                 const uint32_t rows = min(NT, P.T - tt * NT), rows16 = (rows + 15) / 16 * 16;
                 const uint32_t b_bytes = rows16 * DG_KS * 2;
                 const uint16_t* xsrc = P.xb + (size_t)tt * NT * P.K;
                 bool ok = true;
-                for (uint32_t ks = part_begin(part); ks < part_begin(part + 1); ++ks) {
+                for (uint32_t ks = part_begin(part0); ks < part_begin(part1); ++ks) {
                     if (!mbar_wait_bounded(&empty_bar[s], ph ^ 1u, &s_abort, 64, P.poll_limit)) { give_up(ST_WAIT_EMPTY); ok = false; break; }
                     mbar_expect_tx(&full_bar[s], DG_A_STAGE + b_bytes);
                     if (NPROJ == 2) {
@@ -205,31 +218,34 @@ __global__ void __launch_bounds__(64 + DG_EPI_WARPS * 32, 1) dense_gemm_kernel(c
             const uint32_t a_s = smem_u32(a_ring), b_s = smem_u32(b_ring);
             // gate / up interleave per 8-row group: a projection's core matrices of one K group are 2 KB apart
             constexpr uint32_t A_SBO = NPROJ == 2 ? 2048u : 1024u, A_LBO = 128u, A_GROUP = NPROJ == 2 ? 1024u : (uint32_t)DG_A_TILE;
-            for (uint32_t unit = blockIdx.x; unit < n_units && !s_abort; unit += gridDim.x, ++n_done) {
-                uint32_t tt, fb, part;
-                decode_unit(unit, tt, fb, part);
+            for (uint32_t unit = blockIdx.x; unit < n_units && !s_abort; unit += gridDim.x) {
+                uint32_t tt, fb;
+                decode_unit(unit, tt, fb);
                 const uint32_t rows = min(NT, P.T - tt * NT), rows16 = (rows + 15) / 16 * 16;
                 const uint32_t idesc = umma_idesc(UMMA_BF16, rows16), lbo_b = rows16 * 16;
-                if (!mbar_wait_bounded(&acc_empty, (n_done & 1u) ^ 1u, &s_abort, 64, P.poll_limit)) { give_up(ST_WAIT_EMPTY); break; }
-                tc_fence_after();
                 bool ok = true;
-                const uint32_t nk = part_begin(part + 1) - part_begin(part);
-                for (uint32_t kk = 0; kk < nk; ++kk) {
-                    if (!mbar_wait_bounded(&full_bar[s], ph, &s_abort, 0, P.poll_limit)) { give_up(ST_WAIT_FULL); ok = false; break; }
+                for (uint32_t part = part0; part < part1 && ok; ++part) {
+                    const uint32_t buf = n_done % n_buf, acc = tmem + (CL ? part - part0 : buf) * 2 * NT;
+                    if (!CL && !mbar_wait_bounded(&acc_empty[buf], (n_done / n_buf & 1u) ^ 1u, &s_abort, 64, P.poll_limit)) { give_up(ST_WAIT_EMPTY); ok = false; break; }
                     tc_fence_after();
-                    const uint32_t a0 = a_s + s * DG_A_STAGE, b0 = b_s + s * b_stage;
+                    const uint32_t ks0 = part_begin(part), ks1 = part_begin(part + 1);
+                    for (uint32_t ks = ks0; ks < ks1; ++ks) {
+                        if (!mbar_wait_bounded(&full_bar[s], ph, &s_abort, 0, P.poll_limit)) { give_up(ST_WAIT_FULL); ok = false; break; }
+                        tc_fence_after();
+                        const uint32_t a0 = a_s + s * DG_A_STAGE, b0 = b_s + s * b_stage;
 #pragma unroll
-                    for (int gq = 0; gq < 2; ++gq) {
+                        for (int gq = 0; gq < 2; ++gq) {
 #pragma unroll
-                        for (int i = 0; i < DG_KS / 16; ++i)
-                            umma_f16(tmem + gq * DG_NT, umma_smem_desc(a0 + gq * A_GROUP + i * 2 * A_LBO, A_LBO, A_SBO),
-                                     umma_smem_desc(b0 + i * 2 * lbo_b, lbo_b, 128), idesc, (kk | (uint32_t)i) ? 1u : 0u);
+                            for (int i = 0; i < DG_KS / 16; ++i)
+                                umma_f16(acc + gq * NT, umma_smem_desc(a0 + gq * A_GROUP + i * 2 * A_LBO, A_LBO, A_SBO),
+                                         umma_smem_desc(b0 + i * 2 * lbo_b, lbo_b, 128), idesc, ks != ks0 || i ? 1u : 0u);
+                        }
+                        umma_commit(&empty_bar[s]);
+                        if (++s == NS) { s = 0; ph ^= 1u; }
                     }
-                    umma_commit(&empty_bar[s]);
-                    if (++s == NS) { s = 0; ph ^= 1u; }
+                    if (ok && (!CL || part + 1 == part1)) { umma_commit(&acc_full[buf]); ++n_done; }
                 }
                 if (!ok) break;
-                umma_commit(&acc_full);
             }
         }
     } else {
@@ -238,31 +254,30 @@ __global__ void __launch_bounds__(64 + DG_EPI_WARPS * 32, 1) dense_gemm_kernel(c
         // the tile alternate between the two halves
         const uint32_t ew = warp - 2, q = warp & 3u, half = ew >> 2;
         uint32_t n_done = 0;
-        for (uint32_t unit = blockIdx.x; unit < n_units && !s_abort; unit += gridDim.x, ++n_done) {
-            uint32_t tt, fb, part;
-            decode_unit(unit, tt, fb, part);
-            const uint32_t rows = min(NT, P.T - tt * NT), rows16 = (rows + 15) / 16 * 16, nch = rows16 / 16;
-            if (!mbar_wait_bounded(&acc_full, n_done & 1u, &s_abort, 0, P.poll_limit)) { give_up(ST_WAIT_FULL); break; }
+        const uint32_t fl = q * 32u + lane;                     // feature inside the block
+        auto wait_acc = [&](uint32_t buf) -> bool {
+            if (!mbar_wait_bounded(&acc_full[buf], n_done / n_buf & 1u, &s_abort, 0, P.poll_limit)) { give_up(ST_WAIT_FULL); return false; }
             tc_fence_after();
-            const uint32_t fl = q * 32u + lane;                 // feature inside the block
-            for (uint32_t c = half; c < nch; c += 2) {
-                uint32_t r0[16], r1[16];
-                tmem_ld16(tmem + ((q * 32u) << 16) + 0 * DG_NT + c * 16, r0);
-                tmem_ld16(tmem + ((q * 32u) << 16) + 1 * DG_NT + c * 16, r1);
-                if (CL) {
-                    // this part's tile into the ring's memory (its MMAs are complete): [group][row][128 features]
-                    float* z = reinterpret_cast<float*>(smem_raw) + (size_t)c * 16 * 128 + fl;
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        z[i * 128] = __uint_as_float(r0[i]);
-                        z[(rows16 + i) * 128] = __uint_as_float(r1[i]);
-                    }
-                } else if (NPROJ == 2) {
+            return true;
+        };
+        auto release_acc = [&](uint32_t buf) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_empty[buf]);
+            ++n_done;
+        };
+        for (uint32_t unit = blockIdx.x; unit < n_units && !s_abort; unit += gridDim.x) {
+            uint32_t tt, fb;
+            decode_unit(unit, tt, fb);
+            const uint32_t rows = min(NT, P.T - tt * NT), rows16 = (rows + 15) / 16 * 16, nch = rows16 / 16;
+            // 16 rows (chunk c) of this thread's feature, both groups
+            auto emit = [&](uint32_t c, const float (&v0)[16], const float (&v1)[16]) {
+                if (NPROJ == 2) {
                     const uint32_t f = fb * 128 + fl;
 #pragma unroll
                     for (int i = 0; i < 16; ++i) {
                         const uint32_t r = c * 16 + i;
-                        const __nv_bfloat16 hv = __float2bfloat16_rn(dg_act(__uint_as_float(r0[i]), __uint_as_float(r1[i]), P.limit));
+                        const __nv_bfloat16 hv = __float2bfloat16_rn(dg_act(v0[i], v1[i], P.limit));
                         // padding rows of the tile are written as zeros: the down product reads whole 16-row groups
                         P.hb[dg_b_off(P.n_out, NT, tt, rows16, r, f)] = r < rows ? __bfloat16_as_ushort(hv) : (uint16_t)0;
                     }
@@ -273,37 +288,95 @@ __global__ void __launch_bounds__(64 + DG_EPI_WARPS * 32, 1) dense_gemm_kernel(c
                         const uint32_t f = 2 * fb * 128 + fl;
                         if (r < rows) {
                             float* o = P.out + (size_t)(tt * NT + r) * P.n_out + f;
-                            if (f < P.n_out) o[0] = __uint_as_float(r0[i]);
-                            if (f + 128 < P.n_out) o[128] = __uint_as_float(r1[i]);
+                            if (f < P.n_out) o[0] = v0[i];
+                            if (f + 128 < P.n_out) o[128] = v1[i];
                         }
                     }
                 }
+            };
+            auto load = [&](uint32_t col, float (&v)[16]) {
+                uint32_t r[16];
+                tmem_ld16(tmem + ((q * 32u) << 16) + col, r);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+            };
+            if (CL) {
+                // the parts' tiles into the ring's memory (all MMAs are complete): [part][group][row][128 features]
+                if (!wait_acc(0)) break;
+                for (uint32_t c = half; c < nch; c += 2)
+                    for (uint32_t l = 0; l < n_parts; ++l) {
+                        float v0[16], v1[16];
+                        load(2 * l * NT + c * 16, v0);
+                        load((2 * l + 1) * NT + c * 16, v1);
+                        float* z = reinterpret_cast<float*>(smem_raw) + ((size_t)2 * l * rows16 + c * 16) * 128 + fl;
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) {
+                            z[i * 128] = v0[i];
+                            z[(rows16 + i) * 128] = v1[i];
+                        }
+                    }
+                release_acc(0);
+            } else if (MODE == DG_WHOLE) {
+                const uint32_t buf = n_done % n_buf;
+                if (!wait_acc(buf)) break;
+                for (uint32_t c = half; c < nch; c += 2) {
+                    float v0[16], v1[16];
+                    load(buf * 2 * NT + c * 16, v0);
+                    load((buf * 2 + 1) * NT + c * 16, v1);
+                    emit(c, v0, v1);
+                }
+                release_acc(buf);
+            } else {
+                // at most 64 rows: two chunks per warp; the parts are added in part order
+                static_assert(DG_FOLD_NT <= 64, "two chunks of 16 rows per half of the warps");
+                float sum[2][2][16];
+                bool ok = true;
+                for (uint32_t part = 0; part < KP; ++part) {
+                    const uint32_t buf = n_done % n_buf;
+                    if (!(ok = wait_acc(buf))) break;
+#pragma unroll
+                    for (int j = 0; j < 2; ++j)
+#pragma unroll
+                        for (int g = 0; g < 2; ++g)
+                            if (half + 2 * j < nch) {
+                                float v[16];
+                                load((buf * 2 + g) * NT + (half + 2 * j) * 16, v);
+#pragma unroll
+                                for (int i = 0; i < 16; ++i) sum[j][g][i] = part ? __fadd_rn(sum[j][g][i], v[i]) : v[i];
+                            }
+                    release_acc(buf);
+                }
+                if (!ok) break;
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+                    if (half + 2 * j < nch) emit(half + 2 * j, sum[j][0], sum[j][1]);
             }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&acc_empty);
         }
     }
     // every thread comes here, also after a give-up: the cluster's barriers are always met, the tensor memory is always released
     if (CL) {
         __syncwarp();
         cluster_barrier();
-        // the sums of a slice of the tile's rows over the cluster's parts, in part order
-        uint32_t tt, fb, part;
-        decode_unit(blockIdx.x, tt, fb, part);
+        // the sums of a slice of the tile's rows over the item's parts, in part order
+        uint32_t tt, fb;
+        decode_unit(blockIdx.x, tt, fb);
         const uint32_t rows = min(NT, P.T - tt * NT), rows16 = (rows + 15) / 16 * 16;
-        const uint32_t row0 = part * rows16 / KP, n_rows = (part + 1) * rows16 / KP - row0, base = smem_u32(smem_raw);
+        const uint32_t row0 = cl_rank * rows16 / NCL, n_rows = (cl_rank + 1) * rows16 / NCL - row0, base = smem_u32(smem_raw);
         for (uint32_t i = threadIdx.x; i < n_rows * 16; i += blockDim.x) {
             const uint32_t r = row0 + i / 16, f8 = i % 16;      // eight features of a row, of both groups
             float v[16];
+            for (uint32_t rank = 0; rank < NCL; ++rank) {
+                const uint32_t src = cluster_addr(base + (r * 128 + f8 * 8) * 4, rank), n = cl_part(rank + 1) - cl_part(rank);
+                for (uint32_t l = 0; l < n; ++l) {
+                    const bool init = (rank | l) == 0;
 #pragma unroll
-            for (int k = 0; k < 16; ++k) v[k] = 0.f;
-            for (uint32_t pp = 0; pp < KP; ++pp) {
-                const uint32_t src = cluster_addr(base + (r * 128 + f8 * 8) * 4, pp);
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const float4 w = ld_cluster4(src + (k >> 1) * (rows16 * 512) + (k & 1) * 16);
-                    v[4 * k] += w.x; v[4 * k + 1] += w.y; v[4 * k + 2] += w.z; v[4 * k + 3] += w.w;
+                    for (int k = 0; k < 4; ++k) {
+                        const float4 w = ld_cluster4(src + (2 * l + (k >> 1)) * (rows16 * 512) + (k & 1) * 16);
+                        v[4 * k] = init ? w.x : __fadd_rn(v[4 * k], w.x);
+                        v[4 * k + 1] = init ? w.y : __fadd_rn(v[4 * k + 1], w.y);
+                        v[4 * k + 2] = init ? w.z : __fadd_rn(v[4 * k + 2], w.z);
+                        v[4 * k + 3] = init ? w.w : __fadd_rn(v[4 * k + 3], w.w);
+                    }
                 }
             }
             if (NPROJ == 2) {
@@ -330,89 +403,108 @@ __global__ void __launch_bounds__(64 + DG_EPI_WARPS * 32, 1) dense_gemm_kernel(c
     if (warp == 0) tmem_free(tmem, 512);
 }
 
-// ---- how a product is cut: rows per token tile and CTAs (of a cluster) per item ----
+// ---- how a product is cut ----
 struct DgShape { uint32_t n_fb, n_ks; };             // feature-block pairs, stages of 64 inputs
-// clusters of kp CTAs that the device holds at once (an SM holds one CTA; clusters do not cross GPCs)
-template <int NPROJ>
-static uint32_t dg_max_clusters(uint32_t kp, int sm_count) {
-    static uint32_t known[9] = {0};
-    if (kp == 1) return (uint32_t)sm_count;
-    if (!known[kp]) {
+// Parts of the reduction: as many as give every SM a weight stream with tiles of 256 rows, each part at least 4 stages long.
+// The bits of a sum go by this count, so it is a function of the item count and the SM count alone and no measurement enters:
+// calls of up to 256 tokens always split the same way.
+static uint32_t dg_parts(DgShape s, uint32_t T, int sm_count) {
+    const uint32_t items = (T + DG_NT - 1) / DG_NT * s.n_fb;
+    uint32_t kp = (uint32_t)sm_count / (items ? items : 1u);
+    if (kp > s.n_ks / 4) kp = s.n_ks / 4;
+    if (kp > 16) kp = 16;
+    return kp ? kp : 1u;
+}
+// Estimated cycles of a product of kp parts cut into tiles of nt rows and spread over clusters of n_cl CTAs: per stage the
+// larger of the bytes an SM takes in (55 a cycle) and its eight MMAs with the turn-around of a stage; per wave a constant for
+// the pipeline's fill and the epilogue; for a cluster the tiles' way through distributed shared memory.  The constants are a
+// fit to 1188 timings at (H, I) = (5120, 2304), (4096, 2048), (6144, 2048), 65 to 8192 tokens, every tile and cluster that
+// fits (and 21000 cycles for what all have in common): spread of measured over predicted 11 %, the cut taken 1.01 times the
+// best one's time on average and 1.18 times at most.
+static double dg_cost(DgShape s, uint32_t T, uint32_t nt, uint32_t kp, uint32_t n_cl, uint32_t max_clusters) {
+    const uint32_t rows = nt < T ? nt : (T + 15) / 16 * 16, per = (kp + n_cl - 1) / n_cl;
+    const double load = (DG_A_STAGE + rows * 128.0) / 55.0, mma = 8.0 * (rows > 96 ? rows / 2.0 : 48.0) + 140.0;
+    const uint32_t items = (T + nt - 1) / nt * s.n_fb, waves = (items + max_clusters - 1) / max_clusters;
+    return waves * ((s.n_ks * per + kp - 1) / kp * (load > mma ? load : mma) + 8000.0 + rows * (n_cl > 1 ? per : 1) * 8.0 +
+                    (n_cl > 1 ? 4300.0 + rows * per * 60.0 : 0.0));
+}
+// CTAs per item for tiles of nt rows; 0: the parts' tiles do not fit
+static uint32_t dg_pick_cluster(DgShape s, uint32_t T, uint32_t nt, int sm_count, const DenseCaps& caps, double* cost) {
+    const uint32_t kp = dg_parts(s, T, sm_count);
+    uint32_t best = 0;
+    for (uint32_t per = 1; per <= kp; ++per) {            // parts of a CTA
+        const uint32_t n_cl = (kp + per - 1) / per;
+        if (n_cl > (uint32_t)DG_CL_MAX || (n_cl > 1 ? per * nt > (uint32_t)DG_CL_NT : kp > 1 && nt > (uint32_t)DG_FOLD_NT)) continue;
+        const double c = dg_cost(s, T, nt, kp, n_cl, caps.clusters[n_cl]);
+        if (!best || c < *cost) { *cost = c; best = n_cl; }
+    }
+    return best;
+}
+// rows per tile for one or two products of the same rows; 64 rows and fewer always fit
+static uint32_t dg_pick_rows(const DgShape* s, int n, uint32_t T, int sm_count, const DenseCaps& caps) {
+    static const uint32_t tiles[] = {DG_NT, DG_CL_NT, 160, 128, 96, 64, 48, 32};
+    uint32_t best = 32;
+    double c0 = 0;
+    bool any = false;
+    for (const uint32_t nt : tiles) {
+        double c = 0, one = 0;
+        bool fits = true;
+        for (int i = 0; i < n && fits; ++i) { fits = dg_pick_cluster(s[i], T, nt, sm_count, caps, &one) != 0; c += one; }
+        if (fits && (!any || c < c0)) { c0 = c; best = nt; any = true; }
+    }
+    return best;
+}
+uint32_t dense_shared_rows(uint32_t T, uint32_t H, uint32_t I, int sm_count, const DenseCaps& caps) {
+    const DgShape s[2] = {{I / 128, H / DG_KS}, {H / 256, I / DG_KS}};
+    return dg_pick_rows(s, 2, T, sm_count, caps);
+}
+uint32_t dense_logits_rows(uint32_t T, uint32_t E, uint32_t H, int sm_count, const DenseCaps& caps) {
+    const DgShape s{(E + 255) / 256, H / DG_KS};
+    return dg_pick_rows(&s, 1, T, sm_count, caps);
+}
+// clusters of n CTAs that the device holds at once (an SM holds one CTA; clusters do not cross GPCs)
+cudaError_t dense_caps(int sm_count, DenseCaps* caps) {
+    const cudaError_t e = cudaFuncSetAttribute(dense_gemm_kernel<2, DG_CLUSTER>, cudaFuncAttributeMaxDynamicSharedMemorySize, DG_RING);
+    if (e != cudaSuccess) return e;
+    caps->clusters[0] = 0;
+    caps->clusters[1] = (uint32_t)sm_count;
+    for (uint32_t n_cl = 2; n_cl <= (uint32_t)DG_CL_MAX; ++n_cl) {
         cudaLaunchAttribute attr;
         attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = kp; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+        attr.val.clusterDim.x = n_cl; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
         cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(kp * 64); cfg.blockDim = dim3(64 + DG_EPI_WARPS * 32); cfg.dynamicSmemBytes = DG_RING; cfg.attrs = &attr; cfg.numAttrs = 1;
+        cfg.gridDim = dim3(n_cl * 64); cfg.blockDim = dim3(64 + DG_EPI_WARPS * 32); cfg.dynamicSmemBytes = DG_RING; cfg.attrs = &attr; cfg.numAttrs = 1;
         int n = 0;
-        cudaFuncSetAttribute(dense_gemm_kernel<NPROJ, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, DG_RING);
-        if (cudaOccupancyMaxActiveClusters(&n, dense_gemm_kernel<NPROJ, true>, &cfg) != cudaSuccess || n < 1) { cudaGetLastError(); n = sm_count / (int)kp; }
-        known[kp] = (uint32_t)(n > 0 ? n : 1);
+        if (cudaOccupancyMaxActiveClusters(&n, dense_gemm_kernel<2, DG_CLUSTER>, &cfg) != cudaSuccess || n < 1) { cudaGetLastError(); n = sm_count / (int)n_cl; }
+        caps->clusters[n_cl] = (uint32_t)(n > 0 ? n : 1);
     }
-    return known[kp];
-}
-// Estimated cycles of a product cut into tiles of nt rows and kp parts: per stage the larger of the bytes an SM takes in (about
-// 50 a cycle) and its eight MMAs with the turn-around of a stage; a constant per wave for the pipeline's fill and the
-// epilogue; for a cluster the tile's way through distributed shared memory.  Measured at H 5120, I 2304 (gate/up + down).
-static double dg_cost(DgShape s, uint32_t T, uint32_t nt, uint32_t kp, uint32_t max_clusters) {
-    const uint32_t rows = nt < T ? nt : (T + 15) / 16 * 16;
-    const double load = (DG_A_STAGE + rows * 128.0) / 50.0, mma = 8.0 * (rows / 2.0 > 48.0 ? rows / 2.0 : 48.0) + 120.0;
-    const uint32_t items = (T + nt - 1) / nt * s.n_fb, waves = (items + max_clusters - 1) / max_clusters;
-    return waves * ((s.n_ks + kp - 1) / kp * (load > mma ? load : mma) + 5000.0 + rows * 16.0) + (kp > 1 ? 3000.0 + rows * 1024.0 / 25.0 : 0.0);
-}
-template <int NPROJ>
-static uint32_t dg_pick_parts(DgShape s, uint32_t T, uint32_t nt, int sm_count, double* cost) {
-    uint32_t best = 1;
-    double c0 = dg_cost(s, T, nt, 1, (uint32_t)sm_count);
-    for (uint32_t kp = 2; kp <= 8 && nt <= (uint32_t)DG_CL_NT && kp * 4 <= s.n_ks; kp *= 2) {
-        const double c = dg_cost(s, T, nt, kp, dg_max_clusters<NPROJ>(kp, sm_count));
-        if (c < c0) { c0 = c; best = kp; }
-    }
-    *cost = c0;
-    return best;
-}
-static uint32_t dg_pick_rows(const DgShape* gu, const DgShape* plain, int n_plain, uint32_t T, int sm_count) {
-    uint32_t best = DG_NT;
-    double c0 = 0;
-    for (uint32_t nt = DG_NT; nt >= 64; nt -= nt > (uint32_t)DG_CL_NT ? nt - DG_CL_NT : 32) {
-        double c = 0, one = 0;
-        if (gu) { dg_pick_parts<2>(*gu, T, nt, sm_count, &one); c += one; }
-        for (int i = 0; i < n_plain; ++i) { dg_pick_parts<1>(plain[i], T, nt, sm_count, &one); c += one; }
-        if (nt == (uint32_t)DG_NT || c < c0) { c0 = c; best = nt; }
-    }
-    return best;
-}
-uint32_t dense_shared_rows(uint32_t T, uint32_t H, uint32_t I, int sm_count) {
-    const DgShape gu{I / 128, H / DG_KS}, dn{H / 256, I / DG_KS};
-    return dg_pick_rows(&gu, &dn, 1, T, sm_count);
-}
-uint32_t dense_logits_rows(uint32_t T, uint32_t E, uint32_t H, int sm_count) {
-    const DgShape lg{(E + 255) / 256, H / DG_KS};
-    return dg_pick_rows(nullptr, &lg, 1, T, sm_count);
+    return cudaSuccess;
 }
 
 template <int NPROJ>
-static cudaError_t dg_launch(DenseParams P, int sm_count, cudaStream_t st) {
+static cudaError_t dg_launch(DenseParams P, int sm_count, const DenseCaps& caps, cudaStream_t st) {
     const DgShape s{NPROJ == 2 ? P.n_blocks : P.n_blocks / 2, P.n_ks};
     double cost = 0;
-    P.k_parts = dg_pick_parts<NPROJ>(s, P.T, P.nt, sm_count, &cost);
+    P.k_parts = dg_parts(s, P.T, sm_count);
+    P.n_cl = dg_pick_cluster(s, P.T, P.nt, sm_count, caps, &cost);
+    if (!P.n_cl) return cudaErrorInvalidValue;
     const size_t stage = DG_A_STAGE + (size_t)P.nt * DG_KS * 2;
     P.n_stages = (uint32_t)(DG_RING / stage < (size_t)DG_STAGES ? DG_RING / stage : (size_t)DG_STAGES);
     const uint32_t n_items = (P.T + P.nt - 1) / P.nt * s.n_fb;
-    cudaError_t e;
-    if (P.k_parts == 1) {
-        if ((e = cudaFuncSetAttribute(dense_gemm_kernel<NPROJ, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, DG_RING)) != cudaSuccess) return e;
-        const uint32_t grid = n_items < (uint32_t)sm_count ? n_items : (uint32_t)sm_count;
-        dense_gemm_kernel<NPROJ, false><<<grid, 64 + DG_EPI_WARPS * 32, DG_RING, st>>>(P);
+    const auto kernel = P.n_cl > 1 ? dense_gemm_kernel<NPROJ, DG_CLUSTER> : P.k_parts > 1 ? dense_gemm_kernel<NPROJ, DG_FOLD> : dense_gemm_kernel<NPROJ, DG_WHOLE>;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DG_RING);
+    if (e != cudaSuccess) return e;
+    if (P.n_cl == 1) {
+        kernel<<<n_items < (uint32_t)sm_count ? n_items : (uint32_t)sm_count, 64 + DG_EPI_WARPS * 32, DG_RING, st>>>(P);
         return cudaGetLastError();
     }
-    if ((e = cudaFuncSetAttribute(dense_gemm_kernel<NPROJ, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, DG_RING)) != cudaSuccess) return e;
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = P.k_parts; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+    attr.val.clusterDim.x = P.n_cl; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(n_items * P.k_parts); cfg.blockDim = dim3(64 + DG_EPI_WARPS * 32); cfg.dynamicSmemBytes = DG_RING; cfg.stream = st;
+    cfg.gridDim = dim3(n_items * P.n_cl); cfg.blockDim = dim3(64 + DG_EPI_WARPS * 32); cfg.dynamicSmemBytes = DG_RING; cfg.stream = st;
     cfg.attrs = &attr; cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, dense_gemm_kernel<NPROJ, true>, P);
+    return cudaLaunchKernelEx(&cfg, kernel, P);
 }
 static_assert(DG_RING >= 2 * DG_CL_NT * 128 * 4, "a cluster's partial tile in the ring's memory");
 
@@ -430,14 +522,14 @@ cudaError_t launch_dense_shared_expert(const DenseSharedArgs& a, cudaStream_t st
     P.status = a.status; P.poll_limit = 1u << 20; P.limit = a.limit; P.T = a.T; P.nt = a.nt;
     // gate / up -> h (B-operand order over I inputs)
     P.w = static_cast<const uint8_t*>(a.w_gu); P.n_blocks = a.I / 128; P.n_ks = a.H / DG_KS; P.xb = a.xb; P.K = a.H; P.hb = a.hb; P.out = nullptr; P.n_out = a.I;
-    if ((e = dg_launch<2>(P, a.sm_count, st)) != cudaSuccess) return e;
+    if ((e = dg_launch<2>(P, a.sm_count, *a.caps, st)) != cudaSuccess) return e;
     // down -> out f32 [T, H]
     P.w = static_cast<const uint8_t*>(a.w_d); P.n_blocks = a.H / 128; P.n_ks = a.I / DG_KS; P.xb = a.hb; P.K = a.I; P.hb = nullptr; P.out = a.out; P.n_out = a.H;
-    return dg_launch<1>(P, a.sm_count, st);
+    return dg_launch<1>(P, a.sm_count, *a.caps, st);
 }
 
 cudaError_t launch_dense_logits(const __nv_bfloat16* x, const void* w_tiled, uint32_t T, uint32_t E, uint32_t H, uint32_t nt, uint16_t* xb,
-                                float* logits, uint32_t* status, int sm_count, cudaStream_t st) {
+                                float* logits, uint32_t* status, int sm_count, const DenseCaps& caps, cudaStream_t st) {
     if (T == 0) return cudaSuccess;
     const cudaError_t e = dg_stage_rows(x, T, H, nt, xb, sm_count, st);
     if (e != cudaSuccess) return e;
@@ -445,7 +537,7 @@ cudaError_t launch_dense_logits(const __nv_bfloat16* x, const void* w_tiled, uin
     P.status = status; P.poll_limit = 1u << 20; P.limit = 0.f; P.T = T; P.nt = nt;
     P.w = static_cast<const uint8_t*>(w_tiled); P.n_blocks = (E + 255) / 256 * 2; P.n_ks = H / DG_KS; P.xb = xb; P.K = H; P.hb = nullptr;
     P.out = logits; P.n_out = E;
-    return dg_launch<1>(P, sm_count, st);
+    return dg_launch<1>(P, sm_count, caps, st);
 }
 
 bool dense_gemm_supported(uint32_t n_out, uint32_t K, int two_blocks) {

@@ -65,9 +65,9 @@ struct mlxs_moe {
     uint32_t pf_min_rows = 0;   // experts with at least this many rows of a call take the tensor-core lane (0: lane off)
     uint32_t chunk_rows = CHUNK_ROWS, group_chunks = GROUP_CHUNKS;
     __nv_bfloat16* sh_h = nullptr;
-    // dense tensor-core products (shared expert, router logits): rows / h in the MMA's B-operand order, the scratch of
-    // the split reduction
+    // dense tensor-core products (shared expert, router logits): rows / h in the MMA's B-operand order
     uint16_t *dg_xb = nullptr, *dg_hb = nullptr;
+    mlxs::DenseCaps dg_caps{};    // filled with dg_xb
     uint32_t dg_staged_nt = 0;    // inside mlxs_moe_forward_x: dg_xb holds this call's rows in tiles of that many (0: it does not)
     // small batches: the shared expert runs beside the routed kernels on a second stream (they leave SMs free)
     float* logits_ws = nullptr;       // [max_tokens, E] logits of mlxs_moe_forward_x

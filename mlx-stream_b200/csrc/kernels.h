@@ -279,6 +279,8 @@ cudaError_t launch_shared_expert(const __nv_bfloat16* x, const __nv_bfloat16* w1
                                  __nv_bfloat16* h_ws, float* out, cudaStream_t st);
 // ---- dense bf16 products on tcgen05 (dense_gemm.cu): the shared expert at every batch size, the router's logits ----
 // weights re-tiled at load: w_gu = [I/128][H/64] stages of gate and up interleaved, w_d = [H/128][I/64]; see the file
+struct DenseCaps { uint32_t clusters[9]; };   // clusters of n CTAs of a dense product that the device holds at once
+cudaError_t dense_caps(int sm_count, DenseCaps* caps);
 struct DenseSharedArgs {
     const __nv_bfloat16* x;  // [T, H]
     const void* w_gu;        // re-tiled gate + up, 2 * H * I bf16
@@ -288,14 +290,15 @@ struct DenseSharedArgs {
     uint16_t* xb;            // [T rounded to 16, H] rows in the MMA's B-operand order (scratch)
     uint16_t* hb;            // [T rounded to 16, I] h in the same order (scratch)
     float* out;              // [T, H] f32
-    uint32_t nt;             // rows per token tile: dense_shared_rows(T, H, I, sm_count)
+    uint32_t nt;             // rows per token tile: dense_shared_rows(T, H, I, sm_count, caps)
     bool rows_staged;        // xb already holds x in tiles of nt rows
     uint32_t* status;
     int sm_count;
+    const DenseCaps* caps;
 };
 // rows per token tile of the shared expert's products, of the logits product alone
-uint32_t dense_shared_rows(uint32_t T, uint32_t H, uint32_t I, int sm_count);
-uint32_t dense_logits_rows(uint32_t T, uint32_t E, uint32_t H, int sm_count);
+uint32_t dense_shared_rows(uint32_t T, uint32_t H, uint32_t I, int sm_count, const DenseCaps& caps);
+uint32_t dense_logits_rows(uint32_t T, uint32_t E, uint32_t H, int sm_count, const DenseCaps& caps);
 bool dense_gemm_supported(uint32_t n_out, uint32_t K, int two_blocks);
 // W[n_out, K] row-major bf16 (w1 = a second matrix interleaved per 8-row group, or null) -> the tiled order
 cudaError_t launch_dense_retile(const __nv_bfloat16* w0, const __nv_bfloat16* w1, uint32_t n_out, uint32_t K, void* dst,
@@ -303,7 +306,7 @@ cudaError_t launch_dense_retile(const __nv_bfloat16* w0, const __nv_bfloat16* w1
 cudaError_t launch_dense_shared_expert(const DenseSharedArgs& a, cudaStream_t st);
 // logits[T, E] f32 = x . W_g^T with W_g re-tiled (single projection); E a multiple of 256
 cudaError_t launch_dense_logits(const __nv_bfloat16* x, const void* w_tiled, uint32_t T, uint32_t E, uint32_t H, uint32_t nt, uint16_t* xb,
-                                float* logits, uint32_t* status, int sm_count, cudaStream_t st);
+                                float* logits, uint32_t* status, int sm_count, const DenseCaps& caps, cudaStream_t st);
 // y[t] = sum_k ro[t,k] w[t,k] (+ shared[t]) -> bf16
 cudaError_t launch_combine(const void* ro, int ro_bf16, const float* weights, const float* shared, uint32_t T,
                            uint32_t K, uint32_t H, int chain, __nv_bfloat16* y, cudaStream_t st);

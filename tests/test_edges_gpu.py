@@ -141,3 +141,33 @@ def test_fp4_scale_bytes_at_the_ends_of_their_range(cls, scales):
             assert rel_l2(y, case.cpu_layer(x, ids, w)) < 1e-2, T
     finally:
         case.close()
+
+
+@pytest.mark.parametrize("H,I", [(1280, 768), (4096, 2048)])
+def test_dense_products_of_a_row_do_not_depend_on_the_batch(H, I):
+    """A row of the shared expert and of the router's logits has the same bits in every call of 65 to 256 tokens, whatever
+    tiles and clusters serve it (5 and 3, 9 and 8 parts of the sums; 5 and 16 for the logits); larger calls split into fewer
+    parts and are checked against the plain product."""
+    import torch
+    case = Exl3Case(H, I, 256, 1, seed=11, shared=True, max_tokens=1030, experts_to_load=[0, 1])
+    try:
+        x, _ = case.inputs(1025, seed=5)
+        ref = _shared_ref(x, case.shared, case.limit)
+        wg = O.f32_to_bf16_bits((np.random.default_rng(5).standard_normal((256, H)) * H ** -0.5).astype(np.float32))
+        case.moe.set_router_weight(0, wg.ctypes.data)
+        lref = x.astype(np.float64) @ O.bf16_bits_to_f32(wg).astype(np.float64).T
+        first = None
+        for T in (65, 70, 96, 97, 128, 129, 160, 161, 192, 193, 200, 256, 257, 300, 512, 513, 768, 769, 1024, 1025):
+            y = case.gpu_experts(x[:T], np.zeros((T, 1), np.int32), np.zeros((T, 1), np.float32))
+            lg = torch.empty((T, 256), dtype=torch.float32, device=case.dev)
+            case.moe.logits(0, case.to_dev_bf16(x[:T]).data_ptr(), T, lg.data_ptr(), None)
+            torch.cuda.synchronize()
+            got = lg.cpu().numpy()
+            assert case.status() == 0
+            assert rel_l2(y, ref[:T]) < 4e-3, T
+            assert rel_l2(got, lref[:T]) < 5e-7, T      # 20 sums in f32 per part and 16 parts: a random walk of 36 roundings of 2^-24 is 3.6e-7
+            if T <= 256:
+                first = (y[:65], got[:65]) if first is None else first
+                assert (y[:65] == first[0]).all() and (got[:65] == first[1]).all(), T
+    finally:
+        case.close()
