@@ -143,8 +143,8 @@ int mlxs_moe_bank_layer_bits_text(const char *manifest_json, uint32_t *bits_out,
 int mlxs_moe_set_router_bias(mlxs_moe *h, uint32_t layer, const float *bias_host);
 /* Router weight W_g bf16 [n_experts, hidden] (src/arch/deepseek_v41/graph.zig:2033): with it the layer can start from x. */
 int mlxs_moe_set_router_weight(mlxs_moe *h, uint32_t layer, const void *w_gate_bf16, int on_device);
-/* logits[T, n_experts] f32 = f32(x) . f32(W_g)^T, f32 accumulate in a fixed order (row by row up to 16 tokens, a tcgen05
- * product above) */
+/* logits[T, n_experts] f32 = f32(x) . f32(W_g)^T, f32 accumulate in a fixed order (above 64 tokens, and when n_experts is a
+ * multiple of 256, a tcgen05 product) */
 int mlxs_moe_logits(mlxs_moe *h, uint32_t layer, const void *x_dev, uint32_t T, float *logits_dev, void *stream);
 /* mlxs_moe_logits into the handle's workspace, then mlxs_moe_forward: the whole layer from x
  * (Source.forward's real caller, src/arch/glm5_next/experts.zig:566-595) */

@@ -555,9 +555,10 @@ extern "C" int mlxs_moe_plan_placement(const uint64_t* counts, uint32_t n_expert
     return MLXS_OK;
 }
 
-// more tokens than this take the tcgen05 product of dense_gemm.cu for the router's logits (32 tokens of H 6144: 61 -> 12 us),
-// fewer the row-by-row kernel (or the fused front, which has the same code)
-static constexpr uint32_t LOGITS_DENSE_FROM = 16;
+// More tokens than this take the tcgen05 product of dense_gemm.cu for the router's logits, where the expert count fills its
+// feature blocks; all others the f32 kernels of router.cu (or the fused front, with the same sums).  The product rounds four
+// times as much (3e-7 of the logits' norm against 8e-8 at H 5120), so it stays where it always was.
+static constexpr uint32_t LOGITS_DENSE_FROM = 64;
 extern "C" int mlxs_moe_set_router_weight(mlxs_moe* h, uint32_t layer, const void* w_gate_bf16, int on_device) {
     if (!h || !w_gate_bf16) return fail(MLXS_E_ARG, "set_router_weight: null argument");
     if (layer >= h->cfg.n_layers) return fail(MLXS_E_ARG, "set_router_weight: layer %u of %u", layer, h->cfg.n_layers);
@@ -568,9 +569,9 @@ extern "C" int mlxs_moe_set_router_weight(mlxs_moe* h, uint32_t layer, const voi
     if (!L.router_w && (rc = h->alloc(&L.router_w, n))) return rc;
     if (!h->logits_ws && (rc = h->alloc(&h->logits_ws, (size_t)h->cfg.max_tokens * h->cfg.n_experts * 4))) return rc;
     CU(cudaMemcpy(L.router_w, w_gate_bf16, n, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice));
-    if (h->cfg.max_tokens > LOGITS_DENSE_FROM && h->cfg.n_experts % 8 == 0) {
+    if (h->cfg.max_tokens > LOGITS_DENSE_FROM && dense_gemm_supported(h->cfg.n_experts, h->cfg.hidden, 1)) {
         if ((rc = dense_workspace(h))) return rc;
-        if (!L.router_w_t && (rc = h->alloc(&L.router_w_t, ((size_t)h->cfg.n_experts + 255) / 256 * 256 * h->cfg.hidden * 2))) return rc;
+        if (!L.router_w_t && (rc = h->alloc(&L.router_w_t, n))) return rc;
         CU(launch_dense_retile(L.router_w, nullptr, h->cfg.n_experts, h->cfg.hidden, L.router_w_t, 0));
         CU(cudaStreamSynchronize(0));
     }

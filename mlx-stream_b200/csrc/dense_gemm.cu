@@ -44,7 +44,7 @@ constexpr int DG_EPI_WARPS = 8;
 // ---- load-time re-tiling of a weight matrix W[n_out, K] (row-major bf16) ----
 // np = 2: w0 and w1 interleaved per 8-row group ([rc][p][kc][8][8]); np = 1: w0 alone ([rc][kc][8][8])
 __global__ void dense_retile_kernel(const __nv_bfloat16* __restrict__ w0, const __nv_bfloat16* __restrict__ w1, uint32_t n_out,
-                                    uint32_t n_valid, uint32_t K, int np, uint4* __restrict__ dst) {
+                                    uint32_t K, int np, uint4* __restrict__ dst) {
     const size_t n_vec = (size_t)np * n_out * K / 8;
     const uint32_t nks = K / DG_KS;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_vec; i += (size_t)gridDim.x * blockDim.x) {
@@ -55,18 +55,15 @@ __global__ void dense_retile_kernel(const __nv_bfloat16* __restrict__ w0, const 
         const uint32_t rc = r % 16; r /= 16;
         const uint32_t ks = r % nks; r /= nks;
         const uint32_t nb = (uint32_t)r;
-        const uint32_t f = nb * 128 + rc * 8 + r8;
-        const __nv_bfloat16* src = (p ? w1 : w0) + (size_t)f * K + (size_t)ks * DG_KS + kc * 8;
-        dst[i] = f < n_valid ? *reinterpret_cast<const uint4*>(src) : make_uint4(0, 0, 0, 0);
+        const __nv_bfloat16* src = (p ? w1 : w0) + (size_t)(nb * 128 + rc * 8 + r8) * K + (size_t)ks * DG_KS + kc * 8;
+        dst[i] = *reinterpret_cast<const uint4*>(src);
     }
 }
 
 cudaError_t launch_dense_retile(const __nv_bfloat16* w0, const __nv_bfloat16* w1, uint32_t n_out, uint32_t K, void* dst,
                                 cudaStream_t st) {
-    if (K % DG_KS || (w1 && n_out % 128)) return cudaErrorInvalidValue;
-    // a single matrix is cut into pairs of blocks: padded with zero features to a whole pair
-    const uint32_t n_pad = w1 ? n_out : (n_out + 255) / 256 * 256;
-    dense_retile_kernel<<<592, 256, 0, st>>>(w0, w1, n_pad, n_out, K, w1 ? 2 : 1, static_cast<uint4*>(dst));
+    if (n_out % (w1 ? 128 : 256) || K % DG_KS) return cudaErrorInvalidValue;
+    dense_retile_kernel<<<592, 256, 0, st>>>(w0, w1, n_out, K, w1 ? 2 : 1, static_cast<uint4*>(dst));
     return cudaGetLastError();
 }
 
@@ -288,8 +285,8 @@ __global__ void __launch_bounds__(64 + DG_EPI_WARPS * 32, 1) dense_gemm_kernel(c
                         const uint32_t f = 2 * fb * 128 + fl;
                         if (r < rows) {
                             float* o = P.out + (size_t)(tt * NT + r) * P.n_out + f;
-                            if (f < P.n_out) o[0] = v0[i];
-                            if (f + 128 < P.n_out) o[128] = v1[i];
+                            o[0] = v0[i];
+                            o[128] = v1[i];
                         }
                     }
                 }
@@ -388,10 +385,10 @@ __global__ void __launch_bounds__(64 + DG_EPI_WARPS * 32, 1) dense_gemm_kernel(c
                 }
                 *reinterpret_cast<uint4*>(P.hb + dg_b_off(P.n_out, NT, tt, rows16, r, fb * 128 + f8 * 8)) = make_uint4(h[0], h[1], h[2], h[3]);
             } else if (r < rows) {
-                const uint32_t f = 2 * fb * 128 + f8 * 8;           // n_out is a multiple of 8
+                const uint32_t f = 2 * fb * 128 + f8 * 8;
                 float4* o = reinterpret_cast<float4*>(P.out + (size_t)(tt * NT + r) * P.n_out + f);
-                if (f < P.n_out) { o[0] = make_float4(v[0], v[1], v[2], v[3]); o[1] = make_float4(v[4], v[5], v[6], v[7]); }
-                if (f + 128 < P.n_out) { o[32] = make_float4(v[8], v[9], v[10], v[11]); o[33] = make_float4(v[12], v[13], v[14], v[15]); }
+                o[0] = make_float4(v[0], v[1], v[2], v[3]); o[1] = make_float4(v[4], v[5], v[6], v[7]);
+                o[32] = make_float4(v[8], v[9], v[10], v[11]); o[33] = make_float4(v[12], v[13], v[14], v[15]);
             }
         }
         __syncwarp();
@@ -459,7 +456,7 @@ uint32_t dense_shared_rows(uint32_t T, uint32_t H, uint32_t I, int sm_count, con
     return dg_pick_rows(s, 2, T, sm_count, caps);
 }
 uint32_t dense_logits_rows(uint32_t T, uint32_t E, uint32_t H, int sm_count, const DenseCaps& caps) {
-    const DgShape s{(E + 255) / 256, H / DG_KS};
+    const DgShape s{E / 256, H / DG_KS};
     return dg_pick_rows(&s, 1, T, sm_count, caps);
 }
 // clusters of n CTAs that the device holds at once (an SM holds one CTA; clusters do not cross GPCs)
@@ -535,7 +532,7 @@ cudaError_t launch_dense_logits(const __nv_bfloat16* x, const void* w_tiled, uin
     if (e != cudaSuccess) return e;
     DenseParams P{};
     P.status = status; P.poll_limit = 1u << 20; P.limit = 0.f; P.T = T; P.nt = nt;
-    P.w = static_cast<const uint8_t*>(w_tiled); P.n_blocks = (E + 255) / 256 * 2; P.n_ks = H / DG_KS; P.xb = xb; P.K = H; P.hb = nullptr;
+    P.w = static_cast<const uint8_t*>(w_tiled); P.n_blocks = E / 128; P.n_ks = H / DG_KS; P.xb = xb; P.K = H; P.hb = nullptr;
     P.out = logits; P.n_out = E;
     return dg_launch<1>(P, sm_count, caps, st);
 }

@@ -34,7 +34,8 @@ def test_rows_of_an_expert_around_the_lanes_tiles(cls, limit, rows):
 
 @pytest.mark.parametrize("E", [16, 64, 120, 256, 288])
 def test_router_logits_around_the_change_of_kernel(E):
-    """16 and 17 tokens (row kernel, tensor-core product) and the product's token tiles, the expert count padded to 256."""
+    """Few tokens (rows staged), tiles of 8 x 8 and, for 256 experts, 64 and 65 (tiles, tensor-core product); expert counts
+    that leave a tile half empty."""
     import torch
     case = Exl3Case(640, 256, E, 4, seed=2, shared=False, max_tokens=1030, experts_to_load=[])
     try:
@@ -169,5 +170,35 @@ def test_dense_products_of_a_row_do_not_depend_on_the_batch(H, I):
             if T <= 256:
                 first = (y[:65], got[:65]) if first is None else first
                 assert (y[:65] == first[0]).all() and (got[:65] == first[1]).all(), T
+    finally:
+        case.close()
+
+
+@pytest.mark.parametrize("E,H", [(256, 4096), (252, 1152), (60, 640), (288, 2176)])
+def test_router_logits_keep_their_f32_sums(E, H):
+    """Up to 64 tokens, and at any count when the experts do not fill the tensor-core product's blocks, a token's logits are
+    the bits of a call of that token alone, and off a 64-bit product by no more than f32 sums of H / 128 terms per lane."""
+    import torch
+    case = Exl3Case(H, 128, E, 4, seed=2, shared=False, max_tokens=1030, experts_to_load=[])
+    try:
+        wg = O.f32_to_bf16_bits((np.random.default_rng(5).standard_normal((E, H)) * H ** -0.5).astype(np.float32))
+        case.moe.set_router_weight(0, wg.ctypes.data)
+        x, _ = case.inputs(1025, seed=7)
+        xd = case.to_dev_bf16(x)
+        ref = x.astype(np.float64) @ O.bf16_bits_to_f32(wg).astype(np.float64).T
+
+        def logits(t0, T):
+            lg = torch.full((T + 1, E), 7.0, dtype=torch.float32, device=case.dev)
+            case.moe.logits(0, xd.data_ptr() + t0 * H * 2, T, lg.data_ptr(), None)
+            torch.cuda.synchronize()
+            assert (lg[T] == 7.0).all()
+            return lg[:T].cpu().numpy()
+        one = np.concatenate([logits(t, 1) for t in range(80)])
+        for T in (4, 5, 8, 9, 16, 17, 25, 31, 64) + (() if E % 256 == 0 else (65, 200, 1025)):
+            got = logits(0, T)
+            assert (got[:80] == one[:T]).all(), T
+            # a lane's H / 128 sums, the butterfly's 5 and the fold's 3, as a random walk of roundings of 2^-24
+            assert rel_l2(got, ref[:T]) < 2.0 ** -24 * (H / 128 + 8) ** 0.5, T
+        assert case.status() == 0
     finally:
         case.close()
