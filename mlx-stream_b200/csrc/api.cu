@@ -585,6 +585,7 @@ static int logits_impl(mlxs_moe* h, uint32_t layer, const void* x_dev, uint32_t 
     if (rc) return rc;
     if (T == 0) return MLXS_OK;
     if (!x_dev || !logits_dev) return fail(MLXS_E_ARG, "logits: null buffer");
+    if ((rc = check_aligned(x_dev, 16, "logits", "x_dev")) || (rc = check_aligned(logits_dev, 4, "logits", "logits_dev"))) return rc;
     const mlxs_moe_config& c = h->cfg;
     LayerBank& L = h->layers[layer];
     if (!L.router_w) return fail(MLXS_E_NOT_LOADED, "logits: layer %u has no router weight (mlxs_moe_set_router_weight)", layer);

@@ -100,6 +100,7 @@ struct DenseParams {
     uint16_t* hb;              // gate/up: h in B-operand order over n_out inputs
     float* out;                // plain: [T, n_out] f32
     uint32_t n_out;
+    bool out_vec;              // out is 16-byte aligned (the caller's logits need only 4)
     uint32_t nt;               // rows per token tile (a multiple of 16)
     uint32_t n_stages;         // ring stages
     uint32_t k_parts;          // parts of the reduction, each summed by itself
@@ -386,9 +387,15 @@ __global__ void __launch_bounds__(64 + DG_EPI_WARPS * 32, 1) dense_gemm_kernel(c
                 *reinterpret_cast<uint4*>(P.hb + dg_b_off(P.n_out, NT, tt, rows16, r, fb * 128 + f8 * 8)) = make_uint4(h[0], h[1], h[2], h[3]);
             } else if (r < rows) {
                 const uint32_t f = 2 * fb * 128 + f8 * 8;
-                float4* o = reinterpret_cast<float4*>(P.out + (size_t)(tt * NT + r) * P.n_out + f);
-                o[0] = make_float4(v[0], v[1], v[2], v[3]); o[1] = make_float4(v[4], v[5], v[6], v[7]);
-                o[32] = make_float4(v[8], v[9], v[10], v[11]); o[33] = make_float4(v[12], v[13], v[14], v[15]);
+                float* o = P.out + (size_t)(tt * NT + r) * P.n_out + f;
+                if (P.out_vec) {
+                    float4* o4 = reinterpret_cast<float4*>(o);
+                    o4[0] = make_float4(v[0], v[1], v[2], v[3]); o4[1] = make_float4(v[4], v[5], v[6], v[7]);
+                    o4[32] = make_float4(v[8], v[9], v[10], v[11]); o4[33] = make_float4(v[12], v[13], v[14], v[15]);
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) { o[k] = v[k]; o[128 + k] = v[8 + k]; }
+                }
             }
         }
         __syncwarp();
@@ -482,6 +489,7 @@ template <int NPROJ>
 static cudaError_t dg_launch(DenseParams P, int sm_count, const DenseCaps& caps, cudaStream_t st) {
     const DgShape s{NPROJ == 2 ? P.n_blocks : P.n_blocks / 2, P.n_ks};
     double cost = 0;
+    P.out_vec = reinterpret_cast<uintptr_t>(P.out) % 16 == 0;
     P.k_parts = dg_parts(s, P.T, sm_count);
     P.n_cl = dg_pick_cluster(s, P.T, P.nt, sm_count, caps, &cost);
     if (!P.n_cl) return cudaErrorInvalidValue;

@@ -202,3 +202,32 @@ def test_router_logits_keep_their_f32_sums(E, H):
         assert case.status() == 0
     finally:
         case.close()
+
+
+def test_router_logits_into_a_buffer_of_four_byte_alignment():
+    """Logits need 4-byte alignment alone, at every count of tokens (row kernel, tiles, the tensor-core product with and
+    without a cluster): the same values as in an aligned buffer, and nothing beside them.  Less alignment, or rows of x off
+    16 bytes, is refused by name."""
+    import torch
+    case = Exl3Case(4096, 256, 256, 4, seed=2, shared=False, max_tokens=2400, experts_to_load=[])
+    try:
+        wg = O.f32_to_bf16_bits((np.random.default_rng(5).standard_normal((256, 4096)) * 4096 ** -0.5).astype(np.float32))
+        case.moe.set_router_weight(0, wg.ctypes.data)
+        x, _ = case.inputs(2400, seed=7)
+        xd = case.to_dev_bf16(x)
+        for T in (1, 17, 65, 200, 600, 2400):
+            a = torch.empty((T, 256), dtype=torch.float32, device=case.dev)
+            b = torch.full((T * 256 + 5,), 7.0, dtype=torch.float32, device=case.dev)
+            case.moe.logits(0, xd.data_ptr(), T, a.data_ptr(), None)
+            for off in (1, 2, 3):
+                b.fill_(7.0)
+                case.moe.logits(0, xd.data_ptr(), T, b.data_ptr() + 4 * off, None)
+                torch.cuda.synchronize()
+                assert torch.equal(b[off:off + T * 256], a.view(-1)), (T, off)
+                assert (b[:off] == 7.0).all() and (b[off + T * 256:] == 7.0).all(), (T, off)
+        for dx, dl, name in ((2, 0, "x_dev"), (8, 0, "x_dev"), (0, 2, "logits_dev")):
+            with pytest.raises(case.pkg.MlxsError, match=name):
+                case.moe.logits(0, xd.data_ptr() + dx, 70, b.data_ptr() + dl, None)
+        assert case.status() == 0
+    finally:
+        case.close()
