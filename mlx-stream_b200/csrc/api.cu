@@ -162,6 +162,7 @@ extern "C" int mlxs_moe_create(const mlxs_moe_config* c, mlxs_moe** out) {
             return bail(rc);
         if (cudaMemset(h->ks_count, 0, ksplit_count_words(h->sm_count) * 4) != cudaSuccess) return bail(fail(MLXS_E_CUDA, "create: cudaMemset failed"));
     } else {
+        if ((rc = h->alloc(&h->inf_flag, 4))) return bail(rc);
         if ((rc = h->alloc(&h->xa_gu, (size_t)max_chunks * (H / 32) * 512)) ||
             (rc = h->alloc(&h->xa_d, (size_t)max_chunks * (I / 32) * 512)) || (rc = h->alloc(&h->ro, A * H * 4)))
             return bail(rc);
@@ -300,6 +301,7 @@ extern "C" int mlxs_moe_load_expert(mlxs_moe* h, uint32_t layer, uint32_t expert
     }
     // the expert's entry of the per-expert table: 1 = resident; the FP4 repack may raise it to 3 (see takes_tensor_lane)
     const uint8_t one = 1;
+    uint32_t inf_scale = 0;
     CU(cudaMemcpyAsync(L.loaded_dev + le, &one, 1, cudaMemcpyHostToDevice, 0));
     if (is_exl3(h->cfg.bank_kind)) {
         const Exl3Dims d{h->cfg.hidden, h->cfg.inter, L.kbits};
@@ -307,12 +309,15 @@ extern "C" int mlxs_moe_load_expert(mlxs_moe* h, uint32_t layer, uint32_t expert
                               L.d_code + (size_t)le * exl3_code_words(d), L.scales + (size_t)le * exl3_scales_per_expert(d), 0));
     } else {
         const int nv = h->cfg.bank_kind == MLXS_BANK_NVFP4;
+        if (!nv) CU(cudaMemsetAsync(h->inf_flag, 0, 4, 0));
         CU(launch_fp4_repack(src, h->cfg.hidden, h->cfg.inter, nv,
                              L.f4_gu + (size_t)le * fp4_stream_bytes_per_expert(h->cfg.hidden, h->cfg.inter, nv, 0),
                              L.f4_dn + (size_t)le * fp4_stream_bytes_per_expert(h->cfg.hidden, h->cfg.inter, nv, 1),
-                             L.f4_gscale + (size_t)le * 3, L.loaded_dev + le, 0));
+                             L.f4_gscale + (size_t)le * 3, L.loaded_dev + le, nv ? nullptr : h->inf_flag, 0));
+        if (!nv) CU(cudaMemcpyAsync(&inf_scale, h->inf_flag, 4, cudaMemcpyDeviceToHost, 0));
     }
     CU(cudaStreamSynchronize(0));
+    L.inf_scales = L.inf_scales || inf_scale;
     L.loaded[expert] = 1;
     return MLXS_OK;
 }
@@ -718,7 +723,7 @@ int mlxs_run_routed(mlxs_moe* h, uint32_t layer, const void* x_dev, const int32_
         Fp4GemvArgs a{};
         a.gu = L.f4_gu; a.dn = L.f4_dn; a.nv = c.bank_kind == MLXS_BANK_NVFP4; a.gscale = a.nv ? L.f4_gscale : nullptr;
         a.H = c.hidden; a.I = c.inter; a.t = h->tabs; a.xa = h->xa_gu; a.xa_d = h->xa_d; a.ro = ro;
-        a.ro_bf16 = ro_bf16; a.limit = limit; a.dependent = !two_lanes;
+        a.ro_bf16 = ro_bf16; a.limit = limit; a.dependent = !two_lanes; a.inf_scales = L.inf_scales;
         a.status = h->status; a.sm_count = h->sm_count; a.ks_scratch = h->ks_scratch; a.ks_count = h->ks_count;
         {
             StageTimer tm(h, MLXS_STAGE_GATE_UP, st);

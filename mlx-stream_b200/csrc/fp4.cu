@@ -36,7 +36,7 @@ __host__ __device__ inline uint32_t f4_scale_stage_bytes(bool nv) { return nv ? 
 //   a thread of the tensor-core lane reads the four words of one output row (r, g) as one 16-byte load.
 __global__ void fp4_repack_kernel(const uint8_t* __restrict__ rec, uint32_t H, uint32_t I, int nv,
                                   uint8_t* __restrict__ gu, uint8_t* __restrict__ dn, float* __restrict__ gscale,
-                                  uint8_t* lane_flag) {
+                                  uint8_t* lane_flag, uint32_t* inf_flag) {
     const size_t wbytes = (size_t)H * I / 2, sbytes = (size_t)H * I / (nv ? 16 : 32), tail = nv ? 4 : 0;
     const size_t part = wbytes + sbytes + tail;
     const uint32_t sstage = f4_scale_stage_bytes(nv != 0);
@@ -70,14 +70,15 @@ __global__ void fp4_repack_kernel(const uint8_t* __restrict__ rec, uint32_t H, u
                 d[((wr * 4 + sb) * 8 + g) * 2 + r] = s[i];
                 // the tensor-core lane forms 2^(b-1) as a bf16: b > 128 keeps this expert in the streaming lane
                 if (lane_flag && s[i] > 128u) *lane_flag = 3;
+                if (inf_flag && s[i] == 255u) *inf_flag = 1;
             }
         }
     }
 }
 
 cudaError_t launch_fp4_repack(const uint8_t* record_dev, uint32_t H, uint32_t I, int nv, uint8_t* gu_e, uint8_t* dn_e,
-                              float* gscale_e, uint8_t* lane_flag, cudaStream_t st) {
-    fp4_repack_kernel<<<592, 256, 0, st>>>(record_dev, H, I, nv, gu_e, dn_e, gscale_e, lane_flag);
+                              float* gscale_e, uint8_t* lane_flag, uint32_t* inf_flag, cudaStream_t st) {
+    fp4_repack_kernel<<<592, 256, 0, st>>>(record_dev, H, I, nv, gu_e, dn_e, gscale_e, lane_flag, inf_flag);
     return cudaGetLastError();
 }
 
@@ -156,8 +157,10 @@ __device__ __forceinline__ uint32_t hmul2_u32(uint32_t a, __half2 s) {
 
 // One ring slot of SUB 128-input sub-stages: [sub-stage][projection codes, projection scales], then the rows [chunk][sub-stage].
 // w, sc: this lane's first code word and scale pair of the slot; xs: its first row word.  The block scales come through the
-// conversion instructions (two bytes at once: this lane's two output rows).
-template <int NPROJ, bool NV, int MC, int SUB>
+// conversion instructions (two bytes at once: this lane's two output rows).  INF: an MXFP4 layer in which a scale byte is 255,
+// the infinity that its bits are (src/arch/mimo_v2/moe.zig:410-413); the conversion gives a NaN, which the minimum with infinity
+// puts right.  A form of its own: the one instruction costs every other bank 3 to 6 %.
+template <int NPROJ, bool NV, bool INF, int MC, int SUB>
 __device__ __forceinline__ void fp4_slot(const uint32_t* __restrict__ wv, const uint8_t* __restrict__ sc, const uint4* __restrict__ xv,
                                          float (&acc)[F4_GROUP][4]) {
     constexpr uint32_t W_BYTES = NPROJ * (F4_W_STAGE + (NV ? 1024u : 512u));
@@ -183,6 +186,7 @@ __device__ __forceinline__ void fp4_slot(const uint32_t* __restrict__ wv, const 
                 uint32_t s2;
                 const uint16_t bb = *reinterpret_cast<const uint16_t*>(sc + u * W_BYTES + sb * 16);
                 asm("cvt.rn.bf16x2.ue8m0x2 %0, %1;" : "=r"(s2) : "h"(bb));
+                if (INF) asm("min.bf16x2 %0, %0, %1;" : "+r"(s2) : "r"(0x7F807F80u));
                 s_lo = __uint_as_float(s2 << 16);
                 s_hi = __uint_as_float(s2 & 0xFFFF0000u);
             }
@@ -210,7 +214,7 @@ __device__ __forceinline__ float sigmoid_ref(float x) {  // src/arch/mimo_v2/moe
     return x < 0.f ? y : 1.0f - y;
 }
 
-template <int NPROJ, bool NV>
+template <int NPROJ, bool NV, bool INF>
 __global__ void __launch_bounds__(NPROJ * 256 + 32, NPROJ == 1 ? 3 : 2) fp4_gemv_kernel(const Fp4Params P) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     constexpr int NCW = NPROJ * 8;
@@ -347,13 +351,13 @@ __global__ void __launch_bounds__(NPROJ * 256 + 32, NPROJ == 1 ? 3 : 2) fp4_gemv
         const uint8_t* sc = st + s_off;
         const uint4* xv = reinterpret_cast<const uint4*>(st + x_off);
         if (flags & 8u) {
-            if (P.sub == 2) fp4_slot<NPROJ, NV, 2, 2>(wv, sc, xv, acc);
-            else if (P.sub == 4) fp4_slot<NPROJ, NV, 2, 4>(wv, sc, xv, acc);
-            else fp4_slot<NPROJ, NV, 2, 1>(wv, sc, xv, acc);
+            if (P.sub == 2) fp4_slot<NPROJ, NV, INF, 2, 2>(wv, sc, xv, acc);
+            else if (P.sub == 4) fp4_slot<NPROJ, NV, INF, 2, 4>(wv, sc, xv, acc);
+            else fp4_slot<NPROJ, NV, INF, 2, 1>(wv, sc, xv, acc);
         } else {
-            if (P.sub == 2) fp4_slot<NPROJ, NV, 1, 2>(wv, sc, xv, acc);
-            else if (P.sub == 4) fp4_slot<NPROJ, NV, 1, 4>(wv, sc, xv, acc);
-            else fp4_slot<NPROJ, NV, 1, 1>(wv, sc, xv, acc);
+            if (P.sub == 2) fp4_slot<NPROJ, NV, INF, 1, 2>(wv, sc, xv, acc);
+            else if (P.sub == 4) fp4_slot<NPROJ, NV, INF, 1, 4>(wv, sc, xv, acc);
+            else fp4_slot<NPROJ, NV, INF, 1, 1>(wv, sc, xv, acc);
         }
         // the slot may be refilled once this warp has arrived below
         F4Meta m;
@@ -513,19 +517,14 @@ cudaError_t launch_fp4_gemv(const Fp4GemvArgs& a, int down, cudaStream_t st) {
     P.n_ring = ns;
     const size_t smem = zs_bytes + (size_t)ns * P.stage_bytes;
     const int ctas = per_sm * a.sm_count;
-    cudaError_t e;
-#define MLXS_F4_LAUNCH(NP, NVV)                                                                               \
-    do {                                                                                                      \
-        e = cudaFuncSetAttribute(fp4_gemv_kernel<NP, NVV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-        if (e != cudaSuccess) return e;                                                                       \
-        e = launch_dependent(!down || a.dependent, fp4_gemv_kernel<NP, NVV>, ctas, NP * 256 + 32, smem, st, P); \
-        if (e != cudaSuccess) return e;                                                                       \
-    } while (0)
-    if (!down && a.nv) MLXS_F4_LAUNCH(2, true);
-    else if (!down) MLXS_F4_LAUNCH(2, false);
-    else if (a.nv) MLXS_F4_LAUNCH(1, true);
-    else MLXS_F4_LAUNCH(1, false);
-#undef MLXS_F4_LAUNCH
+    auto launch = [&](auto kernel) -> cudaError_t {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        return e != cudaSuccess ? e : launch_dependent(!down || a.dependent, kernel, ctas, nproj * 256 + 32, smem, st, P);
+    };
+    const cudaError_t e = a.nv ? (down ? launch(fp4_gemv_kernel<1, true, false>) : launch(fp4_gemv_kernel<2, true, false>))
+                          : a.inf_scales ? (down ? launch(fp4_gemv_kernel<1, false, true>) : launch(fp4_gemv_kernel<2, false, true>))
+                                         : (down ? launch(fp4_gemv_kernel<1, false, false>) : launch(fp4_gemv_kernel<2, false, false>));
+    if (e != cudaSuccess) return e;
     return cudaGetLastError();
 }
 

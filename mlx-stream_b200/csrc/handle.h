@@ -21,6 +21,7 @@ struct LayerBank {
     __half* scales = nullptr;
     uint8_t *f4_gu = nullptr, *f4_dn = nullptr;  // FP4 banks: the two streams
     float* f4_gscale = nullptr;                  // NVFP4 [E_local][3]
+    bool inf_scales = false;                     // MXFP4: an expert loaded here holds a scale of byte 255
     uint8_t* loaded_dev = nullptr;  // [E_local] per local slot: 1 = loaded (bit 1: see takes_tensor_lane)
     std::vector<uint8_t> loaded;    // [E] by expert id, host copy
     // EXL3: this layer's bits per weight and record size (a bank may mix widths; mlxs_moe_set_layer_bits)
@@ -73,6 +74,7 @@ struct mlxs_moe {
     float* logits_ws = nullptr;       // [max_tokens, E] logits of mlxs_moe_forward_x
     float* ks_scratch = nullptr;      // K-split workspace of the streaming kernels (exl3.cu)
     uint32_t* ks_count = nullptr;
+    uint32_t* inf_flag = nullptr;     // what a load found in its record (launch_fp4_repack)
     cudaStream_t aux_stream = nullptr;
     cudaEvent_t aux_fork = nullptr, aux_join = nullptr;
     // the tensor-core lane runs on a stream of its own beside the streaming lane

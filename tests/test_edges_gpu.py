@@ -231,3 +231,28 @@ def test_router_logits_into_a_buffer_of_four_byte_alignment():
         assert case.status() == 0
     finally:
         case.close()
+
+
+@pytest.mark.parametrize("scale", [253, 254, 255])
+def test_mxfp4_scale_bytes_beyond_f32(scale):
+    """Block scales whose products leave f32: the gate saturates at the activation's limit, byte 255 too (2^128, an infinity,
+    and no NaN), in every form of the streaming kernel; with 20 rows an expert of such scales still streams."""
+    H, I = 512, 256
+    case = Mxfp4Case(H, I, 2, 1, seed=4, shared=False, scoring=O.SCORE_SIGMOID, max_tokens=32, routed_scale=1.0, limit=10.0, chain=True)
+    try:
+        off = O.mxfp4_record_bytes(H, I)[1]
+        rec = case.records[0].copy()
+        rec[off[0]:off[0] + H * I // 2] = 0x77         # the gate projection: 6 everywhere
+        rec[off[1]:off[1] + H * I // 32] = scale
+        case.records[0] = rec
+        case.moe.load_expert(0, 0, rec.ctypes.data, rec.size, on_device=False)
+        for T in (1, 7, 9, 16, 20):
+            x, _ = case.inputs(T, seed=T)
+            x = np.abs(x) + 0.125
+            x = O.bf16_bits_to_f32(O.f32_to_bf16_bits(x.astype(np.float32)))
+            ids, w = np.zeros((T, 1), np.int32), np.ones((T, 1), np.float32)
+            y = case.gpu_experts(x, ids, w)
+            assert case.status() == 0 and np.isfinite(y).all(), T
+            assert rel_l2(y, case.cpu_layer(x, ids, w)) < 1e-2, T
+    finally:
+        case.close()
