@@ -93,6 +93,7 @@ extern "C" int mlxs_moe_create(const mlxs_moe_config* c, mlxs_moe** out) {
     if (!h) return fail(MLXS_E_ARG, "create: out of host memory");
     h->cfg = *c;
     h->sm_count = prop.multiProcessorCount;
+    h->front_smem_max = prop.sharedMemPerBlockOptin - 1024;   // less what the kernel holds statically
     h->e_local = c->n_experts / c->ep_world;
     h->e_first = c->ep_rank * h->e_local;
     const uint64_t H = c->hidden, I = c->inter;
@@ -328,11 +329,11 @@ struct FrontCall {
 };
 
 // Can this call take the fused front kernel (front.cu)?  One rank, a decode-sized batch, no route tally to feed.  MLXS_FRONT_MAX moves the batch limit (0: never).
-static bool front_applies(const mlxs_moe* h, uint32_t T) {
+static bool front_applies(const mlxs_moe* h, uint32_t T, bool from_x) {
     static const uint32_t front_max = getenv("MLXS_FRONT_MAX") ? (uint32_t)atoi(getenv("MLXS_FRONT_MAX")) : 16u;
     if (T == 0 || T > front_max || h->cfg.ep_world != 1 || h->usage_on || h->front_off) return false;
     if (T * h->cfg.top_k > 2048) return false;
-    return true;
+    return front_fits((int)h->cfg.n_experts, (int)h->cfg.top_k, T, h->cfg.hidden, from_x, h->front_smem_max);
 }
 
 static int experts_impl(mlxs_moe* h, uint32_t layer, const void* x_dev, const int32_t* ids_dev, const float* weights_dev,
@@ -615,7 +616,7 @@ extern "C" int mlxs_moe_logits(mlxs_moe* h, uint32_t layer, const void* x_dev, u
 extern "C" int mlxs_moe_forward_x(mlxs_moe* h, uint32_t layer, const void* x_dev, uint32_t T, void* y_dev, void* stream) {
     if (!h) return fail(MLXS_E_ARG, "forward_x: null handle");
     if (!h->logits_ws) return fail(MLXS_E_NOT_LOADED, "forward_x: no router weight was set (mlxs_moe_set_router_weight)");
-    if (layer < h->cfg.n_layers && front_applies(h, T)) {
+    if (layer < h->cfg.n_layers && front_applies(h, T, true)) {
         // decode-sized: the logits product is the first phase of the fused front kernel (no [T, E] round trip, no launch)
         if (!h->layers[layer].router_w) return fail(MLXS_E_NOT_LOADED, "forward_x: layer %u has no router weight (mlxs_moe_set_router_weight)", layer);
         const FrontCall fc{nullptr};
@@ -820,17 +821,17 @@ static int experts_impl(mlxs_moe* h, uint32_t layer, const void* x_dev, const in
         fa.heavy = (h->pf_tiles && T >= h->pf_min_rows) ? h->pf_min_rows : 0u;   // the lane choice of mlxs_run_routed
         fa.x = static_cast<const __nv_bfloat16*>(x_dev); fa.H = c.hidden; fa.bank_exl3 = is_exl3(c.bank_kind) ? 1 : 0;
         fa.scales = L.scales; fa.scales_stride = is_exl3(c.bank_kind) ? exl3_scales_per_expert(Exl3Dims{c.hidden, c.inter, L.kbits}) : 0;
-        fa.xa = h->xa_gu; fa.bar = h->front_bar;
+        fa.xa = h->xa_gu; fa.bar = h->front_bar; fa.smem_max = h->front_smem_max;
         StageTimer tm(h, MLXS_STAGE_ROUTER, st);
         const cudaError_t fe = launch_front(fa, st);
         h->stats.route_calls += 1;
         if (fe == cudaSuccess) {
             h->front_done = true;
         } else {
-            // the cooperative launch was refused (no room for all of its CTAs at once): the same work as separate
-            // kernels, now and from here on
+            // refused: the same work as separate kernels; from here on too where the device has no room for all CTAs of a
+            // cooperative launch at once
             cudaGetLastError();
-            h->front_off = true;
+            if (fe == cudaErrorCooperativeLaunchTooLarge) h->front_off = true;
             const float* lg = front->logits;
             if (!lg) {
                 CU(launch_router_logits(fa.x, L.router_w, T, c.n_experts, c.hidden, h->logits_ws, st));
@@ -874,7 +875,7 @@ extern "C" int mlxs_moe_experts(mlxs_moe* h, uint32_t layer, const void* x_dev, 
 
 extern "C" int mlxs_moe_forward(mlxs_moe* h, uint32_t layer, const void* x_dev, const float* logits_dev, uint32_t T,
                                 void* y_dev, void* stream) {
-    if (h && layer < h->cfg.n_layers && front_applies(h, T)) {
+    if (h && layer < h->cfg.n_layers && front_applies(h, T, false)) {
         if (!logits_dev) return fail(MLXS_E_ARG, "forward: null buffer");
         int rc = check_aligned(logits_dev, 4, "forward", "logits_dev");
         if (rc) return rc;

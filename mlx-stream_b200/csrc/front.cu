@@ -10,7 +10,8 @@
 //   phase 3: all warps stage the rows for the streaming lane (the prep kernels' code).
 // Phases 1 and 2 are a few microseconds whoever does them; done by every CTA for itself they cost no grid barrier (two of
 // them, with the round trips of ids and tables through L2, were half of the 17 us this kernel took at one token), and without
-// phase 0 the launch is an ordinary one.  More than 256 experts or top_k > 32: a CTA per token routes, then a barrier.
+// phase 0 the launch is an ordinary one.  More than 256 experts, top_k > 32, or more tokens than shared memory holds scores of
+// (165 at 256 experts and top-8): a CTA per token routes, then a barrier.
 // The grid barrier is a counter and a generation word in global memory: the last CTA to arrive resets the counter and
 // bumps the generation, the others poll the generation with a bound.  A launch with a barrier is cooperative, so all CTAs
 // are resident together; a barrier that runs out still records the status word and lets the kernel finish.
@@ -197,13 +198,20 @@ __global__ void __launch_bounds__(1024, 1) front_kernel(const FrontParams P) {
     }
 }
 
+static int front_route_threads(int E, int K) { return ((E > K ? E : K) + 31) / 32 * 32; }
 // smem: the larger of the phases' needs
-static size_t front_smem_bytes(const FrontArgs& a, int rthreads) {
-    size_t s = router_smem_floats(a.E, a.K, rthreads) * sizeof(float);
-    const size_t d = ((size_t)8 * a.T * a.K + (size_t)a.E + 17 + dispatch_words(a.T * (uint32_t)a.K, (uint32_t)a.E) + (size_t)a.T * (a.E + 2)) * sizeof(uint32_t);
+static size_t front_smem_bytes(int E, int K, uint32_t T, uint32_t H, bool from_x, bool by_warp) {
+    size_t s = router_smem_floats(E, K, front_route_threads(E, K)) * sizeof(float);
+    const size_t d = ((size_t)8 * T * K + (size_t)E + 17 + dispatch_words(T * (uint32_t)K, (uint32_t)E) + (by_warp ? (size_t)T * (E + 2) : 0)) * sizeof(uint32_t);
     if (d > s) s = d;
-    if (a.w_router) { const size_t l = logits_smem_bytes(a.H, 32); if (l > s) s = l; }
+    if (from_x) { const size_t l = logits_smem_bytes(H, 32); if (l > s) s = l; }
     return s;
+}
+static bool front_by_warp(int E, int K, uint32_t T, uint32_t H, bool from_x, size_t smem_max) {
+    return route_by_warp(E, K) && front_smem_bytes(E, K, T, H, from_x, true) <= smem_max;
+}
+bool front_fits(int E, int K, uint32_t T, uint32_t H, bool from_x, size_t smem_max) {
+    return front_smem_bytes(E, K, T, H, from_x, front_by_warp(E, K, T, H, from_x, smem_max)) <= smem_max;
 }
 
 cudaError_t launch_front(const FrontArgs& a, cudaStream_t st) {
@@ -214,12 +222,11 @@ cudaError_t launch_front(const FrontArgs& a, cudaStream_t st) {
     P.loaded = a.loaded; P.t = a.t; P.chunk_rows = a.chunk_rows; P.group_chunks = a.group_chunks; P.heavy = a.heavy; P.status = a.status;
     P.x = a.x; P.H = a.H; P.bank_exl3 = a.bank_exl3; P.scales = a.scales; P.scales_stride = a.scales_stride; P.xa = a.xa;
     P.bar = a.bar; P.poll_limit = 1u << 22;
-    const int rt = ((a.E > a.K ? a.E : a.K) + 31) / 32 * 32;
-    P.rthreads = rt;
-    const size_t smem = front_smem_bytes(a, rt);
+    P.rthreads = front_route_threads(a.E, a.K);
+    P.by_warp = front_by_warp(a.E, a.K, a.T, a.H, a.w_router, a.smem_max) ? 1 : 0;
+    const size_t smem = front_smem_bytes(a.E, a.K, a.T, a.H, a.w_router, P.by_warp);
     cudaError_t e = cudaFuncSetAttribute(front_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    P.by_warp = route_by_warp(a.E, a.K) ? 1 : 0;
     const bool barrier = a.w_router || !P.by_warp;
     // a warp per staging task (a row's 128-block, or a quarter of a row for the FP4 banks), at most a CTA per SM; with a
     // barrier 32 to 64 CTAs: one round of expert rows, and room beside the shared expert's kernels

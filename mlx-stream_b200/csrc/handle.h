@@ -93,6 +93,7 @@ struct mlxs_moe {
     bool front_done = false;          // the fused front kernel of this call has built the tables and staged the rows
     bool mxfp4_native = false;        // MXFP4 tensor-core lane on the block-scaled kind (MLXS_MXFP4_NATIVE=1 at create) instead of the decoded-operand lane
     bool front_off = false;           // a cooperative launch was refused once: separate kernels from then on
+    size_t front_smem_max = 0;        // shared memory that the front kernel may ask for
     uint32_t dbg_poll_limit = 0, dbg_withhold = 0;  // mlxs_moe_debug_wait (self-test of the bounded waits)
     uint32_t rows_cap = 0;  // rows the expert kernels' workspaces hold (assignments of one call, or received rows)
     // per-stage timing (off by default)

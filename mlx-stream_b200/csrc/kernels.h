@@ -61,7 +61,9 @@ struct FrontArgs {
     uint32_t* xa;
     uint32_t* bar;
     int sm_count;
+    size_t smem_max;                // dynamic shared memory that a block may ask for
 };
+bool front_fits(int E, int K, uint32_t T, uint32_t H, bool from_x, size_t smem_max);   // does a call's front fit that?
 cudaError_t launch_front(const FrontArgs& a, cudaStream_t st);
 
 // ids [A] (A = T*k) -> tables; expert ids outside [0, E) set *status and are treated as expert 0.

@@ -256,3 +256,41 @@ def test_mxfp4_scale_bytes_beyond_f32(scale):
             assert rel_l2(y, case.cpu_layer(x, ids, w)) < 1e-2, T
     finally:
         case.close()
+
+
+FRONT_SCRIPT = r"""
+import sys
+import numpy as np
+sys.path.insert(0, "tests")
+import oracle_lib as O
+from moe_cases import Exl3Case
+E, k, counts = int(sys.argv[1]), int(sys.argv[2]), [int(t) for t in sys.argv[3].split(",")]
+case = Exl3Case(256, 128, E, k, seed=6, shared=False, scoring=O.SCORE_SOFTMAX, max_tokens=256)
+wg = O.f32_to_bf16_bits((np.random.default_rng(5).standard_normal((E, 256)) / 16).astype(np.float32))
+case.moe.set_router_weight(0, wg.ctypes.data)
+case.moe.profile_enable(True)
+for T in counts:
+    x, logits = case.inputs(T, seed=T)
+    case.moe.profile_read()
+    y = case.gpu_forward(x, logits)
+    fused = case.moe.profile_read()["dispatch"][1] == 0
+    assert fused == (T * k <= 2048), T
+    ids, w = case.gpu_route(logits)
+    assert (ids == case.cpu_route(logits)[0]).all(), T
+    assert (y == case.gpu_experts(x, ids, w)).all(), T
+    assert case.status() == 0
+print("ok")
+"""
+
+
+@pytest.mark.parametrize("E,k,counts", [(256, 8, "164,165,166,200,256,1"), (256, 16, "128,129,1"), (1024, 8, "64,256,1"), (1024, 64, "32,1")])
+def test_front_of_more_tokens_than_shared_memory_holds_scores_of(E, k, counts):
+    """With the front's limit raised (in a process of its own: the limit is read once), up to 2048 assignments start with the
+    fused kernel whatever the experts, and a call that does not leaves it to the calls after it."""
+    import os
+    import subprocess
+    import sys
+    from pathlib import Path
+    r = subprocess.run([sys.executable, "-c", FRONT_SCRIPT, str(E), str(k), counts], cwd=Path(__file__).resolve().parent.parent,
+                       env=dict(os.environ, MLXS_FRONT_MAX="256"), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "ok" in r.stdout, r.stderr[-2000:]
