@@ -176,7 +176,6 @@ extern "C" int mlxs_moe_create(const mlxs_moe_config* c, mlxs_moe** out) {
         // tensor-core lane up to 192; the two lanes run side by side, so the row count from which an expert takes the
         // tensor-core lane is the one that evens them out.
         const bool exl3 = is_exl3(c->bank_kind);
-        if (const char* nv = getenv("MLXS_MXFP4_NATIVE")) h->mxfp4_native = atoi(nv) != 0;
         // measured (24-layer Zipf stack at 64 tokens, EXL3: 9 rows 14.20, 13 rows 14.28, 17 rows 14.79, 21 rows 15.42 ms;
         // FP4 banks are within 1.5 % either way between 13 and 17)
         const char* ev = getenv("MLXS_PREFILL_MIN_ROWS");
@@ -186,12 +185,8 @@ extern "C" int mlxs_moe_create(const mlxs_moe_config* c, mlxs_moe** out) {
             h->pf_min_rows = (uint32_t)min_rows;
             const size_t heavy_max = A / (size_t)min_rows < h->e_local ? A / (size_t)min_rows : h->e_local;
             h->pf_max_tiles = (uint32_t)(A / PREFILL_TILE_ROWS + heavy_max + 1);
-            size_t xa_bytes = exl3 ? exl3_prefill_xa_bytes(d, A, h->pf_max_tiles) : fp4_prefill_xa_bytes(c->hidden, A, h->pf_max_tiles);
-            size_t xd_bytes = exl3 ? exl3_prefill_xd_bytes(d, A, h->pf_max_tiles) : fp4_prefill_xa_bytes(c->inter, A, h->pf_max_tiles);
-            if (h->mxfp4_native && c->bank_kind == MLXS_BANK_MXFP4) {   // the block-scaled lane stages 132 bytes per row per 64 inputs
-                xa_bytes = std::max(xa_bytes, mxfp4_native_xa_bytes(c->hidden, A, h->pf_max_tiles));
-                xd_bytes = std::max(xd_bytes, mxfp4_native_xa_bytes(c->inter, A, h->pf_max_tiles));
-            }
+            const size_t xa_bytes = exl3 ? exl3_prefill_xa_bytes(d, A, h->pf_max_tiles) : fp4_prefill_xa_bytes(c->hidden, A, h->pf_max_tiles);
+            const size_t xd_bytes = exl3 ? exl3_prefill_xd_bytes(d, A, h->pf_max_tiles) : fp4_prefill_xa_bytes(c->inter, A, h->pf_max_tiles);
             if ((rc = h->alloc(&h->pf_tiles, prefill_tile_words(h->pf_max_tiles) * 4)) || (rc = h->alloc(&h->pf_xa, xa_bytes)) ||
                 (rc = h->alloc(&h->pf_xd, xd_bytes)))
                 return bail(rc);
@@ -209,10 +204,7 @@ extern "C" int mlxs_moe_create(const mlxs_moe_config* c, mlxs_moe** out) {
             cudaEventCreateWithFlags(&h->aux_join, cudaEventDisableTiming) != cudaSuccess ||
             cudaStreamCreateWithFlags(&h->lane_stream, cudaStreamNonBlocking) != cudaSuccess ||
             cudaEventCreateWithFlags(&h->lane_fork, cudaEventDisableTiming) != cudaSuccess ||
-            cudaEventCreateWithFlags(&h->lane_join, cudaEventDisableTiming) != cudaSuccess ||
-            cudaStreamCreateWithFlags(&h->lane2_stream, cudaStreamNonBlocking) != cudaSuccess ||
-            cudaEventCreateWithFlags(&h->lane2_fork, cudaEventDisableTiming) != cudaSuccess ||
-            cudaEventCreateWithFlags(&h->lane2_join, cudaEventDisableTiming) != cudaSuccess)
+            cudaEventCreateWithFlags(&h->lane_join, cudaEventDisableTiming) != cudaSuccess)
             return bail(fail(MLXS_E_CUDA, "create: second stream"));
     }
     if (cudaDeviceSynchronize() != cudaSuccess) return bail(fail(MLXS_E_CUDA, "create: device synchronize failed"));
@@ -227,9 +219,6 @@ extern "C" void mlxs_moe_destroy(mlxs_moe* h) {
     mlxs_ep_destroy(h);
     if (h->lane_fork) cudaEventDestroy(h->lane_fork);
     if (h->lane_join) cudaEventDestroy(h->lane_join);
-    if (h->lane2_fork) cudaEventDestroy(h->lane2_fork);
-    if (h->lane2_join) cudaEventDestroy(h->lane2_join);
-    if (h->lane2_stream) cudaStreamDestroy(h->lane2_stream);
     if (h->aux_fork) cudaEventDestroy(h->aux_fork);
     if (h->aux_join) cudaEventDestroy(h->aux_join);
     if (h->aux_stream) cudaStreamDestroy(h->aux_stream);
@@ -710,12 +699,8 @@ int mlxs_run_routed(mlxs_moe* h, uint32_t layer, const void* x_dev, const int32_
             pa.xa = reinterpret_cast<uint16_t*>(h->pf_xa); pa.xd = reinterpret_cast<uint16_t*>(h->pf_xd);
             pa.ro = ro; pa.ro_bf16 = ro_bf16; pa.limit = limit; pa.status = h->status; pa.sm_count = h->sm_count;
             pa.act = h->pf_act;
-            if (lane_aside) { pa.side = h->lane2_stream; pa.side_fork = h->lane2_fork; pa.side_join = h->lane2_join; }
             StageTimer tm(h, MLXS_STAGE_TENSOR_LANE, tl);
-            // MXFP4 decodes to bf16 operands like NVFP4 to f16 ones; the block-scaled tensor-core kind on the codes as stored is
-            // opt-in (MLXS_MXFP4_NATIVE=1 at create): 8.0 against 6.4 ms at 16384 tokens, 1.68 against 1.38 ms at 2048
-            if (!pa.nv && h->mxfp4_native) CU(launch_mxfp4_native(pa, tl));
-            else CU(launch_fp4_prefill(pa, tl));
+            CU(launch_fp4_prefill(pa, tl));
         }
         if (!front_done) {
             StageTimer tm(h, MLXS_STAGE_PREP, st);

@@ -25,11 +25,7 @@ namespace mlxs {
 // ------------------------------------------------------------------------------------------------------------
 // plan: row tiles per expert from the dispatch tables
 // ------------------------------------------------------------------------------------------------------------
-// Tile table: [2] = most rows of a tile of list 0 (a multiple of 16); [3], [4] = items that the gate/up, the down kernel has
-// given out; [0] = tiles of list 0 (experts with up to cap0 rows: one tile each; with cap1 = 0 every expert, in tiles
-// of up to cap0 rows), [1] = tiles of list 1 (the other experts, tiles of up to cap1 rows), then the entries {expert,
-// first sorted row, rows, first staging row}: list 0 from entry 0, list 1 from entry max_tiles.  An expert's rows are
-// split evenly over its tiles (a 16-row remainder tile would cost a full decode).
+// An expert's rows are split evenly over its tiles (a 16-row remainder tile would cost a full decode).
 // Staging rows: a tile's rows padded to 16, tiles in sorted order, so tile number n starts at its first row + 16 n.
 // narrow: with tiles of up to that many rows the lane has another operand slot (lane.cuh), worth about as much as a
 // twentieth of the tiles: taken when the call gets at most one tile in sixteen more.  (300 Zipf-routed tokens, one expert
@@ -37,31 +33,28 @@ namespace mlxs {
 // it were taken there.)
 // One thread per expert; with one thread adding up the tile counts the kernel took 8 us for 256 experts.
 __global__ void __launch_bounds__(DTHREADS) pf_plan_kernel(DispatchTables t, uint32_t E, const uint8_t* __restrict__ flags, uint32_t min_rows,
-                                                           uint32_t cap0, uint32_t cap1, uint32_t narrow, uint32_t max_tiles,
-                                                           uint32_t* __restrict__ tiles, uint32_t* status) {
+                                                           uint32_t cap, uint32_t narrow, uint32_t max_tiles, uint32_t* __restrict__ tiles,
+                                                           uint32_t* status) {
     __shared__ uint32_t ws[99], s_most;
     const uint32_t e = threadIdx.x;
     if (e == 0) s_most = 0;
     const uint32_t r0 = e < E ? t.offsets[e] : 0u, c = e < E ? t.offsets[e + 1] - r0 : 0u;
-    const bool lane = e < E && takes_tensor_lane(c, min_rows, flags, e), list1 = cap1 && c > cap0;
-    const uint32_t v[3] = {lane && !list1 ? (c + cap0 - 1) / cap0 : 0u, lane && list1 ? (c + cap1 - 1) / cap1 : 0u,
-                           lane && narrow ? (c + narrow - 1) / narrow : 0u};
+    const bool lane = e < E && takes_tensor_lane(c, min_rows, flags, e);
+    const uint32_t v[3] = {lane ? (c + cap - 1) / cap : 0u, lane ? (c + narrow - 1) / narrow : 0u, 0u};
     uint32_t base[3], tot[3];
     block_scan3(v, base, tot, ws);
-    const int k = narrow && tot[2] * 16u <= tot[0] * 17u ? 2 : 0;   // the scan that list 0 goes by
-    const bool ok = tot[k] <= max_tiles && tot[1] <= max_tiles;
-    const uint32_t nt = list1 ? v[1] : v[k], first = list1 ? base[1] : base[k], ordinal = base[k] + base[1];
-    const uint32_t per = nt ? ((c + nt - 1) / nt + 15) / 16 * 16 : 0u;
-    if (!list1 && nt) atomicMax(&s_most, per);
+    const int k = tot[1] * 16u <= tot[0] * 17u ? 1 : 0;
+    const bool ok = tot[k] <= max_tiles;
+    const uint32_t nt = v[k], first = base[k], per = nt ? ((c + nt - 1) / nt + 15) / 16 * 16 : 0u;
+    if (nt) atomicMax(&s_most, per);
     if (ok)
         for (uint32_t i = 0; i < nt; ++i)
-            *reinterpret_cast<uint4*>(prefill_tile(tiles, list1 ? 1 : 0, max_tiles, first + i)) =
-                make_uint4(e, r0 + i * per, min(per, c - i * per), r0 + i * per + 16 * (ordinal + i));
+            *reinterpret_cast<uint4*>(prefill_tile(tiles, first + i)) =
+                make_uint4(e, r0 + i * per, min(per, c - i * per), r0 + i * per + 16 * (first + i));
     __syncthreads();
     if (e == 0) {
         if (!ok) atomicMax(status, (uint32_t)ST_WORKLIST_OVERFLOW);
         tiles[0] = ok ? tot[k] : 0u;
-        tiles[1] = ok ? tot[1] : 0u;
         tiles[2] = s_most;
         tiles[3] = tiles[4] = 0;
     }
@@ -140,11 +133,10 @@ __device__ __forceinline__ void pf_load_scale4(const __half* p, uint32_t lane, f
 constexpr int PREP_WARPS = 8;
 __global__ void __launch_bounds__(PREP_WARPS * 32, 3) pf_prep_kernel(const __nv_bfloat16* __restrict__ x, uint32_t top_k, uint32_t H,
                                                                   const __half* __restrict__ scales, size_t scales_stride,
-                                                                  DispatchTables t, const uint32_t* __restrict__ tiles, uint32_t max_tiles,
-                                                                  size_t proj_stride, __half* __restrict__ xa) {
+                                                                  DispatchTables t, const uint32_t* __restrict__ tiles, size_t proj_stride, __half* __restrict__ xa) {
     const uint32_t tile = blockIdx.x;
     if (tile >= tiles[0]) return;
-    const uint32_t* te = prefill_tile(tiles, 0, max_tiles, tile);
+    const uint32_t* te = prefill_tile(tiles, tile);
     const uint32_t e = te[0], row0 = te[1], rows = te[2];
     const uint32_t rows16 = (rows + 15) / 16 * 16, warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, nblk = H / 128;
     const uint32_t r8 = lane >> 2, seg = lane & 3u;
@@ -377,18 +369,17 @@ bool exl3_prefill_supported(Exl3Dims d) { return d.I % LN_KST == 0 && d.H % LN_K
 
 size_t lane_act_bytes(int sm_count) { return (size_t)sm_count * LN_ACT_BYTES; }
 
-cudaError_t launch_prefill_plan(DispatchTables t, uint32_t n_experts, const uint8_t* lane_flags, uint32_t min_rows,
-                                uint32_t cap0, uint32_t cap1, uint32_t narrow, uint32_t max_tiles, uint32_t* tiles,
-                                uint32_t* status, cudaStream_t st) {
+cudaError_t launch_prefill_plan(DispatchTables t, uint32_t n_experts, const uint8_t* lane_flags, uint32_t min_rows, uint32_t cap,
+                                uint32_t narrow, uint32_t max_tiles, uint32_t* tiles, uint32_t* status, cudaStream_t st) {
     if (n_experts > (uint32_t)DTHREADS) return cudaErrorInvalidValue;
-    pf_plan_kernel<<<1, DTHREADS, 0, st>>>(t, n_experts, lane_flags, min_rows, cap0, cap1, narrow, max_tiles, tiles, status);
+    pf_plan_kernel<<<1, DTHREADS, 0, st>>>(t, n_experts, lane_flags, min_rows, cap, narrow, max_tiles, tiles, status);
     return cudaGetLastError();
 }
 
 template <int KB>
 static cudaError_t pf_launch_all(const Exl3PrefillArgs& a, cudaStream_t st) {
     LaneParams P{};
-    P.tiles = a.tiles; P.next = a.tiles + 3; P.max_tiles = a.max_tiles; P.t = a.t; P.scales = a.L.scales; P.scales_stride = exl3_scales_per_expert(a.d);
+    P.tiles = a.tiles; P.next = a.tiles + 3; P.t = a.t; P.scales = a.L.scales; P.scales_stride = exl3_scales_per_expert(a.d);
     P.H = a.d.H; P.I = a.d.I; P.limit = a.limit; P.status = a.status; P.act = a.act;
     P.code = reinterpret_cast<const uint8_t*>(a.L.gu_code); P.expert_stride = 8 * exl3_code_words(a.d); P.n_blocks = a.d.I / 128; P.n_stages = a.d.H / LN_KST;
     P.xa = reinterpret_cast<const uint16_t*>(a.xa); P.xa_proj_stride = exl3_prefill_staging_rows(a.rows_cap, a.max_tiles) * a.d.H;
@@ -402,10 +393,10 @@ static cudaError_t pf_launch_all(const Exl3PrefillArgs& a, cudaStream_t st) {
 }
 
 cudaError_t launch_exl3_prefill(const Exl3PrefillArgs& a, cudaStream_t st) {
-    cudaError_t e = launch_prefill_plan(a.t, a.n_experts, nullptr, a.min_rows, LN_ROWS, 0, LN_ROWS_NARROW, a.max_tiles, a.tiles, a.status, st);
+    cudaError_t e = launch_prefill_plan(a.t, a.n_experts, nullptr, a.min_rows, LN_ROWS, LN_ROWS_NARROW, a.max_tiles, a.tiles, a.status, st);
     if (e != cudaSuccess) return e;
     pf_prep_kernel<<<dim3(a.max_tiles, 8), PREP_WARPS * 32, 0, st>>>(a.x, a.top_k, a.d.H, a.L.scales, exl3_scales_per_expert(a.d), a.t,
-                                                                     a.tiles, a.max_tiles,
+                                                                     a.tiles,
                                                                      exl3_prefill_staging_rows(a.rows_cap, a.max_tiles) * a.d.H, a.xa);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     return a.d.K == 3 ? pf_launch_all<3>(a, st) : pf_launch_all<2>(a, st);

@@ -33,11 +33,11 @@ __device__ __forceinline__ uint4 q_order8(uint4 r) {
 // a warp moves 32 consecutive inputs of eight rows: four lanes read 64 bytes of a row, eight lanes write one core matrix
 template <bool NV>
 __global__ void __launch_bounds__(256) q_prep_kernel(const __nv_bfloat16* __restrict__ x, uint32_t top_k, uint32_t H,
-                                                     DispatchTables t, const uint32_t* __restrict__ tiles, uint32_t max_tiles,
+                                                     DispatchTables t, const uint32_t* __restrict__ tiles,
                                                      uint16_t* __restrict__ xa) {
     const uint32_t tile = blockIdx.x;
     if (tile >= tiles[0]) return;
-    const uint32_t* te = prefill_tile(tiles, 0, max_tiles, tile);
+    const uint32_t* te = prefill_tile(tiles, tile);
     const uint32_t row0 = te[1], rows = te[2], rows16 = (rows + 15) / 16 * 16;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, r8 = lane >> 2, c = lane & 3u;
     uint16_t* dst = xa + (size_t)te[3] * H;
@@ -245,11 +245,11 @@ bool fp4_prefill_supported(uint32_t H, uint32_t I) { return H % 128 == 0 && I % 
 
 template <bool NV>
 static cudaError_t q_launch_all(const Fp4PrefillArgs& a, cudaStream_t st) {
-    q_prep_kernel<NV><<<dim3(a.max_tiles, 8), 256, 0, st>>>(a.x, a.top_k, a.H, a.t, a.tiles, a.max_tiles, a.xa);
+    q_prep_kernel<NV><<<dim3(a.max_tiles, 8), 256, 0, st>>>(a.x, a.top_k, a.H, a.t, a.tiles, a.xa);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     LaneParams P{};
-    P.gscale = a.gscale; P.tiles = a.tiles; P.next = a.tiles + 3; P.max_tiles = a.max_tiles; P.t = a.t; P.H = a.H; P.I = a.I; P.limit = a.limit;
+    P.gscale = a.gscale; P.tiles = a.tiles; P.next = a.tiles + 3; P.t = a.t; P.H = a.H; P.I = a.I; P.limit = a.limit;
     P.status = a.status; P.act = a.act;
     P.code = a.gu; P.n_blocks = a.I / 128; P.n_stages = a.H / LN_KST;
     P.expert_stride = (size_t)P.n_blocks * P.n_stages * 2 * Fp4LaneBank<NV>::RAW_BYTES;
@@ -263,7 +263,7 @@ static cudaError_t q_launch_all(const Fp4PrefillArgs& a, cudaStream_t st) {
 }
 
 cudaError_t launch_fp4_prefill(const Fp4PrefillArgs& a, cudaStream_t st) {
-    const cudaError_t e = launch_prefill_plan(a.t, a.n_experts, a.lane_flags, a.min_rows, LN_ROWS, 0, LN_ROWS_NARROW, a.max_tiles, a.tiles, a.status, st);
+    const cudaError_t e = launch_prefill_plan(a.t, a.n_experts, a.lane_flags, a.min_rows, LN_ROWS, LN_ROWS_NARROW, a.max_tiles, a.tiles, a.status, st);
     if (e != cudaSuccess) return e;
     return a.nv ? q_launch_all<true>(a, st) : q_launch_all<false>(a, st);
 }

@@ -80,8 +80,6 @@ struct mlxs_moe {
     // the tensor-core lane runs on a stream of its own beside the streaming lane
     cudaStream_t lane_stream = nullptr;
     cudaEvent_t lane_fork = nullptr, lane_join = nullptr;
-    cudaStream_t lane2_stream = nullptr;   // the tensor-core lane's large-tile kernels beside its small-tile kernels
-    cudaEvent_t lane2_fork = nullptr, lane2_join = nullptr;
     float* sh_out = nullptr;
     uint32_t* status = nullptr;
     uint8_t* staging = nullptr;
@@ -91,7 +89,6 @@ struct mlxs_moe {
     EpState* ep = nullptr;
     uint32_t* front_bar = nullptr;    // grid barrier of the fused front kernel (two words)
     bool front_done = false;          // the fused front kernel of this call has built the tables and staged the rows
-    bool mxfp4_native = false;        // MXFP4 tensor-core lane on the block-scaled kind (MLXS_MXFP4_NATIVE=1 at create) instead of the decoded-operand lane
     bool front_off = false;           // a cooperative launch was refused once: separate kernels from then on
     size_t front_smem_max = 0;        // shared memory that the front kernel may ask for
     uint32_t dbg_poll_limit = 0, dbg_withhold = 0;  // mlxs_moe_debug_wait (self-test of the bounded waits)

@@ -144,21 +144,15 @@ constexpr int PREFILL_TILE_ROWS = 128;
 __host__ __device__ inline bool takes_tensor_lane(uint32_t rows, uint32_t min_rows, const uint8_t* flags, uint32_t e) {
     return min_rows && rows >= min_rows && !(flags && (flags[e] & 2u));
 }
-// Row tiles of the experts that take the tensor-core lane.  tiles[2] = most rows of a tile of list 0, rounded up to 16;
-// tiles[0], tiles[1] = tiles of list 0 (experts with up to
-// cap0 rows; with cap1 = 0 all experts, in tiles of up to cap0 rows) and list 1 (the others, tiles of up to cap1 rows);
-// entries {expert, first sorted row, rows, first staging row}, list 1 from entry max_tiles.  The table holds
-// prefill_tile_words(max_tiles) words.
-__host__ __device__ inline size_t prefill_tile_words(uint32_t max_tiles) { return 8 + 8 * (size_t)max_tiles; }
-__host__ __device__ inline uint32_t* prefill_tile(uint32_t* tiles, int list, uint32_t max_tiles, uint32_t i) {
-    return tiles + 8 + 4 * ((size_t)(list ? max_tiles : 0) + i);
-}
-__host__ __device__ inline const uint32_t* prefill_tile(const uint32_t* tiles, int list, uint32_t max_tiles, uint32_t i) {
-    return tiles + 8 + 4 * ((size_t)(list ? max_tiles : 0) + i);
-}
-cudaError_t launch_prefill_plan(DispatchTables t, uint32_t n_experts, const uint8_t* lane_flags, uint32_t min_rows,
-                                uint32_t cap0, uint32_t cap1, uint32_t narrow, uint32_t max_tiles, uint32_t* tiles,
-                                uint32_t* status, cudaStream_t st);
+// Row tiles of the experts that take the tensor-core lane: tiles[0] = tiles, tiles[2] = most rows of a tile, rounded up to 16;
+// tiles[3], tiles[4] = items that the gate/up, the down kernel has given out; then the entries {expert, first sorted row, rows,
+// first staging row}.  The table holds prefill_tile_words(max_tiles) words.
+__host__ __device__ inline size_t prefill_tile_words(uint32_t max_tiles) { return 8 + 4 * (size_t)max_tiles; }
+__host__ __device__ inline uint32_t* prefill_tile(uint32_t* tiles, uint32_t i) { return tiles + 8 + 4 * (size_t)i; }
+__host__ __device__ inline const uint32_t* prefill_tile(const uint32_t* tiles, uint32_t i) { return tiles + 8 + 4 * (size_t)i; }
+// cap: most rows of a tile; narrow: the tighter cap that a call takes where it costs few tiles
+cudaError_t launch_prefill_plan(DispatchTables t, uint32_t n_experts, const uint8_t* lane_flags, uint32_t min_rows, uint32_t cap,
+                                uint32_t narrow, uint32_t max_tiles, uint32_t* tiles, uint32_t* status, cudaStream_t st);
 struct Exl3PrefillArgs {
     Exl3Layer L;
     Exl3Dims d;
@@ -180,7 +174,7 @@ struct Exl3PrefillArgs {
 };
 size_t lane_act_bytes(int sm_count);
 // staging rows: every tile's rows padded to 16, tiles in sorted order
-static inline size_t exl3_prefill_staging_rows(size_t rows_cap, uint32_t max_tiles) { return rows_cap + 16 * (size_t)(2 * max_tiles + 1); }
+static inline size_t exl3_prefill_staging_rows(size_t rows_cap, uint32_t max_tiles) { return rows_cap + 16 * ((size_t)max_tiles + 1); }
 static inline size_t exl3_prefill_xa_bytes(Exl3Dims d, size_t rows_cap, uint32_t max_tiles) { return 2 * exl3_prefill_staging_rows(rows_cap, max_tiles) * d.H * 2; }
 static inline size_t exl3_prefill_xd_bytes(Exl3Dims d, size_t rows_cap, uint32_t max_tiles) { return exl3_prefill_staging_rows(rows_cap, max_tiles) * d.I * 2; }
 cudaError_t launch_exl3_prefill(const Exl3PrefillArgs& a, cudaStream_t st);
@@ -236,8 +230,7 @@ struct Fp4PrefillArgs {
     uint32_t top_k;
     uint32_t* tiles;         // [prefill_tile_words(max_tiles)]
     uint32_t max_tiles;
-    uint16_t* xa;            // [staging rows][H] rows in the MMA's B-operand order (bf16 MXFP4, f16 NVFP4; the block-scaled
-                             // MXFP4 lane keeps E4M3 high / low parts and scale bytes here, mxfp4_native_xa_bytes)
+    uint16_t* xa;            // [staging rows][H] rows in the MMA's B-operand order (bf16 MXFP4, f16 NVFP4)
     uint16_t* xd;            // [staging rows][I], the same for the down product
     uint32_t rows_cap;       // assignment rows the staging was sized for
     void* ro;                // [A, H] bf16 (chain combine) or f32
@@ -245,36 +238,13 @@ struct Fp4PrefillArgs {
     float limit;
     uint32_t* status;
     int sm_count;
-    void* act;               // lane_act_bytes(sm_count): act(gate) between a CTA's gate and up passes (not used by launch_mxfp4_native)
-    // launch_mxfp4_native, optional: a stream for the kernels of the large tiles (they touch other experts than the small-tile kernels), with
-    // the events that fork it from and join it into the call's stream; null: one stream
-    cudaStream_t side = nullptr;
-    cudaEvent_t side_fork = nullptr, side_join = nullptr;
+    void* act;               // lane_act_bytes(sm_count): act(gate) between a CTA's gate and up passes
 };
-// the large-tile kernels beside the small-tile ones: fork before, join after (always, also after a refused launch)
-template <class F>
-static inline cudaError_t prefill_lists_side_by_side(cudaStream_t st, cudaStream_t side, cudaEvent_t fork_ev, cudaEvent_t join_ev, F&& launches) {
-    cudaError_t e = cudaSuccess;
-    if (side && ((e = cudaEventRecord(fork_ev, st)) != cudaSuccess || (e = cudaStreamWaitEvent(side, fork_ev, 0)) != cudaSuccess)) return e;
-    e = launches(side ? side : st);
-    if (side) {
-        const cudaError_t j1 = cudaEventRecord(join_ev, side);
-        const cudaError_t j2 = j1 == cudaSuccess ? cudaStreamWaitEvent(st, join_ev, 0) : j1;
-        if (e == cudaSuccess) e = j2;
-    }
-    return e;
-}
 // staging rows: every tile's rows padded to 16
 static inline size_t fp4_prefill_xa_bytes(uint32_t width, size_t rows_cap, uint32_t max_tiles) {
-    return (rows_cap + 16 * (size_t)(2 * max_tiles + 1)) * width * 2;
+    return (rows_cap + 16 * ((size_t)max_tiles + 1)) * width * 2;
 }
 cudaError_t launch_fp4_prefill(const Fp4PrefillArgs& a, cudaStream_t st);
-// MXFP4 on the block-scaled tensor-core kind (fp4_native.cu): the same arguments; xa / xd hold the rows split into E4M3
-// high and low parts with their block scales, 132 bytes per row per 64 inputs
-static inline size_t mxfp4_native_xa_bytes(uint32_t width, size_t rows_cap, uint32_t max_tiles) {
-    return (rows_cap + 16 * (size_t)(2 * max_tiles + 1)) * (width / 64) * 132;
-}
-cudaError_t launch_mxfp4_native(const Fp4PrefillArgs& a, cudaStream_t st);
 bool fp4_prefill_supported(uint32_t H, uint32_t I);
 
 // ---- shared expert (bf16 dense) + combine ----

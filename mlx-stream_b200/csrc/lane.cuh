@@ -71,9 +71,8 @@ struct LaneParams {
     uint32_t n_blocks, n_stages; // out / 128, in / 128
     const uint16_t* xa;          // staged rows, pass p at p * xa_proj_stride elements
     size_t xa_proj_stride;
-    const uint32_t* tiles;       // list 0 of the tile table
+    const uint32_t* tiles;       // the tile table
     uint32_t* next;              // items given out so far
-    uint32_t max_tiles;
     DispatchTables t;
     uint32_t H, I;
     const __half* scales;        // EXL3: the layer's sign / scale vectors
@@ -278,7 +277,7 @@ __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P)
                 const uint32_t item = it ? atomicAdd(P.next, 1u) : first;
                 const bool more = item < n_items && !s_abort;
                 const uint32_t nb = more ? item % P.n_blocks : LN_NO_ITEM;
-                const uint4 te = *reinterpret_cast<const uint4*>(prefill_tile(P.tiles, 0, P.max_tiles, more ? item / P.n_blocks : 0u));
+                const uint4 te = *reinterpret_cast<const uint4*>(prefill_tile(P.tiles, more ? item / P.n_blocks : 0u));
                 s_tile[it % LN_ITEMS] = te;
                 s_nb[it % LN_ITEMS] = nb;
                 mbar_arrive(&item_full[it % LN_ITEMS]);
