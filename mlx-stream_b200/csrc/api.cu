@@ -163,7 +163,7 @@ extern "C" int mlxs_moe_create(const mlxs_moe_config* c, mlxs_moe** out) {
             return bail(rc);
         if (cudaMemset(h->ks_count, 0, ksplit_count_words(h->sm_count) * 4) != cudaSuccess) return bail(fail(MLXS_E_CUDA, "create: cudaMemset failed"));
     } else {
-        if ((rc = h->alloc(&h->inf_flag, 4))) return bail(rc);
+        if (cudaMallocHost(reinterpret_cast<void**>(&h->inf_flag), 4) != cudaSuccess) return bail(fail(MLXS_E_CUDA, "create: cudaMallocHost failed"));
         if ((rc = h->alloc(&h->xa_gu, (size_t)max_chunks * (H / 32) * 512)) ||
             (rc = h->alloc(&h->xa_d, (size_t)max_chunks * (I / 32) * 512)) || (rc = h->alloc(&h->ro, A * H * 4)))
             return bail(rc);
@@ -224,6 +224,7 @@ extern "C" void mlxs_moe_destroy(mlxs_moe* h) {
     if (h->aux_stream) cudaStreamDestroy(h->aux_stream);
     if (h->lane_stream) cudaStreamDestroy(h->lane_stream);
     for (void* p : h->allocs) cudaFree(p);
+    if (h->inf_flag) cudaFreeHost(h->inf_flag);
     for (auto& s : h->spans) { cudaEventDestroy(s.a); cudaEventDestroy(s.b); }
     for (auto e : h->ev_pool) cudaEventDestroy(e);
     delete h;
@@ -291,7 +292,6 @@ extern "C" int mlxs_moe_load_expert(mlxs_moe* h, uint32_t layer, uint32_t expert
     }
     // the expert's entry of the per-expert table: 1 = resident; the FP4 repack may raise it to 3 (see takes_tensor_lane)
     const uint8_t one = 1;
-    uint32_t inf_scale = 0;
     CU(cudaMemcpyAsync(L.loaded_dev + le, &one, 1, cudaMemcpyHostToDevice, 0));
     if (is_exl3(h->cfg.bank_kind)) {
         const Exl3Dims d{h->cfg.hidden, h->cfg.inter, L.kbits};
@@ -299,15 +299,14 @@ extern "C" int mlxs_moe_load_expert(mlxs_moe* h, uint32_t layer, uint32_t expert
                               L.d_code + (size_t)le * exl3_code_words(d), L.scales + (size_t)le * exl3_scales_per_expert(d), 0));
     } else {
         const int nv = h->cfg.bank_kind == MLXS_BANK_NVFP4;
-        if (!nv) CU(cudaMemsetAsync(h->inf_flag, 0, 4, 0));
+        *h->inf_flag = 0;   // nothing of an earlier load is in flight: every load ends synchronised
         CU(launch_fp4_repack(src, h->cfg.hidden, h->cfg.inter, nv,
                              L.f4_gu + (size_t)le * fp4_stream_bytes_per_expert(h->cfg.hidden, h->cfg.inter, nv, 0),
                              L.f4_dn + (size_t)le * fp4_stream_bytes_per_expert(h->cfg.hidden, h->cfg.inter, nv, 1),
                              L.f4_gscale + (size_t)le * 3, L.loaded_dev + le, nv ? nullptr : h->inf_flag, 0));
-        if (!nv) CU(cudaMemcpyAsync(&inf_scale, h->inf_flag, 4, cudaMemcpyDeviceToHost, 0));
     }
     CU(cudaStreamSynchronize(0));
-    L.inf_scales = L.inf_scales || inf_scale;
+    if (h->inf_flag && *static_cast<volatile uint32_t*>(h->inf_flag)) L.inf_scales = true;
     L.loaded[expert] = 1;
     return MLXS_OK;
 }

@@ -74,7 +74,7 @@ struct mlxs_moe {
     float* logits_ws = nullptr;       // [max_tokens, E] logits of mlxs_moe_forward_x
     float* ks_scratch = nullptr;      // K-split workspace of the streaming kernels (exl3.cu)
     uint32_t* ks_count = nullptr;
-    uint32_t* inf_flag = nullptr;     // what a load found in its record (launch_fp4_repack)
+    uint32_t* inf_flag = nullptr;     // pinned host word: what a load found in its record (launch_fp4_repack)
     cudaStream_t aux_stream = nullptr;
     cudaEvent_t aux_fork = nullptr, aux_join = nullptr;
     // the tensor-core lane runs on a stream of its own beside the streaming lane

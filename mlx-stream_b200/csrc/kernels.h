@@ -188,8 +188,8 @@ static inline size_t fp4_stream_bytes_per_expert(uint32_t H, uint32_t I, int nv,
     return (size_t)(H / 128) * (I / 128) * per_stage;
 }
 // record (device, reference layout) -> the expert's slices of the gate/up stream, the down stream and the global scales
-// lane_flag: the expert's entry of the per-expert table; set to 3 when an MXFP4 block scale exceeds 2^1; inf_flag: set to 1 when
-// one is byte 255
+// lane_flag: the expert's entry of the per-expert table; set to 3 when an MXFP4 block scale exceeds 2^1; inf_flag (a word that
+// the device can write): set to 1 when one is byte 255
 cudaError_t launch_fp4_repack(const uint8_t* record_dev, uint32_t H, uint32_t I, int nv, uint8_t* gu_e, uint8_t* dn_e,
                               float* gscale_e, uint8_t* lane_flag, uint32_t* inf_flag, cudaStream_t st);
 // x bf16 [T, H] -> f16 rows in the kernels' B-fragment order: [chunk][H/32][128] u32
