@@ -626,7 +626,7 @@ int mlxs_run_routed(mlxs_moe* h, uint32_t layer, const void* x_dev, const int32_
     if (A > h->rows_cap) return fail(MLXS_E_TOO_MANY_TOKENS, "experts: %u rows exceed the workspace's %u", A, h->rows_cap);
     // Lane choice per expert by its row count, as the reference decides on logical M (src/sdk_ext/quant.zig:5-6,
     // src/arch/deepseek_v41/experts.zig:1545-1547): experts with `heavy` rows or more go to the tensor-core lane, which
-    // amortises one decode over up to 128 rows; the others stream through the decode-batch lane.
+    // amortises one decode over up to 192 rows; the others stream through the decode-batch lane.
     // a token's experts are distinct, so no expert has more rows than the call has tokens
     const bool two_lanes = h->pf_tiles && T >= h->pf_min_rows;
     const uint32_t heavy = two_lanes ? h->pf_min_rows : 0u;
@@ -646,8 +646,9 @@ int mlxs_run_routed(mlxs_moe* h, uint32_t layer, const void* x_dev, const int32_
     // its two kernels) is queued on a stream of its own beside the streaming lane, forked after the dispatch
     // and joined before the rows are read.  Its launches, most of all the ones that find no heavy expert and return at
     // once, then cost the step nothing, and the lanes' tails overlap.
-    // Prefill-sized calls (nearly every expert in the tensor-core lane, nothing to overlap) keep one stream: with two,
-    // C4 at 16384 tokens went from 13.0 to 14.4 ms.  MLXS_LANES_ASIDE_MAX moves the limit (0: always one stream).
+    // Prefill-sized calls (nearly every expert in the tensor-core lane, nothing to overlap) keep one stream: from 1000 tokens on
+    // one stream and two are within 1 % of each other (2048 EXL3 tokens 3.04 ms either way, 16384 MXFP4 tokens 6.78), but for
+    // Zipf routing, where two are 1.5 % faster at 4096 tokens.  MLXS_LANES_ASIDE_MAX moves the limit (0: always one stream).
     static const uint32_t lanes_aside_max = getenv("MLXS_LANES_ASIDE_MAX") ? (uint32_t)atoi(getenv("MLXS_LANES_ASIDE_MAX")) : 2048u;
     const bool lane_aside = two_lanes && h->lane_stream && T <= lanes_aside_max;
     const cudaStream_t tl = lane_aside ? h->lane_stream : st;

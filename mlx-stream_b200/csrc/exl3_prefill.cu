@@ -11,10 +11,10 @@
 //   * the epilogue: transpose through shared memory, then row-wise Hadamard-128, svh, clamped SwiGLU, suh_d, Hadamard for
 //     gate / up (act(gate) waits in an L2-resident scratch between the two passes, read back by the threads that wrote it);
 //     Hadamard, svh_d for down.
-// What bounds it (about 55 warp instructions per decoded tile, 43 of them the decode): up to about 128 rows per tile the
+// What bounds it (57 to 64 warp instructions per decoded tile with the epilogue, 43 of them the decode; 72 to 81 % of the issue slots): up to about 128 rows per tile the
 // decode's instruction issue, above that the MMAs; calls of thousands of tokens run into the 1 kW power cap (1.55 GHz at
-// 8192 tokens).  Layer of H 5120, I 2304, 256 experts: 2048 tokens 4.06 -> 3.02 ms, 8192 tokens 10.6 -> 7.7 ms against
-// the lane that accumulated gate and up together.
+// 8192 tokens).  Layer of H 5120, I 2304, 256 experts, calls back to back: 2048 tokens 4.04 -> 3.05 ms, 8192 tokens 10.65 ->
+// 7.74 ms against the lane that accumulated gate and up together.
 #include <cstdlib>
 
 #include "dispatch_body.cuh"
@@ -277,92 +277,92 @@ struct Exl3LaneBank {
             const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&s0.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&s0.y));
             svh[0] = a.x; svh[1] = a.y; svh[2] = b.x; svh[3] = b.y;
         }
-                        for (uint32_t rb = 0; rb < rows16; rb += PF_EPI_ROWS, ++E.batch) {
-                            float* z = zs + (E.batch & 1u) * (PF_EPI_ROWS * PF_ZS_STRIDE);
-                            if (rb + half * 16 < rows16) {
-                                uint32_t v[16];
-                                tmem_ld16(C.acc + ((q * 32u) << 16) + rb + half * 16, v);
-        #pragma unroll
-                                for (int i = 0; i < 16; ++i) z[(half * 16 + i) * PF_ZS_STRIDE + q * 32 + lane] = __uint_as_float(v[i]);
-                            }
-                            if (rb + PF_EPI_ROWS >= rows16) C.release(lane);
+        for (uint32_t rb = 0; rb < rows16; rb += PF_EPI_ROWS, ++E.batch) {
+            float* z = zs + (E.batch & 1u) * (PF_EPI_ROWS * PF_ZS_STRIDE);
+            if (rb + half * 16 < rows16) {
+                uint32_t v[16];
+                tmem_ld16(C.acc + ((q * 32u) << 16) + rb + half * 16, v);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) z[(half * 16 + i) * PF_ZS_STRIDE + q * 32 + lane] = __uint_as_float(v[i]);
+            }
+            if (rb + PF_EPI_ROWS >= rows16) C.release(lane);
             // one rendezvous per batch: a staging buffer is written again two batches later, after the next one
-                            if (!E.sync()) return false;
-        #pragma unroll
-                            for (int rr = 0; rr < 4; rr += 2) {
-                                const uint32_t zr = ew * 4 + rr, r = rb + zr;
-                                if (r >= rows16) break;
-                                float v[2][4];
-        #pragma unroll
-                                for (int i = 0; i < 2; ++i) {
-                                    const float* zp = z + (zr + i) * PF_ZS_STRIDE;
-                                    if (NPASS == 2) {
-                                        const float2 a = *reinterpret_cast<const float2*>(zp + pf_lane_col(lane)), b = *reinterpret_cast<const float2*>(zp + pf_lane_col(lane) + 8);
-                                        v[i][0] = a.x; v[i][1] = a.y; v[i][2] = b.x; v[i][3] = b.y;
-                                    } else {
-                                        const float4 a = *reinterpret_cast<const float4*>(zp + lane * 4);
-                                        v[i][0] = a.x; v[i][1] = a.y; v[i][2] = a.z; v[i][3] = a.w;
-                                    }
-                                }
-                                pf_hadamard<NPASS == 2>(v, sg);
-                                if (NPASS == 2 && p == 0) {
-        #pragma unroll
-                                    for (int i = 0; i < 2; ++i) {
-                                        float o[4];
-        #pragma unroll
-                                        for (int k = 0; k < 4; ++k) {
-                                            const float gm = (v[i][k] * S) * svh[k];
-                                            float gate = gm;
-                                            if (P.limit > 0.f) gate = (gm != gm) ? gm : (gm < P.limit ? gm : P.limit);
-                                            const float yv = sigmoid_tail_fast(gate);
-                                            o[k] = gate * (gate < 0.f ? yv : 1.0f - yv);
-                                        }
-                                        __stcg(reinterpret_cast<float4*>(act + (size_t)(r + i) * 128), make_float4(o[0], o[1], o[2], o[3]));
-                                    }
-                                } else if (NPASS == 2) {
-                                    float4 a4[2];
-        #pragma unroll
-                                    for (int i = 0; i < 2; ++i) a4[i] = __ldcg(reinterpret_cast<const float4*>(act + (size_t)(r + i) * 128));
-                                    float h[2][4];
-        #pragma unroll
-                                    for (int i = 0; i < 2; ++i) {
-                                        const float av[4] = {a4[i].x, a4[i].y, a4[i].z, a4[i].w};
-        #pragma unroll
-                                        for (int k = 0; k < 4; ++k) {
-                                            const float um = (v[i][k] * S) * svh[k];
-                                            float up = um;
-                                            if (P.limit > 0.f) {
-                                                const float u0 = (um != um) ? um : (um > -P.limit ? um : -P.limit);
-                                                up = (u0 != u0) ? u0 : (u0 < P.limit ? u0 : P.limit);
-                                            }
-                                            h[i][k] = __fmul_rn(av[k], up);   // 0 in padding rows: their B rows are 0
-                                        }
-                                        // x suh_d and the transform's level 0, the first product of a pair unrounded (written out,
-                                        // so that the bits do not hang on what the compiler contracts)
-        #pragma unroll
-                                        for (int k = 0; k < 4; k += 2) {
-                                            const float t0 = h[i][k], t1 = __fmul_rn(h[i][k + 1], shd[k + 1]);
-                                            h[i][k] = __fmaf_rn(t0, shd[k], t1);
-                                            h[i][k + 1] = __fmaf_rn(t0, shd[k], -t1);
-                                        }
-                                    }
-                                    pf_hadamard<true, false>(h, sg);
-                                    // src/kernels/exl3/header_dig2_x.metal:104: the down input is rounded to f16
-                                    __half* xd = reinterpret_cast<__half*>(P.xd) + (size_t)C.srow0 * P.I + (size_t)nb * (rows16 * LN_KST);
-        #pragma unroll
-                                    for (int i = 0; i < 2; ++i)
-                                        *reinterpret_cast<uint2*>(xd + pf_lane_off(r + i, lane)) = pf_pack4(h[i][0] * S, h[i][1] * S, h[i][2] * S, h[i][3] * S);
-                                } else {
-        #pragma unroll
-                                    for (int i = 0; i < 2; ++i) {
-                                        if (r + i >= rows) continue;
-                                        const uint32_t assign = P.t.order[C.row0 + r + i];
-                                        *reinterpret_cast<float4*>(static_cast<float*>(P.out) + (size_t)assign * P.H + nb * 128 + lane * 4) =
-                                            make_float4((v[i][0] * S) * svh[0], (v[i][1] * S) * svh[1], (v[i][2] * S) * svh[2], (v[i][3] * S) * svh[3]);
-                                    }
-                                }
-                            }
+            if (!E.sync()) return false;
+#pragma unroll
+            for (int rr = 0; rr < 4; rr += 2) {
+                const uint32_t zr = ew * 4 + rr, r = rb + zr;
+                if (r >= rows16) break;
+                float v[2][4];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const float* zp = z + (zr + i) * PF_ZS_STRIDE;
+                    if (NPASS == 2) {
+                        const float2 a = *reinterpret_cast<const float2*>(zp + pf_lane_col(lane)), b = *reinterpret_cast<const float2*>(zp + pf_lane_col(lane) + 8);
+                        v[i][0] = a.x; v[i][1] = a.y; v[i][2] = b.x; v[i][3] = b.y;
+                    } else {
+                        const float4 a = *reinterpret_cast<const float4*>(zp + lane * 4);
+                        v[i][0] = a.x; v[i][1] = a.y; v[i][2] = a.z; v[i][3] = a.w;
+                    }
+                }
+                pf_hadamard<NPASS == 2>(v, sg);
+                if (NPASS == 2 && p == 0) {
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        float o[4];
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            const float gm = (v[i][k] * S) * svh[k];
+                            float gate = gm;
+                            if (P.limit > 0.f) gate = (gm != gm) ? gm : (gm < P.limit ? gm : P.limit);
+                            const float yv = sigmoid_tail_fast(gate);
+                            o[k] = gate * (gate < 0.f ? yv : 1.0f - yv);
                         }
+                        __stcg(reinterpret_cast<float4*>(act + (size_t)(r + i) * 128), make_float4(o[0], o[1], o[2], o[3]));
+                    }
+                } else if (NPASS == 2) {
+                    float4 a4[2];
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) a4[i] = __ldcg(reinterpret_cast<const float4*>(act + (size_t)(r + i) * 128));
+                    float h[2][4];
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        const float av[4] = {a4[i].x, a4[i].y, a4[i].z, a4[i].w};
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            const float um = (v[i][k] * S) * svh[k];
+                            float up = um;
+                            if (P.limit > 0.f) {
+                                const float u0 = (um != um) ? um : (um > -P.limit ? um : -P.limit);
+                                up = (u0 != u0) ? u0 : (u0 < P.limit ? u0 : P.limit);
+                            }
+                            h[i][k] = __fmul_rn(av[k], up);   // 0 in padding rows: their B rows are 0
+                        }
+                        // x suh_d and the transform's level 0, the first product of a pair unrounded (written out,
+                        // so that the bits do not hang on what the compiler contracts)
+#pragma unroll
+                        for (int k = 0; k < 4; k += 2) {
+                            const float t0 = h[i][k], t1 = __fmul_rn(h[i][k + 1], shd[k + 1]);
+                            h[i][k] = __fmaf_rn(t0, shd[k], t1);
+                            h[i][k + 1] = __fmaf_rn(t0, shd[k], -t1);
+                        }
+                    }
+                    pf_hadamard<true, false>(h, sg);
+                    // src/kernels/exl3/header_dig2_x.metal:104: the down input is rounded to f16
+                    __half* xd = reinterpret_cast<__half*>(P.xd) + (size_t)C.srow0 * P.I + (size_t)nb * (rows16 * LN_KST);
+#pragma unroll
+                    for (int i = 0; i < 2; ++i)
+                        *reinterpret_cast<uint2*>(xd + pf_lane_off(r + i, lane)) = pf_pack4(h[i][0] * S, h[i][1] * S, h[i][2] * S, h[i][3] * S);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        if (r + i >= rows) continue;
+                        const uint32_t assign = P.t.order[C.row0 + r + i];
+                        *reinterpret_cast<float4*>(static_cast<float*>(P.out) + (size_t)assign * P.H + nb * 128 + lane * 4) =
+                            make_float4((v[i][0] * S) * svh[0], (v[i][1] * S) * svh[1], (v[i][2] * S) * svh[2], (v[i][3] * S) * svh[3]);
+                    }
+                }
+            }
+        }
         return true;
     }
 };

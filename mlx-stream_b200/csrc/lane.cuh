@@ -16,7 +16,7 @@
 //     operand slots there are four teams of four warps, a warp decoding both halves of a stage, with two slots two teams of
 //     eight (a team of four keeps its slot for twice as long).  The barriers around a stage were a quarter of the instructions
 //     of a warp that decoded one half (EXL3: 60 per 16x16 tile, 43 of them the decode), and their latencies showed where the
-//     decode is short: EXL3 at 2048 tokens 2927 -> 2690 us, at 8192 7660 -> 7355, MXFP4 at 2048 1649 -> 1315, at 3500 1840 -> 1625.
+//     decode is short: EXL3 8 % at 2048 tokens and 4 % at 8192, MXFP4 20 % at 2048 and 12 % at 3500.
 //     (Decoding in smaller pieces, or with 5 or 6 warps per lane quarter, measured slower or equal.)
 //   * The MMA warp runs its loop with all lanes and issues under elect.sync (see elect_one); one commit per stage frees the
 //     operand slot and the rows' slot.

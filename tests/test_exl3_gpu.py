@@ -475,8 +475,8 @@ def test_limits_empty_call_too_many_tokens_and_the_widest_router():
 
 
 def test_router_logits_product_and_the_layer_from_x():
-    """logits = f32(x) . f32(W_g)^T (src/arch/deepseek_v41/graph.zig:2033) in both forms (own kernel up to 64 tokens, the
-    library GEMM above), and the layer started from x.  The f32 sum order is the kernel's own, so ids are compared only
+    """logits = f32(x) . f32(W_g)^T (src/arch/deepseek_v41/graph.zig:2033) in both forms (f32 kernels up to 64 tokens, the
+    tensor-core product above), and the layer started from x.  The f32 sum order is the kernel's own, so ids are compared only
     where the k-th and (k+1)-th keys are not a near-tie."""
     import torch
     case = Exl3Case(512, 256, 8, 2, seed=6, shared=True, max_tokens=128)
