@@ -105,80 +105,79 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
 // ---- EXL3 mul1: two 16-bit trellis states -> half2 (lo = a, hi = b) ----
 // value = f16( (1024 + bytesum(state * 0x83DCD12D)) * h(0x1EEE) + h(0xC931) ), one rounding
 // (src/exl3/kernels.zig:963-971; src/kernels/exl3/dsv41_exl3_mul1h_k3_2304.metal:27-31)
-// PRMT: the two halves are put together by a byte permute (logic pipe) instead of a multiply-add: with 16 of a tile's
-// instructions on the half-rate multiply pipe the streaming kernels are 1 % (K = 3) to 4 % (K = 2) faster that way, the
-// tensor-core lane, whose epilogue warps use the logic pipe, is not.
-template <bool PRMT>
+// The two halves are put together by a byte permute (logic pipe), not a multiply-add: the half-rate multiply pipe has 20 of a
+// tile's instructions already (46.8 against 48.5 cycles per tile at K = 3, 43.8 against 45.5 at K = 2; in the tensor-core
+// lane, whose epilogue warps use the logic pipe, the two are within 0.7 %).
 __device__ __forceinline__ uint32_t mul1_pair(uint32_t sa, uint32_t sb) {
     uint32_t xa = sa * MUL1, xb = sb * MUL1;
     uint32_t ha = __dp4a(xa, 0x01010101u, 0x6400u);  // 0x6400 + byte sum = the half bits of 1024 + s
     uint32_t hb = __dp4a(xb, 0x01010101u, 0x6400u);
-    uint32_t pk = PRMT ? __byte_perm(ha, hb, 0x5410) : hb * 65536u + ha;
+    uint32_t pk = __byte_perm(ha, hb, 0x5410);
     const uint32_t kinv = 0x1EEE1EEEu, kbias = 0xC931C931u;
     __half2 r = __hfma2(*reinterpret_cast<__half2*>(&pk), *reinterpret_cast<const __half2*>(&kinv),
                         *reinterpret_cast<const __half2*>(&kbias));
     return *reinterpret_cast<uint32_t*>(&r);
 }
 
-// One lane's share of a 16x16 K=3 tile: lane L owns code positions 8L..8L+7, i.e. the 37 stream bits ending at
-// stream bit 24(L+1); `lo` is the tile word holding that last bit, `hi` the word before it (circular), lp the
-// distance of the last bit from the word's bit 0.  Returns the two B fragments (k16 x n8) of the tile's column
-// halves for mma m16n8k16: b[0], b[1] = columns 0..7, b[2], b[3] = columns 8..15 (the exllamav3 tensor-core order,
-// src/exl3/kernels.zig:978-986).
-template <bool PRMT = false>
-__device__ __forceinline__ void exl3_decode_lane(uint32_t lo, uint32_t hi, uint32_t lp, uint32_t (&b)[4]) {
-    uint32_t v0 = __funnelshift_r(lo, hi, lp);  // stream bits, window m at bits [3m, 3m+16)
-    uint32_t vh = hi >> lp;
-    uint32_t v1 = __funnelshift_r(v0, vh, 18);  // windows 6, 7 at bits 0 and 3
-    uint32_t w0 = v0 & 0xFFFFu;
-    uint32_t w1 = (v0 >> 3) & 0xFFFFu;
-    uint32_t w2 = (v0 >> 6) & 0xFFFFu;
-    uint32_t w3 = (v0 >> 9) & 0xFFFFu;
-    uint32_t w4 = (v0 >> 12) & 0xFFFFu;
-    uint32_t w5 = (v0 >> 15) & 0xFFFFu;
-    uint32_t w6 = v1 & 0xFFFFu;
-    uint32_t w7 = (v1 >> 3) & 0xFFFFu;
-    // code position j = 7 - m; positions (0,1),(2,3) -> columns 0..7 rows (r0,r0+1),(r0+8,r0+9); (4,5),(6,7) -> 8..15
-    b[0] = mul1_pair<PRMT>(w7, w6);
-    b[1] = mul1_pair<PRMT>(w5, w4);
-    b[2] = mul1_pair<PRMT>(w3, w2);
-    b[3] = mul1_pair<PRMT>(w1, w0);
-}
-__device__ __forceinline__ void exl3_lane_plan(uint32_t lane, uint32_t& wi, uint32_t& wj, uint32_t& lp) {
-    wi = (3u * lane + 2u) >> 2;        // word of the lane's last stream bit
-    wj = (wi + 23u) % 24u;             // the word before it, circular
-    lp = 8u * ((lane + 1u) & 3u);
-}
-// The same for K = 2 (a tile is 16 words): lane L's 8 states end at stream bits 16 L + 2 .. 16 L + 16, i.e. they live in
-// the 30 bits ending with halfword L.  `lo` = the word holding halfword L, `hi` = the word before it (circular),
-// lp = 0 when halfword L is the word's low half, 16 when it is the high half; window m at bits [2m, 2m + 16).
-// Bit-level definition: src/exl3/kernels.zig:988-1020 (tileStates at K = 2), generic window formulas
-// scripts/dsv41_exl3_k2_gen.py:96-112.
-template <bool PRMT = false>
-__device__ __forceinline__ void exl3_decode_lane_k2(uint32_t lo, uint32_t hi, uint32_t lp, uint32_t (&b)[4]) {
-    const uint32_t v0 = __funnelshift_r(lo, hi, lp);
-    const uint32_t w0 = v0 & 0xFFFFu, w1 = (v0 >> 2) & 0xFFFFu, w2 = (v0 >> 4) & 0xFFFFu, w3 = (v0 >> 6) & 0xFFFFu;
-    const uint32_t w4 = (v0 >> 8) & 0xFFFFu, w5 = (v0 >> 10) & 0xFFFFu, w6 = (v0 >> 12) & 0xFFFFu, w7 = (v0 >> 14) & 0xFFFFu;
-    b[0] = mul1_pair<PRMT>(w7, w6);
-    b[1] = mul1_pair<PRMT>(w5, w4);
-    b[2] = mul1_pair<PRMT>(w3, w2);
-    b[3] = mul1_pair<PRMT>(w1, w0);
-}
-__device__ __forceinline__ void exl3_lane_plan_k2(uint32_t lane, uint32_t& wi, uint32_t& wj, uint32_t& lp) {
-    wi = lane >> 1;
-    wj = (wi + 15u) % 16u;
-    lp = (lane & 1u) ? 0u : 16u;
-}
-// by code width
-template <int KB, bool PRMT = false>
-__device__ __forceinline__ void exl3_decode_lane_kb(uint32_t lo, uint32_t hi, uint32_t lp, uint32_t (&b)[4]) {
-    if (KB == 3) exl3_decode_lane<PRMT>(lo, hi, lp, b);
-    else exl3_decode_lane_k2<PRMT>(lo, hi, lp, b);
-}
+// ---- the lane's share of a quad: four k-tiles (64 inputs) of one 16-column tile ----
+// A tile's 256 states follow each other in its code (K bits apart, the 16 bits of state i end at stream bit K (i + 1),
+// circular; src/exl3/kernels.zig:978-1020).  Lane l = 4 u + j takes the 32 consecutive states 32 u .. 32 u + 31 of k-tile j:
+// the 16 inputs of the output columns u and u + 8 (the exllamav3 tensor-core order).  They lie in K whole words and the last
+// bits of the word before, so every window has a constant place: no shift by a lane's own distance, no two words per eight
+// states.  States 8 c .. 8 c + 7 are b[0..3] = the weights of column u, inputs (2c, 2c+1), (2c+8, 2c+9), then column u + 8's.
+// Lanes 4u .. 4u + 3 hold the same columns of four k-tiles, which is one mma A fragment (or one tcgen05.st.16x256b fragment)
+// per c with inputs of all four k-tiles; whoever multiplies takes the rows in that order (position 16 c + 4 j + 2 h + b of
+// the 64 = input 16 j + 2 c + 8 h + b).
+// Measured with operands in shared memory, cycles per tile and scheduler, against eight states per lane and tile (two words, a
+// funnel shift by the lane): K = 3 51.7 -> 46.7, K = 2 51.7 -> 43.8; with one mma per tile 58.5 -> 55.3 and 57.4 -> 52.5.
+// The quad in memory: 32 K words, [lane][first two words], then the lanes' third words (K = 3).
 template <int KB>
-__device__ __forceinline__ void exl3_lane_plan_kb(uint32_t lane, uint32_t& wi, uint32_t& wj, uint32_t& lp) {
-    if (KB == 3) exl3_lane_plan(lane, wi, wj, lp);
-    else exl3_lane_plan_k2(lane, wi, wj, lp);
+__device__ __forceinline__ void exl3_quad_words(const uint32_t* __restrict__ quad, uint32_t lane, uint32_t (&z)[4]) {
+    // z: the stream's words from its last on, z[KB] = the word before the lane's first (its neighbour's last)
+    const uint2 w = reinterpret_cast<const uint2*>(quad)[lane];
+    z[KB - 1] = w.x; z[KB - 2] = w.y;
+    if (KB == 3) { z[0] = quad[64 + lane]; z[3] = quad[64 + ((lane - 4u) & 31u)]; }
+    else { z[2] = quad[2u * ((lane - 4u) & 31u) + 1u]; z[3] = 0u; }
+}
+// 32 stream bits from bit O on (counted from the last)
+template <int O>
+__device__ __forceinline__ uint32_t exl3_bits(const uint32_t (&z)[4]) {
+    return O % 32 == 0 ? z[O / 32] : __funnelshift_r(z[O / 32], z[O / 32 + 1 < 4 ? O / 32 + 1 : 3], O % 32);
+}
+// the state at bit O: one byte permute or shift where it is byte-aligned inside a word, else a funnel shift and a mask
+template <int O>
+__device__ __forceinline__ uint32_t exl3_state(const uint32_t (&z)[4]) {
+    return O % 32 == 8 ? __byte_perm(z[O / 32], 0u, 0x4421) : O % 32 == 16 ? z[O / 32] >> 16 : exl3_bits<O>(z) & 0xFFFFu;
+}
+template <int KB, int C>
+__device__ __forceinline__ void exl3_decode8(const uint32_t (&z)[4], uint32_t (&b)[4]) {
+    constexpr int B = KB * (24 - 8 * C);   // of the group's last state
+    if (KB == 3) {
+        b[0] = mul1_pair(exl3_state<B + 21>(z), exl3_state<B + 18>(z));
+        b[1] = mul1_pair(exl3_state<B + 15>(z), exl3_state<B + 12>(z));
+        b[2] = mul1_pair(exl3_state<B + 9>(z), exl3_state<B + 6>(z));
+        b[3] = mul1_pair(exl3_state<B + 3>(z), exl3_state<B>(z));
+    } else {
+        // states four apart are a byte apart: one funnel shift serves both
+        const uint32_t f0 = exl3_bits<B>(z), f1 = exl3_bits<B + 2>(z), f2 = exl3_bits<B + 4>(z), f3 = exl3_bits<B + 6>(z);
+        b[0] = mul1_pair(__byte_perm(f3, 0u, 0x4421), __byte_perm(f2, 0u, 0x4421));
+        b[1] = mul1_pair(__byte_perm(f1, 0u, 0x4421), __byte_perm(f0, 0u, 0x4421));
+        b[2] = mul1_pair(f3 & 0xFFFFu, f2 & 0xFFFFu);
+        b[3] = mul1_pair(f1 & 0xFFFFu, f0 & 0xFFFFu);
+    }
+}
+// all of it: v[4 c + i] = b[i] of group c
+template <int KB>
+__device__ __forceinline__ void exl3_decode_quad(const uint32_t (&z)[4], uint32_t (&v)[16]) {
+    uint32_t b[4];
+    auto put = [&](int c) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[4 * c + i] = b[i];
+    };
+    exl3_decode8<KB, 0>(z, b); put(0);
+    exl3_decode8<KB, 1>(z, b); put(1);
+    exl3_decode8<KB, 2>(z, b); put(2);
+    exl3_decode8<KB, 3>(z, b); put(3);
 }
 
 // ---- 128-point Sylvester-natural Hadamard over a warp: lane holds elements 4*lane .. 4*lane+3 ----

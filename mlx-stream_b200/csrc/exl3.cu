@@ -4,12 +4,13 @@
 // of the decode chain: src/arch/deepseek_v41/experts.zig:449-467).  The weight stream is the bound: a CTA owns one
 // 128-wide output block of one expert for up to 16 of its rows, streams that block's code once through a ring of
 // bulk-copied (TMA 1-D) shared-memory stages, decodes each 16x16 tile in registers straight into one mma A fragment
-// (the trellis' tensor-core order makes a lane's 8 code positions exactly its fragment of W^T: 16 output columns x 16
+// (the trellis' tensor-core order makes eight consecutive states exactly a lane's fragment of W^T: 16 output columns x 16
 // inputs) and multiplies with the rows' rotated activations as the B operand: 8 token slots = 4 rows as f16 hi + the
 // same rows as f16 lo, so the f32 precision of the reference's decode chain is kept while the FMAs run on the tensor
 // pipe, one mma per tile for up to 4 rows.  The output-side Hadamard, svh, the clamped SwiGLU and the down
 // projection's input rotation are fused into the gate/up epilogue; H128 . svh into the down epilogue.
 #include <cstdlib>
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -23,54 +24,65 @@ constexpr int ZS_STRIDE = 132;    // padded row stride of the epilogue's f32 sta
 // ------------------------------------------------------------------------------------------------------------
 // load-time repack: reference record -> kernel layout (bit-preserving: words move, no bit changes)
 // ------------------------------------------------------------------------------------------------------------
-// V = uint4 (the record is 16-byte aligned: eight tiles of a k-tile are 48 or 32 vectors, contiguous on both sides) or uint32_t
-template <class V>
-__global__ void exl3_repack_kernel(const uint8_t* __restrict__ rec, uint32_t H, uint32_t I, uint32_t TW,
+// A block moves one quad column at a time: the four k-tiles x eight tiles of a 128-wide output block (eight tiles of a k-tile are
+// contiguous in the record), through shared memory into quad order (common.cuh).
+// V = uint4 (the record is 16-byte aligned: eight tiles of a k-tile are 48 or 32 vectors) or uint32_t
+template <class V, int KB>
+__global__ void __launch_bounds__(256) exl3_repack_kernel(const uint8_t* __restrict__ rec, uint32_t H, uint32_t I,
                                    uint32_t* __restrict__ gu, uint32_t* __restrict__ dn, __half* __restrict__ sc) {
-    const size_t code_bytes = (size_t)(H / 16) * (I / 16) * TW * 4;   // TW words per 16x16 tile (24 at K = 3, 16 at K = 2)
+    constexpr uint32_t TW = 8 * KB, QUAD = 4 * TW, UNIT = 8 * QUAD;   // words of a tile, of a quad, of the eight quads of a block
+    __shared__ __align__(16) uint32_t tiles[UNIT];
+    const size_t code_bytes = (size_t)(H / 16) * (I / 16) * TW * 4;
     // record offsets (src/expert/bank.zig:116-141): per projection code, rout [out], rin [in]
     const size_t off_g = 0, off_g_rout = code_bytes, off_g_rin = off_g_rout + 2 * (size_t)I;
     const size_t off_u = off_g_rin + 2 * (size_t)H, off_u_rout = off_u + code_bytes, off_u_rin = off_u_rout + 2 * (size_t)I;
     const size_t off_d = off_u_rin + 2 * (size_t)H, off_d_rout = off_d + code_bytes, off_d_rin = off_d_rout + 2 * (size_t)H;
-    const uint32_t per = 8u * TW * 4u / (uint32_t)sizeof(V);          // vectors of one k-tile of one 128-wide output block
-    const uint32_t n_code = (uint32_t)(code_bytes / sizeof(V)), n_all = 3 * n_code, n_sc = 3 * H + 3 * I;
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_all + n_sc; i += stride) {
-        if (i < n_all) {
-            // destination: gate / up [block][projection][k-tile][vector], down [block][k-tile][vector]
-            const bool down = i >= 2 * n_code;
-            uint32_t r = down ? i - 2 * n_code : i;
-            const uint32_t v = r % per; r /= per;
-            const uint32_t nkt = (down ? I : H) / 16, n_out = (down ? H : I) / 16;
-            const uint32_t kt = r % nkt; r /= nkt;
-            uint32_t p = 2;
-            if (!down) { p = r % 2; r /= 2; }
-            const V* src = reinterpret_cast<const V*>(rec + (p == 0 ? off_g : p == 1 ? off_u : off_d));
-            const V w = src[((size_t)kt * n_out + r * 8) * TW * 4 / sizeof(V) + v];
-            if (down) reinterpret_cast<V*>(dn)[i - 2 * n_code] = w;
-            else reinterpret_cast<V*>(gu)[i] = w;
-        } else {
-            const size_t s = i - n_all;
-            const __half* h;
-            if (s < H) h = reinterpret_cast<const __half*>(rec + off_g_rin) + s;                        // suh_g
-            else if (s < 2 * (size_t)H) h = reinterpret_cast<const __half*>(rec + off_u_rin) + (s - H);  // suh_u
-            else if (s < 2 * (size_t)H + I) h = reinterpret_cast<const __half*>(rec + off_g_rout) + (s - 2 * (size_t)H);
-            else if (s < 2 * (size_t)H + 2 * (size_t)I)
-                h = reinterpret_cast<const __half*>(rec + off_u_rout) + (s - 2 * (size_t)H - I);
-            else if (s < 2 * (size_t)H + 3 * (size_t)I)
-                h = reinterpret_cast<const __half*>(rec + off_d_rin) + (s - 2 * (size_t)H - 2 * (size_t)I);  // suh_d
-            else h = reinterpret_cast<const __half*>(rec + off_d_rout) + (s - 2 * (size_t)H - 3 * (size_t)I);  // svh_d
-            sc[s] = *h;
+    const uint32_t n_unit = (uint32_t)(code_bytes / 4 / UNIT);        // of one projection
+    for (uint32_t i = blockIdx.x; i < 3 * n_unit; i += gridDim.x) {
+        // destination: gate / up [block][projection][quad][tile][words], down [block][quad][tile][words]
+        const bool down = i >= 2 * n_unit;
+        uint32_t r = down ? i - 2 * n_unit : i;
+        const uint32_t nq = (down ? I : H) / 64, n_out = (down ? H : I) / 16;
+        const uint32_t q = r % nq; r /= nq;
+        uint32_t p = 2;
+        if (!down) { p = r % 2; r /= 2; }
+        const uint32_t* src = reinterpret_cast<const uint32_t*>(rec + (p == 0 ? off_g : p == 1 ? off_u : off_d)) + ((size_t)q * 4 * n_out + r * 8) * TW;
+        constexpr uint32_t PER = 8 * TW * 4 / sizeof(V);              // vectors of one k-tile
+        for (uint32_t v = threadIdx.x; v < 4 * PER; v += blockDim.x)
+            reinterpret_cast<V*>(tiles)[v] = reinterpret_cast<const V*>(src + (size_t)(v / PER) * n_out * TW)[v % PER];
+        __syncthreads();
+        uint32_t* dst = (down ? dn + (size_t)(i - 2 * n_unit) * UNIT : gu + (size_t)i * UNIT);
+        for (uint32_t w = threadIdx.x; w < UNIT; w += blockDim.x) {
+            const uint32_t t = w / QUAD, in = w % QUAD, l = in < 64 ? in / 2 : in - 64, wd = in < 64 ? in % 2 : 2;   // exl3_quad_words
+            dst[w] = tiles[((l & 3u) * 8 + t) * TW + KB * (l >> 2) + wd];
         }
+        __syncthreads();
+    }
+    const uint32_t n_sc = 3 * H + 3 * I;
+    for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < n_sc; s += gridDim.x * blockDim.x) {
+        const __half* h;
+        if (s < H) h = reinterpret_cast<const __half*>(rec + off_g_rin) + s;                        // suh_g
+        else if (s < 2 * (size_t)H) h = reinterpret_cast<const __half*>(rec + off_u_rin) + (s - H);  // suh_u
+        else if (s < 2 * (size_t)H + I) h = reinterpret_cast<const __half*>(rec + off_g_rout) + (s - 2 * (size_t)H);
+        else if (s < 2 * (size_t)H + 2 * (size_t)I)
+            h = reinterpret_cast<const __half*>(rec + off_u_rout) + (s - 2 * (size_t)H - I);
+        else if (s < 2 * (size_t)H + 3 * (size_t)I)
+            h = reinterpret_cast<const __half*>(rec + off_d_rin) + (s - 2 * (size_t)H - 2 * (size_t)I);  // suh_d
+        else h = reinterpret_cast<const __half*>(rec + off_d_rout) + (s - 2 * (size_t)H - 3 * (size_t)I);  // svh_d
+        sc[s] = *h;
     }
 }
 
 cudaError_t launch_exl3_repack(const uint8_t* record_dev, Exl3Dims d, uint32_t* gu_code_e, uint32_t* d_code_e,
                                __half* scales_e, cudaStream_t st) {
-    if (reinterpret_cast<uintptr_t>(record_dev) % 16 == 0)
-        exl3_repack_kernel<uint4><<<592, 256, 0, st>>>(record_dev, d.H, d.I, exl3_tile_words(d), gu_code_e, d_code_e, scales_e);
-    else
-        exl3_repack_kernel<uint32_t><<<592, 256, 0, st>>>(record_dev, d.H, d.I, exl3_tile_words(d), gu_code_e, d_code_e, scales_e);
+    const bool wide = reinterpret_cast<uintptr_t>(record_dev) % 16 == 0;
+    if (d.K == 3) {
+        if (wide) exl3_repack_kernel<uint4, 3><<<1184, 256, 0, st>>>(record_dev, d.H, d.I, gu_code_e, d_code_e, scales_e);
+        else exl3_repack_kernel<uint32_t, 3><<<1184, 256, 0, st>>>(record_dev, d.H, d.I, gu_code_e, d_code_e, scales_e);
+    } else {
+        if (wide) exl3_repack_kernel<uint4, 2><<<1184, 256, 0, st>>>(record_dev, d.H, d.I, gu_code_e, d_code_e, scales_e);
+        else exl3_repack_kernel<uint32_t, 2><<<1184, 256, 0, st>>>(record_dev, d.H, d.I, gu_code_e, d_code_e, scales_e);
+    }
     return cudaGetLastError();
 }
 
@@ -148,37 +160,47 @@ struct StageMeta { int32_t item; uint32_t flags, mc, chunk0, expert, nb, part, p
 // (chunks of rows, sub-stages of KT k-tiles) -> 0 .. 7; rows in 3 or 4 chunks always come one sub-stage per slot
 __device__ __forceinline__ uint32_t slot_form(uint32_t mc, uint32_t sub) { return mc <= 2 ? (mc - 1) * 3 + sub - 1 : mc + 3; }
 
-// one pipeline stage (KT k-tiles) of one warp's 16-column tile, MC chunks of activations
+// one pipeline stage (KT k-tiles: two quads) of one warp's 16-column tile, MC chunks of activations
 template <int NPROJ, int KB, int MC>
-__device__ __forceinline__ void gemv_stage(const uint32_t* __restrict__ wt, const uint2* __restrict__ at, uint32_t mt_stride,
-                                           uint32_t wi, uint32_t wj, uint32_t lp, float (&acc)[GROUP_CHUNKS][4]) {
-    constexpr int KSTRIDE = 64 * KB;   // words per k-tile: 8 tiles of 8 KB words
-    // at: this projection's KT activation tiles of the first chunk (B-fragment order), the next chunk's mt_stride uint2 on
+__device__ __forceinline__ void gemv_stage(const uint32_t* __restrict__ wt, const uint32_t* __restrict__ at, uint32_t mt_stride,
+                                           uint32_t lane, float (&acc)[GROUP_CHUNKS][4]) {
+    constexpr int QSTRIDE = 8 * 32 * KB;   // words of a quad's eight tiles
+    // at: this projection's activations of the first chunk, 4 A_TILE_WORDS words per quad, the next chunk's mt_stride words on
 #pragma unroll
-    for (int kt = 0; kt < KT; ++kt) {
-        const uint32_t lo = wt[kt * KSTRIDE + wi], hi = wt[kt * KSTRIDE + wj];
-        uint32_t b[4];
-        exl3_decode_lane_kb<KB, true>(lo, hi, lp, b);
+    for (int q = 0; q < KT / 4; ++q) {
+        uint32_t z[4], b[4];
+        exl3_quad_words<KB>(wt + q * QSTRIDE, lane, z);
         // W^T as the A operand: rows = the tile's 16 output columns
-        const uint32_t a[4] = {b[0], b[2], b[1], b[3]};
+        auto product = [&](auto cc, const uint32_t* xp, uint2 first) {
+            exl3_decode8<KB, decltype(cc)::value>(z, b);
+            const uint32_t a[4] = {b[0], b[2], b[1], b[3]};
 #pragma unroll
-        for (int mt = 0; mt < MC; ++mt) {
-            const uint2 xv = at[mt * mt_stride + kt * 32];
-            mma_f16(acc[mt], a, xv.x, xv.y);
-        }
+            for (int mt = 0; mt < MC; ++mt) {
+                const uint2 xv = MC == 1 ? first : *reinterpret_cast<const uint2*>(xp + mt * mt_stride);
+                mma_f16(acc[mt], a, xv.x, xv.y);
+            }
+        };
+        auto products = [&](auto cc) {   // c and c + 1; of one chunk both fragments in one load (more do not fit the registers)
+            constexpr int C2 = decltype(cc)::value;
+            const uint32_t* xp = at + q * (4 * A_TILE_WORDS) + C2 * 64 + lane * 4;
+            const uint4 x = MC == 1 ? *reinterpret_cast<const uint4*>(xp) : make_uint4(0, 0, 0, 0);
+            product(cc, xp, make_uint2(x.x, x.y));
+            product(std::integral_constant<int, C2 + 1>(), xp + 2, make_uint2(x.z, x.w));
+        };
+        products(std::integral_constant<int, 0>());
+        products(std::integral_constant<int, 2>());
     }
 }
 
 // SUB sub-stages of one ring slot, unrolled: [projection][SUB x KT k-tiles of codes][chunk][projection][SUB x KT row tiles]
 template <int NPROJ, int KB, int MC, int SUB>
-__device__ __forceinline__ void gemv_slot(const uint8_t* __restrict__ st, uint32_t p, uint32_t lane, uint32_t wi, uint32_t wj,
-                                          uint32_t lp, float (&acc)[GROUP_CHUNKS][4]) {
+__device__ __forceinline__ void gemv_slot(const uint8_t* __restrict__ st, uint32_t p, uint32_t lane, uint32_t tile, float (&acc)[GROUP_CHUNKS][4]) {
     constexpr uint32_t CODE = SUB * KT * (64 * KB) * 4, ROWS = SUB * KT * A_TILE_WORDS * 4;   // bytes of one projection
-    const uint32_t* wt = reinterpret_cast<const uint32_t*>(st + (NPROJ == 2 ? p * CODE : 0u));
-    const uint2* at = reinterpret_cast<const uint2*>(st + NPROJ * CODE + (NPROJ == 2 ? p * ROWS : 0u)) + lane;
+    const uint32_t* wt = reinterpret_cast<const uint32_t*>(st + (NPROJ == 2 ? p * CODE : 0u)) + tile;
+    const uint32_t* at = reinterpret_cast<const uint32_t*>(st + NPROJ * CODE + (NPROJ == 2 ? p * ROWS : 0u));
 #pragma unroll
     for (int u = 0; u < SUB; ++u)
-        gemv_stage<NPROJ, KB, MC>(wt + u * KT * (64 * KB), at + u * KT * 32, NPROJ * SUB * KT * 32, wi, wj, lp, acc);
+        gemv_stage<NPROJ, KB, MC>(wt + u * KT * (64 * KB), at + u * KT * A_TILE_WORDS, NPROJ * SUB * KT * A_TILE_WORDS, lane, acc);
 }
 
 // KB = bits per weight
@@ -298,8 +320,7 @@ __global__ void __launch_bounds__(NPROJ * 256 + 32, NPROJ == 1 ? 3 : 2) exl3_gem
 
     // ---------------- consumer warps ----------------
     const uint32_t p = NPROJ == 2 ? warp >> 3 : 0u, j = warp & 7u;  // projection, 16-column tile
-    uint32_t wi, wj, lp;
-    exl3_lane_plan_kb<KB>(lane, wi, wj, lp);
+    const uint32_t tile = j * (32 * KB);   // words of this warp's quad inside a quad's eight
     float acc[GROUP_CHUNKS][4];
     const float S = __uint_as_float(SCALE_BITS);
     uint32_t epi_ph = 0;
@@ -315,7 +336,6 @@ __global__ void __launch_bounds__(NPROJ * 256 + 32, NPROJ == 1 ? 3 : 2) exl3_gem
     // ring slot, its barriers, its meta and its phase advance by increment-and-wrap (the ring depth is a run-time value: no
     // division per stage, and as little else as possible: the decode leaves no free issue slots)
     const uint32_t full0 = smem_u32(&full_bar[0]), full_end = full0 + 8 * NS;
-    wi += j * TW; wj += j * TW;            // words of this warp's tile inside a k-tile
     uint32_t bar = full0, ph = 0;
     const uint8_t* st = ring;
     const StageMeta* mp = &meta[0];
@@ -338,17 +358,17 @@ __global__ void __launch_bounds__(NPROJ * 256 + 32, NPROJ == 1 ? 3 : 2) exl3_gem
         static_assert(GROUP_CHUNKS == 4, "the stage dispatch below enumerates the chunk counts");
         // straight-line code per slot_form
         if (form < 3) {
-            if (form == 1) gemv_slot<NPROJ, KB, 1, 2>(st, p, lane, wi, wj, lp, acc);
-            else if (form == 2) gemv_slot<NPROJ, KB, 1, 3>(st, p, lane, wi, wj, lp, acc);
-            else gemv_slot<NPROJ, KB, 1, 1>(st, p, lane, wi, wj, lp, acc);
+            if (form == 1) gemv_slot<NPROJ, KB, 1, 2>(st, p, lane, tile, acc);
+            else if (form == 2) gemv_slot<NPROJ, KB, 1, 3>(st, p, lane, tile, acc);
+            else gemv_slot<NPROJ, KB, 1, 1>(st, p, lane, tile, acc);
         } else if (form < 6) {
-            if (form == 4) gemv_slot<NPROJ, KB, 2, 2>(st, p, lane, wi, wj, lp, acc);
-            else if (form == 5) gemv_slot<NPROJ, KB, 2, 3>(st, p, lane, wi, wj, lp, acc);
-            else gemv_slot<NPROJ, KB, 2, 1>(st, p, lane, wi, wj, lp, acc);
+            if (form == 4) gemv_slot<NPROJ, KB, 2, 2>(st, p, lane, tile, acc);
+            else if (form == 5) gemv_slot<NPROJ, KB, 2, 3>(st, p, lane, tile, acc);
+            else gemv_slot<NPROJ, KB, 2, 1>(st, p, lane, tile, acc);
         } else if (form == 6) {
-            gemv_slot<NPROJ, KB, 3, 1>(st, p, lane, wi, wj, lp, acc);
+            gemv_slot<NPROJ, KB, 3, 1>(st, p, lane, tile, acc);
         } else {
-            gemv_slot<NPROJ, KB, 4, 1>(st, p, lane, wi, wj, lp, acc);
+            gemv_slot<NPROJ, KB, 4, 1>(st, p, lane, tile, acc);
         }
         // the slot may be refilled once this warp has arrived below.  (Gate/up has 56 registers a thread: the copy of the
         // whole struct spilled, 4 % at K = 2)

@@ -5,22 +5,22 @@
 
 namespace mlxs {
 
-constexpr int A_TILE_WORDS = 64;   // one chunk x k-tile of activations in B-fragment order: 32 lanes x 2 u32
+constexpr int A_TILE_WORDS = 64;   // activations of one chunk and 16 inputs: 8 slots x 16 f16
 
-// One chunk x k-tile block is 32 lanes x 2 u32: lane (g = token slot, c) holds b0 = x[slot g][k 2c,2c+1],
-// b1 = x[slot g][k 2c+8,2c+9]; slots 0..3 are the f16 hi halves of rows 0..3, slots 4..7 their lo halves.  A warp lane
+// A chunk's 64 inputs of a quad (four k-tiles) are 256 words [c / 2][32 lanes][c % 2][2]: lane (g = token slot, j) holds, for
+// each of the quad's four products c, b0 = x[slot g][k-tile j, inputs 2c, 2c+1] and b1 = x[slot g][2c+8, 2c+9], the B fragment
+// that goes with exl3_decode8<c>; slots 0..3 are the f16 hi halves of rows 0..3, slots 4..7 their lo halves.  A warp lane
 // that owns elements 4*lane..4*lane+3 of a 128-block writes k-tile lane/4, k = 4*(lane&3) + q.
-__device__ __forceinline__ void store_frag4(uint32_t* tile_base /* the 128-block's first k-tile */, uint32_t row,
+__device__ __forceinline__ void store_frag4(uint32_t* block_base /* the 128-block's two quads */, uint32_t row,
                                             uint32_t lane, const float (&v)[4]) {
-    const uint32_t cq = lane & 3u;
-    uint32_t* kt = tile_base + (lane >> 2) * A_TILE_WORDS;
-    const uint32_t c0 = 2u * (cq & 1u), reg = cq >> 1;
+    const uint32_t cq = lane & 3u, j = (lane >> 2) & 3u;
+    uint32_t* w = block_base + (lane >> 4) * (4u * A_TILE_WORDS) + (cq & 1u) * 128u + (row * 4u + j) * 4u + (cq >> 1);
     __half h0, l0, h1, l1, h2, l2, h3, l3;
     split_hi_lo(v[0], h0, l0); split_hi_lo(v[1], h1, l1); split_hi_lo(v[2], h2, l2); split_hi_lo(v[3], h3, l3);
-    kt[(row * 4u + c0) * 2u + reg] = pack_h2(h0, h1);
-    kt[((row + 4u) * 4u + c0) * 2u + reg] = pack_h2(l0, l1);
-    kt[(row * 4u + c0 + 1u) * 2u + reg] = pack_h2(h2, h3);
-    kt[((row + 4u) * 4u + c0 + 1u) * 2u + reg] = pack_h2(l2, l3);
+    w[0] = pack_h2(h0, h1);
+    w[2] = pack_h2(h2, h3);
+    w[64] = pack_h2(l0, l1);    // four slots on
+    w[66] = pack_h2(l2, l3);
 }
 
 // One warp stages one 128-block b of one row of a chunk (both projections, or the raw row): xg = H128(x * suh) *

@@ -11,30 +11,33 @@ int mlxs_fail(int rc, const char* fmt, ...);
 
 namespace mlxs {
 
-// One warp decodes `tiles` 16x16 tiles.  The two code words of a lane evolve by a cheap recurrence that does not
-// depend on the decode's result (so the compiler can neither hoist nor fold the decode), the decoded fragments are
+// One warp decodes `quads` quads (four 16x16 tiles each).  The code words of a lane evolve by a cheap recurrence that does
+// not depend on the decode's result (so the compiler can neither hoist nor fold the decode), the decoded fragments are
 // folded into a checksum that is stored once.
 template <int KB, bool MMA>
-__global__ void __launch_bounds__(512, 2) exl3_decode_probe_kernel(uint32_t tiles, uint32_t seed, uint32_t* __restrict__ sink) {
-    const uint32_t lane = threadIdx.x & 31u;
-    uint32_t wi, wj, lp;
-    exl3_lane_plan_kb<KB>(lane, wi, wj, lp);
-    uint32_t lo = seed ^ (blockIdx.x * 2654435761u + threadIdx.x * 40503u), hi = lo * 747796405u + 2891336453u;
+__global__ void __launch_bounds__(512, 2) exl3_decode_probe_kernel(uint32_t quads, uint32_t seed, uint32_t* __restrict__ sink) {
+    uint32_t z[4];
+    z[0] = seed ^ (blockIdx.x * 2654435761u + threadIdx.x * 40503u);
+#pragma unroll
+    for (int i = 1; i < 4; ++i) z[i] = z[i - 1] * 747796405u + 2891336453u;
     uint32_t chk = 0;
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    const uint32_t bx = lo | 0x3C003C00u, by = hi | 0x3C003C00u;   // stand-ins for the rows' fragment
-#pragma unroll 8
-    for (uint32_t t = 0; t < tiles; ++t) {
-        uint32_t b[4];
-        exl3_decode_lane_kb<KB>(lo, hi, lp, b);
-        if (MMA) {
-            const uint32_t a[4] = {b[0], b[2], b[1], b[3]};
-            mma_f16(acc, a, bx, by);
-        } else {
-            chk ^= b[0] ^ b[1] ^ b[2] ^ b[3];
+    const uint32_t bx = z[0] | 0x3C003C00u, by = z[1] | 0x3C003C00u;   // stand-ins for the rows' fragment
+#pragma unroll 2
+    for (uint32_t t = 0; t < quads; ++t) {
+        uint32_t v[16];
+        exl3_decode_quad<KB>(z, v);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            if (MMA) {
+                const uint32_t a[4] = {v[4 * c], v[4 * c + 2], v[4 * c + 1], v[4 * c + 3]};
+                mma_f16(acc, a, bx, by);
+            } else {
+                chk ^= v[4 * c] ^ v[4 * c + 1] ^ v[4 * c + 2] ^ v[4 * c + 3];
+            }
         }
-        lo += 0x9E3779B9u;      // one add per word stands in for the two shared-memory loads of the real loop
-        hi += 0x7F4A7C15u;
+#pragma unroll
+        for (int i = 0; i <= KB; ++i) z[i] += 0x9E3779B9u + 0x1F123BB4u * i;   // one add per word stands in for the shared-memory loads of the real loop
     }
     if (MMA) chk = __float_as_uint(acc[0]) ^ __float_as_uint(acc[1]) ^ __float_as_uint(acc[2]) ^ __float_as_uint(acc[3]);
     if (chk == 0x12345u) sink[0] = chk;   // practically never: keeps the loop alive
@@ -59,20 +62,21 @@ extern "C" int mlxs_moe_exl3_decode_rate(int32_t device, uint32_t bits, int with
     cudaEventCreate(&a);
     cudaEventCreate(&b);
     const int grid = 2 * prop.multiProcessorCount, threads = 512;   // the gate/up kernel's residency: 32 decode warps per SM
-    auto launch = [&](uint32_t tiles) {
+    auto launch = [&](uint32_t quads) {
         if (bits == 3) {
-            if (with_mma) exl3_decode_probe_kernel<3, true><<<grid, threads>>>(tiles, 1u, sink);
-            else exl3_decode_probe_kernel<3, false><<<grid, threads>>>(tiles, 1u, sink);
+            if (with_mma) exl3_decode_probe_kernel<3, true><<<grid, threads>>>(quads, 1u, sink);
+            else exl3_decode_probe_kernel<3, false><<<grid, threads>>>(quads, 1u, sink);
         } else {
-            if (with_mma) exl3_decode_probe_kernel<2, true><<<grid, threads>>>(tiles, 1u, sink);
-            else exl3_decode_probe_kernel<2, false><<<grid, threads>>>(tiles, 1u, sink);
+            if (with_mma) exl3_decode_probe_kernel<2, true><<<grid, threads>>>(quads, 1u, sink);
+            else exl3_decode_probe_kernel<2, false><<<grid, threads>>>(quads, 1u, sink);
         }
     };
-    launch(tiles_per_warp / 8 + 1);   // warm-up
+    const uint32_t quads = (tiles_per_warp + 3) / 4;
+    launch(quads / 8 + 1);   // warm-up
     float best = 0.f;
     for (int rep = 0; rep < 3; ++rep) {
         cudaEventRecord(a, 0);
-        launch(tiles_per_warp);
+        launch(quads);
         cudaEventRecord(b, 0);
         if ((e = cudaEventSynchronize(b)) != cudaSuccess) break;
         float ms = 0.f;
@@ -85,6 +89,6 @@ extern "C" int mlxs_moe_exl3_decode_rate(int32_t device, uint32_t bits, int with
     cudaFree(sink);
     if (e != cudaSuccess) return mlxs_fail(MLXS_E_CUDA, "exl3_decode_rate: %s", cudaGetErrorString(e));
     const double warps = (double)grid * (threads / 32);
-    *tiles_per_s = warps * (double)tiles_per_warp / ((double)best * 1e-3);
+    *tiles_per_s = warps * 4.0 * (double)quads / ((double)best * 1e-3);
     return MLXS_OK;
 }

@@ -16,18 +16,17 @@
 
 #include "../../include/mlxs_moe.h"
 #include "common.cuh"
+#include "exl3_prep_body.cuh"
 
 namespace mlxs {
 
 constexpr uint32_t NA_MAX_ROWS = 32;    // rows per call
 constexpr uint32_t NA_MAX_IN = 8192;    // input width
-constexpr uint32_t NA_FRAG_WORDS = 64;  // one 4-row chunk x one 16-input tile: 32 lanes x 2 u32
-constexpr size_t NA_SCRATCH_WORDS = (size_t)(NA_MAX_ROWS / 4) * (NA_MAX_IN / 16) * NA_FRAG_WORDS;  // 262,144 = 1 MiB
+constexpr size_t NA_SCRATCH_WORDS = (size_t)(NA_MAX_ROWS / 4) * (NA_MAX_IN / 16) * A_TILE_WORDS;  // 262,144 = 1 MiB
 
 static __device__ __align__(256) uint32_t g_scratch[NA_SCRATCH_WORDS];
 
-// rows -> fragment order: lane (g = token slot, c) of a (chunk, k-tile) block holds x[slot g][k 2c,2c+1] and
-// x[slot g][k 2c+8,2c+9]; slots 0..3 are the f16 hi halves of the chunk's rows, slots 4..7 their lo halves
+// rows -> fragment order (store_frag4), a 128-block of a chunk at a time
 __global__ void __launch_bounds__(128) na_stage_kernel(const float* __restrict__ xh, uint32_t rows, uint32_t in_dim,
                                                        uint32_t* __restrict__ xa) {
     const uint32_t chunk = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
@@ -39,14 +38,7 @@ __global__ void __launch_bounds__(128) na_stage_kernel(const float* __restrict__
             const float4 f = *reinterpret_cast<const float4*>(xh + (size_t)r * in_dim + b * 128 + lane * 4);
             v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
         }
-        const uint32_t cq = lane & 3u, c0 = 2u * (cq & 1u), reg = cq >> 1;
-        uint32_t* kt = xa + ((size_t)chunk * nkt + b * 8 + (lane >> 2)) * NA_FRAG_WORDS;
-        __half h0, l0, h1, l1, h2, l2, h3, l3;
-        split_hi_lo(v[0], h0, l0); split_hi_lo(v[1], h1, l1); split_hi_lo(v[2], h2, l2); split_hi_lo(v[3], h3, l3);
-        kt[(warp * 4u + c0) * 2u + reg] = pack_h2(h0, h1);
-        kt[((warp + 4u) * 4u + c0) * 2u + reg] = pack_h2(l0, l1);
-        kt[(warp * 4u + c0 + 1u) * 2u + reg] = pack_h2(h2, h3);
-        kt[((warp + 4u) * 4u + c0 + 1u) * 2u + reg] = pack_h2(l2, l3);
+        store_frag4(xa + ((size_t)chunk * nkt + b * 8) * A_TILE_WORDS, warp, lane, v);
     }
 }
 
@@ -58,9 +50,7 @@ __global__ void __launch_bounds__(128) na_gemv_kernel(const uint32_t* __restrict
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t tn = blockIdx.x * 4 + warp, chunk = blockIdx.y, nkt = in_dim / 16, ntn = out_dim / 16;
     if (tn >= ntn) return;
-    uint32_t wi, wj, lp;
-    exl3_lane_plan(lane, wi, wj, lp);
-    const uint2* xv = reinterpret_cast<const uint2*>(xa + (size_t)chunk * nkt * NA_FRAG_WORDS) + lane;
+    const uint4* xv = reinterpret_cast<const uint4*>(xa + (size_t)chunk * nkt * A_TILE_WORDS) + lane;
     // the sum over the inputs in the same equal parts, folded left, as the handle's streaming kernel takes it (4 parts
     // when the k-tiles divide by 32, else 2 by 16, else one): the two entries then agree bit for bit
     const uint32_t parts = nkt % 32 == 0 ? 4u : (nkt % 16 == 0 ? 2u : 1u), part_kt = nkt / parts;
@@ -68,13 +58,19 @@ __global__ void __launch_bounds__(128) na_gemv_kernel(const uint32_t* __restrict
     float v[4] = {0.f, 0.f, 0.f, 0.f};
     for (uint32_t part = 0; part < parts; ++part) {
         float acc[4] = {0.f, 0.f, 0.f, 0.f};
-        for (uint32_t kt = part * part_kt; kt < (part + 1) * part_kt; ++kt) {
-            const uint32_t* tile = code + ((size_t)kt * ntn + tn) * 24;
-            uint32_t b[4];
-            exl3_decode_lane(tile[wi], tile[wj], lp, b);
-            const uint32_t a[4] = {b[0], b[2], b[1], b[3]};
-            const uint2 x2 = xv[(size_t)kt * 32];
-            mma_f16(acc, a, x2.x, x2.y);
+        for (uint32_t kt = part * part_kt; kt < (part + 1) * part_kt; kt += 4) {
+            // the lane's words straight from the tiles: the group u = g of k-tile kt + c
+            const uint32_t* tile = code + ((size_t)(kt + c) * ntn + tn) * 24;
+            const uint32_t z[4] = {tile[3 * g + 2], tile[3 * g + 1], tile[3 * g], tile[(3 * g + 23) % 24]};
+            uint32_t w[16];
+            exl3_decode_quad<3>(z, w);
+            const uint4 x0 = xv[(size_t)kt * 16], x1 = xv[(size_t)kt * 16 + 32];
+            const uint32_t x[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const uint32_t a[4] = {w[4 * q], w[4 * q + 2], w[4 * q + 1], w[4 * q + 3]};
+                mma_f16(acc, a, x[2 * q], x[2 * q + 1]);
+            }
         }
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
