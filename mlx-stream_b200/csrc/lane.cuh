@@ -19,7 +19,10 @@
 //     decode is short: EXL3 8 % at 2048 tokens and 4 % at 8192, MXFP4 20 % at 2048 and 12 % at 3500.
 //     (Decoding in smaller pieces, or with 5 or 6 warps per lane quarter, measured slower or equal.)
 //   * The MMA warp runs its loop with all lanes and issues under elect.sync (see elect_one); one commit per stage frees the
-//     operand slot and the rows' slot.
+//     operand slot and the rows' slot.  What its operands come from goes through a shuffle from lane 0, so that the compiler
+//     knows that the warp has one value: they stay in uniform registers instead of being moved there for every MMA (cycles
+//     from a stage's operands to its eight MMAs issued, 64 / 128 / 256 rows: EXL3 659 / 749 / 778 -> 578 / 728 / 703, NVFP4 at
+//     128 554 -> 499; the layer at 2048 EXL3 tokens 2911 -> 2842 us, 8192 7480 -> 7258, NVFP4 at 4093 3033 -> 2974).
 //   * One producer lane streams the code, another the rows: bulk copies into rings.
 //   * The code producer takes the CTA's items one by one from a counter and passes them on to the other roles.  Beside the
 //     streaming lane the CTAs start when SMs come free, up to a third of the kernel apart, and with items dealt out in
@@ -140,13 +143,14 @@ __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P)
     uint64_t *full = bar_stage, *done = bar_stage + LN_DONE;             // of the stages in flight: operands complete, MMAs complete
     __shared__ uint32_t s_tmem;
     __shared__ volatile int s_abort;
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    const uint32_t warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31u;
     const uint32_t n_items = P.tiles[0] * P.n_blocks;
     // a CTA that cannot get work leaves before it takes tensor memory (the whole CTA reads the same count)
     if (blockIdx.x >= n_items) return;
 
+    const uint32_t most = __shfl_sync(0xFFFFFFFFu, P.tiles[2], 0);
     // columns of an accumulator buffer (the call's largest tile), operand slots in what is left
-    const uint32_t acc_cols = P.tiles[2] <= 128u ? 128u : P.tiles[2] <= (uint32_t)LN_ROWS_NARROW ? (uint32_t)LN_ROWS_NARROW : (uint32_t)LN_ROWS, slots = (512u - 2u * acc_cols) / LN_A_COLS;
+    const uint32_t acc_cols = most <= 128u ? 128u : most <= (uint32_t)LN_ROWS_NARROW ? (uint32_t)LN_ROWS_NARROW : (uint32_t)LN_ROWS, slots = (512u - 2u * acc_cols) / LN_A_COLS;
     const uint32_t teams = slots >= 3 ? 4u : 2u, raw_stages = 2u * teams, b_slot = acc_cols * (LN_KST * 2u);
     uint8_t* b_ring = smem_raw;                                          // [stage][rows16 x 256 B]
     uint8_t* raw_ring = b_ring + LN_B_STAGES * b_slot;                   // [stage][BK::RAW_BYTES]
@@ -165,7 +169,7 @@ __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P)
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = s_tmem, tmem_a = tmem + 2 * acc_cols;
+    const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, s_tmem, 0), tmem_a = tmem + 2 * acc_cols;
     const uint32_t nstage = P.n_stages, width = nstage * LN_KST;
     auto give_up = [&](uint32_t code) { if (!s_abort) atomicMax(P.status, code); s_abort = 1; };
     // item number n of this CTA, once it is known; false: there is none (or the CTA has given up)
@@ -308,7 +312,7 @@ __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P)
             uint4 te;
             uint32_t nb;
             if (!__all_sync(0xFFFFFFFFu, next_item(it, te, nb, 0))) break;
-            const uint32_t idesc = umma_idesc(BK::FORMAT, (te.z + 15) / 16 * 16);
+            const uint32_t idesc = umma_idesc(BK::FORMAT, __shfl_sync(0xFFFFFFFFu, (te.z + 15) / 16 * 16, 0));
             for (int p = 0; p < NPASS && ok; ++p, ++pass_n) {
                 const uint32_t buf = pass_n & 1u, acc = tmem + buf * acc_cols;
                 if (!mbar_wait_warp(&acc_empty[buf], ((pass_n >> 1) & 1u) ^ 1u, &s_abort)) { give_up(ST_WAIT_EMPTY); ok = false; break; }
