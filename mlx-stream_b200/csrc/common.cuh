@@ -47,6 +47,18 @@ __device__ __forceinline__ bool mbar_try_wait_at(uint32_t bar, uint32_t parity) 
         : "memory");
     return ok != 0;
 }
+// a test that never suspends the warp (try_wait may, for a time that the hardware chooses)
+__device__ __forceinline__ bool mbar_test_at(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) { return mbar_try_wait_at(smem_u32(bar), parity); }
 // Bounded wait: gives up after `limit` polls (each poll itself blocks for a hardware-defined slice) or as soon as
 // *abort_flag is set by another thread of the CTA.  Returns false when it gave up.

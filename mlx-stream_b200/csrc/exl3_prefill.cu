@@ -222,6 +222,8 @@ struct Exl3LaneBank {
     static constexpr uint32_t FORMAT = UMMA_F16;
     static constexpr uint32_t TW = 8 * KB, KT_WORDS = 8 * TW;   // words per 16x16 tile, per k-tile of a block
     static constexpr uint32_t RAW_BYTES = (LN_KST / 16) * KT_WORDS * 4;
+    static constexpr uint32_t AHEAD = 2;   // pieces of a stage decoded before the operand slot is waited for
+    static constexpr int MID = 8;          // MMAs of a stage before the next one's barrier is tested (8: not before the stage)
     static constexpr size_t EPI_SMEM = 2 * PF_EPI_ROWS * PF_ZS_STRIDE * sizeof(float);
 
     // the passes' k-tiles follow each other in the stream: stage ks of both passes together
@@ -235,23 +237,17 @@ struct Exl3LaneBank {
         __device__ __forceinline__ Decoder(uint32_t q, uint32_t half, uint32_t lane_) : lane(lane_) {
             off = half * (LN_KST / 32) * KT_WORDS + 2 * q * (4 * TW);   // lanes 32 q .. hold the 16-column tiles 2 q, 2 q + 1
         }
-        // h: halves of a stage behind the constructor's
-        __device__ __forceinline__ void decode(const uint8_t* raw, uint32_t slot_bytes, uint32_t h, uint32_t (&v)[2][16]) const {
-            const uint32_t* w = reinterpret_cast<const uint32_t*>(raw + slot_bytes) + off + h * ((LN_KST / 32) * KT_WORDS);
-#pragma unroll
-            for (int jj = 0; jj < 2; ++jj) {
-                uint32_t z[4];
-                exl3_quad_words<KB>(w + jj * (4 * TW), lane, z);
-                exl3_decode_quad<KB>(z, v[jj]);
-            }
+        // piece pc of the stage (or of the constructor's half): a quad of one of the two tiles
+        __device__ __forceinline__ void decode(const uint8_t* raw, uint32_t slot_bytes, uint32_t pc, uint32_t (&v)[16]) const {
+            uint32_t z[4];
+            exl3_quad_words<KB>(reinterpret_cast<const uint32_t*>(raw + slot_bytes) + off + (pc >> 1) * ((LN_KST / 32) * KT_WORDS) + (pc & 1u) * (4 * TW), lane, z);
+            exl3_decode_quad<KB>(z, v);
         }
-        static __device__ __forceinline__ void store(uint32_t ta, const uint32_t (&v)[2][16]) {
-#pragma unroll
-            for (int jj = 0; jj < 2; ++jj)
-                asm volatile("tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(ta + ((jj * 16u) << 16)),
-                             "r"(v[jj][0]), "r"(v[jj][1]), "r"(v[jj][2]), "r"(v[jj][3]), "r"(v[jj][4]), "r"(v[jj][5]), "r"(v[jj][6]), "r"(v[jj][7]), "r"(v[jj][8]),
-                             "r"(v[jj][9]), "r"(v[jj][10]), "r"(v[jj][11]), "r"(v[jj][12]), "r"(v[jj][13]), "r"(v[jj][14]), "r"(v[jj][15])
-                             : "memory");
+        static __device__ __forceinline__ void store(uint32_t ta, uint32_t pc, const uint32_t (&v)[16]) {
+            asm volatile("tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(ta + (pc >> 1) * (LN_A_COLS / 2) + ((pc & 1u) << 20)),
+                         "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
+                         "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+                         : "memory");
         }
     };
 

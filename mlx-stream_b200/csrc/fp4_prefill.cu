@@ -121,6 +121,8 @@ struct Fp4LaneBank {
     static constexpr uint32_t FORMAT = NV ? UMMA_F16 : UMMA_BF16;
     static constexpr uint32_t S_STAGE = NV ? 1024u : 512u;      // scale bytes of a projection's (block, stage)
     static constexpr uint32_t RAW_BYTES = Q_W_STAGE + S_STAGE;
+    static constexpr uint32_t AHEAD = 1;   // pieces of a stage decoded before the operand slot is waited for
+    static constexpr int MID = 4;          // MMAs of a stage before the next one's barrier is tested (8: not before the stage)
     static constexpr size_t EPI_SMEM = LN_EPI_WARPS * Q_T_WARP;
 
     // the stream holds, per stage, the projections' codes, then their scales
@@ -139,37 +141,32 @@ struct Fp4LaneBank {
             w_off = (((wr * 4 + sb) * 2 + r) * 32 + g * 4) * 4;                       // words [wr][block][r][g][4]
             s_off = Q_W_STAGE + (NV ? (wr * 4 + sb) * 32 + g * 2 + r : ((wr * 4 + sb) * 8 + g) * 2 + r);
         }
-        // h: halves of a stage behind the constructor's
-        __device__ __forceinline__ void decode(const uint8_t* raw, uint32_t slot_bytes, uint32_t h, uint32_t (&v)[2][16]) const {
-            const uint8_t *w = raw + slot_bytes + w_off + h * 512u, *s = raw + slot_bytes + s_off + h * (NV ? 64u : 32u);
+        // piece pc of the stage (or of the constructor's half): a 32-block, 32 codes of this column
+        __device__ __forceinline__ void decode(const uint8_t* raw, uint32_t slot_bytes, uint32_t pc, uint32_t (&v)[16]) const {
+            const uint4 ww = *reinterpret_cast<const uint4*>(raw + slot_bytes + w_off + pc * 256u);
+            const uint8_t* s = raw + slot_bytes + s_off + pc * (NV ? 32u : 16u);
+            const uint32_t wds[4] = {ww.x, ww.y, ww.z, ww.w};
+            uint32_t s0, s1;
+            if (NV) {
+                s0 = q_e4m3_f16x2(s[0]);
+                s1 = q_e4m3_f16x2(s[16]);
+            } else {
+                s0 = s1 = ((s[0] + 126u) << 7) * 0x00010001u;   // 2^(b - 1) in both halves
+            }
 #pragma unroll
-            for (int b = 0; b < 2; ++b) {
-                const uint4 ww = *reinterpret_cast<const uint4*>(w + b * 256);
-                const uint32_t wds[4] = {ww.x, ww.y, ww.z, ww.w};
-                uint32_t s0, s1;
-                if (NV) {
-                    s0 = q_e4m3_f16x2(s[b * 32]);
-                    s1 = q_e4m3_f16x2(s[b * 32 + 16]);
-                } else {
-                    s0 = s1 = ((s[b * 16] + 126u) << 7) * 0x00010001u;   // 2^(b - 1) in both halves
-                }
+            for (int c = 0; c < 4; ++c) {
+                uint32_t h[4];
+                if (NV) q_decode8_f16(wds[c], h);
+                else q_decode8_bf16(wds[c], h);
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    uint32_t h[4];
-                    if (NV) q_decode8_f16(wds[c], h);
-                    else q_decode8_bf16(wds[c], h);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) v[b][4 * c + i] = NV ? q_mul_f16x2(h[i], c < 2 ? s0 : s1) : q_mul_bf16x2(h[i], s0);
-                }
+                for (int i = 0; i < 4; ++i) v[4 * c + i] = NV ? q_mul_f16x2(h[i], c < 2 ? s0 : s1) : q_mul_bf16x2(h[i], s0);
             }
         }
-        static __device__ __forceinline__ void store(uint32_t ta, const uint32_t (&v)[2][16]) {
-#pragma unroll
-            for (int b = 0; b < 2; ++b)
-                asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(ta + b * 16),
-                             "r"(v[b][0]), "r"(v[b][1]), "r"(v[b][2]), "r"(v[b][3]), "r"(v[b][4]), "r"(v[b][5]), "r"(v[b][6]), "r"(v[b][7]), "r"(v[b][8]),
-                             "r"(v[b][9]), "r"(v[b][10]), "r"(v[b][11]), "r"(v[b][12]), "r"(v[b][13]), "r"(v[b][14]), "r"(v[b][15])
-                             : "memory");
+        static __device__ __forceinline__ void store(uint32_t ta, uint32_t pc, const uint32_t (&v)[16]) {
+            asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(ta + pc * 16),
+                         "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
+                         "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+                         : "memory");
         }
     };
 

@@ -11,8 +11,8 @@
 //     further ahead and a stage's round trip (decode, store, MMAs, slot free) no longer shows.
 //     With gate and up accumulated together (2 x 192, one buffer) the K loop stood still for the epilogue, a fifth of an
 //     item's time, and experts of 65 .. 96 rows paid for it most.
-//   * 16 decode warps in teams that take the stages in turn.  A warp decodes half a stage of its 32 columns into 32 registers
-//     and only then waits for its operand slot: the MMAs of the slot's last stage run under the decode.  With three or four
+//   * 16 decode warps in teams that take the stages in turn.  A warp decodes a first piece of its 32 columns into registers
+//     (BK::AHEAD quarters of a stage) and only then waits for its operand slot: the MMAs of the slot's last stage run under the decode.  With three or four
 //     operand slots there are four teams of four warps, a warp decoding both halves of a stage, with two slots two teams of
 //     eight (a team of four keeps its slot for twice as long).  The barriers around a stage were a quarter of the instructions
 //     of a warp that decoded one half (EXL3: 60 per 16x16 tile, 43 of them the decode), and their latencies showed where the
@@ -23,6 +23,11 @@
 //     knows that the warp has one value: they stay in uniform registers instead of being moved there for every MMA (cycles
 //     from a stage's operands to its eight MMAs issued, 64 / 128 / 256 rows: EXL3 659 / 749 / 778 -> 578 / 728 / 703, NVFP4 at
 //     128 554 -> 499; the layer at 2048 EXL3 tokens 2911 -> 2842 us, 8192 7480 -> 7258, NVFP4 at 4093 3033 -> 2974).
+//     The FP4 banks, whose decode is short, test the next stage's barrier in the middle of a stage's MMAs and decode and store a
+//     quarter of a stage at a time (the first waits for the slot): NVFP4 at 4093 tokens 2979 -> 2949 us, MXFP4 at 16384 6280 -> 6150.
+//     What is left there is the copy of rows and codes from L2, 55 to 62 bytes per clock and SM (41 and 53 KB per stage of 760
+//     and 870 cycles; the MMAs alone are 520 and 700).  EXL3 is bound by the decode: neither helps, half a stage at a time is 1 %
+//     faster at 8192 tokens.
 //   * One producer lane streams the code, another the rows: bulk copies into rings.
 //   * The code producer takes the CTA's items one by one from a counter and passes them on to the other roles.  Beside the
 //     streaming lane the CTAs start when SMs come free, up to a third of the kernel apart, and with items dealt out in
@@ -124,7 +129,8 @@ struct LanePass {
     }
 };
 
-// shared memory of the two rings: four code stages beside tiles of up to 192 rows, eight where four teams decode
+// shared memory of the two rings: four code stages beside tiles of up to 192 rows, eight where four teams decode.  (As many stages of
+// rows as fit, up to eight, with a slot of the call's largest tile: no faster, and NVFP4 at 4093 tokens 3004 -> 3045 us.)
 template <class BK>
 constexpr size_t ln_ring_bytes() {
     constexpr size_t two = (size_t)LN_B_STAGES * LN_B_SLOT + 4 * BK::RAW_BYTES;
@@ -198,9 +204,11 @@ __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P)
         bool code_ready = false;
         uint32_t woff = 0, slot = team % slots;            // of stage g: g % slots
         uint32_t items = 0, known = 0;                     // items so far and the stages they have
+        LC(long long t_item = 0, t_code = 0, t_slot = 0; uint32_t n_st = 0; long long t0;)
         for (uint32_t i = 0;; ++i) {
             const uint32_t g = team + TEAMS * i;
             bool more = true;
+            LC(t0 = clock64(); ++n_st;)
             while (more && g >= known) {
                 uint4 tile;
                 uint32_t nb;
@@ -208,28 +216,32 @@ __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P)
                 known += NPASS * nstage;
             }
             if (!more) break;
+            LC(t_item += clock64() - t0; t0 = clock64();)
             if (!code_ready && !mbar_wait_bounded_at(b_raw, (i >> 1) & 1u, &s_abort)) { give_up(ST_WAIT_FULL); break; }
+            LC(t_code += clock64() - t0;)
             // this slot's last MMAs are stage d = g - slots
             const uint32_t d = g - slots, b_done = bar0 + 8 * LN_DONE + 8 * (d % LN_DONE), ph_done = (d / LN_DONE) & 1u;
-            uint32_t v[2][16];
-            dec.decode(raw, woff, 0, v);
-            const bool slot_ready = g < slots || mbar_try_wait_at(b_done, ph_done);
-            b_raw ^= x_raw;
-            if (TEAMS == 2) {
-                code_ready = mbar_try_wait_at(b_raw, ((i + 1) >> 1) & 1u);
-                __syncwarp();
-                if (lane == 0) mbar_arrive_at(b_emp);
+            constexpr uint32_t GROUPS = (TEAMS == 4 ? 4u : 2u) / BK::AHEAD;
+            bool ok = true;
+#pragma unroll
+            for (uint32_t gr = 0; gr < GROUPS; ++gr) {
+                uint32_t v[BK::AHEAD][16];
+#pragma unroll
+                for (uint32_t k = 0; k < BK::AHEAD; ++k) dec.decode(raw, woff, gr * BK::AHEAD + k, v[k]);
+                if (gr + 1 == GROUPS) {
+                    b_raw ^= x_raw;
+                    code_ready = mbar_test_at(b_raw, ((i + 1) >> 1) & 1u);
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_at(b_emp);
+                }
+                if (gr == 0) {
+                    if (g >= slots && !mbar_wait_bounded_at(b_done, ph_done, &s_abort)) { give_up(ST_WAIT_EMPTY); ok = false; break; }
+                    tc_fence_after();
+                }
+#pragma unroll
+                for (uint32_t k = 0; k < BK::AHEAD; ++k) BK::Decoder::store(ta0 + slot * LN_A_COLS, gr * BK::AHEAD + k, v[k]);
             }
-            if (!slot_ready && !mbar_wait_bounded_at(b_done, ph_done, &s_abort)) { give_up(ST_WAIT_EMPTY); break; }
-            tc_fence_after();
-            BK::Decoder::store(ta0 + slot * LN_A_COLS, v);
-            if (TEAMS == 4) {
-                dec.decode(raw, woff, 1, v);
-                code_ready = mbar_try_wait_at(b_raw, ((i + 1) >> 1) & 1u);
-                __syncwarp();
-                if (lane == 0) mbar_arrive_at(b_emp);
-                BK::Decoder::store(ta0 + slot * LN_A_COLS + LN_A_COLS / 2, v);
-            }
+            if (!ok) break;
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             tc_fence_before();
             __syncwarp();
@@ -237,6 +249,7 @@ __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P)
             b_emp ^= x_emp; woff ^= TEAMS * BK::RAW_BYTES;
             if (TEAMS == 4 && slots == 3) slot = slot == 2 ? 0u : slot + 1;   // else the slot stays the team's
         }
+        LC(if (blockIdx.x == 3 && lane == 0 && (warp == 13 || warp == 16) && n_st) printf("LANE<%d> decode warp %u: %u stages, cycles per stage: item %lld code %lld slot %lld\n", NPASS, warp, n_st, t_item / n_st, t_code / n_st, t_slot / n_st);)
     };
 
     if (warp >= LN_SERVICE && warp < LN_SERVICE + LN_DEC_WARPS) {
@@ -304,21 +317,25 @@ __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P)
         const uint64_t bdesc = umma_smem_desc(smem_u32(b_ring), LN_LBO, LN_SBO);
         const uint32_t bd_hi = (uint32_t)(bdesc >> 32), bd_lo0 = (uint32_t)bdesc, bd_step = b_slot >> 4, bd_end = bd_lo0 + LN_B_STAGES * bd_step;
         const uint32_t a_end = tmem_a + slots * LN_A_COLS;
-        uint32_t bd_lo = bd_lo0, a0 = tmem_a, bars = smem_u32(&bar_stage[0]), par = 0;   // bars: full[g % 4] at + 0, done[g % 4] at + 32
+        uint32_t bd_lo = bd_lo0, a0 = tmem_a, bars = smem_u32(&bar_stage[0]), par = 0;   // bars: full[g % LN_DONE], done[g % LN_DONE] 8 LN_DONE bytes on
         const uint32_t bars_end = bars + 8 * LN_DONE;
-        bool ok = true;
-        LC(long long m_a = 0, m_issue = 0; uint32_t g = 0;)
+        bool ok = true, ready = false;
+        LC(long long m_a = 0, m_issue = 0, m_acc = 0, m_item = 0, m_all = clock64(); uint32_t g = 0;)
         for (uint32_t it = 0; ok; ++it) {
             uint4 te;
             uint32_t nb;
+            LC(long long w0 = clock64();)
             if (!__all_sync(0xFFFFFFFFu, next_item(it, te, nb, 0))) break;
+            LC(m_item += clock64() - w0;)
             const uint32_t idesc = umma_idesc(BK::FORMAT, __shfl_sync(0xFFFFFFFFu, (te.z + 15) / 16 * 16, 0));
             for (int p = 0; p < NPASS && ok; ++p, ++pass_n) {
                 const uint32_t buf = pass_n & 1u, acc = tmem + buf * acc_cols;
+                LC(w0 = clock64();)
                 if (!mbar_wait_warp(&acc_empty[buf], ((pass_n >> 1) & 1u) ^ 1u, &s_abort)) { give_up(ST_WAIT_EMPTY); ok = false; break; }
+                LC(m_acc += clock64() - w0;)
                 for (uint32_t ks = 0; ks < nstage; ++ks) {
                     LC(const long long w1 = clock64(); ++g;)
-                    if (!mbar_wait_warp_at(bars, par, &s_abort)) { give_up(ST_WAIT_FULL); ok = false; break; }
+                    if (!ready && !mbar_wait_warp_at(bars, par, &s_abort)) { give_up(ST_WAIT_FULL); ok = false; break; }
                     tc_fence_after();
                     LC(const long long w2 = clock64();)
                     const uint32_t bars_n = bars + 8 == bars_end ? bars_end - 8 * LN_DONE : bars + 8, par_n = bars + 8 == bars_end ? par ^ 1u : par;
@@ -326,17 +343,25 @@ __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P)
                     if (elect_one()) {
                         umma_f16_ts_lohi(acc, a0, bd_lo, bd_hi, idesc, ks);
 #pragma unroll
-                        for (int i = 1; i < LN_KST / 16; ++i) umma_f16_ts_lohi(acc, a0 + i * 8, bd_lo + ((i * 2 * LN_LBO) >> 4), bd_hi, idesc, 1u);
+                        for (int i = 1; i < BK::MID; ++i) umma_f16_ts_lohi(acc, a0 + i * 8, bd_lo + ((i * 2 * LN_LBO) >> 4), bd_hi, idesc, 1u);
+                    }
+                    // the test of the next stage's barrier goes out between the MMAs: behind the last one its latency would show
+                    bool next = false;
+                    if (BK::MID < LN_KST / 16) next = mbar_test_at(bars_n, par_n);
+                    if (elect_one()) {
+#pragma unroll
+                        for (int i = BK::MID; i < LN_KST / 16; ++i) umma_f16_ts_lohi(acc, a0 + i * 8, bd_lo + ((i * 2 * LN_LBO) >> 4), bd_hi, idesc, 1u);
                         // one commit per stage frees the operand slot and the rows' slot
                         umma_commit_at(bars + 8 * LN_DONE);
                         if (ks + 1 == nstage) umma_commit(&acc_full[buf]);
                     }
+                    ready = __all_sync(0xFFFFFFFFu, next);
                     bars = bars_n; par = par_n; bd_lo = bd_n; a0 = a0 + LN_A_COLS == a_end ? tmem_a : a0 + LN_A_COLS;
                     LC(m_a += w2 - w1; m_issue += clock64() - w2;)
                 }
             }
         }
-        LC(if (blockIdx.x == 3 && g && lane == 0) printf("LANE<%d> mma warp: %u stages, cycles per stage: operand wait %lld issue %lld\n", NPASS, g, m_a / g, m_issue / g);)
+        LC(if (blockIdx.x == 3 && g && lane == 0) printf("LANE<%d> mma warp: %u stages, cycles per stage: operand wait %lld issue %lld acc %lld item %lld all %lld\n", NPASS, g, m_a / g, m_issue / g, m_acc / g, m_item / g, (clock64() - m_all) / g);)
     } else if (warp == 2) {
         // ---------------- rows' producer ----------------
         if (lane == 0) {
