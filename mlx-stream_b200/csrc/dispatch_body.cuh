@@ -117,11 +117,103 @@ __device__ __forceinline__ void place_block(uint32_t id, bool valid, uint32_t a,
     __syncthreads();
 }
 
+// Few assignments (a decode step of up to four tokens of top-8): a thread per assignment finds its place by looking at all of
+// them, a few barriers instead of fourteen.  What the scan and the placement write is written here entry by entry: the thread of
+// an expert's rank-th assignment writes the chunk that starts there, if one does, and the group.  The code of a decode step's
+// small kernels comes cold, so its length counts: the loops are not unrolled (unrolled, 8 rows took 9,500 cycles).  Inside the
+// front kernel, against the scan: 8 rows 7,700 -> 3,600 cycles, 56 rows 7,500 -> 7,400, 128 rows 8,100 -> 13,300.
+constexpr uint32_t DISPATCH_FEW = 32;
+__device__ __forceinline__ void dispatch_few(const int32_t* __restrict__ ids, uint32_t A, uint32_t E, const uint8_t* __restrict__ loaded,
+                                             DispatchTables t, uint32_t CHUNK_ROWS, uint32_t GROUP_CHUNKS, uint32_t HEAVY,
+                                             uint32_t* status, uint32_t* dsm) {
+    uint4* ids4 = reinterpret_cast<uint4*>((reinterpret_cast<uintptr_t>(dsm) + 15) / 16 * 16);   // [DISPATCH_FEW] ids
+    uint4* key4 = ids4 + DISPATCH_FEW / 4;                                                     // [DISPATCH_FEW] id << 2 | starts a group << 1 | starts a chunk
+    const uint32_t a = threadIdx.x, n4 = (A + 3) / 4;
+    uint32_t id = 0x3FFFFFFFu;   // behind every expert
+    if (a < A) {
+        const int32_t v = ids[a];
+        const bool good = v >= 0 && (uint32_t)v < E;
+        id = good ? (uint32_t)v : 0u;
+        if (!good) atomicMax(status, (uint32_t)ST_BAD_EXPERT_ID);
+        else if (loaded && !loaded[v]) atomicMax(status, (uint32_t)ST_NOT_LOADED);
+    }
+    if (a < DISPATCH_FEW) reinterpret_cast<uint32_t*>(ids4)[a] = id;
+    __syncthreads();
+    if (a < E) {   // E <= DTHREADS
+        uint32_t less = 0;
+#pragma unroll 1
+        for (uint32_t i = 0; i < n4; ++i) {
+            const uint4 w = ids4[i];
+            less += (w.x < a) + (w.y < a) + (w.z < a) + (w.w < a);
+        }
+        t.offsets[a] = less;
+    }
+    uint32_t less = 0, rank = 0, c = 0;
+    bool chunk = false, group = false;
+    if (a < A) {
+#pragma unroll 1
+        for (uint32_t i = 0; i < n4; ++i) {
+            const uint4 q = ids4[i];
+            const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+            for (uint32_t k = 0; k < 4; ++k) {
+                less += w[k] < id;
+                c += w[k] == id;
+                rank += w[k] == id && 4 * i + k < a;
+            }
+        }
+        t.order[less + rank] = a;
+        chunk = !takes_tensor_lane(c, HEAVY, loaded, id) && rank % CHUNK_ROWS == 0;
+        group = chunk && rank % (CHUNK_ROWS * GROUP_CHUNKS) == 0;
+    }
+    if (a < DISPATCH_FEW) reinterpret_cast<uint32_t*>(key4)[a] = id << 2 | (group ? 2u : 0u) | (chunk ? 1u : 0u);
+    const uint32_t n_chunks = (uint32_t)__syncthreads_count(chunk), n_groups = (uint32_t)__syncthreads_count(group);
+    const uint32_t distinct = (uint32_t)__syncthreads_count(a < A && rank == 0);
+    const bool ok = n_chunks <= t.max_chunks;
+    if (a == 0) {
+        t.offsets[E] = A;
+        if (!ok) atomicMax(status, (uint32_t)ST_WORKLIST_OVERFLOW);
+        t.header[HDR_NCHUNKS] = ok ? n_chunks : 0u;
+        t.header[HDR_NGROUPS] = ok ? n_groups : 0u;
+        t.header[HDR_CTR_GU] = 0;
+        t.header[HDR_CTR_DOWN] = 0;
+        t.header[HDR_CTR_AUX] = 0;
+        t.header[HDR_DISTINCT] = distinct;
+    }
+    if (chunk && ok) {
+        uint32_t ch = rank / CHUNK_ROWS, g = ch / GROUP_CHUNKS;
+        const uint32_t in = g * GROUP_CHUNKS, nc = (c + CHUNK_ROWS - 1) / CHUNK_ROWS;
+#pragma unroll 1
+        for (uint32_t i = 0; i < n4; ++i) {
+            const uint4 q = key4[i];
+            const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+            for (uint32_t k = 0; k < 4; ++k) {
+                const bool before = (w[k] >> 2) < id;
+                ch += before && (w[k] & 1u);
+                g += before && (w[k] & 2u);
+            }
+        }
+        t.chunk_expert[ch] = id;
+        t.chunk_row0[ch] = less + rank;
+        t.chunk_rows[ch] = min(CHUNK_ROWS, c - rank);
+        if (group) {
+            t.group_chunk0[g] = ch;
+            t.group_mc[g] = min(GROUP_CHUNKS, nc - in) | id << 16;
+        }
+    }
+    __syncthreads();
+}
+
 // The whole sort by one CTA of DTHREADS threads (A <= 2048 rows in practice); dsm: dispatch_words(A, E) words of shared memory
-__host__ __device__ inline size_t dispatch_words(uint32_t A, uint32_t E) { return (size_t)E + 99 + place_words(place_warps(A), E); }
+__host__ __device__ inline size_t dispatch_words(uint32_t A, uint32_t E) {
+    const size_t scan = (size_t)E + 99 + place_words(place_warps(A), E), few = 2 * DISPATCH_FEW + 3;
+    return scan > few ? scan : few;
+}
 __device__ __forceinline__ void dispatch_body(const int32_t* __restrict__ ids, uint32_t A, uint32_t E,
                                               const uint8_t* __restrict__ loaded, DispatchTables t, uint32_t CHUNK_ROWS,
                                               uint32_t GROUP_CHUNKS, uint32_t HEAVY, uint32_t* status, uint32_t* dsm) {
+    if (A <= DISPATCH_FEW) return dispatch_few(ids, A, E, loaded, t, CHUNK_ROWS, GROUP_CHUNKS, HEAVY, status, dsm);
     uint32_t* cnt = dsm;                // [E] counts, then running write positions
     uint32_t* ws = dsm + E;             // [99] scan scratch
     const uint32_t tid = threadIdx.x;

@@ -54,6 +54,7 @@ struct FrontParams {
     uint32_t poll_limit;
     int rthreads;
     int by_warp;                     // phases 1 and 2 in every CTA
+    uint32_t parts;                  // FP4: warps per staged row
 };
 
 __device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p) {
@@ -188,12 +189,13 @@ __global__ void __launch_bounds__(1024, 1) front_kernel(const FrontParams P) {
                                        lane, P.xa);
         }
     } else {
-        // a row's 8-input groups are split over 4 warps
-        for (uint32_t task = gw; task < n_chunks * P.chunk_rows * 4u; task += gstride) {
-            const uint32_t chunk = task / (P.chunk_rows * 4u), rem = task % (P.chunk_rows * 4u), row = rem / 4u, part = rem % 4u;
+        // a row's 8-input groups are split over `parts` warps
+        const uint32_t parts = P.parts, per_chunk = P.chunk_rows * parts;
+        for (uint32_t task = gw; task < n_chunks * per_chunk; task += gstride) {
+            const uint32_t chunk = task / per_chunk, rem = task % per_chunk, row = rem / parts, part = rem % parts;
             const bool valid = row < S.chunk_rows[chunk];
             const uint32_t tok = valid ? x_row_of(S, S.order[S.chunk_row0[chunk] + row], (uint32_t)P.K) : 0u;
-            fp4_prep_row(P.x, tok, valid, P.H, chunk, row, part * 32u + lane, 128u, P.xa);
+            fp4_prep_row(P.x, tok, valid, P.H, chunk, row, part * 32u + lane, parts * 32u, P.xa);
         }
     }
 }
@@ -228,11 +230,14 @@ cudaError_t launch_front(const FrontArgs& a, cudaStream_t st) {
     cudaError_t e = cudaFuncSetAttribute(front_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     const bool barrier = a.w_router || !P.by_warp;
-    // a warp per staging task (a row's 128-block, or a quarter of a row for the FP4 banks), at most a CTA per SM; with a
+    // a warp per staging task (a row's 128-block; for the FP4 banks a sixteenth of a row, or a quarter where that would be more
+    // warps than the SMs hold), at most a CTA per SM; with a
     // barrier 32 to 64 CTAs: one round of expert rows, and room beside the shared expert's kernels
     const unsigned sms = (unsigned)(a.sm_count > 0 ? a.sm_count : 32);
-    unsigned grid = ((unsigned)(a.T * a.K) * a.chunk_rows * (a.bank_exl3 ? a.H / 128 : 4u) + 31u) / 32u;
-    if (barrier) grid = grid < 32u ? 32u : grid > 64u ? 64u : grid;
+    const unsigned rows = (unsigned)(a.T * a.K) * a.chunk_rows;
+    P.parts = rows * 16u <= 32u * sms ? 16u : 4u;
+    unsigned grid = (rows * (a.bank_exl3 ? a.H / 128 : P.parts) + 31u) / 32u;
+    if (barrier) grid = grid < 32u ? 32u : grid > 64u || (a.w_router && a.T > 1) ? 64u : grid;   // 64: two CTAs per set of expert rows
     if (grid > sms) grid = sms;
     if (!barrier) {
         return launch_dependent(true, front_kernel, grid, 1024, smem, st, P);

@@ -19,36 +19,56 @@ __host__ __device__ inline size_t logits_smem_bytes(uint32_t H, uint32_t nwarps)
 
 // For few tokens: up to LG_TOK token rows are staged in shared memory per pass.  All threads of the CTA call this (it holds
 // CTA-wide barriers).  The CTA's warps form nwarps / 4 expert slots; CTA
-// `cta` of `n_cta` takes the experts e = (cta * slots + slot), stepping by n_cta * slots.
+// `cta` of `n_cta` takes the experts e = (cta * slots + slot), stepping by n_cta * slots.  Where the grid has twice the slots
+// that the experts need, neighbouring CTAs share them and take half of the tokens each.
+// A lane's first LG_AHEAD vectors of its row are asked for before the rows are staged: one trip to memory for both (a trip per
+// vector, after the staging, was 5,600 of 11,400 cycles at one token of H 5120, and 15,000 of 25,000 went to seven tokens of H 6144).
+constexpr int LG_AHEAD = 6;
 __device__ __forceinline__ void logits_rows(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                                             uint32_t T, uint32_t E, uint32_t H, float* __restrict__ logits, uint8_t* sm,
                                             uint32_t cta, uint32_t n_cta) {
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, nwarps = blockDim.x >> 5;
     const uint32_t slots = nwarps / LG_PARTS, slot = warp / LG_PARTS, part = warp % LG_PARTS;
+    const bool shared_out = T > 1 && n_cta % 2 == 0 && (n_cta / 2) * slots >= E;
+    const uint32_t t_half = (T + 1) / 2, t_begin = shared_out && (cta & 1u) ? t_half : 0u, t_end = shared_out && !(cta & 1u) ? t_half : T;
+    if (shared_out) { cta /= 2; n_cta /= 2; }
     const uint32_t nv = H / 8;
     uint4* xs = reinterpret_cast<uint4*>(sm);                                  // [LG_TOK][nv] vectors of 8 bf16
     float* ps = reinterpret_cast<float*>(sm + (size_t)LG_TOK * H * 2);         // [nwarps][LG_TOK]
     const uint32_t v_begin = part * nv / LG_PARTS, v_end = (part + 1) * nv / LG_PARTS;
     const uint32_t e_step = n_cta * slots, rounds = (E + e_step - 1) / e_step;
-    for (uint32_t t0 = 0; t0 < T; t0 += LG_TOK) {
-        const uint32_t nt = T - t0 < (uint32_t)LG_TOK ? T - t0 : (uint32_t)LG_TOK;
+    uint4 wv[LG_AHEAD];
+    auto fetch = [&](uint32_t e, uint32_t v) {
+        const uint4* wrow = reinterpret_cast<const uint4*>(w + (size_t)e * H);
+#pragma unroll
+        for (int i = 0; i < LG_AHEAD; ++i)
+            if (v + 32 * i < v_end) wv[i] = wrow[v + 32 * i];
+    };
+    for (uint32_t t0 = t_begin; t0 < t_end; t0 += LG_TOK) {
+        const uint32_t nt = t_end - t0 < (uint32_t)LG_TOK ? t_end - t0 : (uint32_t)LG_TOK;
+        const uint32_t e0 = cta * slots + slot;
+        if (e0 < E) fetch(e0, v_begin + lane);
         __syncthreads();
         for (uint32_t v = threadIdx.x; v < nt * nv; v += blockDim.x) xs[v] = reinterpret_cast<const uint4*>(x + (size_t)t0 * H)[v];
         __syncthreads();
         for (uint32_t rd = 0; rd < rounds; ++rd) {
-            const uint32_t e = rd * e_step + cta * slots + slot;
-            const bool live = slot < slots && e < E;
+            const uint32_t e = rd * e_step + e0;
+            const bool live = e < E;
             float acc[LG_TOK];
 #pragma unroll
             for (int tt = 0; tt < LG_TOK; ++tt) acc[tt] = 0.f;
             if (live) {
-                const uint4* wrow = reinterpret_cast<const uint4*>(w + (size_t)e * H);
-                for (uint32_t v = v_begin + lane; v < v_end; v += 32) {
-                    const uint4 wv = wrow[v];
-                    const uint32_t ww[4] = {wv.x, wv.y, wv.z, wv.w};
+                for (uint32_t v0 = v_begin + lane; v0 < v_end; v0 += 32 * LG_AHEAD) {
+                    if (rd || v0 != v_begin + lane) fetch(e, v0);
+#pragma unroll 1
+                    for (uint32_t v = v0; v < v_end && v < v0 + 32 * LG_AHEAD; v += 32) {
+                        // the vectors move up by one: a short loop (unrolled over them, the code alone took longer to fetch)
+                        const uint32_t ww[4] = {wv[0].x, wv[0].y, wv[0].z, wv[0].w};
 #pragma unroll
-                    for (int tt = 0; tt < LG_TOK; ++tt) {
-                        if ((uint32_t)tt < nt) {
+                        for (int i = 0; i + 1 < LG_AHEAD; ++i) wv[i] = wv[i + 1];
+#pragma unroll
+                        for (int tt = 0; tt < LG_TOK; ++tt) {
+                            if ((uint32_t)tt >= nt) break;
                             const uint4 xv = xs[tt * nv + v];
                             const uint32_t xw[4] = {xv.x, xv.y, xv.z, xv.w};
 #pragma unroll

@@ -91,6 +91,7 @@ __device__ __forceinline__ void route_row_warp(const float* __restrict__ row, co
         }
     }
     float total = 0.0f, mine = 0.0f;
+#pragma unroll 1
     for (int r = 0; r < K; ++r) {
         // this lane's best live expert (a lower i is a lower index), then the warp's
         uint32_t bk = 0, bi = 0xFFFFFFFFu;

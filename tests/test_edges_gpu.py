@@ -294,3 +294,78 @@ def test_front_of_more_tokens_than_shared_memory_holds_scores_of(E, k, counts):
     r = subprocess.run([sys.executable, "-c", FRONT_SCRIPT, str(E), str(k), counts], cwd=Path(__file__).resolve().parent.parent,
                        env=dict(os.environ, MLXS_FRONT_MAX="256"), capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "ok" in r.stdout, r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("cls,E", [(Exl3Case, 256), (Exl3Case, 40), (Mxfp4Case, 256), (Nvfp4Case, 24)])
+def test_few_rows_are_sorted_as_many(cls, E):
+    """Up to 32 rows a thread per row finds its place, above that the scan does: the same permutation, and the rows of the
+    tokens that both calls hold are the same bits (experts with one row to several chunks of rows)."""
+    import torch
+    fp4 = cls is not Exl3Case
+    case = cls(512, 256, E, 8, seed=4, shared=False, scoring=O.SCORE_SIGMOID, max_tokens=64, routed_scale=1.0, chain=fp4)
+    try:
+        rng = np.random.default_rng(E)
+        for n in (1, 4, 8, 31, 32, 33):
+            slot = rng.integers(0, E, n).astype(np.int32)
+            d = torch.from_numpy(slot).cuda()
+            order = torch.full((n,), -1, dtype=torch.int32, device="cuda")
+            offs = torch.full((E + 1,), -1, dtype=torch.int32, device="cuda")
+            case.moe.sort_rows(d.data_ptr(), n, E, order.data_ptr(), offs.data_ptr(), None)
+            torch.cuda.synchronize()
+            assert (order.cpu().numpy() == np.argsort(slot, kind="stable")).all(), n
+            assert (offs.cpu().numpy() == np.concatenate([[0], np.cumsum(np.bincount(slot, minlength=E))])).all(), n
+        hot = min(E, 20)   # 17 tokens of 8 experts among 20: fewer than 13 rows each with these seeds, so all of them stream
+        ids = np.stack([np.random.default_rng(100 + t).permutation(hot)[:8] for t in range(17)]).astype(np.int32)
+        assert np.bincount(ids.ravel()).max() < 13
+        x, _ = case.inputs(17, seed=3)
+        w = np.full(ids.shape, 0.125, np.float32)
+        many = case.gpu_experts(x, ids, w)
+        for T in (1, 3, 4, 5):
+            assert (case.gpu_experts(x[:T], ids[:T], w[:T]) == many[:T]).all(), T
+        same = np.broadcast_to(ids[0], (4, 8)).copy()   # four tokens of the same experts
+        wide = np.concatenate([same, ids[4:9]])
+        assert (case.gpu_experts(x[:4], same, w[:4]) == case.gpu_experts(x[:9], wide, w[:9])[:4]).all()
+        assert rel_l2(many, case.cpu_layer(x, ids, w)) < 1e-2
+        assert case.status() == 0
+    finally:
+        case.close()
+
+
+@pytest.mark.parametrize("E,H", [(256, 1024), (256, 6144), (64, 7168), (9, 1664)])
+def test_layer_from_x_of_a_few_tokens(E, H):
+    """From x the front's CTAs share out experts, tokens and (beyond 6144 inputs) a row's vectors in more than one round: the
+    layer is the one that the logits alone give, 1 to 16 tokens."""
+    import torch
+    case = Exl3Case(H, 128, E, 4, seed=2, shared=False, scoring=O.SCORE_SIGMOID, max_tokens=32)
+    try:
+        wg = O.f32_to_bf16_bits((np.random.default_rng(5).standard_normal((E, H)) * H ** -0.5).astype(np.float32))
+        case.moe.set_router_weight(0, wg.ctypes.data)
+        for T in (1, 2, 7, 8, 9, 15, 16):
+            x, _ = case.inputs(T, seed=20 + T)
+            xd = case.to_dev_bf16(x)
+            lg = torch.empty((T, E), dtype=torch.float32, device=case.dev)
+            case.moe.logits(0, xd.data_ptr(), T, lg.data_ptr(), None)
+            y = torch.empty((T, H), dtype=torch.bfloat16, device=case.dev)
+            case.moe.forward_x(0, xd.data_ptr(), T, y.data_ptr(), None)
+            torch.cuda.synchronize()
+            assert (y.float().cpu().numpy() == case.gpu_forward(x, lg.cpu().numpy())).all(), T
+        assert case.status() == 0
+    finally:
+        case.close()
+
+
+@pytest.mark.parametrize("cls", [Exl3Case, Exl3K2Case])
+def test_records_of_four_byte_alignment_load_the_same_bank(cls):
+    """The repack reads a record in 16-byte vectors where its address allows, else in words."""
+    import torch
+    case = cls(384, 256, 2, 1, seed=9, shared=False, max_tokens=32, experts_to_load=[0])
+    try:
+        rec = torch.from_numpy(np.concatenate([np.zeros(4, np.uint8), case.records[0]])).cuda()
+        case.moe.load_expert(0, 1, rec.data_ptr() + 4, rec.numel() - 4, on_device=True)
+        x, _ = case.inputs(5, seed=1)
+        w = np.ones((5, 1), np.float32)
+        a, b = (case.gpu_experts(x, np.full((5, 1), e, np.int32), w) for e in (0, 1))
+        assert np.isfinite(a).all() and np.abs(a).max() > 0 and (a == b).all()
+        assert case.status() == 0
+    finally:
+        case.close()
