@@ -140,16 +140,24 @@ __device__ __forceinline__ uint32_t mul1_pair(uint32_t sa, uint32_t sb) {
 // Lanes 4u .. 4u + 3 hold the same columns of four k-tiles, which is one mma A fragment (or one tcgen05.st.16x256b fragment)
 // per c with inputs of all four k-tiles; whoever multiplies takes the rows in that order (position 16 c + 4 j + 2 h + b of
 // the 64 = input 16 j + 2 c + 8 h + b).
-// Measured with operands in shared memory, cycles per tile and scheduler, against eight states per lane and tile (two words, a
-// funnel shift by the lane): K = 3 51.7 -> 46.7, K = 2 51.7 -> 43.8; with one mma per tile 58.5 -> 55.3 and 57.4 -> 52.5.
-// The quad in memory: 32 K words, [lane][first two words], then the lanes' third words (K = 3).
+// Against eight states per lane and tile (two words, a funnel shift by the lane) 64 tokens take 1941 -> 1852 us, 16 of K = 2
+// 955 -> 887.  In the bare loop with one mma per tile 58.5 -> 55.3 cycles per tile and scheduler (K = 2 57.4 -> 52.5), 46.7 and 43.8
+// of them the decode: an mma.sync costs 8.7 whatever its shape.
+// The quad in memory: word w of the four k-tiles beside each other, [8 K words][4 k-tiles]: four 4-byte loads here, two 16-byte
+// loads for four tiles in the tensor-core lane.  (A lane's first two words as one 8-byte load: 1834 and 870 us, but the
+// tensor-core lane would need eight loads again.)
+// The tensor-core lane multiplies 16 inputs of one k-tile at a time instead (exl3_decode_lane): with the quad's order the grouping of
+// its sums over the inputs changes, and the f16 and bf16 roundings behind them turn that into 2e-4 of a layer's rows and, layer by
+// layer, into as much as 1e-2 after four (the streaming kernel's order alone: 5e-6 to 5e-5, 6e-3).
 template <int KB>
 __device__ __forceinline__ void exl3_quad_words(const uint32_t* __restrict__ quad, uint32_t lane, uint32_t (&z)[4]) {
     // z: the stream's words from its last on, z[KB] = the word before the lane's first (its neighbour's last)
-    const uint2 w = reinterpret_cast<const uint2*>(quad)[lane];
-    z[KB - 1] = w.x; z[KB - 2] = w.y;
-    if (KB == 3) { z[0] = quad[64 + lane]; z[3] = quad[64 + ((lane - 4u) & 31u)]; }
-    else { z[2] = quad[2u * ((lane - 4u) & 31u) + 1u]; z[3] = 0u; }
+    const uint32_t u = lane >> 2, j = lane & 3u;
+    const uint32_t* w = quad + (KB * 4u) * u + j;
+#pragma unroll
+    for (int i = 0; i < KB; ++i) z[i] = w[4 * (KB - 1 - i)];
+    z[KB] = quad[(u ? KB * 4u * u : KB * 32u) - 4u + j];
+    if (KB == 2) z[3] = 0u;
 }
 // 32 stream bits from bit O on (counted from the last)
 template <int O>
@@ -190,6 +198,68 @@ __device__ __forceinline__ void exl3_decode_quad(const uint32_t (&z)[4], uint32_
     exl3_decode8<KB, 1>(z, b); put(1);
     exl3_decode8<KB, 2>(z, b); put(2);
     exl3_decode8<KB, 3>(z, b); put(3);
+}
+
+// ---- one lane's share of one tile (the tensor-core lane) ----
+// A 16x16 K=3 tile: lane L owns code positions 8L..8L+7, i.e. the 37 stream bits ending at
+// stream bit 24(L+1); `lo` is the tile word holding that last bit, `hi` the word before it (circular), lp the
+// distance of the last bit from the word's bit 0.  Returns the two B fragments (k16 x n8) of the tile's column
+// halves for mma m16n8k16: b[0], b[1] = columns 0..7, b[2], b[3] = columns 8..15 (the exllamav3 tensor-core order,
+// src/exl3/kernels.zig:978-986).
+__device__ __forceinline__ void exl3_decode_lane(uint32_t lo, uint32_t hi, uint32_t lp, uint32_t (&b)[4]) {
+    uint32_t v0 = __funnelshift_r(lo, hi, lp);  // stream bits, window m at bits [3m, 3m+16)
+    uint32_t vh = hi >> lp;
+    uint32_t v1 = __funnelshift_r(v0, vh, 18);  // windows 6, 7 at bits 0 and 3
+    uint32_t w0 = v0 & 0xFFFFu;
+    uint32_t w1 = (v0 >> 3) & 0xFFFFu;
+    uint32_t w2 = (v0 >> 6) & 0xFFFFu;
+    uint32_t w3 = (v0 >> 9) & 0xFFFFu;
+    uint32_t w4 = (v0 >> 12) & 0xFFFFu;
+    uint32_t w5 = (v0 >> 15) & 0xFFFFu;
+    uint32_t w6 = v1 & 0xFFFFu;
+    uint32_t w7 = (v1 >> 3) & 0xFFFFu;
+    // code position j = 7 - m; positions (0,1),(2,3) -> columns 0..7 rows (r0,r0+1),(r0+8,r0+9); (4,5),(6,7) -> 8..15
+    b[0] = mul1_pair(w7, w6);
+    b[1] = mul1_pair(w5, w4);
+    b[2] = mul1_pair(w3, w2);
+    b[3] = mul1_pair(w1, w0);
+}
+__device__ __forceinline__ void exl3_lane_plan(uint32_t lane, uint32_t& wi, uint32_t& wj, uint32_t& lp) {
+    wi = (3u * lane + 2u) >> 2;        // word of the lane's last stream bit
+    wj = (wi + 23u) % 24u;             // the word before it, circular
+    lp = 8u * ((lane + 1u) & 3u);
+}
+// The same for K = 2 (a tile is 16 words): lane L's 8 states end at stream bits 16 L + 2 .. 16 L + 16, i.e. they live in
+// the 30 bits ending with halfword L.  `lo` = the word holding halfword L, `hi` = the word before it (circular),
+// lp = 0 when halfword L is the word's low half, 16 when it is the high half; window m at bits [2m, 2m + 16).
+// Bit-level definition: src/exl3/kernels.zig:988-1020 (tileStates at K = 2), generic window formulas
+// scripts/dsv41_exl3_k2_gen.py:96-112.
+__device__ __forceinline__ void exl3_decode_lane_k2(uint32_t lo, uint32_t hi, uint32_t lp, uint32_t (&b)[4]) {
+    const uint32_t v0 = __funnelshift_r(lo, hi, lp);
+    // states four apart are a byte apart: one shift serves both
+    const uint32_t v2 = v0 >> 2, v4 = v0 >> 4, v6 = v0 >> 6;
+    const uint32_t w0 = v0 & 0xFFFFu, w1 = v2 & 0xFFFFu, w2 = v4 & 0xFFFFu, w3 = v6 & 0xFFFFu;
+    const uint32_t w4 = __byte_perm(v0, 0u, 0x4421), w5 = __byte_perm(v2, 0u, 0x4421), w6 = __byte_perm(v4, 0u, 0x4421), w7 = __byte_perm(v6, 0u, 0x4421);
+    b[0] = mul1_pair(w7, w6);
+    b[1] = mul1_pair(w5, w4);
+    b[2] = mul1_pair(w3, w2);
+    b[3] = mul1_pair(w1, w0);
+}
+__device__ __forceinline__ void exl3_lane_plan_k2(uint32_t lane, uint32_t& wi, uint32_t& wj, uint32_t& lp) {
+    wi = lane >> 1;
+    wj = (wi + 15u) % 16u;
+    lp = (lane & 1u) ? 0u : 16u;
+}
+// by code width
+template <int KB>
+__device__ __forceinline__ void exl3_decode_lane_kb(uint32_t lo, uint32_t hi, uint32_t lp, uint32_t (&b)[4]) {
+    if (KB == 3) exl3_decode_lane(lo, hi, lp, b);
+    else exl3_decode_lane_k2(lo, hi, lp, b);
+}
+template <int KB>
+__device__ __forceinline__ void exl3_lane_plan_kb(uint32_t lane, uint32_t& wi, uint32_t& wj, uint32_t& lp) {
+    if (KB == 3) exl3_lane_plan(lane, wi, wj, lp);
+    else exl3_lane_plan_k2(lane, wi, wj, lp);
 }
 
 // ---- 128-point Sylvester-natural Hadamard over a warp: lane holds elements 4*lane .. 4*lane+3 ----

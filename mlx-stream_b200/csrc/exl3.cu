@@ -53,8 +53,8 @@ __global__ void __launch_bounds__(256) exl3_repack_kernel(const uint8_t* __restr
         __syncthreads();
         uint32_t* dst = (down ? dn + (size_t)(i - 2 * n_unit) * UNIT : gu + (size_t)i * UNIT);
         for (uint32_t w = threadIdx.x; w < UNIT; w += blockDim.x) {
-            const uint32_t t = w / QUAD, in = w % QUAD, l = in < 64 ? in / 2 : in - 64, wd = in < 64 ? in % 2 : 2;   // exl3_quad_words
-            dst[w] = tiles[((l & 3u) * 8 + t) * TW + KB * (l >> 2) + wd];
+            const uint32_t t = w / QUAD, in = w % QUAD;   // word in / 4 of k-tile in % 4
+            dst[w] = tiles[((in & 3u) * 8 + t) * TW + (in >> 2)];
         }
         __syncthreads();
     }

@@ -3,10 +3,11 @@
 // The reference's prefill lane (src/exl3/quant.zig:1040-1271; texts dsv41_prefill_dig_gemm_*_m128*.metal) decodes
 // trellis tiles to f16 in threadgroup memory per K stage and feeds its MMA units with f16 rotated activations and an
 // f32 accumulator.  Here the pipeline is lane.cuh's; this file supplies
-//   * the decode: a lane that has decoded its share of a quad (common.cuh: 32 states, the 16 inputs of columns u and u + 8 of
-//     one of four k-tiles) holds four tcgen05.st.16x256b fragments (thread (u, j): lanes u and u + 8, two adjacent 32-bit
-//     columns) once the K order inside 64 inputs is taken as 16 c + 4 j + 2 h + b for input 16 j + 2 c + 8 h + b; the rows are
-//     staged in the same order.  The stores go out a quad at a time (16x256b.x4);
+//   * the decode: a lane (g, c) that has decoded a 16x16 tile holds W[k 2c,2c+1 | 2c+8,2c+9][column g | g+8]: that is one
+//     tcgen05.st.16x256b fragment (thread (g, c): lanes g and g + 8, two adjacent 32-bit columns) once the K order inside a
+//     16-block is taken as k' = 4c + 2 (k / 8) + k % 2, c = (k % 8) / 2; the rows are staged in the same order.  Four k-tiles of a
+//     column tile lie word by word beside each other (common.cuh): two 16-byte loads serve four tiles, and their stores go out
+//     together (16x256b.x4);
 //   * the row staging: H128(x suh) 128^-0.5, f16, once per projection;
 //   * the epilogue: transpose through shared memory, then row-wise Hadamard-128, svh, clamped SwiGLU, suh_d, Hadamard for
 //     gate / up (act(gate) waits in an L2-resident scratch between the two passes, read back by the threads that wrote it);
@@ -105,11 +106,12 @@ __device__ __forceinline__ void pf_hadamard(float (&v)[R][4], const float (&sg)[
 // ------------------------------------------------------------------------------------------------------------
 // prep: rows -> rotated f16 activations in the MMA's B-operand order
 // ------------------------------------------------------------------------------------------------------------
-// Positions inside 64 inputs: the order of a decoded quad (common.cuh).  A lane (t = lane / 4, c = lane % 4) that holds the
-// inputs 16 t + {2c, 2c + 1, 2c + 8, 2c + 9} of a 128-block has the four consecutive positions 64 (t / 4) + 16 c + 4 (t % 4):
-// one 8-byte store at this element offset inside the stage.
+// The position of input k inside its 16-block is 4 ((k % 8) / 2) + 2 ((k % 16) / 8) + k % 2, the order in which the decode's
+// registers fill a tensor-memory fragment.  A lane (t = lane / 4, c = lane % 4) that holds the inputs 16 t + {2c, 2c + 1,
+// 2c + 8, 2c + 9} of a 128-block has the four consecutive positions 16 t + 4 c: one 8-byte store at this element offset
+// inside the stage.
 __device__ __forceinline__ uint32_t pf_lane_off(uint32_t row, uint32_t lane) {
-    return ln_row_off(row, (lane >> 4) * 8u + (lane & 3u) * 2u + ((lane >> 3) & 1u)) + ((lane >> 2) & 1u) * 4u;
+    return ln_row_off(row, (lane >> 2) * 2u + ((lane >> 1) & 1u)) + (lane & 1u) * 4u;
 }
 __device__ __forceinline__ uint32_t pf_lane_col(uint32_t lane) { return (lane >> 2) * 16u + (lane & 3u) * 2u; }   // and + 1, + 8, + 9
 __device__ __forceinline__ uint2 pf_pack4(float v0, float v1, float v2, float v3) {
@@ -127,9 +129,8 @@ __device__ __forceinline__ void pf_load_scale4(const __half* p, uint32_t lane, f
 // registers.  For a level of s the two lanes swap half their registers: each then has both sides of 16 butterflies, and the
 // lane bit has become a bit of i, whose level is done.  The kernel is bound by the L1's data path, which the shuffles share:
 // 32 of them per row group and projection (one per input and level, with a last exchange before the stores, was 72).
-// After both levels a lane holds the inputs {2 c, 2 c + 1, 2 c + 8, 2 c + 9} of every 16-block, c = lane % 4 with its two bits
-// swapped: four consecutive positions, those of two neighbouring 16-blocks next to each other (one 16-byte store); the stores
-// of a warp fill whole lines.
+// After both levels a lane holds exactly the four consecutive positions of pf_lane_off in every 16-block: with c = lane % 4,
+// {2 c', 2 c' + 1, 2 c' + 8, 2 c' + 9}, c' = c with its two bits swapped; the 8-byte stores of a warp fill whole lines.
 // Two CTAs per SM: with three (80 registers) 60 bytes a thread spilled into the data path that bounds the kernel (300 tokens of
 // 64 experts 28.0 -> 26.1 us, 2048 tokens 124 -> 121, 8192 447 -> 451, under ncu).
 constexpr int PREP_WARPS = 8;
@@ -199,13 +200,12 @@ __global__ void __launch_bounds__(PREP_WARPS * 32, 2) pf_prep_kernel(const __nv_
             for (int k = 0; k < 32; ++k) v[k] *= (k & 6) == 6 ? S01 : (k & 4) ? S0 : (k & 2) ? S1 : S;
             // src/kernels/exl3/dsv41_prefill_dig_take2v_5120.metal:57-58: the rotated input is rounded to f16
             const uint32_t c = (seg & 1u) * 2u + (seg >> 1);
-            __half* dst = xa + p * proj_stride + (size_t)te[3] * H + (size_t)b * (rows16 * LN_KST) + ln_row_off(r, c * 2u);
-            // registers 8 j + 4 (bit 3 of the input) + 2 (bit 4) + bit 0; 16-blocks 2 s and 2 s + 1
+            __half* dst = xa + p * proj_stride + (size_t)te[3] * H + (size_t)b * (rows16 * LN_KST) + ln_row_off(r, c >> 1) + (c & 1u) * 4u;
+            // registers 8 j + 4 (bit 3 of the input) + 2 (bit 4) + bit 0
 #pragma unroll
-            for (int s = 0; s < 4; ++s) {
-                const int k = 8 * s;
-                const uint2 lo = pf_pack4(v[k], v[k + 1], v[k + 4], v[k + 5]), hi = pf_pack4(v[k + 2], v[k + 3], v[k + 6], v[k + 7]);
-                *reinterpret_cast<uint4*>(dst + (s >> 1) * 512 + (s & 1) * 64) = make_uint4(lo.x, lo.y, hi.x, hi.y);
+            for (int t16 = 0; t16 < 8; ++t16) {
+                const int k = (t16 >> 1) * 8 + (t16 & 1) * 2;
+                *reinterpret_cast<uint2*>(dst + t16 * 128) = pf_pack4(v[k], v[k + 1], v[k + 4], v[k + 5]);
             }
         }
     }
@@ -233,15 +233,23 @@ struct Exl3LaneBank {
     }
 
     struct Decoder {
-        uint32_t lane, off;
-        __device__ __forceinline__ Decoder(uint32_t q, uint32_t half, uint32_t lane_) : lane(lane_) {
+        uint32_t wi, wj, lp, off;
+        __device__ __forceinline__ Decoder(uint32_t q, uint32_t half, uint32_t lane) {
+            exl3_lane_plan_kb<KB>(lane, wi, wj, lp);
             off = half * (LN_KST / 32) * KT_WORDS + 2 * q * (4 * TW);   // lanes 32 q .. hold the 16-column tiles 2 q, 2 q + 1
         }
         // piece pc of the stage (or of the constructor's half): a quad of one of the two tiles
         __device__ __forceinline__ void decode(const uint8_t* raw, uint32_t slot_bytes, uint32_t pc, uint32_t (&v)[16]) const {
-            uint32_t z[4];
-            exl3_quad_words<KB>(reinterpret_cast<const uint32_t*>(raw + slot_bytes) + off + (pc >> 1) * ((LN_KST / 32) * KT_WORDS) + (pc & 1u) * (4 * TW), lane, z);
-            exl3_decode_quad<KB>(z, v);
+            const uint4* w = reinterpret_cast<const uint4*>(reinterpret_cast<const uint32_t*>(raw + slot_bytes) + off + (pc >> 1) * ((LN_KST / 32) * KT_WORDS) + (pc & 1u) * (4 * TW));
+            const uint4 lo = w[wi], hi = w[wj];
+            const uint32_t l4[4] = {lo.x, lo.y, lo.z, lo.w}, h4[4] = {hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+            for (int kt = 0; kt < 4; ++kt) {
+                uint32_t bq[4];
+                exl3_decode_lane_kb<KB>(l4[kt], h4[kt], lp, bq);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) v[4 * kt + k] = bq[k];
+            }
         }
         static __device__ __forceinline__ void store(uint32_t ta, uint32_t pc, const uint32_t (&v)[16]) {
             asm volatile("tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(ta + (pc >> 1) * (LN_A_COLS / 2) + ((pc & 1u) << 20)),

@@ -22,7 +22,7 @@
 //     operand slot and the rows' slot.  What its operands come from goes through a shuffle from lane 0, so that the compiler
 //     knows that the warp has one value: they stay in uniform registers instead of being moved there for every MMA (cycles
 //     from a stage's operands to its eight MMAs issued, 64 / 128 / 256 rows: EXL3 659 / 749 / 778 -> 578 / 728 / 703, NVFP4 at
-//     128 554 -> 499; the layer at 2048 EXL3 tokens 2911 -> 2842 us, 8192 7480 -> 7258, NVFP4 at 4093 3033 -> 2974).
+//     128 554 -> 499; the layer at 2048 EXL3 tokens 2.4 %, 8192 3.0 %, NVFP4 at 4093 3033 -> 2974 us).
 //     The FP4 banks, whose decode is short, test the next stage's barrier in the middle of a stage's MMAs and decode and store a
 //     quarter of a stage at a time (the first waits for the slot): NVFP4 at 4093 tokens 2979 -> 2949 us, MXFP4 at 16384 6280 -> 6150.
 //     What is left there is the copy of rows and codes from L2, 55 to 62 bytes per clock and SM (41 and 53 KB per stage of 760
