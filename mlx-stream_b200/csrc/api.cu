@@ -806,7 +806,7 @@ static int experts_impl(mlxs_moe* h, uint32_t layer, const void* x_dev, const in
         fa.heavy = (h->pf_tiles && T >= h->pf_min_rows) ? h->pf_min_rows : 0u;   // the lane choice of mlxs_run_routed
         fa.x = static_cast<const __nv_bfloat16*>(x_dev); fa.H = c.hidden; fa.bank_exl3 = is_exl3(c.bank_kind) ? 1 : 0;
         fa.scales = L.scales; fa.scales_stride = is_exl3(c.bank_kind) ? exl3_scales_per_expert(Exl3Dims{c.hidden, c.inter, L.kbits}) : 0;
-        fa.xa = h->xa_gu; fa.bar = h->front_bar; fa.smem_max = h->front_smem_max;
+        fa.xa = h->xa_gu; fa.bar = h->front_bar; fa.beside = shared_aside; fa.smem_max = h->front_smem_max;
         StageTimer tm(h, MLXS_STAGE_ROUTER, st);
         const cudaError_t fe = launch_front(fa, st);
         h->stats.route_calls += 1;

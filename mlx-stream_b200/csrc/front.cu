@@ -231,13 +231,23 @@ cudaError_t launch_front(const FrontArgs& a, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     const bool barrier = a.w_router || !P.by_warp;
     // a warp per staging task (a row's 128-block; for the FP4 banks a sixteenth of a row, or a quarter where that would be more
-    // warps than the SMs hold), at most a CTA per SM; with a
-    // barrier 32 to 64 CTAs: one round of expert rows, and room beside the shared expert's kernels
+    // warps than the SMs hold), at most a CTA per SM.  From x, two tokens and more beside the shared expert's kernels, an FP4
+    // row always goes by quarters.  The front then ends 2 us later, which is better: gate/up's units belong to its CTAs by
+    // number, so while the shared expert's first kernel (35 us, from the front's start on) holds SMs some of them wait, and
+    // gate/up takes 60 us from the front's end instead of 53.  NVFP4, H 6144, two tokens, sixteenths -> quarters: of 32 and 128
+    // experts 113.9 -> 106.7 and 116.2 -> 108.4 us; handles on whose streams the shared expert's kernel runs before the front
+    // or behind gate/up 120.1 -> 121.5 (256 experts).  One token: nothing lost by sixteenths (85.1, 96.9 with 100.8 by quarters).
     const unsigned sms = (unsigned)(a.sm_count > 0 ? a.sm_count : 32);
     const unsigned rows = (unsigned)(a.T * a.K) * a.chunk_rows;
-    P.parts = rows * 16u <= 32u * sms ? 16u : 4u;
+    P.parts = rows * 16u <= 32u * sms && !(a.w_router && a.beside && a.T > 1) ? 16u : 4u;
     unsigned grid = (rows * (a.bank_exl3 ? a.H / 128 : P.parts) + 31u) / 32u;
-    if (barrier) grid = grid < 32u ? 32u : grid > 64u || (a.w_router && a.T > 1) ? 64u : grid;   // 64: two CTAs per set of expert rows
+    // with a barrier 32 to 64 CTAs: one round of expert rows, and room beside the shared expert's kernels; from x two CTAs per set
+    // of eight expert rows where that is within the bounds, so that they share out the tokens (logits_body.cuh)
+    if (barrier) {
+        const unsigned want = a.w_router && a.T > 1 ? 2u * ((unsigned)(a.E + 7) / 8u) : 0u;
+        grid = ((grid > want ? grid : want) + 1u) / 2u * 2u;
+        grid = grid < 32u ? 32u : grid > 64u ? 64u : grid;
+    }
     if (grid > sms) grid = sms;
     if (!barrier) {
         return launch_dependent(true, front_kernel, grid, 1024, smem, st, P);

@@ -61,6 +61,7 @@ struct FrontArgs {
     uint32_t* xa;
     uint32_t* bar;
     int sm_count;
+    bool beside;                    // the shared expert's kernels run beside it
     size_t smem_max;                // dynamic shared memory that a block may ask for
 };
 bool front_fits(int E, int K, uint32_t T, uint32_t H, bool from_x, size_t smem_max);   // does a call's front fit that?
