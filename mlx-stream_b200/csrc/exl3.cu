@@ -24,20 +24,21 @@ constexpr int ZS_STRIDE = 132;    // padded row stride of the epilogue's f32 sta
 // ------------------------------------------------------------------------------------------------------------
 // load-time repack: reference record -> kernel layout (bit-preserving: words move, no bit changes)
 // ------------------------------------------------------------------------------------------------------------
-// A block moves one quad column at a time: the four k-tiles x eight tiles of a 128-wide output block (eight tiles of a k-tile are
-// contiguous in the record), through shared memory into quad order (common.cuh).
-// V = uint4 (the record is 16-byte aligned: eight tiles of a k-tile are 48 or 32 vectors) or uint32_t
-template <class V, int KB>
-__global__ void __launch_bounds__(256) exl3_repack_kernel(const uint8_t* __restrict__ rec, uint32_t H, uint32_t I,
-                                   uint32_t* __restrict__ gu, uint32_t* __restrict__ dn, __half* __restrict__ sc) {
-    constexpr uint32_t TW = 8 * KB, QUAD = 4 * TW, UNIT = 8 * QUAD;   // words of a tile, of a quad, of the eight quads of a block
-    __shared__ __align__(16) uint32_t tiles[UNIT];
+// A thread moves one word of a tile of four k-tiles, four loads and one 16-byte store; a block the eight tiles of a 128-wide output
+// block for four k-tiles.  The eight tiles of a k-tile are contiguous in the record and so are the quads in the layout
+// (common.cuh): both sides are coalesced, whatever the record's alignment beyond its words.  load_expert of a device record of
+// H 5120, I 2304: 22.2 us at K = 3 and 20.0 at K = 2, most of it the call's own copies and waits; through shared memory, with
+// 16-byte loads where the record allows them, 25 to 29 and 24 to 27.
+template <int KB>
+__global__ void __launch_bounds__(64 * KB) exl3_repack_kernel(const uint8_t* __restrict__ rec, uint32_t H, uint32_t I,
+                                                              uint4* __restrict__ gu, uint4* __restrict__ dn, __half* __restrict__ sc) {
+    constexpr uint32_t TW = 8 * KB, UNIT = 8 * TW;   // words of a tile, of a k-tile of a block (= vectors of the block's eight quads)
     const size_t code_bytes = (size_t)(H / 16) * (I / 16) * TW * 4;
     // record offsets (src/expert/bank.zig:116-141): per projection code, rout [out], rin [in]
     const size_t off_g = 0, off_g_rout = code_bytes, off_g_rin = off_g_rout + 2 * (size_t)I;
     const size_t off_u = off_g_rin + 2 * (size_t)H, off_u_rout = off_u + code_bytes, off_u_rin = off_u_rout + 2 * (size_t)I;
     const size_t off_d = off_u_rin + 2 * (size_t)H, off_d_rout = off_d + code_bytes, off_d_rin = off_d_rout + 2 * (size_t)H;
-    const uint32_t n_unit = (uint32_t)(code_bytes / 4 / UNIT);        // of one projection
+    const uint32_t n_unit = (uint32_t)(code_bytes / 16 / UNIT);       // of one projection
     for (uint32_t i = blockIdx.x; i < 3 * n_unit; i += gridDim.x) {
         // destination: gate / up [block][projection][quad][tile][words], down [block][quad][tile][words]
         const bool down = i >= 2 * n_unit;
@@ -46,17 +47,10 @@ __global__ void __launch_bounds__(256) exl3_repack_kernel(const uint8_t* __restr
         const uint32_t q = r % nq; r /= nq;
         uint32_t p = 2;
         if (!down) { p = r % 2; r /= 2; }
-        const uint32_t* src = reinterpret_cast<const uint32_t*>(rec + (p == 0 ? off_g : p == 1 ? off_u : off_d)) + ((size_t)q * 4 * n_out + r * 8) * TW;
-        constexpr uint32_t PER = 8 * TW * 4 / sizeof(V);              // vectors of one k-tile
-        for (uint32_t v = threadIdx.x; v < 4 * PER; v += blockDim.x)
-            reinterpret_cast<V*>(tiles)[v] = reinterpret_cast<const V*>(src + (size_t)(v / PER) * n_out * TW)[v % PER];
-        __syncthreads();
-        uint32_t* dst = (down ? dn + (size_t)(i - 2 * n_unit) * UNIT : gu + (size_t)i * UNIT);
-        for (uint32_t w = threadIdx.x; w < UNIT; w += blockDim.x) {
-            const uint32_t t = w / QUAD, in = w % QUAD;   // word in / 4 of k-tile in % 4
-            dst[w] = tiles[((in & 3u) * 8 + t) * TW + (in >> 2)];
-        }
-        __syncthreads();
+        const uint32_t* src = reinterpret_cast<const uint32_t*>(rec + (p == 0 ? off_g : p == 1 ? off_u : off_d)) + ((size_t)q * 4 * n_out + r * 8) * TW + threadIdx.x;
+        const size_t kt = (size_t)n_out * TW;
+        uint4* dst = down ? dn + (size_t)(i - 2 * n_unit) * UNIT : gu + (size_t)i * UNIT;
+        dst[threadIdx.x] = make_uint4(src[0], src[kt], src[2 * kt], src[3 * kt]);
     }
     const uint32_t n_sc = 3 * H + 3 * I;
     for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < n_sc; s += gridDim.x * blockDim.x) {
@@ -75,14 +69,11 @@ __global__ void __launch_bounds__(256) exl3_repack_kernel(const uint8_t* __restr
 
 cudaError_t launch_exl3_repack(const uint8_t* record_dev, Exl3Dims d, uint32_t* gu_code_e, uint32_t* d_code_e,
                                __half* scales_e, cudaStream_t st) {
-    const bool wide = reinterpret_cast<uintptr_t>(record_dev) % 16 == 0;
-    if (d.K == 3) {
-        if (wide) exl3_repack_kernel<uint4, 3><<<1184, 256, 0, st>>>(record_dev, d.H, d.I, gu_code_e, d_code_e, scales_e);
-        else exl3_repack_kernel<uint32_t, 3><<<1184, 256, 0, st>>>(record_dev, d.H, d.I, gu_code_e, d_code_e, scales_e);
-    } else {
-        if (wide) exl3_repack_kernel<uint4, 2><<<1184, 256, 0, st>>>(record_dev, d.H, d.I, gu_code_e, d_code_e, scales_e);
-        else exl3_repack_kernel<uint32_t, 2><<<1184, 256, 0, st>>>(record_dev, d.H, d.I, gu_code_e, d_code_e, scales_e);
-    }
+    uint4 *gu = reinterpret_cast<uint4*>(gu_code_e), *dn = reinterpret_cast<uint4*>(d_code_e);   // an expert's code is a multiple of 2 KB
+    const size_t units = 3 * exl3_code_words(d) / (32 * exl3_tile_words(d));
+    const unsigned grid = (unsigned)(units < 1480 ? units : 1480);   // ten blocks per SM; 740, 2960 and one per unit measured the same
+    if (d.K == 3) exl3_repack_kernel<3><<<grid, 192, 0, st>>>(record_dev, d.H, d.I, gu, dn, scales_e);
+    else exl3_repack_kernel<2><<<grid, 128, 0, st>>>(record_dev, d.H, d.I, gu, dn, scales_e);
     return cudaGetLastError();
 }
 

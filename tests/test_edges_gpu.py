@@ -356,7 +356,7 @@ def test_layer_from_x_of_a_few_tokens(E, H):
 
 @pytest.mark.parametrize("cls", [Exl3Case, Exl3K2Case])
 def test_records_of_four_byte_alignment_load_the_same_bank(cls):
-    """The repack reads a record in 16-byte vectors where its address allows, else in words."""
+    """The repack reads a record in words, at any address that they allow."""
     import torch
     case = cls(384, 256, 2, 1, seed=9, shared=False, max_tokens=32, experts_to_load=[0])
     try:
