@@ -109,7 +109,7 @@ int mlxs_moe_layer_record_bytes(const mlxs_moe *h, uint32_t layer, uint32_t *bit
 
 /* Replaces the expert source's fill of a slot row (src/sdk_ext/expert.zig:226-264; csrc/q3_lookahead4_exl3.c): one
  * expert's record, in the reference's layout, becomes HBM resident.  `record` is a host pointer (on_device = 0) or a
- * device pointer (1); nbytes >= logical bytes.  Experts outside this rank's shard are accepted and ignored. */
+ * device pointer (1, 4-byte aligned, refused by name otherwise); nbytes >= logical bytes.  Experts outside this rank's shard are accepted and ignored. */
 int mlxs_moe_load_expert(mlxs_moe *h, uint32_t layer, uint32_t expert, const void *record, uint64_t nbytes,
                          int on_device);
 /* Bank.open + stream fill (src/expert/bank.zig:208-324, src/arch/mimo_v2/bank.zig:172-260,

@@ -282,6 +282,8 @@ extern "C" int mlxs_moe_load_expert(mlxs_moe* h, uint32_t layer, uint32_t expert
     if (nbytes < L.logical_bytes)
         return fail(MLXS_E_BANK, "load_expert: record has %llu bytes, the layer's record is %llu (RecordGeometry)",
                     (unsigned long long)nbytes, (unsigned long long)L.logical_bytes);
+    if (on_device && (reinterpret_cast<uintptr_t>(record) & 3u))   // the repack kernels read words
+        return fail(MLXS_E_ARG, "load_expert: a device record must be 4-byte aligned");
     if (L.place_rank[expert] != h->cfg.ep_rank) return MLXS_OK;  // another rank's shard
     CU(cudaSetDevice(h->cfg.device));
     const uint32_t le = L.place_slot[expert];

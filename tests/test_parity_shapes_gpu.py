@@ -342,6 +342,11 @@ def test_misaligned_buffers_are_refused_by_name():
         with pytest.raises(case.pkg.MlxsError) as ei:
             case.moe.forward(0, x.data_ptr(), lg.data_ptr(), 4, y.data_ptr() + 4, None)
         assert "y_dev" in ei.value.msg
+        rec = torch.zeros(case.records[0].size + 4, dtype=torch.uint8, device=case.dev)
+        for off in (1, 2, 3):   # refused before anything is copied or launched
+            with pytest.raises(case.pkg.MlxsError) as ei:
+                case.moe.load_expert(0, 1, rec.data_ptr() + off, case.records[0].size, on_device=True)
+            assert ei.value.rc == case.pkg.E_ARG and "aligned" in ei.value.msg
         case.moe.forward(0, x.data_ptr() + 16, lg.data_ptr() + 4, 4, y.data_ptr() + 16, None)
         torch.cuda.synchronize()
         assert case.status() == 0
