@@ -207,8 +207,8 @@ __device__ __forceinline__ void dispatch_few(const int32_t* __restrict__ ids, ui
 
 // The whole sort by one CTA of DTHREADS threads (A <= 2048 rows in practice); dsm: dispatch_words(A, E) words of shared memory
 __host__ __device__ inline size_t dispatch_words(uint32_t A, uint32_t E) {
-    const size_t scan = (size_t)E + 99 + place_words(place_warps(A), E), few = 2 * DISPATCH_FEW + 3;
-    return scan > few ? scan : few;
+    static_assert(2 * DISPATCH_FEW + 3 <= 99, "the short sort's ids and keys fit where the scan's scratch is");
+    return (size_t)E + 99 + place_words(place_warps(A), E);
 }
 __device__ __forceinline__ void dispatch_body(const int32_t* __restrict__ ids, uint32_t A, uint32_t E,
                                               const uint8_t* __restrict__ loaded, DispatchTables t, uint32_t CHUNK_ROWS,

@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(1024) ep_dedup_kernel(const uint32_t* __restri
 }
 // The plan of one exchange for decode-sized calls in one launch: destination rank and local slot of every assignment,
 // the stable sort by rank (the dispatch kernel's code), the first assignment of every (token, rank) pair.  One CTA; the
-// three steps read what the one before wrote to global memory after a CTA barrier.  dsm: W + 99 words.
+// three steps read what the one before wrote to global memory after a CTA barrier.  dsm: dispatch_words(A, W) words.
 __global__ void __launch_bounds__(DTHREADS) ep_plan_kernel(const int32_t* __restrict__ ids, uint32_t A, uint32_t E,
                                                            const uint32_t* __restrict__ place, int32_t* __restrict__ dest,
                                                            int32_t* __restrict__ meta, DispatchTables rtab, uint32_t W, uint32_t k,

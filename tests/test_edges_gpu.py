@@ -299,7 +299,7 @@ def test_front_of_more_tokens_than_shared_memory_holds_scores_of(E, k, counts):
 @pytest.mark.parametrize("cls,E", [(Exl3Case, 256), (Exl3Case, 40), (Mxfp4Case, 256), (Nvfp4Case, 24)])
 def test_few_rows_are_sorted_as_many(cls, E):
     """Up to 32 rows a thread per row finds its place, above that the scan does: the same permutation, and the rows of the
-    tokens that both calls hold are the same bits (experts with one row to several chunks of rows)."""
+    tokens that both calls hold are the same bits (a chunk of rows per expert; more in the next test)."""
     import torch
     fp4 = cls is not Exl3Case
     case = cls(512, 256, E, 8, seed=4, shared=False, scoring=O.SCORE_SIGMOID, max_tokens=64, routed_scale=1.0, chain=fp4)
@@ -331,16 +331,82 @@ def test_few_rows_are_sorted_as_many(cls, E):
         case.close()
 
 
-@pytest.mark.parametrize("E,H", [(256, 1024), (256, 6144), (64, 7168), (9, 1664)])
-def test_layer_from_x_of_a_few_tokens(E, H):
-    """From x the front's CTAs share out experts, tokens and (beyond 6144 inputs) a row's vectors in more than one round: the
-    layer is the one that the logits alone give, 1 to 16 tokens."""
+@pytest.mark.parametrize("cls,counts", [(Exl3Case, (12, 9, 5, 4, 1, 1)), (Exl3Case, (8, 12, 12)), (Exl3K2Case, (4, 11, 8, 9)), (Mxfp4Case, (16, 9, 5, 1, 1)),
+                                        (Mxfp4Case, (8, 15, 9)), (Nvfp4Case, (1, 16, 8, 7))])
+def test_experts_of_several_chunks_in_a_short_call(cls, counts):
+    """32 rows, experts with up to three chunks of rows: the bits that the same rows have in a call of 37, whose sort is the scan."""
+    fp4 = cls in (Mxfp4Case, Nvfp4Case)
+    case = cls(512, 256, 8, 1, seed=6, shared=False, scoring=O.SCORE_SIGMOID, max_tokens=64, routed_scale=1.0, limit=10.0, chain=fp4)
+    try:
+        ids = np.random.default_rng(sum(counts[:2])).permutation(np.repeat(np.arange(len(counts)), counts)).astype(np.int32)
+        assert ids.size == 32
+        more = np.concatenate([ids, np.full(5, 7, np.int32)])[:, None]
+        x, _ = case.inputs(37, seed=8)
+        w = np.full(more.shape, 0.75, np.float32)
+        few = case.gpu_experts(x[:32], more[:32], w[:32])
+        assert (few == case.gpu_experts(x, more, w)[:32]).all()
+        ref = case.cpu_layer(x[:32], more[:32], w[:32])
+        for e in range(len(counts)):
+            assert rel_l2(few[ids == e], ref[ids == e]) < 1e-2, e
+        assert case.status() == 0
+    finally:
+        case.close()
+
+
+@pytest.mark.parametrize("cls", [Exl3Case, Exl3K2Case, Mxfp4Case, Nvfp4Case])
+@pytest.mark.parametrize("split", [32, 20, 17, 16])
+def test_experts_of_several_groups_in_a_short_call(cls, split):
+    """Four tokens that name an expert eight times over: up to 32 rows of one expert in the streaming lane, two groups of chunks
+    (16 rows), against five tokens (40 rows, the scan)."""
+    fp4 = cls in (Mxfp4Case, Nvfp4Case)
+    case = cls(512, 256, 8, 8, seed=7, shared=False, scoring=O.SCORE_SIGMOID, max_tokens=64, routed_scale=1.0, limit=10.0, chain=fp4)
+    try:
+        ids = np.random.default_rng(split).permutation(np.repeat([2, 5], [split, 32 - split])).reshape(4, 8).astype(np.int32)
+        more = np.concatenate([ids, np.arange(8, dtype=np.int32)[None] % 2 * 6])   # experts 0 and 6
+        x, _ = case.inputs(5, seed=9)
+        w = np.random.default_rng(1).random(more.shape).astype(np.float32)
+        few = case.gpu_experts(x[:4], ids, w[:4])
+        assert (few == case.gpu_experts(x, more, w)[:4]).all()
+        assert rel_l2(few, case.cpu_layer(x[:4], ids, w[:4])) < 1e-2
+        assert case.status() == 0
+    finally:
+        case.close()
+
+
+@pytest.mark.parametrize("W", [1, 2, 3, 8])
+def test_few_rows_into_few_bins(W):
+    """The short sort with the bin counts that an exchange between ranks has."""
     import torch
-    case = Exl3Case(H, 128, E, 4, seed=2, shared=False, scoring=O.SCORE_SIGMOID, max_tokens=32)
+    case = Exl3Case(128, 128, 8, 1, seed=1, shared=False, max_tokens=64, experts_to_load=[])
+    try:
+        rng = np.random.default_rng(W)
+        for n in range(1, 34):
+            slot = rng.integers(0, W, n).astype(np.int32)
+            d = torch.from_numpy(slot).cuda()
+            order = torch.full((n,), -1, dtype=torch.int32, device="cuda")
+            offs = torch.full((W + 1,), -1, dtype=torch.int32, device="cuda")
+            case.moe.sort_rows(d.data_ptr(), n, W, order.data_ptr(), offs.data_ptr(), None)
+            torch.cuda.synchronize()
+            assert (order.cpu().numpy() == np.argsort(slot, kind="stable")).all(), n
+            assert (offs.cpu().numpy() == np.concatenate([[0], np.cumsum(np.bincount(slot, minlength=W))])).all(), n
+        assert case.status() == 0
+    finally:
+        case.close()
+
+
+@pytest.mark.parametrize("cls,E,H,shared", [(Exl3Case, 256, 1024, False), (Exl3Case, 256, 6144, False), (Exl3Case, 64, 7168, False), (Exl3Case, 9, 1664, False),
+                                            (Exl3Case, 288, 512, False), (Exl3Case, 1024, 256, False), (Nvfp4Case, 24, 512, True), (Mxfp4Case, 136, 256, False),
+                                            (Nvfp4Case, 300, 256, True)])
+def test_layer_from_x_of_a_few_tokens(cls, E, H, shared):
+    """From x the front's CTAs share out experts, tokens (beyond 256 experts in two passes, a CTA's experts in two or more
+    rounds) and (beyond 6144 inputs) a row's vectors in more than one round: the layer is the one that the logits alone give, 1
+    to 16 tokens.  The FP4 banks' rows are staged by quarters beside the shared expert, from the logits by sixteenths."""
+    import torch
+    case = cls(H, 128, E, 4, seed=2, shared=shared, scoring=O.SCORE_SIGMOID, max_tokens=32, chain=cls is not Exl3Case)
     try:
         wg = O.f32_to_bf16_bits((np.random.default_rng(5).standard_normal((E, H)) * H ** -0.5).astype(np.float32))
         case.moe.set_router_weight(0, wg.ctypes.data)
-        for T in (1, 2, 7, 8, 9, 15, 16):
+        for T in (1, 2, 3, 7, 8, 9, 15, 16):
             x, _ = case.inputs(T, seed=20 + T)
             xd = case.to_dev_bf16(x)
             lg = torch.empty((T, E), dtype=torch.float32, device=case.dev)
