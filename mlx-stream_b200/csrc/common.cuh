@@ -144,8 +144,8 @@ __device__ __forceinline__ uint32_t mul1_pair(uint32_t sa, uint32_t sb) {
 // 955 -> 887.  In the bare loop with one mma per tile 58.5 -> 55.3 cycles per tile and scheduler (K = 2 57.4 -> 52.5), 46.7 and 43.8
 // of them the decode: an mma.sync costs 8.7 whatever its shape.
 // The quad in memory: word w of the four k-tiles beside each other, [8 K words][4 k-tiles]: four 4-byte loads here, two 16-byte
-// loads for four tiles in the tensor-core lane.  (A lane's first two words as one 8-byte load: 1834 and 870 us, but the
-// tensor-core lane would need eight loads again.)
+// loads for four tiles in the tensor-core lane.  At K = 3 a load's lanes take 32 banks, at K = 2 the lanes u and u + 4 share one.
+// (A lane's first two words as one 8-byte load: 1834 and 870 us, but the tensor-core lane would need eight loads again.)
 // The tensor-core lane multiplies 16 inputs of one k-tile at a time instead (exl3_decode_lane): with the quad's order the grouping of
 // its sums over the inputs changes, and the f16 and bf16 roundings behind them turn that into 2e-4 of a layer's rows and, layer by
 // layer, into as much as 1e-2 after four (the streaming kernel's order alone: 5e-6 to 5e-5, 6e-3).

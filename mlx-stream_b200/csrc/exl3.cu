@@ -78,7 +78,7 @@ cudaError_t launch_exl3_repack(const uint8_t* record_dev, Exl3Dims d, uint32_t* 
 }
 
 // ------------------------------------------------------------------------------------------------------------
-// activation staging: rows -> mma A-fragment order, f16 hi / lo
+// activation staging: rows -> mma B-fragment order, f16 hi / lo
 // ------------------------------------------------------------------------------------------------------------
 template <bool RAW>
 __global__ void __launch_bounds__(CHUNK_ROWS * 32) exl3_prep_kernel(const void* __restrict__ xin, uint32_t top_k, uint32_t in_dim,
@@ -118,8 +118,8 @@ struct GemvParams {
     size_t expert_stride_words;
     uint32_t n_blocks;           // out / 128
     uint32_t nkt;                // in / 16
-    uint32_t block_stride_words; // words per 128-wide output block: a projection's k-tiles follow each other (8 tiles each)
-    const uint32_t* xa;          // [chunk][NPROJ][nkt][128]
+    uint32_t block_stride_words; // words per 128-wide output block: a projection's quads follow each other (8 tiles each)
+    const uint32_t* xa;          // [chunk][NPROJ][nkt / 4][256], a quad's inputs in the order of exl3_prep_body.cuh
     DispatchTables t;
     uint32_t counter_idx;
     const __half* scales;        // layer base

@@ -12,7 +12,7 @@
 //   * the epilogue: transpose through shared memory, then row-wise Hadamard-128, svh, clamped SwiGLU, suh_d, Hadamard for
 //     gate / up (act(gate) waits in an L2-resident scratch between the two passes, read back by the threads that wrote it);
 //     Hadamard, svh_d for down.
-// What bounds it (54 to 61 warp instructions per decoded tile with the epilogue, 43 of them the decode; 74 to 80 % of the issue slots): up to about 128 rows per tile the
+// What bounds it (54 to 61 warp instructions per decoded tile with the epilogue, about 42 of them the decode by its source; 74 to 80 % of the issue slots): up to about 128 rows per tile the
 // decode's instruction issue, above that the MMAs; calls of thousands of tokens run into the 1 kW power cap (1.55 GHz at
 // 8192 tokens).  Layer of H 5120, I 2304, 256 experts, calls back to back: 2048 tokens 4.04 -> 3.05 ms, 8192 tokens 10.65 ->
 // 7.74 ms against the lane that accumulated gate and up together, 3 % less with uniform MMA operands and wide code loads.

@@ -86,8 +86,8 @@ cudaError_t launch_usage_count(const int32_t* ids, uint64_t n, uint32_t E, unsig
 
 // ---- EXL3 ----
 struct Exl3Layer {            // one layer's resident bank, in the kernels' layout
-    const uint32_t* gu_code;  // [E][I/128][2][H/16][192] u32: per 128-wide output block, gate's k-tiles, then up's
-    const uint32_t* d_code;   // [E][H/128][I/16][192] u32
+    const uint32_t* gu_code;  // [E][I/128][2][H/64][8][8 K][4] u32: per 128-wide output block, gate's quads, then up's (common.cuh)
+    const uint32_t* d_code;   // [E][H/128][I/64][8][8 K][4] u32
     const __half* scales;     // [E][2H + 2I + I + H]: suh_g, suh_u [H] | svh_g, svh_u [I] | suh_d [I] | svh_d [H]
 };
 struct Exl3Dims { uint32_t H, I, K; };   // K = bits per weight of the trellis code (3 or 2): a 16x16 tile is 8 K words
@@ -99,7 +99,7 @@ static inline size_t exl3_code_words(Exl3Dims d) { return (size_t)(d.H / 16) * (
 cudaError_t launch_exl3_repack(const uint8_t* record_dev, Exl3Dims d, uint32_t* gu_code_e, uint32_t* d_code_e,
                                __half* scales_e, cudaStream_t st);
 
-// activation staging in mma B-fragment order: [chunk][proj][k-tile][32 lanes][2] u32 (256 B per k-tile)
+// activation staging in mma B-fragment order: [chunk][proj][in/64][256] u32, a quad's inputs in the order of exl3_prep_body.cuh
 // gate/up inputs: xg = H128(x * suh_g) * 128^-0.5 and xu likewise, f16 hi/lo
 cudaError_t launch_exl3_prep_in(const __nv_bfloat16* x, uint32_t top_k, Exl3Layer L, Exl3Dims d, DispatchTables t,
                                 uint32_t* xa_gu, cudaStream_t st);
@@ -110,8 +110,8 @@ struct Exl3GemvArgs {
     Exl3Layer L;
     Exl3Dims d;
     DispatchTables t;
-    const uint32_t* xa_gu;  // [chunk][2][H/16][64] u32
-    uint32_t* xa_d;         // [chunk][I/16][64] u32 (written by gate/up, read by down)
+    const uint32_t* xa_gu;  // [chunk][2][H/64][256] u32
+    uint32_t* xa_d;         // [chunk][I/64][256] u32 (written by gate/up, read by down)
     float* ro;              // [A, H] f32 routed outputs in assignment order (CHAIN combine: bf16 [A, H])
     int ro_bf16;
     float limit;            // > 0: clamped SwiGLU

@@ -1,5 +1,5 @@
 // The tensor-core lane of the banks that decode their weights on the SM (exl3_prefill.cu, fp4_prefill.cu): the pipeline that
-// both share.  A bank supplies its code stream's stages, the decode of a half stage, and the epilogue of a pass.
+// both share.  A bank supplies its code stream's stages, the decode of a quarter of a stage, and the epilogue of a pass.
 //
 // A CTA owns (expert, a tile of up to 192 of its rows, a 128-column block) and walks the inputs once per projection (a
 // "pass": gate then up, or down alone).  W^T is the MMA's A operand (M = 128 output columns), decoded straight into tensor
@@ -15,9 +15,9 @@
 //     (BK::AHEAD quarters of a stage) and only then waits for its operand slot: the MMAs of the slot's last stage run under the decode.  With three or four
 //     operand slots there are four teams of four warps, a warp decoding both halves of a stage, with two slots two teams of
 //     eight (a team of four keeps its slot for twice as long).  The barriers around a stage were a quarter of the instructions
-//     of a warp that decoded one half (EXL3: 60 per 16x16 tile, 43 of them the decode), and their latencies showed where the
+//     of a warp that decoded one half (EXL3: 60 per 16x16 tile, about 42 of them the decode), and their latencies showed where the
 //     decode is short: EXL3 8 % at 2048 tokens and 4 % at 8192, MXFP4 20 % at 2048 and 12 % at 3500.
-//     (Decoding in smaller pieces, or with 5 or 6 warps per lane quarter, measured slower or equal.)
+//     (EXL3 with quarters instead of halves between the stores, or with 5 or 6 warps per lane quarter: slower or equal.)
 //   * The MMA warp runs its loop with all lanes and issues under elect.sync (see elect_one); one commit per stage frees the
 //     operand slot and the rows' slot.  What its operands come from goes through a shuffle from lane 0, so that the compiler
 //     knows that the warp has one value: they stay in uniform registers instead of being moved there for every MMA (cycles
@@ -196,8 +196,8 @@ __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P)
         const uint32_t ta0 = tmem_a + ((q * 32u) << 16) + half * (LN_A_COLS / 2);
         // The team's stages are g = team + TEAMS i: code slot and code barriers alternate between team and team + TEAMS, their
         // phases flip every second stage.  The instructions around the decode count (it is issue-bound), so those addresses
-        // advance by an exclusive-or, and the tests of the two barriers that come next (the operand slot, the next stage's
-        // code) go out together: a test of a barrier that is ready costs its latency.
+        // advance by an exclusive-or, and the next stage's code is tested for behind this stage's last decode: a test of a
+        // barrier that is ready costs its latency, which the stores and the arrivals hide.
         const uint32_t bar0 = smem_u32(&bar_stage[0]);
         uint32_t b_raw = smem_u32(&raw_full[team]), b_emp = smem_u32(&raw_empty[team]);
         const uint32_t x_raw = b_raw ^ smem_u32(&raw_full[team + TEAMS]), x_emp = b_emp ^ smem_u32(&raw_empty[team + TEAMS]);
@@ -235,7 +235,9 @@ __global__ void __launch_bounds__(LN_THREADS, 1) lane_kernel(const LaneParams P)
                     if (lane == 0) mbar_arrive_at(b_emp);
                 }
                 if (gr == 0) {
+                    LC(t0 = clock64();)
                     if (g >= slots && !mbar_wait_bounded_at(b_done, ph_done, &s_abort)) { give_up(ST_WAIT_EMPTY); ok = false; break; }
+                    LC(t_slot += clock64() - t0;)
                     tc_fence_after();
                 }
 #pragma unroll
