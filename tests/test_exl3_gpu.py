@@ -109,6 +109,30 @@ def test_gemv_against_f64(c1):
         assert max_err_over_rms(z, ref) < 2.0 ** -16 * 8
 
 
+@pytest.mark.parametrize("cls,K", [(Exl3Case, 3), (Exl3K2Case, 2)])
+@pytest.mark.parametrize("H,I", [(5120, 256), (1920, 2304)])
+def test_streaming_products_hold_f32_precision(cls, K, H, I):
+    """The products' error against 64 bits, in the 2-norm.  A row is f16 hi + lo: 2^-21 of it is lost at most.  A part of the sum
+    is n products of 16 inputs, each added to f32 with the sum cut off below its last bit: 2^-23 of the running sum at most, which
+    grows as the root of the products so far, so n / 3 x 2^-23 of the part with an average loss of half a unit and twice that for
+    the bound."""
+    case = cls(H, I, 1, 1, seed=5, shared=False, max_tokens=64)
+    try:
+        g = O.exl3_geometry(H, I, K)
+        rng = np.random.default_rng(H)
+        for proj, n_in, n_out in ((0, H, I), (1, H, I), (2, I, H)):
+            code = case.records[0][g.off[3 * proj]:g.off[3 * proj] + g.len[3 * proj]].view(np.int16)
+            w = O.reconstruct(code, n_in // 16, n_out // 16, K).view(np.float16).astype(np.float64)
+            tiles = n_in // 16
+            n = tiles // (4 if tiles % 32 == 0 else 2 if tiles % 16 == 0 else 1)
+            for rows in (1, 7, 12, 33):
+                xh = rng.standard_normal((rows, n_in)).astype(np.float32)
+                assert rel_l2(case.gpu_gemv(0, proj, xh), xh.astype(np.float64) @ w) < 2 * n / 3 * 2.0 ** -24 + 2.0 ** -21, (proj, rows)
+        assert case.status() == 0
+    finally:
+        case.close()
+
+
 @pytest.mark.parametrize("T", [1, 8])
 def test_layer_config1(c1, T):
     x, logits = c1.inputs(T, seed=20 + T)
